@@ -37,7 +37,7 @@
 extern "C" {
 #endif
 
-#define PALIMPSA_ABI_VERSION 11
+#define PALIMPSA_ABI_VERSION 12
 
 /* io dtype of q, k, v, b, o, o_var, do, do_var, dq, dk, dv, db */
 #define PALIMPSA_F32 0
@@ -244,6 +244,12 @@ int palimpsa_fwd_tile_rows(int K, int V);
  * 0 if the shape is not supported.  No counterpart in the reference (grid (V/16) x N x H,
  * chunk_palimpsa_forgetting_scalar.py:558). */
 int palimpsa_bwd_tile_rows(int K, int V, int io_dtype, int uncertainty);
+
+/* Bookkeeping of a packed batch on the device, in one launch: chunk_offsets [n] (first checkpoint slot of every
+ * sequence) and order [n] (palimpsa_problem::seq_order: longest sequence first, ties in order; beyond 2048 sequences,
+ * where the tail of a launch no longer depends on it, their own order). */
+int palimpsa_varlen_plan(const int32_t *cu_seqlens, int32_t n, int32_t *chunk_offsets, int32_t *order, void *cuda_stream);
+
 
 /* Upper bound on checkpoint slots for a problem: ceil(total_tokens/16) + num_seqs (varlen needs
  * no host synchronisation to size its buffers). */

@@ -7,7 +7,7 @@ import os
 PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "libpalimpsa_b200.so")
 
-ABI_VERSION = 11
+ABI_VERSION = 12
 F32, BF16, F16 = 0, 1, 2
 FLAG_UNCERTAINTY = 1
 FLAG_EXPLICIT_INIT = 2
@@ -100,6 +100,7 @@ SYMBOLS = {
     "palimpsa_peer_wait": (C.c_int, [C.c_void_p, C.c_uint64, C.c_uint32, C.c_void_p, C.c_void_p]),
     "palimpsa_peer_signal": (C.c_int, [C.c_void_p, C.c_uint64, C.c_void_p]),
     "palimpsa_ckpt_slots": (C.c_longlong, [C.POINTER(Problem)]),
+    "palimpsa_varlen_plan": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]),
     "palimpsa_segment_summary": (C.c_int, [C.POINTER(Problem), C.POINTER(Segments), C.c_void_p]),
     "palimpsa_tensor_core_status": (C.c_int, []),
     "palimpsa_cp_combine": (C.c_int, [C.POINTER(Problem), C.POINTER(Segments), C.c_void_p, C.c_void_p, C.c_void_p,
@@ -130,6 +131,7 @@ SYMBOLS = {
 }
 
 _lib = None
+_torch_ops = None
 
 
 class PalimpsaLibraryError(RuntimeError):
@@ -158,6 +160,24 @@ def lib():
         raise PalimpsaLibraryError(f"{LIB_PATH} has ABI version {v}, Python side expects {ABI_VERSION}; rebuild it")
     _lib = h
     return h
+
+
+def torch_ops():
+    """The native torch front end (csrc/torch_ops.cpp), which also registers ``torch.ops.palimpsa_b200``.  Loading the
+    library first makes a missing build the same loud error as everywhere else."""
+    global _torch_ops
+    if _torch_ops is None:
+        lib()
+        try:
+            from . import _torch_ops as ext
+        except ImportError as e:
+            raise PalimpsaLibraryError("palimpsa_b200._torch_ops is missing or does not load. Build it with "
+                                       f"`python -m palimpsa_b200.build`: {e}") from e
+        if ext.abi_version() != ABI_VERSION:
+            raise PalimpsaLibraryError(f"palimpsa_b200._torch_ops was built for ABI version {ext.abi_version()}, "
+                                       f"Python side expects {ABI_VERSION}; rebuild it")
+        _torch_ops = ext
+    return _torch_ops
 
 
 def check(rc: int, what: str):

@@ -1,21 +1,26 @@
-"""Build libpalimpsa_b200.so in-tree with nvcc for sm_100a.
+"""Build libpalimpsa_b200.so (nvcc, sm_100a) and the torch front end over it (_torch_ops, host C++) in-tree.
 
     python -m palimpsa_b200.build [--force]
 
 Cross-compiles without a GPU.  The library links the CUDA runtime statically and has no other
-dependency (no torch, no Python): its whole surface is the C ABI in include/palimpsa_b200.h.
+dependency (no torch, no Python): its whole surface is the C ABI in include/palimpsa_b200.h.  The front end is a
+Python extension module that links torch and the library.
 """
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 ROOT = os.path.dirname(PKG)
 LIB = os.path.join(PKG, "libpalimpsa_b200.so")
+EXT = os.path.join(PKG, "_torch_ops" + sysconfig.get_config_var("EXT_SUFFIX"))
+EXT_SOURCE = os.path.join(CSRC, "torch_ops.cpp")
+HEADER = os.path.join(ROOT, "include", "palimpsa_b200.h")
 UNITS = ("abi", "fwd", "bwd", "decode", "segments", "summary_tc", "carry_tc", "layer", "peer")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--extended-lambda",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
@@ -27,18 +32,48 @@ def _nvcc() -> str:
 
 
 def _sources():
-    out = [os.path.join(ROOT, "include", "palimpsa_b200.h")]
+    out = [HEADER]
     for f in sorted(os.listdir(CSRC)):
         if f.endswith((".cu", ".cuh", ".h")):
             out.append(os.path.join(CSRC, f))
     return out
 
 
+def _older(target, sources) -> bool:
+    return not os.path.exists(target) or any(os.path.getmtime(s) > os.path.getmtime(target) for s in sources)
+
+
 def needs_build() -> bool:
-    if not os.path.exists(LIB):
-        return True
-    t = os.path.getmtime(LIB)
-    return any(os.path.getmtime(s) > t for s in _sources())
+    return _older(LIB, _sources()) or _older(EXT, [HEADER, EXT_SOURCE])
+
+
+def _run(cmd, what, log=None):
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if log:
+        with open(log, "w") as f:
+            f.write(r.stdout + r.stderr)
+    if r.returncode != 0:
+        raise RuntimeError(f"{what} failed:\n{r.stdout}\n{r.stderr}")
+
+
+def _compile_ext(obj):
+    """The front end's object file: torch's headers, plain host C++."""
+    from torch.utils import cpp_extension as E
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    inc = [*E.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    _run(["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_torch_ops",
+          "-DTORCH_API_INCLUDE_EXTENSION_H", *(f"-I{d}" for d in inc), "-c", EXT_SOURCE, "-o", obj], "g++ on torch_ops.cpp")
+
+
+def _link_ext(obj):
+    import torch
+    from torch.utils import cpp_extension as E
+    tmp = EXT + ".tmp"
+    libs = [f"-L{d}" for d in E.library_paths()]
+    _run(["g++", "-shared", "-o", tmp, obj, f"-L{PKG}", "-l:libpalimpsa_b200.so", *libs, "-ltorch", "-ltorch_cpu",
+          "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN",
+          f"-Wl,-rpath,{os.path.join(os.path.dirname(torch.__file__), 'lib')}"], "link of _torch_ops")
+    os.replace(tmp, EXT)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -54,22 +89,22 @@ def build(force: bool = False, verbose: bool = False) -> str:
         deps = headers + [os.path.join(CSRC, u + ".cu")]
         if not force and os.path.exists(obj) and all(os.path.getmtime(d) <= os.path.getmtime(obj) for d in deps):
             return obj                                # this unit's sources are older than its object
-        cmd = [_nvcc(), *NVCC_FLAGS, "-c", os.path.join(CSRC, u + ".cu"), "-o", obj]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        with open(os.path.join(objdir, u + ".ptxas.log"), "w") as f:
-            f.write(r.stdout + r.stderr)
-        if r.returncode != 0:
-            raise RuntimeError(f"nvcc failed on {u}.cu:\n{r.stdout}\n{r.stderr}")
+        _run([_nvcc(), *NVCC_FLAGS, "-c", os.path.join(CSRC, u + ".cu"), "-o", obj], f"nvcc on {u}.cu",
+             os.path.join(objdir, u + ".ptxas.log"))
         return obj
 
-    with ThreadPoolExecutor(len(UNITS)) as ex:
+    ext_obj = os.path.join(objdir, "torch_ops.o")
+    with ThreadPoolExecutor(len(UNITS) + 1) as ex:
+        ext_job = ex.submit(_compile_ext, ext_obj) if force or _older(ext_obj, [HEADER, EXT_SOURCE]) else None
         objs = list(ex.map(compile_unit, UNITS))
-    cmd = [_nvcc(), "-shared", "-o", LIB, *objs, "-gencode", "arch=compute_100a,code=sm_100a"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+        if ext_job:
+            ext_job.result()
+    tmp = LIB + ".tmp"
+    _run([_nvcc(), "-shared", "-o", tmp, *objs, "-gencode", "arch=compute_100a,code=sm_100a"], "link")
+    os.replace(tmp, LIB)
+    _link_ext(ext_obj)
     if verbose:
-        print("built", LIB)
+        print("built", LIB, EXT)
     return LIB
 
 

@@ -125,6 +125,13 @@ long long palimpsa_ckpt_slots(const palimpsa_problem* p) {
     return ((long long)p->total_tokens + TB - 1) / TB + p->num_seqs;
 }
 
+int palimpsa_varlen_plan(const int32_t* cu_seqlens, int32_t n, int32_t* chunk_offsets, int32_t* order, void* cuda_stream) {
+    if (n < 0) return PALIMPSA_E_SHAPE;
+    if (n == 0) return PALIMPSA_OK;
+    if (!cu_seqlens || !chunk_offsets || !order) return PALIMPSA_E_NULL;
+    return launch_varlen_plan(cu_seqlens, n, chunk_offsets, order, static_cast<cudaStream_t>(cuda_stream));
+}
+
 int palimpsa_chunk_fwd(const palimpsa_fwd_params* prm, void* cuda_stream) {
     int rc = check_fwd(prm);
     if (rc) return rc;

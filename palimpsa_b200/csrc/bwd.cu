@@ -930,9 +930,7 @@ static int launch_bwd_w(const BwdArgs& a, int tiles, int num_seg, bool carry_onl
     dim3 block(32 * W, 1, 1);
 #define PALIMPSA_BWD_LAUNCH(U, C)                                                                                 \
     do {                                                                                                          \
-        if (cudaFuncSetAttribute(bwd_kernel<RK, KG, RV, W, U, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                                 L.total) != cudaSuccess)                                                         \
-            return PALIMPSA_E_LAUNCH;                                                                             \
+        if (!allow_smem<bwd_kernel<RK, KG, RV, W, U, C>>(L.total)) return PALIMPSA_E_LAUNCH;                        \
         bwd_kernel<RK, KG, RV, W, U, C><<<grid, block, L.total, stream>>>(a);                                     \
     } while (0)
     if (carry_only) {

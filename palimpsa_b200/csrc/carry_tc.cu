@@ -420,12 +420,10 @@ int launch_carry_tc(const palimpsa_bwd_params* prm, const palimpsa_segments& sg,
                      make_tensor_map_bf16_rows(&maps.v, p.v, (unsigned long long)p.total_tokens, (unsigned long long)p.H * p.V, CT) &&
                      make_tensor_map_bf16_rows(&maps.b, p.b, (unsigned long long)p.total_tokens, (unsigned long long)p.H * p.V, CT);
     if (tma) {
-        if (cudaFuncSetAttribute(carry_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-            return PALIMPSA_E_LAUNCH;
+        if (!allow_smem<carry_tc_kernel<true>>(smem)) return PALIMPSA_E_LAUNCH;
         carry_tc_kernel<true><<<grid, 128, smem, stream>>>(a, maps);
     } else {
-        if (cudaFuncSetAttribute(carry_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-            return PALIMPSA_E_LAUNCH;
+        if (!allow_smem<carry_tc_kernel<false>>(smem)) return PALIMPSA_E_LAUNCH;
         carry_tc_kernel<false><<<grid, 128, smem, stream>>>(a, maps);
     }
     return cudaGetLastError() == cudaSuccess ? PALIMPSA_OK : PALIMPSA_E_LAUNCH;

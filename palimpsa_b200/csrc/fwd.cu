@@ -508,21 +508,14 @@ static int launch_fwd_w(const FwdArgs& a, int num_seg, bool summary, cudaStream_
     const FwdSmem L = fwd_smem_layout(RK * KG, TV, dtype_size(p.io_dtype), unc);
     dim3 grid((p.V + TV - 1) / TV, p.num_seqs * p.H, num_seg);
     dim3 block(32 * W, 1, 1);
-    cudaError_t e;
     if (summary) {
-        e = cudaFuncSetAttribute(fwd_kernel<RK, KG, RV, W, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 L.total);
-        if (e != cudaSuccess) return PALIMPSA_E_LAUNCH;
+        if (!allow_smem<fwd_kernel<RK, KG, RV, W, false, true>>(L.total)) return PALIMPSA_E_LAUNCH;
         fwd_kernel<RK, KG, RV, W, false, true><<<grid, block, L.total, stream>>>(a);
     } else if (unc) {
-        e = cudaFuncSetAttribute(fwd_kernel<RK, KG, RV, W, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 L.total);
-        if (e != cudaSuccess) return PALIMPSA_E_LAUNCH;
+        if (!allow_smem<fwd_kernel<RK, KG, RV, W, true, false>>(L.total)) return PALIMPSA_E_LAUNCH;
         fwd_kernel<RK, KG, RV, W, true, false><<<grid, block, L.total, stream>>>(a);
     } else {
-        e = cudaFuncSetAttribute(fwd_kernel<RK, KG, RV, W, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 L.total);
-        if (e != cudaSuccess) return PALIMPSA_E_LAUNCH;
+        if (!allow_smem<fwd_kernel<RK, KG, RV, W, false, false>>(L.total)) return PALIMPSA_E_LAUNCH;
         fwd_kernel<RK, KG, RV, W, false, false><<<grid, block, L.total, stream>>>(a);
     }
     return cudaGetLastError() == cudaSuccess ? PALIMPSA_OK : PALIMPSA_E_LAUNCH;

@@ -3,9 +3,31 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "../../include/palimpsa_b200.h"
 
 namespace palimpsa {
+
+// Lets a kernel use `bytes` of dynamic shared memory.  The attribute stays with the kernel on a device, so it is raised
+// once per kernel, device and larger size instead of being set on every launch.
+template <auto Kern>
+bool allow_smem(int bytes) {
+    constexpr int MAX_DEV = 64;
+    static std::atomic<int> granted[MAX_DEV];
+    static std::mutex raising;
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    if (dev < 0 || dev >= MAX_DEV)
+        return cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+    if (granted[dev].load(std::memory_order_acquire) >= bytes) return true;
+    std::lock_guard<std::mutex> lock(raising);
+    if (granted[dev].load(std::memory_order_relaxed) >= bytes) return true;
+    if (cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+    granted[dev].store(bytes, std::memory_order_release);
+    return true;
+}
 
 // Enqueue the forward kernel (fwd.cu).  Parameters are assumed validated.  With `segs` every sequence is
 // cut into segs->num_segments segments that run as separate CTAs: `summary` = false starts each from
@@ -37,6 +59,9 @@ int launch_combine_fwd(const palimpsa_problem& p, const palimpsa_segments& segs,
                        float* out_M, float* out_J, cudaStream_t stream);
 int launch_combine_bwd(const palimpsa_problem& p, const palimpsa_segments& segs, const float* in_M, const float* in_I,
                        float* out_M, float* out_I, cudaStream_t stream);
+
+// Checkpoint slots and start order of a packed batch's sequences (segments.cu).
+int launch_varlen_plan(const int32_t* cu_seqlens, int n, int32_t* chunk_offsets, int32_t* order, cudaStream_t stream);
 
 // Stream-ordered flags in peer-mapped memory (peer.cu): a bounded wait until *flag >= value, and a release store.
 int launch_peer_wait(const void* flag, unsigned long long value, unsigned timeout_ms, float* poison, cudaStream_t stream);

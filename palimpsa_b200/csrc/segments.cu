@@ -175,4 +175,54 @@ int launch_combine_bwd(const palimpsa_problem& p, const palimpsa_segments& segs,
     return cudaGetLastError() == cudaSuccess ? PALIMPSA_OK : PALIMPSA_E_LAUNCH;
 }
 
+// One CTA: exclusive scan of the sequences' block counts, and their rank by decreasing length.  Replaces ~20 small
+// launches of tensor operations (differences, scan, sort, casts) in front of every packed forward and backward.
+constexpr int PLAN_THREADS = 1024, PLAN_SORTED = 2048;
+__global__ void __launch_bounds__(PLAN_THREADS) varlen_plan_kernel(const int32_t* __restrict__ cu, int n,
+                                                                   int32_t* __restrict__ coff, int32_t* __restrict__ order) {
+    __shared__ int32_t part[PLAN_THREADS / 32];
+    __shared__ __align__(16) int32_t lens[PLAN_SORTED];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int per = (n + PLAN_THREADS - 1) / PLAN_THREADS, lo = min(n, tid * per), hi = min(n, lo + per);
+    auto len = [&](int i) { return max(0, cu[i + 1] - cu[i]); };
+    int32_t mine = 0;
+    for (int i = lo; i < hi; ++i) mine += (len(i) + TB - 1) / TB;
+    int32_t incl = mine;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int32_t x = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += x;
+    }
+    if (lane == 31) part[tid >> 5] = incl;
+    const int padded = (n + 3) / 4 * 4;
+    if (n <= PLAN_SORTED)
+        for (int i = tid; i < padded; i += PLAN_THREADS) lens[i] = i < n ? len(i) : -1;
+    __syncthreads();
+    int32_t at = incl - mine;
+    for (int w = 0; w < (tid >> 5); ++w) at += part[w];
+    for (int i = lo; i < hi; ++i) {
+        coff[i] = at;
+        at += (len(i) + TB - 1) / TB;
+    }
+    for (int i = tid; i < n; i += PLAN_THREADS) {
+        if (n > PLAN_SORTED) {
+            order[i] = i;
+            continue;
+        }
+        const int32_t l = lens[i];
+        int rank = 0;
+        for (int j = 0; j < padded; j += 4) {
+            const int4 x = *reinterpret_cast<const int4*>(lens + j);
+            rank += (x.x > l || (x.x == l && j < i)) + (x.y > l || (x.y == l && j + 1 < i)) +
+                    (x.z > l || (x.z == l && j + 2 < i)) + (x.w > l || (x.w == l && j + 3 < i));
+        }
+        order[rank] = i;
+    }
+}
+
+int launch_varlen_plan(const int32_t* cu_seqlens, int n, int32_t* chunk_offsets, int32_t* order, cudaStream_t stream) {
+    varlen_plan_kernel<<<1, PLAN_THREADS, 0, stream>>>(cu_seqlens, n, chunk_offsets, order);
+    return cudaGetLastError() == cudaSuccess ? PALIMPSA_OK : PALIMPSA_E_LAUNCH;
+}
+
 }  // namespace palimpsa

@@ -237,12 +237,10 @@ int launch_summary_tc(const palimpsa_problem& p, const palimpsa_segments& sg, cu
     const bool tma = p.K % 64 == 0 && p.total_tokens > 0 &&
                      make_tensor_map_bf16_rows(&kmap, p.k, (unsigned long long)p.total_tokens, (unsigned long long)p.H * p.K, TCK);
     if (tma) {
-        if (cudaFuncSetAttribute(summary_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-            return PALIMPSA_E_LAUNCH;
+        if (!allow_smem<summary_tc_kernel<true>>(smem)) return PALIMPSA_E_LAUNCH;
         summary_tc_kernel<true><<<grid, 128, smem, stream>>>(a, kmap);
     } else {
-        if (cudaFuncSetAttribute(summary_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-            return PALIMPSA_E_LAUNCH;
+        if (!allow_smem<summary_tc_kernel<false>>(smem)) return PALIMPSA_E_LAUNCH;
         summary_tc_kernel<false><<<grid, 128, smem, stream>>>(a, kmap);
     }
     return cudaGetLastError() == cudaSuccess ? PALIMPSA_OK : PALIMPSA_E_LAUNCH;
