@@ -245,6 +245,10 @@ int palimpsa_fwd_tile_rows(int K, int V);
  * chunk_palimpsa_forgetting_scalar.py:558). */
 int palimpsa_bwd_tile_rows(int K, int V, int io_dtype, int uncertainty);
 
+/* Copies n <= 8 device buffers (src[i] -> dst[i], bytes[i]; not overlapping) in one launch: the token inputs of a
+ * replayed decode step. */
+int palimpsa_copy_buffers(const void *const *src, void *const *dst, const size_t *bytes, int n, void *cuda_stream);
+
 /* Bookkeeping of a packed batch on the device, in one launch: chunk_offsets [n] (first checkpoint slot of every
  * sequence) and order [n] (palimpsa_problem::seq_order: longest sequence first, ties in order; beyond 2048 sequences,
  * where the tail of a launch no longer depends on it, their own order). */

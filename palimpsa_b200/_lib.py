@@ -100,6 +100,8 @@ SYMBOLS = {
     "palimpsa_peer_wait": (C.c_int, [C.c_void_p, C.c_uint64, C.c_uint32, C.c_void_p, C.c_void_p]),
     "palimpsa_peer_signal": (C.c_int, [C.c_void_p, C.c_uint64, C.c_void_p]),
     "palimpsa_ckpt_slots": (C.c_longlong, [C.POINTER(Problem)]),
+    "palimpsa_copy_buffers": (C.c_int, [C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.POINTER(C.c_size_t), C.c_int,
+                                        C.c_void_p]),
     "palimpsa_varlen_plan": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]),
     "palimpsa_segment_summary": (C.c_int, [C.POINTER(Problem), C.POINTER(Segments), C.c_void_p]),
     "palimpsa_tensor_core_status": (C.c_int, []),

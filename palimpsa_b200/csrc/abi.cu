@@ -125,6 +125,15 @@ long long palimpsa_ckpt_slots(const palimpsa_problem* p) {
     return ((long long)p->total_tokens + TB - 1) / TB + p->num_seqs;
 }
 
+int palimpsa_copy_buffers(const void* const* src, void* const* dst, const size_t* bytes, int n, void* cuda_stream) {
+    if (n < 0 || n > 8) return PALIMPSA_E_LIMIT;
+    if (n == 0) return PALIMPSA_OK;
+    if (!src || !dst || !bytes) return PALIMPSA_E_NULL;
+    for (int i = 0; i < n; ++i)
+        if (bytes[i] && (!src[i] || !dst[i])) return PALIMPSA_E_NULL;
+    return launch_copy_buffers(src, dst, bytes, n, static_cast<cudaStream_t>(cuda_stream));
+}
+
 int palimpsa_varlen_plan(const int32_t* cu_seqlens, int32_t n, int32_t* chunk_offsets, int32_t* order, void* cuda_stream) {
     if (n < 0) return PALIMPSA_E_SHAPE;
     if (n == 0) return PALIMPSA_OK;

@@ -37,6 +37,7 @@ int launch_fwd(const palimpsa_fwd_params* prm, const palimpsa_segments* segs, bo
 // Single-token decode step (decode.cu): dedicated HBM-bound kernel, when it covers the call.
 bool decode_supported(const palimpsa_fwd_params* prm);
 int launch_decode(const palimpsa_fwd_params* prm, cudaStream_t stream);
+int launch_copy_buffers(const void* const* src, void* const* dst, const size_t* bytes, int n, cudaStream_t stream);
 
 // Backward (bwd.cu): main kernel (stages bit 0) + the two finishing kernels (bit 1); bit 2: the finishing
 // kernels also sum the extra partial slot that carry_tc.cu fills.

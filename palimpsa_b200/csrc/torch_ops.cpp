@@ -488,6 +488,29 @@ py::object decode_step(const Tensor& q_, const Tensor& k_, const Tensor& v_, con
     return py::cast(std::get<0>(r));
 }
 
+// The token inputs of a replayed step into the graph's static buffers: one launch for those that are plain copies (same
+// dtype, contiguous), tensor copies for the rest.
+void copy_inputs(const std::vector<Tensor>& dst, const std::vector<OptTensor>& src) {
+    const void* from[8];
+    void* to[8];
+    size_t bytes[8];
+    int n = 0;
+    c10::cuda::CUDAGuard guard(dst[0].device());
+    for (size_t i = 0; i < dst.size(); ++i) {
+        if (!given(src[i])) continue;
+        const Tensor &d = dst[i], &s = *src[i];
+        TORCH_CHECK_VALUE(s.numel() == d.numel(), "decode input ", i, ": ", s.numel(), " elements, expected ", d.numel());
+        if (n < 8 && s.device() == d.device() && s.scalar_type() == d.scalar_type() && s.is_contiguous() && plain({&s})) {
+            from[n] = s.const_data_ptr(), to[n] = d.data_ptr(), bytes[n++] = (size_t)d.nbytes();
+            bump_version(d);
+        } else {
+            at::NoGradGuard no_grad;
+            d.copy_(s.reshape(d.sizes()), /*non_blocking=*/true);
+        }
+    }
+    check_rc(palimpsa_copy_buffers(from, to, bytes, n, stream_of(dst[0])), "decode inputs");
+}
+
 // ---- chunk_palimpsa / fused_recurrent_palimpsa ------------------------------------------------------------------
 py::object run(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& gt, const Tensor& g,
                const Tensor& Ip, const OptTensor& mu0, const OptTensor& I0, std::optional<double> scale, bool want_final,
@@ -764,6 +787,7 @@ TORCH_LIBRARY_IMPL(palimpsa_b200, Autograd, m) {
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("run", &run);
     m.def("decode_step", &decode_step);
+    m.def("copy_inputs", &copy_inputs);
     m.def("layer_prologue", &layer_prologue);
     m.def("layer_epilogue", &layer_epilogue);
     m.def("plan_segments", &plan_segments_py);

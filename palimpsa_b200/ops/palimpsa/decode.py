@@ -95,8 +95,6 @@ class DecodeGraph:
     def step(self, q=None, k=None, v=None, b=None, gt=None):
         """Copies the given tensors into the static input buffers (those left ``None`` keep their content) and
         replays the graph on the current stream.  Returns ``self.o`` (and ``self.o_var``)."""
-        for dst, src in ((self.q, q), (self.k, k), (self.v, v), (self.b, b), (self.gt, gt)):
-            if src is not None:
-                dst.copy_(src.reshape(dst.shape), non_blocking=True)
+        _core.native().copy_inputs([self.q, self.k, self.v, self.b, self.gt], [q, k, v, b, gt])
         self.graph.replay()
         return (self.o, self.o_var) if self.unc else self.o
