@@ -732,106 +732,124 @@ __global__ void __launch_bounds__(32 * W) bwd_kernel(const BwdArgs a) {
     }
 }
 
-// ---- finishing kernel 1: one warp per (token, head) row ------------------------------------------------
-__device__ __forceinline__ void st2(void* base, long long idx, float2 x, int dt) {  // idx even, base 8-byte aligned
-    if (dt == PALIMPSA_F32)
-        *reinterpret_cast<float2*>(reinterpret_cast<float*>(base) + idx) = x;
-    else if (dt == PALIMPSA_BF16)
-        *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(base) + idx) = __floats2bfloat162_rn(x.x, x.y);
-    else
-        *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(base) + idx) = __floats2half2_rn(x.x, x.y);
+// ---- finishing kernel 1 ----------------------------------------------------------------------------------
+// CTAs [0, col_ctas): dq, dk = the row tiles' partials summed in tile order and cast.  A thread owns four consecutive
+// columns of a row (16-byte loads, all tiles' loads independent); as many whole rows as fit share a CTA, so that no
+// lane idles whatever d_k is.  The other CTAs: the per-token scalars of a strided share of the tokens, thread = (token
+// lane, head): df and dIp terms summed over the tiles, dgt written, dg and dIp terms accumulated per head and reduced over
+// the CTA's token lanes in a fixed order.  HBM-bound: 8 (KP tiles + 1) bytes read per (token, head), and K io values written
+// twice.  With one warp per row, 48-column rows kept 12 of 32 lanes busy: 336 us at B=8 T=4096 H=16 d_k=d_v=48.
+constexpr int FIN_THREADS = 256, FIN_SCALAR_CTAS = 296;
+
+__device__ __forceinline__ void st4(void* base, long long idx, float4 x, int dt) {  // idx a multiple of 4, base aligned for it
+    if (dt == PALIMPSA_F32) {
+        *reinterpret_cast<float4*>(reinterpret_cast<float*>(base) + idx) = x;
+        return;
+    }
+    uint2 u;
+    if (dt == PALIMPSA_BF16) {
+        const __nv_bfloat162 a = __floats2bfloat162_rn(x.x, x.y), b = __floats2bfloat162_rn(x.z, x.w);
+        u = make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
+    } else {
+        const __half2 a = __floats2half2_rn(x.x, x.y), b = __floats2half2_rn(x.z, x.w);
+        u = make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
+    }
+    *reinterpret_cast<uint2*>(reinterpret_cast<unsigned short*>(base) + idx) = u;
 }
 
-__global__ void __launch_bounds__(256) bwd_finish_rows(const palimpsa_problem p, const float* __restrict__ dq_part,
-                                                       const float* __restrict__ dk_part,
-                                                       const float* __restrict__ df_part,
-                                                       const float* __restrict__ dip_part, void* dq, void* dk,
-                                                       float* dgt, float* w_dg, float* w_dip, int tiles, int tiles_k,
-                                                       int KP, long long rows, int pairs_ok) {
-    const int lane = threadIdx.x & 31;
-    const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= rows) return;
-    const int h = (int)(row % p.H);
-    // per-token scalars: lane t fetches tile t's partial (tiles beyond 32 go round), summed by a fixed butterfly
-    float df = 0.f, dip = 0.f;
-    for (int t = lane; t < tiles_k; t += 32) {
-        df += df_part[(size_t)t * rows + row];
-        dip += dip_part[(size_t)t * rows + row];
-    }
-    const float gtv = p.gt[row], gh = p.g[h];
-    // a lane owns four consecutive columns: one 16-byte load per tile partial, all tiles' loads independent
-    const int KP4 = KP / 4;
-    for (int c4 = lane; c4 < KP4; c4 += 32) {
-        float4 sq = make_float4(0.f, 0.f, 0.f, 0.f), sk = sq;
-        const float4* pq = reinterpret_cast<const float4*>(dq_part) + (size_t)row * KP4 + c4;
-        const float4* pk = reinterpret_cast<const float4*>(dk_part) + (size_t)row * KP4 + c4;
+__global__ void __launch_bounds__(FIN_THREADS)
+bwd_finish_rows(const palimpsa_problem p, const float* __restrict__ dq_part, const float* __restrict__ dk_part,
+                const float* __restrict__ df_part, const float* __restrict__ dip_part, void* dq, void* dk, float* dgt,
+                float* w_dg, float* w_dip, int tiles, int tiles_k, int KP, long long rows, int vec, int col_ctas) {
+    const int tid = threadIdx.x;
+    if ((int)blockIdx.x < col_ctas) {
+        const int KP4 = KP / 4, rpc = FIN_THREADS / KP4, r = tid / KP4, c4 = tid - r * KP4, kc = 4 * c4;
+        if (r >= rpc || kc >= p.K) return;
         const size_t step = (size_t)rows * KP4;
+        for (long long row = (long long)blockIdx.x * rpc + r; row < rows; row += (long long)col_ctas * rpc) {
+            const float4* pq = reinterpret_cast<const float4*>(dq_part) + (size_t)row * KP4 + c4;
+            const float4* pk = reinterpret_cast<const float4*>(dk_part) + (size_t)row * KP4 + c4;
+            float4 sq = make_float4(0.f, 0.f, 0.f, 0.f), sk = sq;
 #pragma unroll 6
-        for (int t = 0; t < tiles; ++t) {
-            const float4 x = pq[t * step], y = pk[t * step];
-            sq.x += x.x, sq.y += x.y, sq.z += x.z, sq.w += x.w;
-            sk.x += y.x, sk.y += y.y, sk.z += y.z, sk.w += y.w;
-        }
-        if (tiles_k > tiles) {  // dk has one slot more than dq: the carried-gradient terms
-            const float4 y = pk[tiles * step];
-            sk.x += y.x, sk.y += y.y, sk.z += y.z, sk.w += y.w;
-        }
-        const int kc = 4 * c4;
-        if (pairs_ok) {          // K even, dq/dk 8-byte aligned: paired stores
-            if (kc < p.K) {
-                st2(dq, row * p.K + kc, make_float2(sq.x, sq.y), p.io_dtype);
-                st2(dk, row * p.K + kc, make_float2(sk.x, sk.y), p.io_dtype);
+            for (int t = 0; t < tiles; ++t) {
+                const float4 x = __ldcs(pq + t * step), y = __ldcs(pk + t * step);
+                sq.x += x.x, sq.y += x.y, sq.z += x.z, sq.w += x.w;
+                sk.x += y.x, sk.y += y.y, sk.z += y.z, sk.w += y.w;
             }
-            if (kc + 2 < p.K) {
-                st2(dq, row * p.K + kc + 2, make_float2(sq.z, sq.w), p.io_dtype);
-                st2(dk, row * p.K + kc + 2, make_float2(sk.z, sk.w), p.io_dtype);
+            if (tiles_k > tiles) {  // dk has one slot more than dq: the carried-gradient terms
+                const float4 y = pk[tiles * step];
+                sk.x += y.x, sk.y += y.y, sk.z += y.z, sk.w += y.w;
             }
-        } else {
-            const float q4[4] = {sq.x, sq.y, sq.z, sq.w}, k4[4] = {sk.x, sk.y, sk.z, sk.w};
+            if (vec) {  // K a multiple of 4, dq and dk aligned for four values
+                st4(dq, row * p.K + kc, sq, p.io_dtype);
+                st4(dk, row * p.K + kc, sk, p.io_dtype);
+            } else {
+                const float q4[4] = {sq.x, sq.y, sq.z, sq.w}, k4[4] = {sk.x, sk.y, sk.z, sk.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (kc + i < p.K) {
-                    st1(dq, row * p.K + kc + i, q4[i], p.io_dtype);
-                    st1(dk, row * p.K + kc + i, k4[i], p.io_dtype);
+                for (int i = 0; i < 4; ++i)
+                    if (kc + i < p.K) {
+                        st1(dq, row * p.K + kc + i, q4[i], p.io_dtype);
+                        st1(dk, row * p.K + kc + i, k4[i], p.io_dtype);
+                    }
+            }
+        }
+        return;
+    }
+    __shared__ float red[2][FIN_THREADS];
+    const int b = blockIdx.x - col_ctas, nb = gridDim.x - col_ctas, H = p.H;
+    const long long tokens = rows / H;
+    const int lanes = H <= FIN_THREADS ? FIN_THREADS / H : 1;  // token lanes
+    for (int h0 = 0; h0 < H; h0 += FIN_THREADS) {              // one turn unless there are more heads than threads
+        const int lane = H <= FIN_THREADS ? tid / H : 0, h = h0 + (H <= FIN_THREADS ? tid - lane * H : tid);
+        float a0 = 0.f, a1 = 0.f;
+        if (lane < lanes && h < H) {
+            const float gh = p.g[h];
+            for (long long tok = (long long)b * lanes + lane; tok < tokens; tok += (long long)nb * lanes) {
+                const long long row = tok * H + h;
+                float df = 0.f, dip = 0.f;
+#pragma unroll 4
+                for (int t = 0; t < tiles_k; ++t) {
+                    df += df_part[(size_t)t * rows + row];
+                    dip += dip_part[(size_t)t * rows + row];
                 }
+                const float gtv = p.gt[row], fdf = expf(-gtv * gh) * df;
+                dgt[row] = -gh * fdf;
+                a0 -= gtv * fdf;
+                a1 += dip;
+            }
         }
-    }
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
-        df += __shfl_xor_sync(0xffffffffu, df, off);
-        dip += __shfl_xor_sync(0xffffffffu, dip, off);
-    }
-    if (lane == 0) {
-        const float f = expf(-gtv * gh);
-        dgt[row] = -gh * f * df;
-        w_dg[row] = -gtv * f * df;
-        w_dip[row] = dip;
-    }
-}
-
-// ---- finishing kernel 2: one CTA per head, ordered sum over all rows -----------------------------------
-__global__ void __launch_bounds__(256) bwd_finish_heads(const float* __restrict__ w_dg, const float* __restrict__ w_dip,
-                                                       float* dg, float* dIp, long long tokens, int H) {
-    __shared__ float s0[256], s1[256];
-    const int h = blockIdx.x, tid = threadIdx.x;
-    float a0 = 0.f, a1 = 0.f;
-    for (long long t = tid; t < tokens; t += 256) {
-        a0 += w_dg[t * H + h];
-        a1 += w_dip[t * H + h];
-    }
-    s0[tid] = a0;
-    s1[tid] = a1;
-    __syncthreads();
-    for (int s = 128; s >= 1; s >>= 1) {
-        if (tid < s) {
-            s0[tid] += s0[tid + s];
-            s1[tid] += s1[tid + s];
+        red[0][tid] = a0;
+        red[1][tid] = a1;
+        __syncthreads();
+        if (lane == 0 && h < H) {
+            for (int l = 1; l < lanes; ++l) {
+                a0 += red[0][l * H + h];
+                a1 += red[1][l * H + h];
+            }
+            w_dg[(size_t)b * H + h] = a0;
+            w_dip[(size_t)b * H + h] = a1;
         }
         __syncthreads();
     }
-    if (tid == 0) {
-        dg[h] = s0[0];
-        dIp[h] = s1[0];
+}
+
+// ---- finishing kernel 2: one warp per head, ordered sum over the scalar CTAs' partials -------------------------
+__global__ void __launch_bounds__(32) bwd_finish_heads(const float* __restrict__ w_dg, const float* __restrict__ w_dip,
+                                                       float* dg, float* dIp, int nb, int H) {
+    const int h = blockIdx.x, lane = threadIdx.x;
+    float a0 = 0.f, a1 = 0.f;
+    for (int b = lane; b < nb; b += 32) {
+        a0 += w_dg[(size_t)b * H + h];
+        a1 += w_dip[(size_t)b * H + h];
+    }
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) {
+        a0 += __shfl_xor_sync(0xffffffffu, a0, off);
+        a1 += __shfl_xor_sync(0xffffffffu, a1, off);
+    }
+    if (lane == 0) {
+        dg[h] = a0;
+        dIp[h] = a1;
     }
 }
 
@@ -913,8 +931,8 @@ BwdWorkspace bwd_workspace_layout(const palimpsa_problem& p) {
     ws.dk_part = take((size_t)(ws.tiles + 1) * rows * ws.KP * 4);
     ws.df_part = take((size_t)(ws.tiles + 1) * rows * 4);
     ws.dip_part = take((size_t)(ws.tiles + 1) * rows * 4);
-    ws.w_dg = take(rows * 4);
-    ws.w_dip = take(rows * 4);
+    ws.w_dg = take((size_t)FIN_SCALAR_CTAS * p.H * 4);
+    ws.w_dip = take((size_t)FIN_SCALAR_CTAS * p.H * 4);
     ws.total = off;
     return ws;
 }
@@ -1019,18 +1037,21 @@ int launch_bwd(const palimpsa_bwd_params* prm, const palimpsa_segments* segs, bo
     if (rc != PALIMPSA_OK) return rc;
     if (!(stages & 2)) return PALIMPSA_OK;
     const long long rows = a.rows_total;
+    int nb = 0;
     if (rows > 0) {
-        const int wpb = 8;
-        bwd_finish_rows<<<(unsigned)((rows + wpb - 1) / wpb), 32 * wpb, 0, stream>>>(
+        const int rpc = FIN_THREADS / (ws.KP / 4), lanes = p.H <= FIN_THREADS ? FIN_THREADS / p.H : 1;
+        const long long groups = (rows + rpc - 1) / rpc, tgroups = (p.total_tokens + lanes - 1) / lanes;
+        const int col_ctas = (int)(groups < 148 * 32 ? groups : 148 * 32);
+        nb = (int)(tgroups < FIN_SCALAR_CTAS ? tgroups : FIN_SCALAR_CTAS);
+        const uintptr_t both = reinterpret_cast<uintptr_t>(prm->dq) | reinterpret_cast<uintptr_t>(prm->dk);
+        bwd_finish_rows<<<col_ctas + nb, FIN_THREADS, 0, stream>>>(
             p, a.dq_part, a.dk_part, a.df_part, a.dip_part, prm->dq, prm->dk, prm->dgt,
             reinterpret_cast<float*>(base + ws.w_dg), reinterpret_cast<float*>(base + ws.w_dip), ws.tiles,
-            ws.tiles + ((stages & 4) ? 1 : 0), ws.KP, rows,
-            (p.K % 2 == 0 && ((reinterpret_cast<uintptr_t>(prm->dq) | reinterpret_cast<uintptr_t>(prm->dk)) & 7) == 0) ? 1 : 0);
+            ws.tiles + ((stages & 4) ? 1 : 0), ws.KP, rows, p.K % 4 == 0 && (both & (4 * es - 1)) == 0, col_ctas);
         if (cudaGetLastError() != cudaSuccess) return PALIMPSA_E_LAUNCH;
     }
-    bwd_finish_heads<<<p.H, 256, 0, stream>>>(reinterpret_cast<float*>(base + ws.w_dg),
-                                              reinterpret_cast<float*>(base + ws.w_dip), prm->dg, prm->dIp,
-                                              p.total_tokens, p.H);
+    bwd_finish_heads<<<p.H, 32, 0, stream>>>(reinterpret_cast<float*>(base + ws.w_dg),
+                                             reinterpret_cast<float*>(base + ws.w_dip), prm->dg, prm->dIp, nb, p.H);
     return cudaGetLastError() == cudaSuccess ? PALIMPSA_OK : PALIMPSA_E_LAUNCH;
 }
 
