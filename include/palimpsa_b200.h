@@ -37,7 +37,7 @@
 extern "C" {
 #endif
 
-#define PALIMPSA_ABI_VERSION 12
+#define PALIMPSA_ABI_VERSION 13
 
 /* io dtype of q, k, v, b, o, o_var, do, do_var, dq, dk, dv, db */
 #define PALIMPSA_F32 0
@@ -64,7 +64,7 @@ extern "C" {
 
 #define PALIMPSA_MAX_K 256
 #define PALIMPSA_CKPT_INTERVAL 16   /* tokens between saved (M, I) checkpoints */
-#define PALIMPSA_STATIC_SCRATCH_BYTES (64u << 20) /* capacity of palimpsa_chunk_bwd_static */
+#define PALIMPSA_STATIC_SCRATCH_BYTES (96u << 20) /* capacity of palimpsa_chunk_bwd_static */
 
 /* Problem description shared by forward and backward. */
 typedef struct palimpsa_problem {
@@ -75,7 +75,9 @@ typedef struct palimpsa_problem {
     int32_t io_dtype;      /* PALIMPSA_F32 / BF16 / F16                                        */
     int32_t flags;
     float scale;           /* multiplies q (default of the Python wrappers: K^-0.5)            */
-    int32_t reserved0;
+    int32_t segments;      /* G of a backward that runs in G segments, else 0 or 1: the backward's tile height depends on
+                              how many CTAs there will be.  The same in every call of one backward, the query of its
+                              workspace among them.                                            */
     const void *q, *k, *v, *b;
     const float *gt, *g, *Ip;
     const int32_t *cu_seqlens;    /* [N+1] device, or NULL                                      */
@@ -245,6 +247,12 @@ int palimpsa_fwd_tile_rows(int K, int V);
  * chunk_palimpsa_forgetting_scalar.py:558). */
 int palimpsa_bwd_tile_rows(int K, int V, int io_dtype, int uncertainty);
 
+/* Estimated time of the backward per token, in units of one warp's token (about 45 ns), from num_seqs, H, K, V,
+ * io_dtype, flags and segments: what planners weigh an uncut backward against one in segments with.  The backward
+ * takes the tile height that this is smallest for; palimpsa_bwd_tile_rows() is the one of a grid of many waves.
+ * 0 if the shape is not supported. */
+double palimpsa_bwd_token_cost(const palimpsa_problem *p);
+
 /* Copies n <= 8 device buffers (src[i] -> dst[i], bytes[i]; not overlapping) in one launch: the token inputs of a
  * replayed decode step. */
 int palimpsa_copy_buffers(const void *const *src, void *const *dst, const size_t *bytes, int n, void *cuda_stream);
@@ -287,14 +295,14 @@ int palimpsa_chunk_bwd_stages(const palimpsa_bwd_params *params, void *cuda_stre
  * fixed at start-up, real-time or interrupt-style service threads, and code running where
  * cudaMalloc is unavailable or would stall the device (it synchronises).  Identical to
  * palimpsa_chunk_bwd, except that params->workspace / workspace_bytes are ignored: the scratch is a
- * fixed PALIMPSA_STATIC_SCRATCH_BYTES (64 MiB) array inside the library, resident on every GPU that
+ * fixed PALIMPSA_STATIC_SCRATCH_BYTES (96 MiB) array inside the library, resident on every GPU that
  * loads the library for as long as the process lives.  The caller still passes every input and
  * output buffer.  It calls no cudaMalloc, cudaFree or any allocating routine.
- *   - Problems whose palimpsa_bwd_workspace_bytes() exceeds the capacity return PALIMPSA_E_LIMIT
- *     (at d_k = d_v = 128 the capacity covers about 9900 (token, head) rows: 6720 bytes per row).
+ *   - Problems that do not fit the capacity even with the tallest row tiles return PALIMPSA_E_LIMIT
+ *     (at d_k = d_v = 128 it covers about 14900 (token, head) rows: 6712 bytes per row).
  *   - The first call on each device looks up the array's device address (once per device, with that
  *     device current); make that first call outside any stream capture.  With the CUDA runtime's
- *     default lazy module loading the 64 MiB are only reserved when the library's backward code is first
+ *     default lazy module loading the 96 MiB are only reserved when the library's backward code is first
  *     loaded on a device, which can be this very call: on a device whose memory is already handed out
  *     the look-up then fails and the call returns PALIMPSA_E_SYMBOL without launching anything.  Hosts
  *     with a fixed pool should therefore make one small call at start-up, before they carve up the

@@ -7,12 +7,12 @@ import os
 PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "libpalimpsa_b200.so")
 
-ABI_VERSION = 12
+ABI_VERSION = 13
 F32, BF16, F16 = 0, 1, 2
 FLAG_UNCERTAINTY = 1
 FLAG_EXPLICIT_INIT = 2
 CKPT_INTERVAL = 16
-STATIC_SCRATCH_BYTES = 64 << 20
+STATIC_SCRATCH_BYTES = 96 << 20
 E_NULL, E_ALIGN, E_LIMIT, E_SYMBOL = -1, -7, -9, -10
 
 
@@ -21,7 +21,7 @@ class Problem(C.Structure):
         ("num_seqs", C.c_int32), ("seq_len", C.c_int32), ("total_tokens", C.c_int32),
         ("H", C.c_int32), ("K", C.c_int32), ("V", C.c_int32),
         ("io_dtype", C.c_int32), ("flags", C.c_int32),
-        ("scale", C.c_float), ("reserved0", C.c_int32),
+        ("scale", C.c_float), ("segments", C.c_int32),
         ("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p), ("b", C.c_void_p),
         ("gt", C.c_void_p), ("g", C.c_void_p), ("Ip", C.c_void_p),
         ("cu_seqlens", C.c_void_p), ("chunk_offsets", C.c_void_p),
@@ -97,6 +97,7 @@ SYMBOLS = {
     "palimpsa_padded_k": (C.c_int, [C.c_int]),
     "palimpsa_fwd_tile_rows": (C.c_int, [C.c_int, C.c_int]),
     "palimpsa_bwd_tile_rows": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int]),
+    "palimpsa_bwd_token_cost": (C.c_double, [C.POINTER(Problem)]),
     "palimpsa_peer_wait": (C.c_int, [C.c_void_p, C.c_uint64, C.c_uint32, C.c_void_p, C.c_void_p]),
     "palimpsa_peer_signal": (C.c_int, [C.c_void_p, C.c_uint64, C.c_void_p]),
     "palimpsa_ckpt_slots": (C.c_longlong, [C.POINTER(Problem)]),

@@ -115,6 +115,12 @@ int palimpsa_bwd_tile_rows(int K, int V, int io_dtype, int uncertainty) {
     return bwd_tile_rows(p);
 }
 
+double palimpsa_bwd_token_cost(const palimpsa_problem* p) {
+    if (!p || p->K <= 0 || p->V <= 0 || p->K > PALIMPSA_MAX_K) return 0;
+    if (p->io_dtype != PALIMPSA_F32 && p->io_dtype != PALIMPSA_BF16 && p->io_dtype != PALIMPSA_F16) return 0;
+    return bwd_token_cost(*p);
+}
+
 int palimpsa_fwd_tile_rows(int K, int V) {
     if (K <= 0 || V <= 0 || K > PALIMPSA_MAX_K) return 0;
     return fwd_tile_rows(K, V);

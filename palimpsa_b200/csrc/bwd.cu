@@ -16,13 +16,18 @@
 // Reductions: over d_k (dv, db) by xor-shuffles inside the lanes of a row; over d_v (dq, dk) first
 // in registers across a thread's rows, then across the CTA's row groups through shared memory, and
 // across the CTAs of different row tiles through fp32 partial buffers in the workspace, which the
-// finishing kernel sums in a fixed order (bitwise reproducible; no atomics).  The CTA-wide barriers of
-// the shared-memory step are mbarriers split into arrive / wait halves (bounded waits), so that the
-// warps of the single resident CTA do not alternate in lockstep between FP32 work and reductions.
-// One CTA per SM: 11 or 12 warps at d_k = 128 (22- or 24-row tiles, whichever pads d_v less).
+// finishing kernel sums in a fixed order (bitwise reproducible; no atomics).
+// Helper warps do all that follows a group's partials in shared memory (sums over the row groups, casts, global
+// stores); the compute warps hand a group over through an mbarrier pair per buffer (bounded waits) and walk on.  What
+// bounds the walk is latency at 2 or 3 warps per scheduler, FP32 pipe and issue slots each half busy, so work and
+// waits taken off the compute warps count, and one scheduler had a warp less than the others (11 warps).  With every
+// warp summing and storing its share behind a split barrier: 7.42 ms a training step at B=8 T=4096 H=6 d=128, now
+// 6.79; 3.99 / 3.51 ms at H=16 d=48.
+// One CTA per SM: up to 11 warps at d_k = 128 (22-row tiles); bwd_config has the choice and its measurements.
 //
 // Finishing kernels: (1) per (token, head) row: sum the row tiles, cast dq/dk, form
 // dgt = -g f df and the per-row terms of dg and dIp; (2) per head: ordered sum over rows.
+#include <cmath>
 #include <mutex>
 
 #include "host.h"
@@ -31,6 +36,7 @@
 namespace palimpsa {
 
 constexpr int GR = 4;  // tokens per register-resident group
+constexpr int BWD_FEWEST_TILES = -1;  // palimpsa_problem::segments, internal: as few row tiles as possible
 
 // 0 ok; 5 / 6: a bounded wait on the split-phase barriers of the backward's group reduction gave up
 __device__ int g_bwd_status = 0;
@@ -40,6 +46,12 @@ __device__ __forceinline__ void mbar_init_n(unsigned long long* bar, unsigned co
 }
 __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
     asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.shared::cta.b64 st, [%0];\n}" ::"r"(tc::smem_u32(bar)) : "memory");
+}
+
+// Barrier over the compute warps of a CTA (the helper warp does not take part).
+template <int N>
+__device__ __forceinline__ void bar_compute() {
+    asm volatile("bar.sync 1, %0;" ::"n"(N) : "memory");
 }
 
 struct BwdArgs {
@@ -62,7 +74,9 @@ struct BwdArgs {
 };
 
 struct BwdSmem {
-    int ks, qs, qqs, vs2, bs2, dys2, dyvs2, fc2, fn2, dvs, dbs, wred, slots, ckb, kred;
+    int ks, qs, qqs, vs2, bs2, dys2, dyvs2, fc2, fn2, slots, ckb;
+    int kred, dvs, dbs, wred, fgr;  // per-group partials handed to the helper warp, kbuf buffers of each
+    int bars;                       // mbarriers: full[2], empty[2]; then the failure flag
     int ck_stage;  // bytes of one (M, I) checkpoint stage
     int raw, rq, rk, rv, rb, rdo, rdov, rgt;
     int total;
@@ -93,13 +107,15 @@ __host__ __device__ inline BwdSmem bwd_smem_layout(int KP, int TV, int NE, int n
     s.dyvs2 = unc ? take(TB * TV * 8) : 0;
     s.fc2 = take(TB * 16);
     s.fn2 = take(TB * 8);
-    s.dvs = take(TB * TV * 4);
-    s.dbs = take(TB * TV * 4);
-    s.wred = take((nthr / 32) * TB * 2 * 4);
     s.slots = take(2 * 2 * NE * nthr * 4);
     s.ck_stage = 2 * TV * KP * 4;
     s.ckb = take(2 * s.ck_stage);
     s.kred = take(kbuf * GR * WV * 2 * KP * 4);  // kbuf = 2 group buffers where they fit (host's choice), else 1
+    s.dvs = take(kbuf * GR * TV * 4);
+    s.dbs = take(kbuf * GR * TV * 4);
+    s.wred = take(kbuf * (nthr / 32) * GR * 2 * 4);
+    s.fgr = take(kbuf * GR * 4);
+    s.bars = take(48);
     s.raw = off;
     int r = 0;
     auto rtake = [&](int bytes) {
@@ -120,10 +136,10 @@ __host__ __device__ inline BwdSmem bwd_smem_layout(int KP, int TV, int NE, int n
 }
 
 // Asynchronous copy of one block's checkpoint rows (M, I) into checkpoint stage `stage_idx`.
-__device__ __forceinline__ void bwd_issue_ckpt(const BwdArgs& a, unsigned char* sm, const BwdSmem& L, int stage_idx,
+__device__ __forceinline__ void bwd_issue_ckpt(const BwdArgs& a, int nthr, unsigned char* sm, const BwdSmem& L, int stage_idx,
                                                int KP, int TV, long long slot, int h, int v0, int tvw) {
     const palimpsa_problem& p = a.p;
-    const int nthr = blockDim.x, tid = threadIdx.x;
+    const int tid = threadIdx.x;
     unsigned char* ck = sm + L.ckb + stage_idx * L.ck_stage;
     const int cr = KP / 4;
     const long long base = ((slot * p.H + h) * (long long)p.V + v0) * KP;
@@ -134,10 +150,10 @@ __device__ __forceinline__ void bwd_issue_ckpt(const BwdArgs& a, unsigned char* 
 }
 
 // Asynchronous copy of one block's raw inputs (aligned path only).
-__device__ __forceinline__ void bwd_issue_raw(const BwdArgs& a, unsigned char* sm, const BwdSmem& L, int es, int KP,
+__device__ __forceinline__ void bwd_issue_raw(const BwdArgs& a, int nthr, unsigned char* sm, const BwdSmem& L, int es, int KP,
                                               int TV, long long tok0, int nt, int nt_ext, int h, int v0, int tvw) {
     const palimpsa_problem& p = a.p;
-    const int nthr = blockDim.x, tid = threadIdx.x;
+    const int tid = threadIdx.x;
     unsigned char* stage = sm + L.raw;
     const int cq = p.K * es / 16;
     const char* gq = reinterpret_cast<const char*>(p.q);
@@ -178,11 +194,11 @@ __device__ __forceinline__ float2 ld2s(const unsigned char* base, int e) {
 }
 
 template <int DT, bool ALIGNED, bool UNC>
-__device__ __forceinline__ void bwd_convert(const BwdArgs& a, unsigned char* sm, const BwdSmem& L, int KP, int TV,
+__device__ __forceinline__ void bwd_convert(const BwdArgs& a, int nthr, unsigned char* sm, const BwdSmem& L, int KP, int TV,
                                             long long tok0, int nt, int nt_ext, int h, int v0, float gh, float iph,
                                             bool carry_block) {
     const palimpsa_problem& p = a.p;
-    const int nthr = blockDim.x, tid = threadIdx.x;
+    const int tid = threadIdx.x;
     const int K4 = KP / 4, V4 = TV / 4;
     const unsigned char* stage = sm + L.raw;
     float4* qs = reinterpret_cast<float4*>(sm + L.qs);
@@ -288,15 +304,21 @@ __device__ __forceinline__ void bwd_convert(const BwdArgs& a, unsigned char* sm,
     }
 }
 
+// Threads of a CTA: W compute warps and, except in the carry-only pass, the helper warps: as many as fit beside the
+// compute warps without costing those registers (8 warps of an SM may have 255 per thread, 12 may have 168).
+__host__ __device__ constexpr int bwd_helpers(int W) { return W < 8 ? 8 - W : 12 - W; }
+__host__ __device__ constexpr int bwd_threads(int W, bool CO) { return 32 * (W + (CO ? 0 : bwd_helpers(W))); }
+
 template <int RV, int NP>
 struct State {
     float2 M[RV][NP], I[RV][NP];
 };
 
 template <int RK, int KG, int RV, int W, bool UNC, bool CO>
-__global__ void __launch_bounds__(32 * W) bwd_kernel(const BwdArgs a) {
+__global__ void __launch_bounds__(bwd_threads(W, CO)) bwd_kernel(const BwdArgs a) {
     constexpr int KP = RK * KG, VG = 32 / KG, NP = RK / 2, NE = RV * RK, KP2 = KP / 2;
     constexpr int TV = W * VG * RV, WV = W * VG, NTHR = 32 * W;
+    static_assert(TV % 2 == 0, "the operand tiles are converted two rows at a time");
     constexpr int NG = TB / GR;       // groups per block
     constexpr int NR1 = GR * RV * 2;  // per-group d_v-indexed partials of a thread: (token, row, dv|db)
     constexpr int NR2 = GR * 2;       // per-group per-token scalars: (token, df|sum GI)
@@ -322,7 +344,7 @@ __global__ void __launch_bounds__(32 * W) bwd_kernel(const BwdArgs a) {
     const long long seg_base = (((long long)n * G + g) * p.H + h) * p.V;  // row index into [N,G,H,V,KP] buffers
     if (s1 <= s0) {  // empty segment: the end-state gradient is the start-state gradient
         if (a.rloc_M) {
-            for (int i = tid; i < tvw * (KP / 4); i += NTHR) {
+            for (int i = tid; i < tvw * (KP / 4); i += bwd_threads(W, CO)) {
                 const long long e = (seg_base + v0) * KP + (long long)i * 4;
                 float4 cm = make_float4(0.f, 0.f, 0.f, 0.f), ci = cm;
                 if (!CO && a.carry_M) {
@@ -343,26 +365,88 @@ __global__ void __launch_bounds__(32 * W) bwd_kernel(const BwdArgs a) {
     const bool has_carry = !CO && a.carry_M != nullptr;
     const bool has_init = p.init_mu != nullptr || (p.flags & PALIMPSA_FLAG_EXPLICIT_INIT);
 
-    // The CTA-wide barriers of the per-group reduction over d_v are split into arrive / wait halves
-    // (mbarriers, one arrival per warp).  A: a warp that has written its partials of a group goes on with its
-    // own shuffle reductions before it waits for the others' partials.  B (single buffer only): a warp that
-    // has read the buffer goes on with the next group's recompute before it waits for the others to finish
-    // reading; with two buffers the next group writes the other one and A alone orders everything.  The warps
-    // of the CTA then drift apart by up to a group and stop hitting the FP32 pipe and the reduction phases
-    // all at the same time.  Waits are bounded; a wait that gives up is recorded.
-    constexpr bool SPLIT_A = !CO;
-    const bool SPLIT_B = KBUF == 1 && !CO;
-    __shared__ __align__(8) unsigned long long gbar[2];
-    unsigned ph_a = 0, ph_b = 0;
+    // Hand-over of a group's partials: full[b] (one arrival per compute warp) and empty[b] (one from the helper),
+    // buffer b = gi & (KBUF - 1).  Waits are bounded; a wait that gives up is recorded below.
+    unsigned long long* full = reinterpret_cast<unsigned long long*>(sm + L.bars);
+    unsigned long long* empty = full + 2;
+    int* fail_flag = reinterpret_cast<int*>(full + 4);
+    unsigned use = 0;  // how often this thread has been through buffer KBUF - 1, the first one of a block
     int wait_fail = 0;
-    if (SPLIT_A) {
+    float* dvs = reinterpret_cast<float*>(sm + L.dvs);
+    float* dbs = reinterpret_cast<float*>(sm + L.dbs);
+    float* wred = reinterpret_cast<float*>(sm + L.wred);
+    float* fgr = reinterpret_cast<float*>(sm + L.fgr);
+    if (!CO) {
         if (tid == 0) {
-            mbar_init_n(&gbar[0], W);
-            mbar_init_n(&gbar[1], W);
+            for (int b = 0; b < 2; ++b) {
+                mbar_init_n(&full[b], W);
+                mbar_init_n(&empty[b], bwd_helpers(W));
+            }
+            *fail_flag = 0;
             tc::mbar_init_fence();
         }
         __syncthreads();
-        if (SPLIT_B && lane == 0) mbar_arrive(&gbar[1]);  // nobody reads before the first group: B starts complete
+    }
+
+    if (!CO && w >= W) {
+        // ---- helper warps: everything a group leaves behind once its partials lie in shared memory --------------
+        // dq / dk summed over the CTA's row groups and written to this row tile's partials, dv / db cast and
+        // written, the per-token scalars summed over the warps.
+        constexpr int KP4 = KP / 4, HT = 32 * bwd_helpers(W);
+        const int ht = tid - NTHR;
+        const float4* kred4 = reinterpret_cast<const float4*>(sm + L.kred);
+        for (int it = 0; it < nblk; ++it) {
+            const int t0 = (blk1 - 1 - it) * TB, nt = min(TB, len - t0);
+            const long long tok0 = (long long)bos + t0;
+#pragma unroll 1
+            for (int gi = NG - 1; gi >= 0; --gi) {
+                const int b = gi & (KBUF - 1);
+                if (!wait_fail && !tc::mbar_wait(&full[b], use & 1)) wait_fail = 5;
+                if (b == 0) ++use;
+                const int ng = min(GR, nt - gi * GR);  // tokens of the group that exist (<= 0 past the sequence end)
+                const long long trow = (tok0 + gi * GR) * p.H + h;  // (token, head) row of the group's first token
+                const size_t prow = (size_t)tile * a.rows_total + trow;
+                for (int i = ht; i < ng * 2 * KP4; i += HT) {
+                    const int j = i / (2 * KP4), which = i / KP4 - 2 * j, c4 = i % KP4;
+                    const float4* src = kred4 + ((b * GR + j) * WV * 2 + which) * KP4 + c4;
+                    float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+#pragma unroll
+                    for (int x = 0; x < WV; ++x) {
+                        const float4 y = src[x * 2 * KP4];
+                        s0 = fadd2(s0, make_float2(y.x, y.y));
+                        s1 = fadd2(s1, make_float2(y.z, y.w));
+                    }
+                    reinterpret_cast<float4*>(which ? a.dk_part : a.dq_part)[(prow + (size_t)j * p.H) * KP4 + c4] =
+                        make_float4(s0.x, s0.y, s1.x, s1.y);
+                }
+                for (int i = ht; i < ng * TV; i += HT) {
+                    const int j = i / TV, r = i - j * TV;
+                    if (r < tvw) {
+                        const long long e = (trow + (long long)j * p.H) * V + v0 + r;
+                        st1(a.dv, e, dvs[b * GR * TV + i], p.io_dtype);
+                        st1(a.db, e, dbs[b * GR * TV + i], p.io_dtype);
+                    }
+                }
+                if (w == W + bwd_helpers(W) - 1 && lane < ng) {
+                    float df = 0.f, s2 = 0.f;
+#pragma unroll
+                    for (int x = 0; x < W; ++x) {
+                        df += wred[((b * W + x) * GR + lane) * 2 + 0];
+                        s2 += wred[((b * W + x) * GR + lane) * 2 + 1];
+                    }
+                    const float f = fgr[b * GR + lane];
+                    float dip = (1.f - f) * s2;
+                    if (t0 + gi * GR + lane == 0 && !has_init) dip += f * s2;  // I_0 = Ip: the start-state gradient reaches Ip
+                    a.df_part[prow + (size_t)lane * p.H] = df;
+                    a.dip_part[prow + (size_t)lane * p.H] = dip;
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty[b]);
+            }
+        }
+        if (wait_fail) *fail_flag = wait_fail;
+        __syncthreads();
+        return;
     }
 
     // this thread's d_k columns are RK*kg .. RK*kg+RK-1: pair q covers columns RK*kg + 2q, +1
@@ -375,9 +459,6 @@ __global__ void __launch_bounds__(32 * W) bwd_kernel(const BwdArgs a) {
     const float2* dyvs2 = reinterpret_cast<const float2*>(sm + L.dyvs2) + row0;
     const float4* fc2 = reinterpret_cast<const float4*>(sm + L.fc2);
     const float2* fn2 = reinterpret_cast<const float2*>(sm + L.fn2);
-    float* dvs = reinterpret_cast<float*>(sm + L.dvs);
-    float* dbs = reinterpret_cast<float*>(sm + L.dbs);
-    float* wred = reinterpret_cast<float*>(sm + L.wred);
     float4* slots4 = reinterpret_cast<float4*>(sm + L.slots) + tid;
     float2* kred2 = reinterpret_cast<float2*>(sm + L.kred);
 
@@ -480,8 +561,8 @@ __global__ void __launch_bounds__(32 * W) bwd_kernel(const BwdArgs a) {
     {
         const int c = blk1 - 1;
         const int nt = min(TB, len - c * TB);
-        bwd_issue_ckpt(a, sm, L, 0, KP, TV, slot0 + c, h, v0, tvw);
-        if (a.aligned) bwd_issue_raw(a, sm, L, es, KP, TV, (long long)bos + c * TB, nt, nt, h, v0, tvw);
+        bwd_issue_ckpt(a, NTHR, sm, L, 0, KP, TV, slot0 + c, h, v0, tvw);
+        if (a.aligned) bwd_issue_raw(a, NTHR, sm, L, es, KP, TV, (long long)bos + c * TB, nt, nt, h, v0, tvw);
         cp_async_commit();
     }
 
@@ -494,29 +575,29 @@ __global__ void __launch_bounds__(32 * W) bwd_kernel(const BwdArgs a) {
         const long long tok0 = (long long)bos + t0;
         const int st = it & 1;
         cp_async_wait<0>();
-        __syncthreads();
+        bar_compute<NTHR>();
         if (a.aligned) {
             if (p.io_dtype == PALIMPSA_BF16)
-                bwd_convert<PALIMPSA_BF16, true, UNC>(a, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
+                bwd_convert<PALIMPSA_BF16, true, UNC>(a, NTHR, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
             else if (p.io_dtype == PALIMPSA_F32)
-                bwd_convert<PALIMPSA_F32, true, UNC>(a, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
+                bwd_convert<PALIMPSA_F32, true, UNC>(a, NTHR, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
             else
-                bwd_convert<PALIMPSA_F16, true, UNC>(a, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
+                bwd_convert<PALIMPSA_F16, true, UNC>(a, NTHR, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
         } else {
             if (p.io_dtype == PALIMPSA_BF16)
-                bwd_convert<PALIMPSA_BF16, false, UNC>(a, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
+                bwd_convert<PALIMPSA_BF16, false, UNC>(a, NTHR, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
             else if (p.io_dtype == PALIMPSA_F32)
-                bwd_convert<PALIMPSA_F32, false, UNC>(a, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
+                bwd_convert<PALIMPSA_F32, false, UNC>(a, NTHR, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
             else
-                bwd_convert<PALIMPSA_F16, false, UNC>(a, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
+                bwd_convert<PALIMPSA_F16, false, UNC>(a, NTHR, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
         }
-        __syncthreads();
+        bar_compute<NTHR>();
         // the raw stage is free again: fetch the next (earlier) block while this one is processed
         if (c > blk0) {
             const int t0n = t0 - TB;
-            bwd_issue_ckpt(a, sm, L, st ^ 1, KP, TV, slot0 + c - 1, h, v0, tvw);
+            bwd_issue_ckpt(a, NTHR, sm, L, st ^ 1, KP, TV, slot0 + c - 1, h, v0, tvw);
             if (a.aligned)
-                bwd_issue_raw(a, sm, L, es, KP, TV, (long long)bos + t0n, TB, min(TB + 1, len - t0n), h, v0, tvw);
+                bwd_issue_raw(a, NTHR, sm, L, es, KP, TV, (long long)bos + t0n, TB, min(TB + 1, len - t0n), h, v0, tvw);
             cp_async_commit();
         }
 
@@ -544,6 +625,7 @@ __global__ void __launch_bounds__(32 * W) bwd_kernel(const BwdArgs a) {
                 P[j + 1] = P[j];
                 fstep(P[j + 1], gi * GR + j);
             }
+            const int b = gi & (KBUF - 1);
             float red1[NR1], red2[NR2];
             // ---- reverse walk over the group ----------------------------------------------------
 #pragma unroll
@@ -605,12 +687,10 @@ __global__ void __launch_bounds__(32 * W) bwd_kernel(const BwdArgs a) {
                     red1[(j * RV + r) * 2 + 1] = -(dba.x + dba.y);
                 }
                 // this row group's share of dq and dk for the token -> shared memory
-                if (SPLIT_B && j == GR - 1) {  // first write of the group: the previous group's readers must be done
-                    if (!wait_fail && !tc::mbar_wait(&gbar[1], ph_b)) wait_fail = 6;  // after one failure: no more waiting
-                    ph_b ^= 1;
-                }
                 if (!CO) {
-                    float2* dst = kred2 + (gi & (KBUF - 1)) * (GR * WV * 2 * KP2) + ((j * WV + wv) * 2) * KP2 + NP * kg;
+                    if (j == GR - 1)  // first write of the group: the helper must be done with the buffer's last contents
+                        if (!wait_fail && !tc::mbar_wait(&empty[b], (use & 1) ^ 1)) wait_fail = 6;  // after one failure: no more waiting
+                    float2* dst = kred2 + b * (GR * WV * 2 * KP2) + ((j * WV + wv) * 2) * KP2 + NP * kg;
                     const float2 sc2 = dup2(p.scale), m2 = dup2(-2.f);
 #pragma unroll
                     for (int q = 0; q < NP; ++q) {
@@ -632,8 +712,6 @@ __global__ void __launch_bounds__(32 * W) bwd_kernel(const BwdArgs a) {
                 red2[j * 2 + 1] = -sc_;
             }
             if (CO) continue;  // carry-only pass: nothing but the state gradients is wanted
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&gbar[0]);  // this warp's partials of the group are written
             // d_v-indexed sums over the KG lanes of a row; per-token scalars over the whole warp
             xreduce<NR1, KG>(red1, lane);
             {
@@ -645,74 +723,31 @@ __global__ void __launch_bounds__(32 * W) bwd_kernel(const BwdArgs a) {
                     for (int i = 0; i < REM; ++i) {
                         const int id = base + i;
                         const int j = id / (RV * 2), r = (id / 2) % RV, which = id & 1;
-                        (which ? dbs : dvs)[(gi * GR + j) * TV + row0 + r] = red1[i];
+                        (which ? dbs : dvs)[(b * GR + j) * TV + row0 + r] = red1[i];
                     }
                 }
             }
             xreduce<NR2, 32>(red2, lane);
             if ((lane & (32 / NR2 - 1)) == 0) {
                 const int id = xreduce_index<NR2, 32>(lane);
-                wred[(w * TB + gi * GR + (id >> 1)) * 2 + (id & 1)] = red2[0];
+                wred[((b * W + w) * GR + (id >> 1)) * 2 + (id & 1)] = red2[0];
             }
-            if (!wait_fail && !tc::mbar_wait(&gbar[0], ph_a)) wait_fail = 5;
-            ph_a ^= 1;
-            // ---- sum the row groups' shares; emit this row tile's dq / dk partials ----------------------
-            const int ng = min(GR, nt - gi * GR);  // tokens of the group that exist (<= 0 past the sequence end)
-            for (int i = tid; i < ng * KP2; i += NTHR) {
-                const int j = i / KP2, pi = i - j * KP2;
-                const float2* src = kred2 + (gi & (KBUF - 1)) * (GR * WV * 2 * KP2) + (j * WV * 2) * KP2 + pi;
-                float2 s0 = make_float2(0.f, 0.f), s1 = s0;
-#pragma unroll
-                for (int x = 0; x < WV; ++x) {
-                    s0 = fadd2(s0, src[(x * 2) * KP2]);
-                    s1 = fadd2(s1, src[(x * 2 + 1) * KP2]);
-                }
-                const size_t e = (((size_t)tile * a.rows_total + (size_t)(tok0 + gi * GR + j) * p.H + h) * KP2) + pi;
-                reinterpret_cast<float2*>(a.dq_part)[e] = s0;
-                reinterpret_cast<float2*>(a.dk_part)[e] = s1;
-            }
-            // with two buffers no second barrier is needed: the next group writes the other buffer, and the
-            // barrier after ITS reverse walk orders this group's reads before the buffer is reused
-            if (SPLIT_B) {
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&gbar[1]);  // this warp has read the buffer
-            }
+            if (tid < GR) fgr[b * GR + tid] = fc2[gi * GR + tid].x;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[b]);  // this warp's partials of the group are written
+            if (b == 0) ++use;
         }
-        if (!CO) __syncthreads();  // dvs / dbs / wred of the whole block are complete
-
-        // ---- block epilogue: dv, db rows and the per-token scalars -----------------------------------
-        if (CO) continue;
-        for (int i = tid; i < nt * TV; i += NTHR) {
-            const int t = i / TV, r = i - t * TV;
-            if (r < tvw) {
-                const long long e = ((tok0 + t) * p.H + h) * (long long)V + v0 + r;
-                st1(a.dv, e, dvs[i], p.io_dtype);
-                st1(a.db, e, dbs[i], p.io_dtype);
-            }
-        }
-        if (tid < nt) {
-            float df = 0.f, s2 = 0.f;
-#pragma unroll
-            for (int x = 0; x < W; ++x) {
-                df += wred[(x * TB + tid) * 2 + 0];
-                s2 += wred[(x * TB + tid) * 2 + 1];
-            }
-            const float f = fc2[tid].x;
-            float dip = (1.f - f) * s2;
-            if (t0 + tid == 0 && !has_init) dip += f * s2;  // I_0 = Ip: the start-state gradient reaches Ip
-            const size_t e = (size_t)tile * a.rows_total + (size_t)(tok0 + tid) * p.H + h;
-            a.df_part[e] = df;
-            a.dip_part[e] = dip;
-        }
-        // the next iteration's first barrier orders these reads before the buffers are reused
     }
 
-    if (SPLIT_A && wait_fail) {
-        // a barrier wait ran out: record it and mark this CTA's results as invalid (NaN in the decay-gradient
-        // partial of its first token, which the finishing kernels carry into dgt and dg)
-        atomicCAS(&g_bwd_status, 0, wait_fail);
-        if (tid == 0)
+    if (!CO) {
+        if (wait_fail) *fail_flag = wait_fail;
+        __syncthreads();
+        if (tid == 0 && *fail_flag) {
+            // a barrier wait ran out: record it and mark this CTA's results as invalid (NaN in the decay-gradient
+            // partial of its first token, which the finishing kernels carry into dgt and dg)
+            atomicCAS(&g_bwd_status, 0, *fail_flag);
             a.df_part[(size_t)tile * a.rows_total + (size_t)((long long)bos + s0) * p.H + h] = __int_as_float(0x7fc00000);
+        }
     }
 
     // ---- gradient w.r.t. the segment's start state: decay the first token's totals once more ----------
@@ -872,45 +907,56 @@ static BwdShape bwd_shape(int KP) {
         default: return {0, 0, 0};
     }
 }
-// Warps per CTA: 8 when d_v is long enough to use them and the shared-memory layout fits, else 4.
+// Compute warps a CTA may have at each tiling (launch_bwd_t instantiates these).  With the helper warps beside them up
+// to 7 leave 255 registers per thread, which 12 state elements need, and 8 to 11 leave 168, which 8 elements need.
+static const int* bwd_warp_choices(int KP) {
+    static const int small[] = {8, 4, 0}, w48[] = {8, 7, 6, 4, 0}, w64[] = {11, 8, 4, 0}, w96[] = {8, 7, 6, 4, 0}, wide[] = {8, 0};
+    return KP <= 32 ? small : KP == 48 ? w48 : KP == 64 || KP == 128 ? w64 : KP == 96 || KP == 192 ? w96 : wide;
+}
 struct BwdConfig {
     BwdShape s;
     int W, TV, smem, kbuf;
+    double cost;
 };
+// The choice that costs least.  A token of a CTA of W warps costs W + 4 (the walk, and what does not grow with the
+// rows; 15 % more where 12 elements per thread spill at W = 8), an SM holds one CTA, and up to three waves are whole
+// ones; a grid beyond that, or one of segments, is charged by its CTAs.  At T = 2048 bf16, ms: 16 sequence-heads of
+// 192x128 4.08 / 3.25 at W = 7 / 8 (160 and 128 CTAs), 32 of 96x192 3.04 / 3.09 / 2.41 at 8 / 7 / 6, 128 of 96x192
+// 8.95 / 8.35 / 8.41, 64 of 128x192 5.33 / 6.45 at 11 / 8; 8 of 64x64 (T = 512, fp32) 0.27 / 0.19 at 8 / 4.
 static BwdConfig bwd_config(const palimpsa_problem& p) {
-    BwdConfig c{};
-    c.s = bwd_shape(palimpsa_padded_k(p.K));
-    if (!c.s.RK) return c;
-    const int VG = 32 / c.s.KG, rpw = VG * c.s.RV, KP = c.s.RK * c.s.KG;
+    BwdConfig best{};
+    best.s = bwd_shape(palimpsa_padded_k(p.K));
+    if (!best.s.RK) return best;
+    const BwdShape s = best.s;
+    const int VG = 32 / s.KG, rpw = VG * s.RV, KP = s.RK * s.KG;
     const bool unc = (p.flags & PALIMPSA_FLAG_UNCERTAINTY) != 0;
     const int es = dtype_size(p.io_dtype);
-    int W = (rpw == 1 || p.V > 4 * rpw) ? 8 : 4;
-    // d_k = 128: 11 or 12 warps (22 / 24 rows) per CTA hide latency better than 8; of the two, the one that
-    // pads d_v with fewer idle rows (d_v = 128: 6 tiles of 22 rows = 132 instead of 144)
-    if (KP == 128 && rpw == 2 && p.V >= 48) {
-        const int pad11 = (p.V + 21) / 22 * 22, pad12 = (p.V + 23) / 24 * 24;
-        W = pad11 < pad12 ? 11 : 12;
-    }
-    // d_k = 48 (8 rows per warp): 6 warps = 48 rows where that pads d_v with fewer idle rows than 64 (d_v = 48, 96, 144)
-    if (KP == 48 && rpw == 8 && W == 8 && (p.V + 47) / 48 * 48 < (p.V + 63) / 64 * 64) W = 6;
-    for (;;) {
-        c.W = W;
-        c.TV = W * rpw;
-        c.kbuf = 2;
-        c.smem = bwd_smem_layout(KP, c.TV, c.s.RV * c.s.RK, 32 * W, W * VG, es, unc, 2).total;
+    const double units = (double)p.num_seqs * p.H;
+    for (const int* w = bwd_warp_choices(KP); *w; ++w) {
+        BwdConfig c{s, *w, *w * rpw, 0, 2, 0};
+        c.smem = bwd_smem_layout(KP, c.TV, s.RV * s.RK, 32 * c.W, c.W * VG, es, unc, 2).total;
         if (c.smem > 227 * 1024) {
             c.kbuf = 1;
-            c.smem = bwd_smem_layout(KP, c.TV, c.s.RV * c.s.RK, 32 * W, W * VG, es, unc, 1).total;
+            c.smem = bwd_smem_layout(KP, c.TV, s.RV * s.RK, 32 * c.W, c.W * VG, es, unc, 1).total;
         }
-        if (c.smem <= 227 * 1024 || W == 4 || rpw == 1 || W >= 11) break;  // 6 and 8 fall back to 4
-        W = 4;
+        if (c.smem > 227 * 1024) continue;
+        const int tiles = (p.V + c.TV - 1) / c.TV;
+        c.cost = (units > 0 ? units : 1) * tiles / 148;
+        if (p.segments != BWD_FEWEST_TILES) {
+            if (units > 0 && p.segments <= 1 && c.cost <= 3) c.cost = ceil(c.cost);
+            c.cost *= c.W + 4;
+            if (c.W == 8 && s.RK * s.RV == 12) c.cost *= 1.15;
+        }
+        if (!best.W || c.cost < best.cost) best = c;
     }
-    return c;
+    return best;
 }
+
+double bwd_token_cost(const palimpsa_problem& p) { return bwd_config(p).cost; }
 
 int bwd_tile_rows(const palimpsa_problem& p) {
     const BwdConfig c = bwd_config(p);
-    return (c.s.RK && c.smem <= 227 * 1024) ? c.TV : 0;
+    return c.TV;  // 0: nothing fits
 }
 
 BwdWorkspace bwd_workspace_layout(const palimpsa_problem& p) {
@@ -945,7 +991,7 @@ static int launch_bwd_w(const BwdArgs& a, int tiles, int num_seg, bool carry_onl
     const BwdSmem L = bwd_smem_layout(RK * KG, TV, RV * RK, 32 * W, W * VG, dtype_size(p.io_dtype), unc, a.kbuf);
     if (L.total > 227 * 1024) return PALIMPSA_E_DIM;
     dim3 grid(tiles, p.num_seqs * p.H, num_seg);
-    dim3 block(32 * W, 1, 1);
+    dim3 block(bwd_threads(W, carry_only), 1, 1);
 #define PALIMPSA_BWD_LAUNCH(U, C)                                                                                 \
     do {                                                                                                          \
         if (!allow_smem<bwd_kernel<RK, KG, RV, W, U, C>>(L.total)) return PALIMPSA_E_LAUNCH;                        \
@@ -965,14 +1011,17 @@ static int launch_bwd_t(const BwdArgs& args, int tiles, int num_seg, bool carry_
     const BwdConfig cfg = bwd_config(args.p);
     BwdArgs a = args;
     a.kbuf = cfg.kbuf;
-    if (cfg.W == 8) return launch_bwd_w<RK, KG, RV, 8>(a, tiles, num_seg, carry_only, stream);
-    if constexpr (RK == 6 && KG == 8 && RV == 2)
-        if (cfg.W == 6) return launch_bwd_w<RK, KG, RV, 6>(a, tiles, num_seg, carry_only, stream);
-    if constexpr (RK == 4 && KG == 32 && RV == 2) {
-        if (cfg.W == 12) return launch_bwd_w<RK, KG, RV, 12>(a, tiles, num_seg, carry_only, stream);
-        if (cfg.W == 11) return launch_bwd_w<RK, KG, RV, 11>(a, tiles, num_seg, carry_only, stream);
+#define PALIMPSA_W(n)                                                                                    \
+    if (cfg.W == n) return launch_bwd_w<RK, KG, RV, n>(a, tiles, num_seg, carry_only, stream)
+    constexpr int KP = RK * KG;
+    PALIMPSA_W(8);
+    if constexpr (RK == 6) {
+        PALIMPSA_W(7);
+        PALIMPSA_W(6);
     }
-    if constexpr (RV > 1) return launch_bwd_w<RK, KG, RV, 4>(a, tiles, num_seg, carry_only, stream);
+    if constexpr (KP == 64 || KP == 128) PALIMPSA_W(11);
+    if constexpr (RV > 1) PALIMPSA_W(4);
+#undef PALIMPSA_W
     return PALIMPSA_E_DIM;
 }
 
@@ -1066,7 +1115,12 @@ int launch_bwd_static(const palimpsa_bwd_params* prm, cudaStream_t stream) {
     constexpr int MAX_DEV = 64;
     static void* addr[MAX_DEV] = {};
     static std::mutex mu;
-    const BwdWorkspace ws = bwd_workspace_layout(prm->p);
+    palimpsa_bwd_params local = *prm;
+    BwdWorkspace ws = bwd_workspace_layout(local.p);
+    if (ws.total > (size_t)PALIMPSA_STATIC_SCRATCH_BYTES) {  // short tiles for a small grid, too many of them: take tall ones
+        local.p.segments = BWD_FEWEST_TILES;
+        ws = bwd_workspace_layout(local.p);
+    }
     if (!ws.tiles) return PALIMPSA_E_DIM;
     if (ws.total > (size_t)PALIMPSA_STATIC_SCRATCH_BYTES) return PALIMPSA_E_LIMIT;
     int dev = -1;
@@ -1086,7 +1140,6 @@ int launch_bwd_static(const palimpsa_bwd_params* prm, cudaStream_t stream) {
         }
         ptr = addr[dev];
     }
-    palimpsa_bwd_params local = *prm;
     local.workspace = ptr;
     local.workspace_bytes = PALIMPSA_STATIC_SCRATCH_BYTES;
     return launch_bwd(&local, nullptr, false, stream, 3);

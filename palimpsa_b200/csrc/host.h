@@ -84,6 +84,7 @@ int fwd_tile_rows(int K, int V);
 
 // State rows (d_v) one backward CTA owns for this problem; the number of row tiles follows.
 int bwd_tile_rows(const palimpsa_problem& p);
+double bwd_token_cost(const palimpsa_problem& p);  // estimated time per token of the backward, 0 if unsupported
 
 // Layout of the backward scratch memory (byte offsets from a 256-byte aligned base).
 struct BwdWorkspace {

@@ -98,8 +98,18 @@ int64_t plan_segments(int64_t N, int64_t T, int64_t H, int64_t K, int64_t V, int
     if (backward) {
         const int64_t brow = palimpsa_bwd_tile_rows((int)K, (int)V, io, unc ? 1 : 0);
         TORCH_CHECK_VALUE(brow > 0, "no backward tiling for d_k = ", K, ", d_v = ", V);
-        const int64_t ctas = N * H * ((V + brow - 1) / brow), waves = (ctas + sms - 1) / sms;
-        if (packed ? ctas >= sms : (double)ctas >= 0.8 * (double)(waves * sms)) return 1;
+        const int64_t ctas = N * H * ((V + brow - 1) / brow);
+        if (packed) {
+            if (ctas >= sms) return 1;
+        } else {
+            palimpsa_problem p{};
+            p.num_seqs = (int)N, p.H = (int)H, p.K = (int)K, p.V = (int)V, p.io_dtype = io;
+            p.flags = unc ? PALIMPSA_FLAG_UNCERTAINTY : 0;
+            const double uncut = palimpsa_bwd_token_cost(&p);
+            p.segments = 2;
+            const double cut = palimpsa_bwd_token_cost(&p);
+            if (uncut <= 1.25 * cut) return 1;
+        }
     } else if (N * H * ((V + rows - 1) / rows) >= sms) {
         return 1;
     }
@@ -234,6 +244,7 @@ BwdOut bwd_impl(const Inputs& x, const BwdIn& in) {
     prm.struct_size = sizeof(prm);
     prm.p = make_problem(x.q, x.k, x.v, x.b, x.gt, x.g, x.Ip, x.cu, in.coff, in.order, Tensor(), Tensor(), in.scale,
                          (unc ? PALIMPSA_FLAG_UNCERTAINTY : 0) | (in.explicit_init ? PALIMPSA_FLAG_EXPLICIT_INIT : 0));
+    if (in.decay.defined() && in.decay.numel() > 0) prm.p.segments = (int)in.decay.size(1);
     prm.d_o = ptr(in.d_o), prm.d_o_var = ptr(in.d_o_var);
     prm.ckpt_M = ptr<float>(in.ckM), prm.ckpt_I = ptr<float>(in.ckI);
     prm.dq = ptr(r.dq), prm.dk = ptr(r.dk), prm.dv = ptr(r.dv), prm.db = ptr(r.db);

@@ -94,10 +94,11 @@ def plan_segments(N: int, T: int, H: int, K: int, V: int, device=None, backward:
     (sequence, head, row-tile) CTAs would leave SMs idle, e.g. one very long sequence or a narrow batch slice.
 
     Forward only: the forward grid has fewer CTAs than the device has SMs.  With a backward to follow
-    (``backward=True``) the backward kernel decides, since it is 3/4 of the step and keeps one CTA of up to 12 warps
-    per SM: segments when its grid fills less than 80 % of the waves it occupies (72 CTAs on 148 SMs, or 192 CTAs =
-    1.3 waves; not 128 CTAs = 0.86 of a wave, nor 288 = 1.95 waves).  Tile heights come from the library, the SM
-    count from the device.
+    (``backward=True``) the backward kernel decides, since it is 3/4 of the step and keeps one CTA per SM: segments
+    when its estimated time per token (``palimpsa_bwd_token_cost``: waves of CTAs times their warps, at the tile height
+    it would take) is more than 1.25 times that of a grid without idle SMs.  That is so for 72 CTAs on 148 SMs, or
+    192 = 1.3 waves that no other tile height fills better; not for 128 CTAs = 0.86 of a wave, nor 288 = 1.95 waves
+    (2 sequences x 16 heads of 96x192, bf16, T = 2048: 3.97 ms in segments, 3.23 uncut with 24-row tiles).
 
     ``packed``: N documents of unequal length in one row of T tokens (``cu_seqlens``).  Only N and T are known
     without a host synchronisation.  With more CTAs than SMs the documents, started longest first, fill the waves by

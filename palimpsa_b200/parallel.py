@@ -237,6 +237,7 @@ class _CudaLocal:
         self.init = (init_mu, init_I) if first_rank and init_mu is not None else (None, None)
         self.prob = _core._problem(q, k, v, b, gt, g, Ip, None, None, self.init[0], self.init[1], self.scale,
                                    L.FLAG_UNCERTAINTY if uncertainty else 0)
+        self.prob.segments = self.G
 
     def state_like(self):
         return torch.empty(2, self.N, self.H, self.V, self.KP, dtype=torch.float32, device=self.dev)

@@ -1,0 +1,48 @@
+"""Every tile height the backward may take (warps per CTA by head size, element type and grid), with one and two group
+buffers, ragged last tiles and tokens past the last whole block, against the float64 oracle."""
+import ctypes as C
+
+import pytest
+import torch
+
+from oracle import palimpsa_oracle as orc
+from tests.gpu_util import compare, run_cuda, run_oracle, tol_for
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("N,H,T,K,V,dtype,unc", [
+    (2, 1, 33, 16, 9, torch.float32, True),       # d_k 16, 4 warps, one row past a lane group
+    (38, 4, 17, 31, 65, torch.float32, False),    # 8 warps, unaligned rows
+    (2, 2, 35, 32, 100, torch.bfloat16, True),
+    (16, 8, 17, 48, 64, torch.bfloat16, False),   # 8 warps of 12 elements
+    (16, 8, 17, 48, 56, torch.float32, True),     # 7 warps
+    (2, 2, 47, 47, 49, torch.float32, False),     # 6 or fewer, second tile of one row
+    (8, 6, 17, 64, 128, torch.bfloat16, False),   # 11 warps of two column groups
+    (5, 1, 31, 64, 66, torch.float32, True),
+    (12, 2, 17, 96, 192, torch.bfloat16, False),  # 8 warps
+    (16, 2, 17, 90, 192, torch.float32, False),   # 6 warps, element loads
+    (32, 4, 5, 96, 196, torch.bfloat16, True),    # 7 warps, ragged last tile
+    (8, 8, 17, 128, 64, torch.float32, True),     # 8 warps, one group buffer
+    (8, 6, 17, 128, 90, torch.bfloat16, False),   # 11 warps
+    (1, 2, 49, 128, 24, torch.bfloat16, True),    # 4 warps
+    (4, 4, 17, 192, 126, torch.bfloat16, False),  # 8 warps, 126 rows
+    (2, 1, 19, 180, 30, torch.float32, True),
+    (2, 2, 18, 256, 20, torch.float32, True),
+])
+def test_backward_tiling_matches_oracle(N, H, T, K, V, dtype, unc):
+    inp = orc.make_inputs(K + V, B=N, T=T, H=H, K=K, V=V, dtype=dtype)
+    compare(run_cuda(inp, "chunk", unc=unc), run_oracle(inp, unc=unc), tol_for(dtype), what=f"{N}x{H} {K}x{V}")
+
+
+@pytest.mark.parametrize("segments", [0, 2])
+def test_tile_height_follows_the_grid_and_the_workspace_query_with_it(segments):
+    """A small grid takes shorter tiles (more row tiles, more scratch) than one of many waves or of segments."""
+    from palimpsa_b200 import _lib as L
+    p = L.Problem()
+    p.num_seqs, p.seq_len, p.total_tokens, p.H, p.K, p.V, p.io_dtype, p.segments = 1, 64, 64, 2, 128, 128, L.BF16, segments
+    tiles = 16 if segments == 0 else 6
+    row = 4 * (128 * (2 * tiles + 1) + 2 * (tiles + 1))
+    need = L.lib().palimpsa_bwd_workspace_bytes(C.byref(p))
+    assert 0 <= need - 128 * row - 2 * 296 * 2 * 4 <= 6 * 256
+    assert L.lib().palimpsa_bwd_token_cost(C.byref(p)) > 0
