@@ -1131,7 +1131,7 @@ int launch_bwd_static(const palimpsa_bwd_params* prm, cudaStream_t stream) {
         if (!addr[dev]) {
             void* sym = nullptr;
             // may be the call that loads this module on the device (lazy loading): the array is reserved now,
-            // and a device without 64 MiB to spare fails here
+            // and a device without 96 MiB to spare fails here
             if (cudaGetSymbolAddress(&sym, g_static_scratch) != cudaSuccess || !sym) {
                 (void)cudaGetLastError();
                 return PALIMPSA_E_SYMBOL;

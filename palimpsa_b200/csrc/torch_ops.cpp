@@ -92,7 +92,8 @@ int64_t segment_len(int64_t T, int64_t G) {
 // How many segments to cut every sequence into on one GPU (plan_segments in _core.py documents the rule).
 int64_t plan_segments(int64_t N, int64_t T, int64_t H, int64_t K, int64_t V, int64_t sms, bool backward, int io, bool unc,
                       bool packed) {
-    if (T < 2048) return 1;
+    const bool shorter = T < 2048;
+    if (shorter && (T < 256 || packed || io == PALIMPSA_BF16)) return 1;
     const int64_t rows = palimpsa_fwd_tile_rows((int)K, (int)V);
     TORCH_CHECK_VALUE(rows > 0, "d_k = ", K, " is above the supported maximum of 256");
     if (backward) {
@@ -108,8 +109,16 @@ int64_t plan_segments(int64_t N, int64_t T, int64_t H, int64_t K, int64_t V, int
             const double uncut = palimpsa_bwd_token_cost(&p);
             p.segments = 2;
             const double cut = palimpsa_bwd_token_cost(&p);
+            if (shorter) {  // one wave of segments; a segment's backward takes its state-gradient pass first
+                const int64_t G = std::min<int64_t>(T / 64, sms / std::max<int64_t>(ctas, 1));
+                const double one_wave = cut * (double)sms / (double)std::max<int64_t>(ctas, 1);
+                return G >= 2 && (double)T * uncut > 1.6 * one_wave * (double)T / (double)G + 400 ? G : 1;
+            }
             if (uncut <= 1.25 * cut) return 1;
         }
+    } else if (shorter) {
+        const int64_t G = std::min<int64_t>(T / 64, sms / std::max<int64_t>(N * H * ((V + rows - 1) / rows), 1));
+        return G >= 3 ? G : 1;
     } else if (N * H * ((V + rows - 1) / rows) >= sms) {
         return 1;
     }

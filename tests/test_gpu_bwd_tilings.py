@@ -46,3 +46,22 @@ def test_tile_height_follows_the_grid_and_the_workspace_query_with_it(segments):
     need = L.lib().palimpsa_bwd_workspace_bytes(C.byref(p))
     assert 0 <= need - 128 * row - 2 * 296 * 2 * 4 <= 6 * 256
     assert L.lib().palimpsa_bwd_token_cost(C.byref(p)) > 0
+
+
+@pytest.mark.parametrize("B,T,H,K,V,dtype,unc", [
+    (2, 256, 2, 64, 64, torch.float32, False),    # the shortest sequence that is cut
+    (1, 257, 3, 31, 65, torch.float32, True),     # ragged last segment, unaligned rows
+    (1, 1000, 2, 128, 128, torch.float16, False),
+    (3, 511, 1, 48, 96, torch.float32, False),
+])
+def test_short_sequences_in_segments_match_oracle(B, T, H, K, V, dtype, unc):
+    """Float32 and float16 sequences under 2048 tokens run in segments (exact float32 boundary states)."""
+    from palimpsa_b200 import _lib as L
+    from palimpsa_b200.ops.palimpsa._core import plan_segments
+    io = L.F32 if dtype == torch.float32 else L.F16
+    assert plan_segments(B, T, H, K, V, backward=True, io_dtype=io, uncertainty=unc) > 1
+    inp = orc.make_inputs(T, B=B, T=T, H=H, K=K, V=V, dtype=dtype)
+    mu0, I0 = orc.make_states(5, B, H, V, K, inp["Ip"])
+    for state in ({}, dict(mu0=mu0, I0=I0)):
+        got = run_cuda(inp, "chunk", unc=unc, **state)
+        compare(got, run_oracle(inp, unc=unc, **state), tol_for(dtype), what=f"{B}x{H} T={T}")
