@@ -596,7 +596,9 @@ __global__ void __launch_bounds__(bwd_threads(W, CO)) bwd_kernel(const BwdArgs a
         const int c = blk1 - 1;
         const int nt = min(TB, len - c * TB);
         bwd_issue_ckpt(a, NTHR, sm, L, 0, KP, TV, slot0 + c, h, v0, tvw);
-        if (a.aligned) bwd_issue_raw(a, NTHR, sm, L, es, KP, TV, (long long)bos + c * TB, nt, nt, h, v0, tvw);
+        // the step size of the token after the block too, where the sequence goes on past this segment
+        if (a.aligned)
+            bwd_issue_raw(a, NTHR, sm, L, es, KP, TV, (long long)bos + c * TB, nt, min(TB + 1, len - c * TB), h, v0, tvw);
         cp_async_commit();
     }
 
