@@ -61,6 +61,16 @@ void require_cuda(std::initializer_list<const Tensor*> ts) {
                     "palimpsa_b200 runs on CUDA (sm_100a) only and has no CPU path; for CPU tensors use "
                     "palimpsa_b200.ops.palimpsa_ref (naive recurrence).");
 }
+// The last check before pointers are taken, whichever way a call came in: the kernels read each argument through a raw
+// pointer, so a host tensor, one of another GPU, another dtype, length or stride would be a fault or garbage there.
+void check_arg(const char* name, const Tensor& t, at::ScalarType dt, at::IntArrayRef sizes, const at::Device& dev) {
+    if (!t.defined()) return;
+    require_cuda({&t});
+    TORCH_CHECK_VALUE(t.device() == dev, name, " is on ", t.device(), ", q on ", dev);
+    TORCH_CHECK_TYPE(t.scalar_type() == dt, name, " has dtype ", t.scalar_type(), ", expected ", dt);
+    TORCH_CHECK_VALUE(t.numel() == c10::multiply_integers(sizes), name, " has shape ", t.sizes(), ", expected ", sizes);
+    TORCH_CHECK_VALUE(t.is_contiguous(), name, " is not contiguous");
+}
 // Nothing between the caller and the kernels: no dispatch mode, no functorch transform, no tensor subclass.
 bool plain(std::initializer_list<const Tensor*> ts) {
     if (c10::impl::dispatch_mode_enabled()) return false;
@@ -76,6 +86,8 @@ Tensor as(const Tensor& t, at::ScalarType dt) {
     return r.is_contiguous() ? r : r.contiguous();
 }
 Tensor as_opt(const OptTensor& t, at::ScalarType dt) { return given(t) ? as(*t, dt) : Tensor(); }
+Tensor dense(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
+Tensor dense(const OptTensor& t) { return given(t) ? dense(*t) : Tensor(); }
 void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 
 int sm_count(const OptTensor& t) {
@@ -176,7 +188,33 @@ struct FwdOut {
     Tensor o, o_var, fmu, fI, ckM, ckI, coff, order, decay;  // undefined where not asked for
 };
 
+void check_inputs(const Inputs& x) {
+    TORCH_CHECK_VALUE(x.q.dim() == 4 && x.k.sizes() == x.q.sizes() && x.v.dim() == 4 && x.b.sizes() == x.v.sizes() &&
+                          x.v.sizes().slice(0, 3) == x.q.sizes().slice(0, 3),
+                      "expected q,k [B,T,H,K] and v,b [B,T,H,V]");
+    const int64_t B = x.q.size(0), T = x.q.size(1), H = x.q.size(2), K = x.q.size(3), V = x.v.size(3);
+    const at::Device dev = x.q.device();
+    const at::ScalarType io = x.q.scalar_type();
+    io_code(io);
+    check_arg("q", x.q, io, {B, T, H, K}, dev);
+    check_arg("k", x.k, io, {B, T, H, K}, dev);
+    check_arg("v", x.v, io, {B, T, H, V}, dev);
+    check_arg("b", x.b, io, {B, T, H, V}, dev);
+    check_arg("gt", x.gt, at::kFloat, {B, T, H}, dev);
+    check_arg("g", x.g, at::kFloat, {H}, dev);
+    check_arg("Ip", x.Ip, at::kFloat, {H}, dev);
+    if (x.cu.defined()) {
+        TORCH_CHECK_VALUE(B == 1 && x.cu.numel() >= 1, "cu_seqlens [N+1] goes with one packed row");
+        check_arg("cu_seqlens", x.cu, at::kInt, {x.cu.numel()}, dev);
+    }
+    const int64_t N = x.cu.defined() ? x.cu.numel() - 1 : B;
+    TORCH_CHECK_VALUE(x.mu0.defined() == x.I0.defined(), "initial_mu_state and initial_I_state must be given together");
+    check_arg("initial_mu_state", x.mu0, at::kFloat, {N, H, V, K}, dev);
+    check_arg("initial_I_state", x.I0, at::kFloat, {N, H, V, K}, dev);
+}
+
 FwdOut fwd_impl(const Inputs& x, const Options& opt) {
+    check_inputs(x);
     const int64_t B = x.q.size(0), T = x.q.size(1), H = x.q.size(2), K = x.q.size(3), V = x.v.size(3);
     const int64_t N = x.cu.defined() ? x.cu.numel() - 1 : B;
     const at::Device dev = x.q.device();
@@ -235,9 +273,27 @@ struct BwdOut {
 };
 
 BwdOut bwd_impl(const Inputs& x, const BwdIn& in) {
+    check_inputs(x);
     const int64_t B = x.q.size(0), T = x.q.size(1), H = x.q.size(2), K = x.q.size(3), V = x.v.size(3);
     const at::Device dev = x.q.device();
     const at::ScalarType io = x.q.scalar_type();
+    const int64_t seqs = x.cu.defined() ? x.cu.numel() - 1 : B;
+    check_arg("the gradient of o", in.d_o, io, {B, T, H, V}, dev);
+    check_arg("the gradient of o_var", in.d_o_var, io, {B, T, H, V}, dev);
+    TORCH_CHECK_VALUE(in.ckM.dim() == 4, "ckpt_M, ckpt_I [slots,H,V,KP]");
+    const int64_t slots = in.ckM.size(0), need_slots = (B * T + PALIMPSA_CKPT_INTERVAL - 1) / PALIMPSA_CKPT_INTERVAL + seqs;
+    TORCH_CHECK_VALUE(slots >= need_slots, "ckpt_M has ", slots, " slots, expected ", need_slots);
+    check_arg("ckpt_M", in.ckM, at::kFloat, {slots, H, V, palimpsa_padded_k((int)K)}, dev);
+    check_arg("ckpt_I", in.ckI, at::kFloat, {slots, H, V, palimpsa_padded_k((int)K)}, dev);
+    if (x.cu.defined()) {
+        TORCH_CHECK_VALUE(in.coff.defined(), "a packed backward needs the forward's chunk_offsets");
+        check_arg("chunk_offsets", in.coff, at::kInt, {seqs}, dev);
+        check_arg("seq_order", in.order, at::kInt, {seqs}, dev);
+    }
+    if (in.decay.defined() && in.decay.numel() > 0) {
+        TORCH_CHECK_VALUE(in.decay.dim() == 3, "seg_decay [N,G,H]");
+        check_arg("seg_decay", in.decay, at::kFloat, {seqs, in.decay.size(1), H}, dev);
+    }
     c10::cuda::CUDAGuard guard(dev);
     void* st = stream_of(x.q);
     BwdOut r;
@@ -297,8 +353,8 @@ FwdTuple fwd_cuda(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
     Options opt;
     opt.scale = scale, opt.unc = uncertainty, opt.save_ckpt = save_ckpt, opt.want_final = want_final;
     opt.recurrent = recurrent, opt.segments = num_segments;
-    FwdOut r = fwd_impl({q, k, v, b, gt, g, Ip, as_opt(init_mu, at::kFloat), as_opt(init_I, at::kFloat),
-                         as_opt(cu_seqlens, at::kInt)}, opt);
+    FwdOut r = fwd_impl({dense(q), dense(k), dense(v), dense(b), dense(gt), dense(g), dense(Ip), as_opt(init_mu, at::kFloat),
+                         as_opt(init_I, at::kFloat), as_opt(cu_seqlens, at::kInt)}, opt);
     auto f = [&](Tensor& t, at::ScalarType dt) { return t.defined() ? t : none_like(q, dt); };
     // the slots are handed out as a tensor of their own: an operator's outputs share no storage
     return {r.o, f(r.o_var, q.scalar_type()), f(r.fmu, at::kFloat), f(r.fI, at::kFloat), f(r.ckM, at::kFloat),
@@ -309,13 +365,14 @@ BwdTuple bwd_cuda(const Tensor& d_o, const OptTensor& d_o_var, const Tensor& q, 
                   const Tensor& b, const Tensor& gt, const Tensor& g, const Tensor& Ip, const OptTensor& cu_seqlens,
                   const OptTensor& chunk_offsets, const Tensor& ckpt_M, const Tensor& ckpt_I, double scale,
                   bool explicit_init, bool recurrent, const OptTensor& seg_decay) {
-    Inputs x{q, k, v, b, gt, g, Ip, Tensor(), Tensor(), as_opt(cu_seqlens, at::kInt)};
+    Inputs x{dense(q), dense(k), dense(v), dense(b), dense(gt), dense(g), dense(Ip), Tensor(), Tensor(), as_opt(cu_seqlens, at::kInt)};
     BwdIn in;
-    in.d_o = d_o, in.d_o_var = given(d_o_var) ? *d_o_var : Tensor();
-    in.coff = given(chunk_offsets) ? *chunk_offsets : Tensor();
-    in.ckM = ckpt_M, in.ckI = ckpt_I, in.decay = given(seg_decay) ? *seg_decay : Tensor();
+    in.d_o = dense(d_o), in.d_o_var = dense(d_o_var);
+    in.coff = dense(chunk_offsets);
+    in.ckM = dense(ckpt_M), in.ckI = dense(ckpt_I), in.decay = dense(seg_decay);
     in.explicit_init = explicit_init, in.recurrent = recurrent, in.scale = scale;
     if (x.cu.defined()) {
+        check_inputs(x);
         const int64_t N = x.cu.numel() - 1;
         c10::cuda::CUDAGuard guard(q.device());
         Tensor plan = empty({2 * N}, at::kInt, q.device());
@@ -433,6 +490,8 @@ std::tuple<Tensor, Tensor> decode_impl(const Tensor& q, const Tensor& k, const T
                                        const Tensor& g, const Tensor& Ip, const Tensor& mu, const Tensor& I, double scale,
                                        bool unc) {
     const at::Device dev = q.device();
+    check_inputs({q, k, v, b, gt, g, Ip, mu, I, Tensor()});
+    TORCH_CHECK_VALUE(q.size(1) == 1, "decode_step takes exactly one token per sequence");
     c10::cuda::CUDAGuard guard(dev);
     const int64_t N = q.size(0), H = q.size(2), V = v.size(3);
     Tensor o = empty({N, 1, H, V}, q.scalar_type(), dev), o_var;
@@ -451,7 +510,8 @@ void bump_version(const Tensor& t) {
 std::tuple<Tensor, Tensor> decode_cuda(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& gt,
                                        const Tensor& g, const Tensor& Ip, const Tensor& mu_state, const Tensor& I_state,
                                        double scale, bool uncertainty) {
-    auto [o, o_var] = decode_impl(q, k, v, b, gt, g, Ip, mu_state, I_state, scale, uncertainty);
+    auto [o, o_var] = decode_impl(dense(q), dense(k), dense(v), dense(b), dense(gt), dense(g), dense(Ip), mu_state, I_state,
+                                  scale, uncertainty);
     return {o, o_var.defined() ? o_var : none_like(q, q.scalar_type())};
 }
 std::tuple<Tensor, Tensor> call_decode_op(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& gt,

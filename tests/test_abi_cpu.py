@@ -123,6 +123,23 @@ def test_python_wrappers_reject_cpu_tensors_and_bad_shapes():
                                  initial_I_state=torch.ones(3, 2, 4, 4))
 
 
+def test_operator_kernels_reject_host_tensors_before_any_launch():
+    """The registered operators' CUDA kernels check every tensor themselves: called with host tensors (as the dispatcher
+    does when one argument of several is on the GPU) they raise instead of handing a host pointer to a kernel."""
+    import torch
+    from palimpsa_b200.ops.palimpsa import _core, decode
+    keys = torch._C.DispatchKeySet(torch._C.DispatchKey.CUDA)
+    q, gt, g = torch.randn(2, 16, 2, 16), torch.rand(2, 16, 2), torch.ones(2)
+    ck, st = torch.zeros(4, 2, 16, 16), torch.zeros(2, 2, 16, 16)
+    with pytest.raises(RuntimeError, match="no CPU path"):
+        _core.fwd_op.redispatch(keys, q, q, q, q, gt, g, g, None, None, None, 0.25, False, True, True, False, 1)
+    with pytest.raises(RuntimeError, match="no CPU path"):
+        _core.bwd_op.redispatch(keys, q, None, q, q, q, q, gt, g, g, None, None, ck, ck, 0.25, False, False, None)
+    t = q[:, :1].contiguous()
+    with pytest.raises(RuntimeError, match="no CPU path"):
+        decode.decode_step_op.redispatch(keys, t, t, t, t, gt[:, :1].contiguous(), g, g, st, st, 0.25, False)
+
+
 def test_naive_ref_matches_fixture():
     import torch
     from oracle import palimpsa_oracle as orc

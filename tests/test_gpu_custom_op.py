@@ -78,3 +78,38 @@ def test_torch_compile_decode_loop_updates_the_cache_in_place():
     assert torch.equal(ref, out)
     assert torch.equal(args[7], ref_args[7]) and torch.equal(args[8], ref_args[8])      # caches advanced identically
     assert not torch.equal(args[7], _decode_args()[7])
+
+
+def _raises_before_launch(op, args, i, bad, exc):
+    args = list(args)
+    args[i] = bad
+    with pytest.raises(exc):
+        op(*args)
+    torch.cuda.synchronize()
+
+
+def test_registered_operators_check_every_tensor():
+    """Called directly, the operators refuse host tensors, another dtype and a wrong length (each would be a bad address or
+    garbage in the kernel), and take rows of any stride."""
+    from palimpsa_b200.ops.palimpsa import _core, decode as D
+    a = _args(grad=False)
+    fwd = (*a, None, None, None, 0.25, False, True, True, False, 1)
+    for i in range(7):
+        _raises_before_launch(_core.fwd_op, fwd, i, a[i].cpu(), (RuntimeError, ValueError))
+    _raises_before_launch(_core.fwd_op, fwd, 4, a[4].bfloat16(), TypeError)
+    _raises_before_launch(_core.fwd_op, fwd, 5, a[5][:1], ValueError)
+    _raises_before_launch(_core.fwd_op, fwd, 2, a[2].bfloat16(), TypeError)
+    o, _, _, _, ckM, ckI, _, _ = _core.fwd_op(*fwd)
+    strided = [x.transpose(1, 2).contiguous().transpose(1, 2) if x.dim() == 4 else x for x in a]
+    assert torch.equal(_core.fwd_op(*strided, *fwd[7:])[0], o)
+    bwd = (torch.ones_like(o), None, *a, None, None, ckM, ckI, 0.25, False, False, None)
+    for i in (0, 2, 7, 8, 11):
+        _raises_before_launch(_core.bwd_op, bwd, i, bwd[i].cpu(), (RuntimeError, ValueError))
+    _raises_before_launch(_core.bwd_op, bwd, 11, ckM[:2], ValueError)
+    ref = _core.bwd_op(*bwd)
+    got = _core.bwd_op(torch.ones_like(o)[..., :1].expand_as(o), *bwd[1:])
+    assert all(torch.equal(x, y) for x, y in zip(ref, got))
+    dec = (*_decode_args(), 0.25, False)
+    for i in (0, 5, 7):
+        _raises_before_launch(D.decode_step_op, dec, i, dec[i].cpu(), (RuntimeError, ValueError))
+    _raises_before_launch(D.decode_step_op, dec, 7, dec[7].bfloat16(), TypeError)
