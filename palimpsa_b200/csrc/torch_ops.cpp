@@ -753,7 +753,7 @@ variable_list layer_prologue(const Tensor& q_raw, const Tensor& k_raw, const Ten
     require_cuda({&q_raw, &k_raw, &x, &b_raw, &dt_raw, &bs_raw, &dt_bias, &b_scale});
     io_code(x.scalar_type());
     const int64_t H = x.size(-2), Hq = q_raw.size(-2);
-    TORCH_CHECK_VALUE(H % Hq == 0 && q_raw.sizes() == k_raw.sizes() && b_raw.sizes() == x.sizes() &&
+    TORCH_CHECK_VALUE(Hq > 0 && H % Hq == 0 && q_raw.sizes() == k_raw.sizes() && b_raw.sizes() == x.sizes() &&
                           q_raw.sizes().slice(0, q_raw.dim() - 2) == x.sizes().slice(0, x.dim() - 2),
                       "layer_prologue: q_raw/k_raw [...,Hq,K], x/b_raw [...,H,V] with H a multiple of Hq");
     const auto rows = x.sizes().slice(0, x.dim() - 1);

@@ -60,6 +60,26 @@ def test_layer_wrappers_reject_cpu_tensors():
         layer_prologue(x, x, x, x, torch.zeros(1, 2, 2), torch.zeros(1, 2, 2), torch.zeros(2), torch.zeros(2))
 
 
+def test_layer_prologue_without_heads_is_an_error():
+    """No query heads at all: an exception (the head ratio is not divided by zero).  Fake tensors stand in for the GPU's;
+    a child process, since an integer division by zero would end it."""
+    import os
+    import subprocess
+    import sys
+    prog = ("import torch\n"
+            "from torch._subclasses.fake_tensor import FakeTensorMode\n"
+            "from palimpsa_b200.layers import layer_prologue\n"
+            "with FakeTensorMode(allow_non_fake_inputs=True):\n"
+            "    e = lambda *s: torch.empty(*s, device='cuda')\n"
+            "    try:\n"
+            "        layer_prologue(e(1, 2, 0, 8), e(1, 2, 0, 8), e(1, 2, 4, 8), e(1, 2, 4, 8), e(1, 2, 4), e(1, 2, 4), e(4), e(4))\n"
+            "    except ValueError as x:\n"
+            "        print('ValueError', x)\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", prog], capture_output=True, text=True, cwd=root)
+    assert r.returncode == 0 and "ValueError layer_prologue" in r.stdout, (r.returncode, r.stderr[-500:])
+
+
 def test_missing_library_is_a_loud_error(monkeypatch, tmp_path):
     """No CPU or PyTorch fallback: without the built CUDA library every entry fails with a clear message."""
     from palimpsa_b200 import _lib
