@@ -532,9 +532,9 @@ std::tuple<Tensor, Tensor> decode_autograd(const Tensor& q, const Tensor& k, con
     return r;
 }
 
-py::object decode_step(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& b_, const Tensor& gt_,
-                       const Tensor& g_, const Tensor& Ip_, const Tensor& mu, const Tensor& I, std::optional<double> scale,
-                       bool unc) {
+std::tuple<Tensor, Tensor> decode_run(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& b_, const Tensor& gt_,
+                                      const Tensor& g_, const Tensor& Ip_, const Tensor& mu, const Tensor& I,
+                                      std::optional<double> scale, bool unc) {
     auto token = [&](const Tensor& t) { return q_.dim() == 3 ? t.unsqueeze(1) : t; };
     const bool grad = at::GradMode::is_enabled();
     at::NoGradGuard no_grad;
@@ -564,6 +564,17 @@ py::object decode_step(const Tensor& q_, const Tensor& k_, const Tensor& v_, con
         r = call_decode_op(d(as(q, io)), d(as(k, io)), d(as(v, io)), d(as(b, io)), d(as(gt, at::kFloat)), d(as(g_, at::kFloat)),
                            d(as(Ip_, at::kFloat)), mu, I, sc, unc);
     }
+    return r;
+}
+// The entries Python calls give the interpreter lock back while they work: an allocation or a launch may wait for the
+// device, and other threads have to be able to feed it meanwhile.
+py::object decode_step(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& gt, const Tensor& g,
+                       const Tensor& Ip, const Tensor& mu, const Tensor& I, std::optional<double> scale, bool unc) {
+    std::tuple<Tensor, Tensor> r;
+    {
+        py::gil_scoped_release no_gil;
+        r = decode_run(q, k, v, b, gt, g, Ip, mu, I, scale, unc);
+    }
     if (unc) return py::cast(r);
     return py::cast(std::get<0>(r));
 }
@@ -592,9 +603,12 @@ void copy_inputs(const std::vector<Tensor>& dst, const std::vector<OptTensor>& s
 }
 
 // ---- chunk_palimpsa / fused_recurrent_palimpsa ------------------------------------------------------------------
-py::object run(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& gt, const Tensor& g,
-               const Tensor& Ip, const OptTensor& mu0, const OptTensor& I0, std::optional<double> scale, bool want_final,
-               bool unc, const OptTensor& cu, bool recurrent, std::optional<int64_t> num_segments, bool carry_tc) {
+struct RunOut {
+    Tensor o, o_var, fmu, fI;  // undefined where not asked for
+};
+RunOut run_impl(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& gt, const Tensor& g,
+                const Tensor& Ip, const OptTensor& mu0, const OptTensor& I0, std::optional<double> scale, bool want_final,
+                bool unc, const OptTensor& cu, bool recurrent, std::optional<int64_t> num_segments, bool carry_tc) {
     if (given(cu)) {
         TORCH_CHECK_VALUE(q.size(0) == 1, recurrent ? "The batch size is expected to be 1 rather than " : "Batch size must be 1 for Varlen, got ",
                           q.size(0), recurrent ? " when using `cu_seqlens`." : "");
@@ -656,8 +670,18 @@ py::object run(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& 
     const at::ScalarType o_dt = recurrent ? v.scalar_type() : q.scalar_type(), var_dt = recurrent ? at::kFloat : q.scalar_type();
     if (o.scalar_type() != o_dt) o = o.to(o_dt);
     if (unc && o_var.scalar_type() != var_dt) o_var = o_var.to(var_dt);
-    py::object out = unc ? py::cast(std::make_tuple(o, o_var)) : py::cast(o);
-    if (want_final) return py::make_tuple(out, fmu, fI);
+    return {o, o_var, fmu, fI};
+}
+py::object run(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& gt, const Tensor& g,
+               const Tensor& Ip, const OptTensor& mu0, const OptTensor& I0, std::optional<double> scale, bool want_final,
+               bool unc, const OptTensor& cu, bool recurrent, std::optional<int64_t> num_segments, bool carry_tc) {
+    RunOut r;
+    {
+        py::gil_scoped_release no_gil;
+        r = run_impl(q, k, v, b, gt, g, Ip, mu0, I0, scale, want_final, unc, cu, recurrent, num_segments, carry_tc);
+    }
+    py::object out = unc ? py::cast(std::make_tuple(r.o, r.o_var)) : py::cast(r.o);
+    if (want_final) return py::make_tuple(out, r.fmu, r.fI);
     return out;
 }
 
@@ -867,9 +891,9 @@ TORCH_LIBRARY_IMPL(palimpsa_b200, Autograd, m) {
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("run", &run);
     m.def("decode_step", &decode_step);
-    m.def("copy_inputs", &copy_inputs);
-    m.def("layer_prologue", &layer_prologue);
-    m.def("layer_epilogue", &layer_epilogue);
+    m.def("copy_inputs", &copy_inputs, py::call_guard<py::gil_scoped_release>());
+    m.def("layer_prologue", &layer_prologue, py::call_guard<py::gil_scoped_release>());
+    m.def("layer_epilogue", &layer_epilogue, py::call_guard<py::gil_scoped_release>());
     m.def("plan_segments", &plan_segments_py);
     m.def("abi_version", [] { return PALIMPSA_ABI_VERSION; });
 }
