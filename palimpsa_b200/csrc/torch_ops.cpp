@@ -7,8 +7,9 @@
 // microseconds plus the launches.
 //
 // Two ways in:
-//   * run(), decode_step(), layer_*(): what the Python functions call.  Plain CUDA tensors with no dispatch mode
-//     active go straight to the implementation (with one autograd node where gradients are wanted).
+//   * run(), decode_step(), layer_*(): what the Python functions call.  Plain CUDA tensors with nothing in between go
+//     straight to the implementation (with one autograd node where gradients are wanted); for anything else run() and
+//     decode_step() hand NotImplemented back, and the Python functions go through the operators.
 //   * torch.ops.palimpsa_b200.{fwd, bwd, decode_step}: the registered operators, which tracing, functorch and
 //     fake-tensor modes see.  Same implementation underneath; their fake kernels are registered from Python.
 #include <ATen/cuda/CUDAContext.h>
@@ -71,16 +72,26 @@ void check_arg(const char* name, const Tensor& t, at::ScalarType dt, at::IntArra
     TORCH_CHECK_VALUE(t.numel() == c10::multiply_integers(sizes), name, " has shape ", t.sizes(), ", expected ", sizes);
     TORCH_CHECK_VALUE(t.is_contiguous(), name, " is not contiguous");
 }
-// Nothing between the caller and the kernels: no dispatch mode, no functorch transform, no tensor subclass.
+// Nothing between the caller and the kernels: dense CUDA tensors and the thread's usual dispatch state.  Everything else
+// (a mode, a transform, a tracer, a fake, negated, batched or wrapped tensor, a kernel that runs below autograd) has a
+// dispatch key of its own, on the thread or on the tensor, and goes through the registered operators, which is where those
+// hook in.  Named by what is allowed, so that a key nobody thought of takes the general route.
 bool plain(std::initializer_list<const Tensor*> ts) {
+    using c10::DispatchKey;
+    using c10::DispatchKeySet;
+    static const DispatchKeySet usual_state = c10::default_included_set | c10::autocast_dispatch_keyset;
+    static const DispatchKeySet usual_tensor = DispatchKeySet(DispatchKey::CUDA) | DispatchKeySet(DispatchKey::AutogradCUDA) |
+                                               DispatchKeySet(DispatchKey::ADInplaceOrView) | DispatchKeySet(DispatchKey::AutocastCUDA);
     if (c10::impl::dispatch_mode_enabled()) return false;
-    if (c10::impl::tls_local_dispatch_key_set().included_.has(c10::DispatchKey::FuncTorchDynamicLayerFrontMode)) return false;
+    const c10::impl::LocalDispatchKeySet tls = c10::impl::tls_local_dispatch_key_set();
+    if (!(tls.included_ - usual_state).empty()) return false;
+    // below autograd no node may be made (inference mode is there too, with gradients off: nothing to make)
+    if (at::GradMode::is_enabled() && !(tls.excluded_ & c10::autograd_dispatch_keyset).empty()) return false;
     for (const Tensor* t : ts)
-        if (t->defined() && (t->key_set().has(c10::DispatchKey::Python) || t->key_set().has(c10::DispatchKey::FuncTorchGradWrapper) ||
-                             t->key_set().has(c10::DispatchKey::FuncTorchBatched) || t->key_set().has(c10::DispatchKey::Functionalize)))
-            return false;
+        if (t->defined() && !(t->key_set() - usual_tensor).empty()) return false;
     return true;
 }
+py::object not_plain() { return py::reinterpret_borrow<py::object>(Py_NotImplemented); }  // the caller takes the general route
 Tensor as(const Tensor& t, at::ScalarType dt) {
     Tensor r = t.scalar_type() == dt ? t : t.to(dt);
     return r.is_contiguous() ? r : r.contiguous();
@@ -536,7 +547,6 @@ std::tuple<Tensor, Tensor> decode_run(const Tensor& q_, const Tensor& k_, const 
                                       const Tensor& g_, const Tensor& Ip_, const Tensor& mu, const Tensor& I,
                                       std::optional<double> scale, bool unc) {
     auto token = [&](const Tensor& t) { return q_.dim() == 3 ? t.unsqueeze(1) : t; };
-    const bool grad = at::GradMode::is_enabled();
     at::NoGradGuard no_grad;
     Tensor q = token(q_), k = token(k_), v = token(v_), b = token(b_), gt = token(gt_);
     TORCH_CHECK_VALUE(q.dim() == 4 && k.sizes() == q.sizes() && v.dim() == 4 && b.sizes() == v.sizes() &&
@@ -545,31 +555,23 @@ std::tuple<Tensor, Tensor> decode_run(const Tensor& q_, const Tensor& k_, const 
     const int64_t N = q.size(0), H = q.size(2), K = q.size(3), V = v.size(3);
     TORCH_CHECK_VALUE(q.size(1) == 1, "decode_step takes exactly one token per sequence");
     TORCH_CHECK_VALUE(gt.numel() == N * H && g_.numel() == H && Ip_.numel() == H, "expected gt [N,1,H] and g, Ip [H]");
-    require_cuda({&q, &k, &v, &b, &gt, &g_, &Ip_, &mu, &I});
     for (const Tensor* s : {&mu, &I})
         TORCH_CHECK_VALUE(s->scalar_type() == at::kFloat && s->is_contiguous() && s->sizes() == at::IntArrayRef({N, H, V, K}),
                           "state cache tensors must be contiguous float32 of shape (", N, ", ", H, ", ", V, ", ", K, ")");
     const at::ScalarType io = q.scalar_type();
     io_code(io);
     const double sc = scale ? *scale : 1.0 / std::sqrt((double)K);
-    std::tuple<Tensor, Tensor> r;
-    if (plain({&q, &k, &v, &b, &gt, &g_, &Ip_, &mu, &I})) {
-        r = decode_impl(as(q, io), as(k, io), as(v, io), as(b, io), as(gt, at::kFloat), as(g_, at::kFloat), as(Ip_, at::kFloat),
-                        mu, I, sc, unc);
-        bump_version(mu);
-        bump_version(I);
-    } else {
-        at::AutoGradMode restore(grad);
-        auto d = [](const Tensor& t) { return t.detach(); };
-        r = call_decode_op(d(as(q, io)), d(as(k, io)), d(as(v, io)), d(as(b, io)), d(as(gt, at::kFloat)), d(as(g_, at::kFloat)),
-                           d(as(Ip_, at::kFloat)), mu, I, sc, unc);
-    }
+    auto r = decode_impl(as(q, io), as(k, io), as(v, io), as(b, io), as(gt, at::kFloat), as(g_, at::kFloat), as(Ip_, at::kFloat),
+                         mu, I, sc, unc);
+    bump_version(mu);
+    bump_version(I);
     return r;
 }
 // The entries Python calls give the interpreter lock back while they work: an allocation or a launch may wait for the
 // device, and other threads have to be able to feed it meanwhile.
 py::object decode_step(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& gt, const Tensor& g,
                        const Tensor& Ip, const Tensor& mu, const Tensor& I, std::optional<double> scale, bool unc) {
+    if (!plain({&q, &k, &v, &b, &gt, &g, &Ip, &mu, &I})) return not_plain();
     std::tuple<Tensor, Tensor> r;
     {
         py::gil_scoped_release no_gil;
@@ -622,7 +624,6 @@ RunOut run_impl(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor&
                       "expected gt [B,T,H] and g, Ip [H]");
     Inputs x;
     x.cu = cu.value_or(Tensor()), x.mu0 = mu0.value_or(Tensor()), x.I0 = I0.value_or(Tensor());
-    require_cuda({&q, &k, &v, &b, &gt, &g, &Ip, &x.mu0, &x.I0, &x.cu});
     io_code(q.scalar_type());
     if (x.cu.defined()) x.cu = as(x.cu, at::kInt);
     const int64_t N = x.cu.defined() ? x.cu.numel() - 1 : B;
@@ -651,12 +652,7 @@ RunOut run_impl(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor&
     opt.segments = num_segments ? *num_segments
                                 : plan_segments(N, T, H, K, V, sm_count(q), opt.save_ckpt, io_code(io), unc, x.cu.defined());
     Tensor o, o_var, fmu, fI;
-    if (!plain({&x.q, &x.k, &x.v, &x.b, &x.gt, &x.g, &x.Ip, &x.mu0, &x.I0, &x.cu})) {
-        auto opt_t = [](const Tensor& t) { return t.defined() ? OptTensor(t) : std::nullopt; };
-        auto r = call_fwd_op(x.q, x.k, x.v, x.b, x.gt, x.g, x.Ip, opt_t(x.mu0), opt_t(x.I0), opt_t(x.cu), opt.scale, unc,
-                             opt.save_ckpt, want_final, recurrent, opt.segments);
-        o = std::get<0>(r), o_var = std::get<1>(r), fmu = std::get<2>(r), fI = std::get<3>(r);
-    } else if (opt.save_ckpt) {
+    if (opt.save_ckpt) {
         auto r = DirectFn::apply(x.q, x.k, x.v, x.b, x.gt, x.g, x.Ip, x, opt);
         size_t i = 0;
         o = r[i++];
@@ -675,6 +671,8 @@ RunOut run_impl(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor&
 py::object run(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& gt, const Tensor& g,
                const Tensor& Ip, const OptTensor& mu0, const OptTensor& I0, std::optional<double> scale, bool want_final,
                bool unc, const OptTensor& cu, bool recurrent, std::optional<int64_t> num_segments, bool carry_tc) {
+    const Tensor mu = mu0.value_or(Tensor()), I = I0.value_or(Tensor()), c = cu.value_or(Tensor());
+    if (!plain({&q, &k, &v, &b, &gt, &g, &Ip, &mu, &I, &c})) return not_plain();
     RunOut r;
     {
         py::gil_scoped_release no_gil;

@@ -1,4 +1,4 @@
-"""What the operator's Python functions share: the native front end and its registered torch operators, the traced
+"""What the operator's Python functions share: the native front end and its registered torch operators, the general
 form of the call, and the planning and parameter helpers for code that drives the C ABI itself.
 
 Eager calls go to the native front end (csrc/torch_ops.cpp), which checks, allocates and launches without Python in
@@ -12,6 +12,7 @@ from typing import Optional
 
 import torch
 from torch import Tensor
+from torch.overrides import has_torch_function_variadic
 
 from ... import _lib as L
 
@@ -111,8 +112,17 @@ def plan_segments(N: int, T: int, H: int, K: int, V: int, device=None, backward:
     themselves (14 or 19 documents in 32 768 tokens: 4.3 ms unsegmented, 5.0-6.0 ms segmented); with fewer, the
     longest document is the critical path and segments of T / G tokens shorten it (7 documents x 16 heads in
     16 384 tokens: 4.16 -> 2.79 ms)."""
-    return L.torch_ops().plan_segments(int(N), int(T), int(H), int(K), int(V), sm_count(device), bool(backward),
-                                       int(io_dtype), bool(uncertainty), bool(packed))
+    sizes = [_known(x) for x in (N, T, H, K, V)]
+    if None in sizes:
+        return 1
+    return L.torch_ops().plan_segments(*sizes, sm_count(device), bool(backward), int(io_dtype), bool(uncertainty),
+                                       bool(packed))
+
+
+def _known(x):
+    """The size a plan is made for: a symbolic one counts with the value it is traced at.  Any number of segments is right
+    for any size, so no guard is put on it and the traced graph holds for the other sizes too."""
+    return x.node.hint if isinstance(x, torch.SymInt) else int(x)
 
 
 def segment_len(T: int, G: int) -> int:
@@ -196,10 +206,16 @@ def _decode_fake(q, k, v, b, gt, g, Ip, mu_state, I_state, scale, uncertainty):
     return q.new_empty(N, 1, H, V), (q.new_empty(N, 1, H, V) if uncertainty else q.new_empty(0))
 
 
-def run_traced(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state, scale, output_final_state, output_uncertainty,
+def takes_general_route(*args) -> bool:
+    """A compiler traces the caller, or an argument's class or an active mode overrides torch functions: the call has to
+    appear as the registered operator.  What else may stand between it and the kernels, the native entries see themselves."""
+    return torch.compiler.is_compiling() or has_torch_function_variadic(*args)
+
+
+def run_general(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state, scale, output_final_state, output_uncertainty,
                cu_seqlens, recurrent: bool, out_dtype, num_segments: Optional[int] = None, var_dtype=None):
-    """chunk_palimpsa / fused_recurrent_palimpsa while ``torch.compile`` / ``torch.export`` trace the caller: the checks
-    and the dtype policy of the native front end in traceable Python around the registered operator."""
+    """chunk_palimpsa / fused_recurrent_palimpsa around the registered operator, with the checks and the dtype policy of the
+    native front end in Python that can be traced: what compilers, tracers, transforms, fake and wrapped tensors take."""
     ensure_ops_registered()
     if q.dim() != 4 or k.shape != q.shape or v.dim() != 4 or b.shape != v.shape or v.shape[:3] != q.shape[:3]:
         raise ValueError("expected q,k [B,T,H,K] and v,b [B,T,H,V]")

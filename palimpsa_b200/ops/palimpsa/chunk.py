@@ -2,8 +2,6 @@
 palimpsa/ops/palimpsa/chunk_palimpsa_forgetting_scalar.py:623."""
 from __future__ import annotations
 
-import torch
-
 from . import _core
 
 
@@ -28,14 +26,16 @@ def chunk_palimpsa(q, k, v, b, gt, g, Ip, initial_mu_state=None, initial_I_state
     cut (segments of ``T / num_segments`` tokens; those past a sequence's end are empty), and the default only does
     so when there are too few documents to fill one wave of CTAs.
     """
-    if torch.compiler.is_compiling():
-        if scale is None:
-            scale = q.shape[-1] ** -0.5
-        if cu_seqlens is not None and q.shape[0] != 1:
-            raise ValueError(f"Batch size must be 1 for Varlen, got {q.shape[0]}")
-        return _core.run_traced(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state, scale, output_final_state,
-                                output_uncertainty, cu_seqlens, recurrent=False, out_dtype=q.dtype,
-                                num_segments=num_segments, var_dtype=q.dtype)
-    return (_core._native or _core.native()).run(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state, scale,
-                                                 output_final_state, output_uncertainty, cu_seqlens, False, num_segments,
-                                                 _core.carry_on_tensor_cores)
+    if not _core.takes_general_route(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state, cu_seqlens):
+        out = (_core._native or _core.native()).run(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state, scale,
+                                                    output_final_state, output_uncertainty, cu_seqlens, False, num_segments,
+                                                    _core.carry_on_tensor_cores)
+        if out is not NotImplemented:
+            return out
+    if scale is None:
+        scale = q.shape[-1] ** -0.5
+    if cu_seqlens is not None and q.shape[0] != 1:
+        raise ValueError(f"Batch size must be 1 for Varlen, got {q.shape[0]}")
+    return _core.run_general(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state, scale, output_final_state,
+                             output_uncertainty, cu_seqlens, recurrent=False, out_dtype=q.dtype, num_segments=num_segments,
+                             var_dtype=q.dtype)

@@ -29,13 +29,16 @@ def decode_step(q, k, v, b, gt, g, Ip, mu_state: torch.Tensor, I_state: torch.Te
     Not differentiable (inference only).  The work is done by the registered op
     ``torch.ops.palimpsa_b200.decode_step`` (declared as mutating the two cache tensors), so the call can sit
     inside a ``torch.compile``d decode loop."""
-    if torch.compiler.is_compiling():
-        return _decode_traced(q, k, v, b, gt, g, Ip, mu_state, I_state, scale, output_uncertainty)
-    return (_core._native or _core.native()).decode_step(q, k, v, b, gt, g, Ip, mu_state, I_state, scale, output_uncertainty)
+    if not _core.takes_general_route(q, k, v, b, gt, g, Ip, mu_state, I_state):
+        out = (_core._native or _core.native()).decode_step(q, k, v, b, gt, g, Ip, mu_state, I_state, scale,
+                                                            output_uncertainty)
+        if out is not NotImplemented:
+            return out
+    return _decode_general(q, k, v, b, gt, g, Ip, mu_state, I_state, scale, output_uncertainty)
 
 
-def _decode_traced(q, k, v, b, gt, g, Ip, mu_state, I_state, scale, output_uncertainty):
-    """The call in traceable Python, around the registered operator."""
+def _decode_general(q, k, v, b, gt, g, Ip, mu_state, I_state, scale, output_uncertainty):
+    """The call in Python that can be traced, around the registered operator."""
     _core.ensure_ops_registered()
     if q.dim() == 3:
         q, k, v, b, gt = q.unsqueeze(1), k.unsqueeze(1), v.unsqueeze(1), b.unsqueeze(1), gt.unsqueeze(1)

@@ -113,3 +113,75 @@ def test_registered_operators_check_every_tensor():
     for i in (0, 5, 7):
         _raises_before_launch(D.decode_step_op, dec, i, dec[i].cpu(), (RuntimeError, ValueError))
     _raises_before_launch(D.decode_step_op, dec, 7, dec[7].bfloat16(), TypeError)
+
+
+def _state():
+    return torch.zeros(2, 2, 16, 32, device=DEV), torch.ones(2, 2, 16, 32, device=DEV)
+
+
+@pytest.mark.parametrize("pre_dispatch", [False, True])
+def test_traced_calls_depend_on_their_inputs(pre_dispatch):
+    """Both fx tracers see the operator; a graph with the traced call's result as a constant would pass on one input."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from palimpsa_b200.ops import chunk_palimpsa, decode_step
+    graph = make_fx(lambda *x: chunk_palimpsa(*x), pre_dispatch=pre_dispatch)(*_args(grad=False))
+    other = [x * 0.5 for x in _args(grad=False)]
+    assert torch.equal(graph(*other), chunk_palimpsa(*other))
+    step = make_fx(lambda *x: decode_step(*x), pre_dispatch=pre_dispatch)(*_args(T=1, grad=False), *_state())
+    other = [x * 0.5 for x in _args(T=1, grad=False)]
+    s1, s2 = _state(), _state()
+    assert torch.equal(step(*other, *s1), decode_step(*other, *s2)) and torch.equal(s1[0], s2[0])
+
+
+def test_jit_trace_records_the_operator():
+    from palimpsa_b200.ops import chunk_palimpsa, decode_step
+    f = torch.jit.trace(lambda *x: chunk_palimpsa(*x), tuple(_args(grad=False)), check_trace=False)
+    other = [x * 0.5 for x in _args(grad=False)]
+    assert "palimpsa_b200::fwd" in str(f.graph) and torch.equal(f(*other), chunk_palimpsa(*other))
+    f = torch.jit.trace(lambda *x: decode_step(*x), (*_args(T=1, grad=False), *_state()), check_trace=False)
+    other = [x * 0.5 for x in _args(T=1, grad=False)]
+    assert torch.equal(f(*other, *_state()), decode_step(*other, *_state()))
+
+
+def test_negated_views_are_read_with_their_sign():
+    from palimpsa_b200.ops import DecodeGraph, chunk_palimpsa, decode_step
+    a = _args(grad=False)
+    neg = [torch._neg_view(a[0]), *a[1:]]
+    assert torch.equal(chunk_palimpsa(*neg), chunk_palimpsa(-a[0], *a[1:]))
+    t = _args(T=1, grad=False)
+    assert torch.equal(decode_step(torch._neg_view(t[0]), *t[1:], *_state()), decode_step(-t[0], *t[1:], *_state()))
+    g1, g2 = DecodeGraph(t[5], t[6], *_state(), dtype=torch.float32), DecodeGraph(t[5], t[6], *_state(), dtype=torch.float32)
+    assert torch.equal(g1.step(torch._neg_view(t[0]), *t[1:5]), g2.step(-t[0], *t[1:5]))
+
+
+def test_subclasses_and_function_modes_see_the_operator():
+    from torch.overrides import TorchFunctionMode
+    from palimpsa_b200.ops import chunk_palimpsa, decode_step
+
+    class Sub(torch.Tensor):
+        pass
+
+    a, t = _args(grad=False), _args(T=1, grad=False)
+    assert type(chunk_palimpsa(a[0].as_subclass(Sub), *a[1:])) is Sub
+    assert type(decode_step(t[0].as_subclass(Sub), *t[1:], *_state())) is Sub
+    seen = []
+
+    class Mode(TorchFunctionMode):
+        def __torch_function__(self, f, types, args=(), kwargs=None):
+            seen.append(str(f))
+            return f(*args, **(kwargs or {}))
+
+    with Mode():
+        chunk_palimpsa(*a)
+    assert any("palimpsa_b200" in s or "fwd" in s for s in seen)
+
+
+def test_a_call_below_autograd_makes_no_graph():
+    """Inside another operator's kernel autograd is off by dispatch key although gradients are enabled."""
+    from palimpsa_b200.ops import chunk_palimpsa
+    a = _args()
+    with torch._C._AutoDispatchBelowAutograd():
+        o = chunk_palimpsa(*a)
+    assert not o.requires_grad
+    with torch.inference_mode():
+        assert torch.equal(chunk_palimpsa(*a), o)

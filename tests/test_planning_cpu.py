@@ -80,6 +80,50 @@ def test_layer_prologue_without_heads_is_an_error():
     assert r.returncode == 0 and "ValueError layer_prologue" in r.stdout, (r.returncode, r.stderr[-500:])
 
 
+def _fake(T, decode=False):
+    import torch
+    e = lambda *s, **kw: torch.empty(*s, device="cuda", **kw)
+    a = [e(2, T, 2, 32), e(2, T, 2, 32), e(2, T, 2, 16), e(2, T, 2, 16), e(2, T, 2), e(2), e(2)]
+    return a + [e(2, 2, 16, 32), e(2, 2, 16, 32)] if decode else a
+
+
+def test_fake_tensors_go_through_the_registered_operators():
+    """Shape propagation without a GPU, outside of any compiler: forward (and backward where there is a GPU), and decode."""
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from palimpsa_b200.ops import chunk_palimpsa, decode_step, fused_recurrent_palimpsa
+    with FakeTensorMode():
+        for fn in (chunk_palimpsa, fused_recurrent_palimpsa):
+            a = [x.requires_grad_() for x in _fake(2100)]
+            o, mu, I = fn(*a, output_final_state=True)
+            assert o.shape == (2, 2100, 2, 16) and mu.shape == I.shape == (2, 2, 16, 32) and o.device.type == "cuda"
+            assert o.requires_grad
+            if torch.cuda.is_available():      # torch's own backward needs a device for fake CUDA tensors too
+                o.sum().backward()
+                assert a[0].grad.shape == a[0].shape and a[5].grad.shape == (2,)
+        assert decode_step(*_fake(1, decode=True)).shape == (2, 1, 2, 16)
+
+
+@pytest.mark.parametrize("T", [64, 600, 3000])
+def test_a_symbolic_length_stays_symbolic(T):
+    """The plan is made for the traced length without fixing it."""
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.fx.experimental.symbolic_shapes import DimDynamic, ShapeEnv, StatelessSymbolicContext
+    from palimpsa_b200.ops import chunk_palimpsa
+    env = ShapeEnv()
+    mode = FakeTensorMode(shape_env=env)
+    like = [torch.empty(s, device="meta") for s in ((2, T, 2, 32), (2, T, 2, 16), (2, T, 2), (2,))]
+    free = lambda t: StatelessSymbolicContext([DimDynamic.DYNAMIC if i == 1 else DimDynamic.STATIC for i in range(t.dim())])
+    with mode:
+        q, v, gt, g = [mode.from_tensor(t, symbolic_context=free(t)) for t in like]
+        s = q.shape[1]
+        cuda = lambda *shape: torch.empty(*shape, device="cuda")
+        o = chunk_palimpsa(cuda(2, s, 2, 32), cuda(2, s, 2, 32), cuda(2, s, 2, 16), cuda(2, s, 2, 16), cuda(2, s, 2), cuda(2),
+                           cuda(2))
+        assert isinstance(o.shape[1], torch.SymInt) and str(o.shape[1]) == str(s) and not str(s).isdigit()
+
+
 def test_missing_library_is_a_loud_error(monkeypatch, tmp_path):
     """No CPU or PyTorch fallback: without the built CUDA library every entry fails with a clear message."""
     from palimpsa_b200 import _lib
