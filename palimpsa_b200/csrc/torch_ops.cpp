@@ -79,16 +79,18 @@ void check_arg(const char* name, const Tensor& t, at::ScalarType dt, at::IntArra
 bool plain(std::initializer_list<const Tensor*> ts) {
     using c10::DispatchKey;
     using c10::DispatchKeySet;
-    static const DispatchKeySet usual_state = c10::default_included_set | c10::autocast_dispatch_keyset;
-    static const DispatchKeySet usual_tensor = DispatchKeySet(DispatchKey::CUDA) | DispatchKeySet(DispatchKey::AutogradCUDA) |
-                                               DispatchKeySet(DispatchKey::ADInplaceOrView) | DispatchKeySet(DispatchKey::AutocastCUDA);
+    // bits, not key-set differences: those leave a set's backends standing
+    static const uint64_t usual_state = (c10::default_included_set | c10::autocast_dispatch_keyset).raw_repr();
+    static const uint64_t usual_tensor = (DispatchKeySet(DispatchKey::CUDA) | DispatchKeySet(DispatchKey::AutogradCUDA) |
+                                          DispatchKeySet(DispatchKey::ADInplaceOrView) | DispatchKeySet(DispatchKey::AutocastCUDA))
+                                             .raw_repr();
     if (c10::impl::dispatch_mode_enabled()) return false;
     const c10::impl::LocalDispatchKeySet tls = c10::impl::tls_local_dispatch_key_set();
-    if (!(tls.included_ - usual_state).empty()) return false;
+    if (tls.included_.raw_repr() & ~usual_state) return false;
     // below autograd no node may be made (inference mode is there too, with gradients off: nothing to make)
-    if (at::GradMode::is_enabled() && !(tls.excluded_ & c10::autograd_dispatch_keyset).empty()) return false;
+    if (at::GradMode::is_enabled() && (tls.excluded_.raw_repr() & c10::autograd_dispatch_keyset.raw_repr())) return false;
     for (const Tensor* t : ts)
-        if (t->defined() && !(t->key_set() - usual_tensor).empty()) return false;
+        if (t->defined() && (t->key_set().raw_repr() & ~usual_tensor)) return false;
     return true;
 }
 py::object not_plain() { return py::reinterpret_borrow<py::object>(Py_NotImplemented); }  // the caller takes the general route

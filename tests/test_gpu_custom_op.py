@@ -185,3 +185,39 @@ def test_a_call_below_autograd_makes_no_graph():
     assert not o.requires_grad
     with torch.inference_mode():
         assert torch.equal(chunk_palimpsa(*a), o)
+
+
+def test_ordinary_calls_take_the_direct_route():
+    """Plain tensors go straight to the kernels, with gradients or without, under autocast, in inference mode, with hooks on
+    saved tensors; the native entry hands everything else back."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from palimpsa_b200.ops.palimpsa import _core
+    ext = _core.native()
+
+    def direct(a):
+        run = ext.run(*a, None, None, None, False, False, None, False, None, True) is not NotImplemented
+        t = [x.detach()[:, :1].contiguous() if x.dim() > 1 else x.detach() for x in a]
+        step = ext.decode_step(*t, *_state(), None, False) is not NotImplemented
+        assert run == step
+        return run
+
+    a = _args()
+    assert direct(a) and direct(_args(grad=False)) and direct([torch.nn.Parameter(x) for x in a])
+    with torch.no_grad():
+        assert direct(a)
+    with torch.inference_mode():
+        assert direct(a) and direct([x + 0 for x in a])
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert direct(a)
+    with torch.autograd.graph.save_on_cpu():
+        assert direct(a)
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, f, types, args=(), kwargs=None):
+            return f(*args, **(kwargs or {}))
+
+    with Mode():
+        assert not direct(a)
+    with torch._C._AutoDispatchBelowAutograd():
+        assert not direct(a)
+    assert not direct([torch._neg_view(a[0].detach()), *a[1:]])
+    assert not direct([x.detach().cpu() for x in a])
