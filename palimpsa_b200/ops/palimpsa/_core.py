@@ -8,6 +8,7 @@ There is no fallback: CPU tensors are rejected and a missing library raises.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from typing import Optional
 
 import torch
@@ -148,17 +149,19 @@ def make_segments(N, G, seg_len, H, V, K, dev, fwd: bool, with_rloc=True):
 
 
 _native = None
+_loading = threading.Lock()
 
 
 def native():
-    """The native front end; the first call loads it and registers the operators' fake kernels."""
+    """The native front end; the first call, of whichever thread, loads it and registers the operators' fake kernels."""
     global _native
-    if _native is None:
-        ext = L.torch_ops()
-        torch.library.register_fake("palimpsa_b200::fwd", _fwd_fake)
-        torch.library.register_fake("palimpsa_b200::bwd", _bwd_fake)
-        torch.library.register_fake("palimpsa_b200::decode_step", _decode_fake)
-        _native = ext
+    with _loading:
+        if _native is None:
+            ext = L.torch_ops()
+            torch.library.register_fake("palimpsa_b200::fwd", _fwd_fake)
+            torch.library.register_fake("palimpsa_b200::bwd", _bwd_fake)
+            torch.library.register_fake("palimpsa_b200::decode_step", _decode_fake)
+            _native = ext
     return _native
 
 

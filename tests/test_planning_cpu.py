@@ -80,6 +80,36 @@ def test_layer_prologue_without_heads_is_an_error():
     assert r.returncode == 0 and "ValueError layer_prologue" in r.stdout, (r.returncode, r.stderr[-500:])
 
 
+def _in_fresh_process(prog):
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", prog], capture_output=True, text=True, cwd=root)
+    assert r.returncode == 0, r.stderr[-1500:]
+    return r.stdout
+
+
+def test_threads_may_make_the_first_call_together():
+    out = _in_fresh_process("""
+import sys, threading
+from palimpsa_b200.ops.palimpsa import _core
+sys.setswitchinterval(1e-6)
+gate, errors = threading.Barrier(8), []
+def first():
+    gate.wait()
+    try:
+        _core.native()
+    except Exception as e:
+        errors.append(e)
+threads = [threading.Thread(target=first) for _ in range(8)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+print("errors", errors)
+""")
+    assert "errors []" in out
+
+
 def _fake(T, decode=False):
     import torch
     e = lambda *s, **kw: torch.empty(*s, device="cuda", **kw)
