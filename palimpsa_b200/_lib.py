@@ -150,7 +150,10 @@ def lib():
         raise PalimpsaLibraryError(
             f"{LIB_PATH} is missing. Build it with `python -m palimpsa_b200.build` (needs nvcc). "
             "palimpsa_b200 has no CPU or PyTorch fallback.")
-    h = C.CDLL(LIB_PATH)
+    try:
+        h = C.CDLL(LIB_PATH)
+    except OSError as e:
+        raise PalimpsaLibraryError(f"{LIB_PATH} does not load: {e}") from e
     for name, (res, args) in SYMBOLS.items():
         try:
             fn = getattr(h, name)

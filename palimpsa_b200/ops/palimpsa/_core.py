@@ -153,7 +153,9 @@ _loading = threading.Lock()
 
 
 def native():
-    """The native front end; the first call, of whichever thread, loads it and registers the operators' fake kernels."""
+    """The native front end; the first call, of whichever thread, loads it and registers the operators' fake kernels.
+    Importing this module makes that call where the package is built: a saved program (torch.export, TorchScript) or code
+    that names ``torch.ops.palimpsa_b200`` needs the operators to exist, not a call of this package first."""
     global _native
     with _loading:
         if _native is None:
@@ -267,3 +269,9 @@ def run_general(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state, scale,
     if output_final_state:
         return out, fmu, fI
     return out
+
+
+try:
+    native()
+except L.PalimpsaLibraryError:      # not built, or for another torch: the first call says so
+    pass

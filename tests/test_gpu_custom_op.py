@@ -196,7 +196,7 @@ def test_ordinary_calls_take_the_direct_route():
 
     def direct(a):
         run = ext.run(*a, None, None, None, False, False, None, False, None, True) is not NotImplemented
-        t = [x.detach()[:, :1].contiguous() if x.dim() > 1 else x.detach() for x in a]
+        t = [x.detach()[:, :1] if x.dim() > 1 else x.detach() for x in a]
         step = ext.decode_step(*t, *_state(), None, False) is not NotImplemented
         assert run == step
         return run
@@ -221,3 +221,21 @@ def test_ordinary_calls_take_the_direct_route():
         assert not direct(a)
     assert not direct([torch._neg_view(a[0].detach()), *a[1:]])
     assert not direct([x.detach().cpu() for x in a])
+
+
+def test_an_exported_program_loads_after_a_bare_import(tmp_path):
+    import os
+    import subprocess
+    import sys
+    from palimpsa_b200.ops import chunk_palimpsa
+
+    class Mod(torch.nn.Module):
+        def forward(self, *x):
+            return chunk_palimpsa(*x)
+
+    path = str(tmp_path / "p.pt2")
+    torch.export.save(torch.export.export(Mod(), tuple(_args(grad=False))), path)
+    prog = f"import palimpsa_b200, torch\nprint('loaded', torch.export.load({path!r}).graph)"
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", prog], capture_output=True, text=True, cwd=root)
+    assert r.returncode == 0 and "palimpsa_b200.fwd" in r.stdout, r.stderr[-1500:]

@@ -110,6 +110,32 @@ print("errors", errors)
     assert "errors []" in out
 
 
+def test_importing_the_package_registers_the_operators():
+    """A program saved with an operator call in it has to load in a process that has only imported the package."""
+    out = _in_fresh_process("""
+import palimpsa_b200, torch
+print([str(getattr(torch.ops.palimpsa_b200, n).default._schema).split("(")[0] for n in ("fwd", "bwd", "decode_step")])
+""")
+    assert "palimpsa_b200::fwd" in out and "palimpsa_b200::bwd" in out and "palimpsa_b200::decode_step" in out
+
+
+def test_an_unbuilt_package_imports_and_says_so_at_the_first_call():
+    out = _in_fresh_process("""
+import ctypes, torch
+real = ctypes.CDLL
+def refuse(path, *a, **k):
+    raise OSError(path)
+ctypes.CDLL = refuse
+import palimpsa_b200
+from palimpsa_b200 import _lib
+try:
+    palimpsa_b200.chunk_palimpsa(*[torch.zeros(1, 1, 1, 16)] * 4, torch.zeros(1, 1, 1), torch.ones(1), torch.ones(1))
+except _lib.PalimpsaLibraryError as e:
+    print("loud", e)
+""")
+    assert "loud" in out
+
+
 def _fake(T, decode=False):
     import torch
     e = lambda *s, **kw: torch.empty(*s, device="cuda", **kw)
