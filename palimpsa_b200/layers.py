@@ -38,4 +38,4 @@ def layer_epilogue(o: Tensor, x: Optional[Tensor], D: Optional[Tensor], weight: 
     ``weight [V]``, multiplied by ``gate * sigmoid(gate)`` when ``gate [..., H, V]`` is given (the gated
     norm of flash-linear-attention's ``FusedRMSNormGated``, activation "swish").  float32 arithmetic, result
     in ``o.dtype``."""
-    return (_core._native or _core.native()).layer_epilogue(o, x, D, weight, gate, eps)
+    return (_core._native or _core.native()).layer_epilogue(o, x, D, weight, gate, float(eps))

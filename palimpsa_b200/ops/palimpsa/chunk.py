@@ -27,8 +27,10 @@ def chunk_palimpsa(q, k, v, b, gt, g, Ip, initial_mu_state=None, initial_I_state
     so when there are too few documents to fill one wave of CTAs.
     """
     if not _core.takes_general_route(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state, cu_seqlens):
-        out = (_core._native or _core.native()).run(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state, scale,
-                                                    output_final_state, output_uncertainty, cu_seqlens, False, num_segments,
+        out = (_core._native or _core.native()).run(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state,
+                                                    None if scale is None else float(scale), bool(output_final_state),
+                                                    bool(output_uncertainty), cu_seqlens, False,
+                                                    None if num_segments is None else int(num_segments),
                                                     _core.carry_on_tensor_cores)
         if out is not NotImplemented:
             return out

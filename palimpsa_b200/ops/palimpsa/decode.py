@@ -30,8 +30,9 @@ def decode_step(q, k, v, b, gt, g, Ip, mu_state: torch.Tensor, I_state: torch.Te
     ``torch.ops.palimpsa_b200.decode_step`` (declared as mutating the two cache tensors), so the call can sit
     inside a ``torch.compile``d decode loop."""
     if not _core.takes_general_route(q, k, v, b, gt, g, Ip, mu_state, I_state):
-        out = (_core._native or _core.native()).decode_step(q, k, v, b, gt, g, Ip, mu_state, I_state, scale,
-                                                            output_uncertainty)
+        out = (_core._native or _core.native()).decode_step(q, k, v, b, gt, g, Ip, mu_state, I_state,
+                                                            None if scale is None else float(scale),
+                                                            bool(output_uncertainty))
         if out is not NotImplemented:
             return out
     return _decode_general(q, k, v, b, gt, g, Ip, mu_state, I_state, scale, output_uncertainty)

@@ -18,8 +18,9 @@ def fused_recurrent_palimpsa(q, k, v, b, gt, g, Ip, scale: Optional[float] = Non
     float32, as in the reference (:247-248); with 16-bit inputs the kernel writes ``o_var`` in that dtype first,
     so its float32 values carry that rounding.  Unlike the reference (:250-253) it is differentiable."""
     if not _core.takes_general_route(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state, cu_seqlens):
-        out = (_core._native or _core.native()).run(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state, scale,
-                                                    output_final_state, output_uncertainty, cu_seqlens, True, None,
+        out = (_core._native or _core.native()).run(q, k, v, b, gt, g, Ip, initial_mu_state, initial_I_state,
+                                                    None if scale is None else float(scale), bool(output_final_state),
+                                                    bool(output_uncertainty), cu_seqlens, True, None,
                                                     _core.carry_on_tensor_cores)
         if out is not NotImplemented:
             return out

@@ -160,6 +160,22 @@ def test_fake_tensors_go_through_the_registered_operators():
         assert decode_step(*_fake(1, decode=True)).shape == (2, 1, 2, 16)
 
 
+def test_options_are_taken_by_their_truth_and_value():
+    """Flags of any type, a float as a segment count and numbers of other types as a scale, as from Python code before the
+    native entries: conversions happen in front of them (fake tensors are handed back, so nothing runs here)."""
+    import numpy as np
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from palimpsa_b200.ops import chunk_palimpsa, decode_step, fused_recurrent_palimpsa
+    with FakeTensorMode():
+        a = _fake(64)
+        for fn in (chunk_palimpsa, fused_recurrent_palimpsa):
+            out, mu, I = fn(*a, output_final_state=object(), output_uncertainty=[1], scale=np.float32(0.5))
+            assert len(out) == 2 and mu.shape == I.shape
+        assert chunk_palimpsa(*a, num_segments=4.0, scale="0.5", output_final_state="").shape == (2, 64, 2, 16)
+        assert len(decode_step(*_fake(1, decode=True), scale="0.5", output_uncertainty="yes")) == 2
+
+
 @pytest.mark.parametrize("T", [64, 600, 3000])
 def test_a_symbolic_length_stays_symbolic(T):
     """The plan is made for the traced length without fixing it."""
