@@ -19,6 +19,7 @@ CSRC = os.path.join(PKG, "csrc")
 ROOT = os.path.dirname(PKG)
 LIB = os.path.join(PKG, "libpalimpsa_b200.so")
 EXT = os.path.join(PKG, "_torch_ops" + sysconfig.get_config_var("EXT_SUFFIX"))
+EXT_STAMP = os.path.join(PKG, "_torch_ops.built_for")      # the torch version EXT was compiled and linked against
 EXT_SOURCE = os.path.join(CSRC, "torch_ops.cpp")
 HEADER = os.path.join(ROOT, "include", "palimpsa_b200.h")
 UNITS = ("abi", "fwd", "bwd", "decode", "segments", "summary_tc", "carry_tc", "layer", "peer")
@@ -43,8 +44,21 @@ def _older(target, sources) -> bool:
     return not os.path.exists(target) or any(os.path.getmtime(s) > os.path.getmtime(target) for s in sources)
 
 
+def _torch_version() -> str:
+    from importlib.metadata import version
+    return version("torch")
+
+
+def _ext_is_for_this_torch() -> bool:
+    """The front end uses torch's C++ interface, which other versions do not keep."""
+    if not os.path.exists(EXT_STAMP):
+        return False
+    with open(EXT_STAMP) as f:
+        return f.read().strip() == _torch_version()
+
+
 def needs_build() -> bool:
-    return _older(LIB, _sources()) or _older(EXT, [HEADER, EXT_SOURCE])
+    return _older(LIB, _sources()) or _older(EXT, [HEADER, EXT_SOURCE]) or not _ext_is_for_this_torch()
 
 
 def _run(cmd, what, log=None):
@@ -74,6 +88,8 @@ def _link_ext(obj):
           "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN",
           f"-Wl,-rpath,{os.path.join(os.path.dirname(torch.__file__), 'lib')}"], "link of _torch_ops")
     os.replace(tmp, EXT)
+    with open(EXT_STAMP, "w") as f:
+        f.write(_torch_version() + "\n")
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -94,8 +110,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return obj
 
     ext_obj = os.path.join(objdir, "torch_ops.o")
+    ext_stale = force or _older(ext_obj, [HEADER, EXT_SOURCE]) or not _ext_is_for_this_torch()
     with ThreadPoolExecutor(len(UNITS) + 1) as ex:
-        ext_job = ex.submit(_compile_ext, ext_obj) if force or _older(ext_obj, [HEADER, EXT_SOURCE]) else None
+        ext_job = ex.submit(_compile_ext, ext_obj) if ext_stale else None
         objs = list(ex.map(compile_unit, UNITS))
         if ext_job:
             ext_job.result()

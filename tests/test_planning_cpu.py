@@ -80,6 +80,17 @@ def test_layer_prologue_without_heads_is_an_error():
     assert r.returncode == 0 and "ValueError layer_prologue" in r.stdout, (r.returncode, r.stderr[-500:])
 
 
+def test_another_torch_version_rebuilds_the_front_end(monkeypatch, tmp_path):
+    from palimpsa_b200 import build as b
+    monkeypatch.setattr(b, "_older", lambda target, sources: False)      # by their times the files are up to date
+    monkeypatch.setattr(b, "EXT_STAMP", str(tmp_path / "stamp"))
+    assert b.needs_build()                                               # built for an unknown version
+    (tmp_path / "stamp").write_text(b._torch_version() + "\n")
+    assert not b.needs_build()
+    monkeypatch.setattr(b, "_torch_version", lambda: "0.0.1")
+    assert b.needs_build()
+
+
 def _in_fresh_process(prog):
     import os
     import subprocess
