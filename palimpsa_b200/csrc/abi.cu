@@ -41,7 +41,10 @@ int check_fwd(const palimpsa_fwd_params* prm) {
     return PALIMPSA_OK;
 }
 
-int check_bwd(const palimpsa_bwd_params* prm, bool caller_workspace = true, bool need_outputs = true) {
+// Validates *prm and copies it to *run, with the tiling that its workspace holds: the tile height follows the grid, so a
+// smaller batch may ask for more scratch than a larger one, and a workspace sized for the largest serves them all by way
+// of the tallest tiles.  Every call of one backward gets the same workspace and so the same tiling.
+int check_bwd(const palimpsa_bwd_params* prm, palimpsa_bwd_params* run, bool caller_workspace = true, bool need_outputs = true) {
     if (!prm) return PALIMPSA_E_NULL;
     if (prm->struct_size != sizeof(palimpsa_bwd_params)) return PALIMPSA_E_VERSION;
     int rc = check_problem(prm->p);
@@ -56,9 +59,13 @@ int check_bwd(const palimpsa_bwd_params* prm, bool caller_workspace = true, bool
     if (misaligned16(prm->ckpt_M) || misaligned16(prm->ckpt_I)) return PALIMPSA_E_ALIGN;
     const size_t need = palimpsa_bwd_workspace_bytes(&p);
     if (need == 0) return PALIMPSA_E_DIM;
+    *run = *prm;
     if (!caller_workspace) return PALIMPSA_OK;
-    if (!prm->workspace || prm->workspace_bytes < need) return PALIMPSA_E_WORKSPACE;
-    if (reinterpret_cast<uintptr_t>(prm->workspace) & 255) return PALIMPSA_E_WORKSPACE;
+    if (!prm->workspace || (reinterpret_cast<uintptr_t>(prm->workspace) & 255)) return PALIMPSA_E_WORKSPACE;
+    if (prm->workspace_bytes < need) {
+        run->p.segments = BWD_FEWEST_TILES;
+        if (prm->workspace_bytes < palimpsa_bwd_workspace_bytes(&run->p)) return PALIMPSA_E_WORKSPACE;
+    }
     return PALIMPSA_OK;
 }
 
@@ -209,13 +216,14 @@ int palimpsa_peer_signal(void* flag, unsigned long long value, void* cuda_stream
 int palimpsa_carry_apply_supported(const palimpsa_problem* p) { return p && carry_tc_supported(*p) ? 1 : 0; }
 
 int palimpsa_carry_apply(const palimpsa_bwd_params* prm, const palimpsa_segments* sg, void* cuda_stream) {
-    int rc = check_bwd(prm);
+    palimpsa_bwd_params run;
+    int rc = check_bwd(prm, &run);
     if (rc) return rc;
     rc = check_segments(prm->p, sg);
     if (rc) return rc;
     if (!sg->carry_M || !sg->carry_I) return PALIMPSA_E_NULL;
     if (!carry_tc_supported(prm->p)) return PALIMPSA_E_DTYPE;
-    return launch_carry_tc(prm, *sg, static_cast<cudaStream_t>(cuda_stream));
+    return launch_carry_tc(&run, *sg, static_cast<cudaStream_t>(cuda_stream));
 }
 
 int palimpsa_cp_combine(const palimpsa_problem* p, const palimpsa_segments* sg, const float* in_M, const float* in_J,
@@ -283,7 +291,8 @@ int palimpsa_chunk_bwd_segments(const palimpsa_bwd_params* prm, const palimpsa_s
                                 void* cuda_stream) {
     if (mode < 0 || mode > 3) return PALIMPSA_E_SHAPE;
     const bool carry_only = mode == 1;
-    int rc = check_bwd(prm, !carry_only, !carry_only);
+    palimpsa_bwd_params run;
+    int rc = check_bwd(prm, &run, !carry_only, !carry_only);
     if (rc) return rc;
     rc = check_segments(prm->p, sg);
     if (rc) return rc;
@@ -294,10 +303,10 @@ int palimpsa_chunk_bwd_segments(const palimpsa_bwd_params* prm, const palimpsa_s
     if (mode == 2) {  // main kernel only, zero end-state gradients
         palimpsa_segments z = *sg;
         z.carry_M = z.carry_I = nullptr;
-        return launch_bwd(prm, &z, false, st, 1);
+        return launch_bwd(&run, &z, false, st, 1);
     }
-    if (mode == 3) return launch_bwd(prm, sg, false, st, 2 | 4);  // finishing kernels, extra slot included
-    return launch_bwd(prm, sg, carry_only, st, 3);
+    if (mode == 3) return launch_bwd(&run, sg, false, st, 2 | 4);  // finishing kernels, extra slot included
+    return launch_bwd(&run, sg, carry_only, st, 3);
 }
 
 size_t palimpsa_bwd_workspace_bytes(const palimpsa_problem* p) {
@@ -306,28 +315,32 @@ size_t palimpsa_bwd_workspace_bytes(const palimpsa_problem* p) {
 }
 
 int palimpsa_chunk_bwd(const palimpsa_bwd_params* prm, void* cuda_stream) {
-    int rc = check_bwd(prm);
+    palimpsa_bwd_params run;
+    int rc = check_bwd(prm, &run);
     if (rc) return rc;
-    return launch_bwd(prm, nullptr, false, static_cast<cudaStream_t>(cuda_stream), 3);
+    return launch_bwd(&run, nullptr, false, static_cast<cudaStream_t>(cuda_stream), 3);
 }
 
 int palimpsa_chunk_bwd_stages(const palimpsa_bwd_params* prm, void* cuda_stream, int stages) {
-    int rc = check_bwd(prm);
+    palimpsa_bwd_params run;
+    int rc = check_bwd(prm, &run);
     if (rc) return rc;
     if (stages < 1 || stages > 3) return PALIMPSA_E_SHAPE;
-    return launch_bwd(prm, nullptr, false, static_cast<cudaStream_t>(cuda_stream), stages);
+    return launch_bwd(&run, nullptr, false, static_cast<cudaStream_t>(cuda_stream), stages);
 }
 
 int palimpsa_chunk_bwd_static(const palimpsa_bwd_params* prm, void* cuda_stream) {
-    int rc = check_bwd(prm, false);
+    palimpsa_bwd_params run;
+    int rc = check_bwd(prm, &run, false);
     if (rc) return rc;
-    return launch_bwd_static(prm, static_cast<cudaStream_t>(cuda_stream));
+    return launch_bwd_static(&run, static_cast<cudaStream_t>(cuda_stream));
 }
 
 int palimpsa_recurrent_bwd(const palimpsa_bwd_params* prm, void* cuda_stream) {
-    int rc = check_bwd(prm);
+    palimpsa_bwd_params run;
+    int rc = check_bwd(prm, &run);
     if (rc) return rc;
-    return launch_bwd(prm, nullptr, false, static_cast<cudaStream_t>(cuda_stream), 3);
+    return launch_bwd(&run, nullptr, false, static_cast<cudaStream_t>(cuda_stream), 3);
 }
 
 }  // extern "C"

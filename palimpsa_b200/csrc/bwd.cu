@@ -36,7 +36,6 @@
 namespace palimpsa {
 
 constexpr int GR = 4;  // tokens per register-resident group
-constexpr int BWD_FEWEST_TILES = -1;  // palimpsa_problem::segments, internal: as few row tiles as possible
 
 // 0 ok; 5 / 6: a bounded wait on the split-phase barriers of the backward's group reduction gave up
 __device__ int g_bwd_status = 0;

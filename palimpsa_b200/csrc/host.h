@@ -39,6 +39,9 @@ bool decode_supported(const palimpsa_fwd_params* prm);
 int launch_decode(const palimpsa_fwd_params* prm, cudaStream_t stream);
 int launch_copy_buffers(const void* const* src, void* const* dst, const size_t* bytes, int n, cudaStream_t stream);
 
+// palimpsa_problem::segments, internal: as few row tiles as possible, the least scratch a backward of this size runs with.
+constexpr int BWD_FEWEST_TILES = -1;
+
 // Backward (bwd.cu): main kernel (stages bit 0) + the two finishing kernels (bit 1); bit 2: the finishing
 // kernels also sum the extra partial slot that carry_tc.cu fills.
 int launch_bwd(const palimpsa_bwd_params* prm, const palimpsa_segments* segs, bool carry_only, cudaStream_t stream,

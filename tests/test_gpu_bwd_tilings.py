@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from oracle import palimpsa_oracle as orc
-from tests.gpu_util import compare, run_cuda, run_oracle, tol_for
+from tests.gpu_util import DEV, compare, run_cuda, run_oracle, tol_for
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +65,38 @@ def test_short_sequences_in_segments_match_oracle(B, T, H, K, V, dtype, unc):
     for state in ({}, dict(mu0=mu0, I0=I0)):
         got = run_cuda(inp, "chunk", unc=unc, **state)
         compare(got, run_oracle(inp, unc=unc, **state), tol_for(dtype), what=f"{B}x{H} T={T}")
+
+
+def test_a_workspace_sized_for_more_sequences_serves_fewer():
+    """A grid takes shorter tiles, and with them more scratch, than one of a sequence more: a workspace that was asked for
+    with the larger batch still runs the smaller one (with taller tiles); one too small for any tiling is refused."""
+    from palimpsa_b200 import _lib as L
+    from palimpsa_b200.ops.palimpsa import _core
+    lib, T, K = L.lib(), 40, 128
+
+    def need(N):
+        p = L.Problem()
+        p.num_seqs, p.seq_len, p.total_tokens, p.H, p.K, p.V, p.io_dtype = N, T, N * T, 1, K, K, L.F32
+        return lib.palimpsa_bwd_workspace_bytes(C.byref(p))
+
+    N = next(n for n in range(8, 80) if need(n) > need(n + 1))
+    own, large = need(N), need(N + 1)
+    inp = {n: x.to(DEV) for n, x in orc.make_inputs(7, B=N, T=T, H=1, K=K, V=K).items()}
+    a = [inp[n] for n in ("q", "k", "v", "b", "gt", "g", "Ip")]
+    p = _core._problem(*a, None, None, None, None, K ** -0.5, 0)
+    _, _, _, _, ckM, ckI, _, _ = _core.fwd_op(*a, None, None, None, K ** -0.5, False, True, False, False, 1)
+    got = []
+    for size in (own, large, 1 << 16):
+        out = [torch.full_like(x, float("nan")) for x in a]
+        ws = torch.empty(size, dtype=torch.uint8, device=DEV)
+        prm = L.BwdParams()
+        prm.struct_size, prm.p, prm.d_o = C.sizeof(L.BwdParams), p, inp["do"].data_ptr()
+        prm.ckpt_M, prm.ckpt_I = ckM.data_ptr(), ckI.data_ptr()
+        prm.dq, prm.dk, prm.dv, prm.db, prm.dgt, prm.dg, prm.dIp = [x.data_ptr() for x in out]
+        prm.workspace, prm.workspace_bytes = ws.data_ptr(), size
+        rc = lib.palimpsa_chunk_bwd(C.byref(prm), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == (-5 if size == 1 << 16 else 0)
+        torch.cuda.synchronize()
+        got.append(out)
+    for x, y in zip(got[0], got[1]):
+        assert orc.rel_err(y, x) <= 1e-5           # float32, sums in another order
