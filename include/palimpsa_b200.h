@@ -258,8 +258,8 @@ double palimpsa_bwd_token_cost(const palimpsa_problem *p);
 int palimpsa_copy_buffers(const void *const *src, void *const *dst, const size_t *bytes, int n, void *cuda_stream);
 
 /* Bookkeeping of a packed batch on the device, in one launch: chunk_offsets [n] (first checkpoint slot of every
- * sequence) and order [n] (palimpsa_problem::seq_order: longest sequence first, ties in order; beyond 2048 sequences,
- * where the tail of a launch no longer depends on it, their own order). */
+ * sequence) and order [n] (palimpsa_problem::seq_order: longest sequence first, ties in order; beyond 2048 sequences
+ * by length class, four classes to a power of two, in order inside a class). */
 int palimpsa_varlen_plan(const int32_t *cu_seqlens, int32_t n, int32_t *chunk_offsets, int32_t *order, void *cuda_stream);
 
 

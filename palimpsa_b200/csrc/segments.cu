@@ -175,48 +175,95 @@ int launch_combine_bwd(const palimpsa_problem& p, const palimpsa_segments& segs,
     return cudaGetLastError() == cudaSuccess ? PALIMPSA_OK : PALIMPSA_E_LAUNCH;
 }
 
-// One CTA: exclusive scan of the sequences' block counts, and their rank by decreasing length.  Replaces ~20 small
-// launches of tensor operations (differences, scan, sort, casts) in front of every packed forward and backward.
-constexpr int PLAN_THREADS = 1024, PLAN_SORTED = 2048;
+// One CTA: exclusive scan of the sequences' block counts, and the sequences by decreasing length.  Replaces ~20 small
+// launches of tensor operations (differences, scan, sort, casts) in front of every packed forward and backward.  Up to
+// PLAN_SORTED sequences a thread ranks its own against all of them; beyond, that grows with the square, and a counting
+// sort by length class takes over: four classes per power of two, in order of their index inside a class.
+constexpr int PLAN_THREADS = 1024, PLAN_WARPS = PLAN_THREADS / 32, PLAN_SORTED = 2048, PLAN_CLASSES = 128;
+
+__device__ __forceinline__ int length_class(int l) {  // increasing; a class spans a quarter of a power of two
+    if (l < 4) return l;
+    const int e = 31 - __clz(l);
+    return 4 * e + ((l >> (e - 2)) & 3);  // at most 4 * 30 + 3
+}
+// Exclusive scan of one value per thread over the CTA (part: one slot per warp).
+__device__ __forceinline__ int plan_scan(int x, int* part) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    int incl = x;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += y;
+    }
+    __syncthreads();
+    if (lane == 31) part[tid >> 5] = incl;
+    __syncthreads();
+    int at = incl - x;
+    for (int w = 0; w < (tid >> 5); ++w) at += part[w];
+    return at;
+}
+
 __global__ void __launch_bounds__(PLAN_THREADS) varlen_plan_kernel(const int32_t* __restrict__ cu, int n,
                                                                    int32_t* __restrict__ coff, int32_t* __restrict__ order) {
-    __shared__ int32_t part[PLAN_THREADS / 32];
+    __shared__ int32_t part[PLAN_WARPS];
     __shared__ __align__(16) int32_t lens[PLAN_SORTED];
-    const int tid = threadIdx.x, lane = tid & 31;
+    __shared__ int32_t slot[PLAN_WARPS][PLAN_CLASSES];  // a warp's sequences per class, then where the next of them goes
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int per = (n + PLAN_THREADS - 1) / PLAN_THREADS, lo = min(n, tid * per), hi = min(n, lo + per);
     auto len = [&](int i) { return max(0, cu[i + 1] - cu[i]); };
     int32_t mine = 0;
     for (int i = lo; i < hi; ++i) mine += (len(i) + TB - 1) / TB;
-    int32_t incl = mine;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int32_t x = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += x;
-    }
-    if (lane == 31) part[tid >> 5] = incl;
-    const int padded = (n + 3) / 4 * 4;
-    if (n <= PLAN_SORTED)
-        for (int i = tid; i < padded; i += PLAN_THREADS) lens[i] = i < n ? len(i) : -1;
-    __syncthreads();
-    int32_t at = incl - mine;
-    for (int w = 0; w < (tid >> 5); ++w) at += part[w];
+    int32_t at = plan_scan(mine, part);
     for (int i = lo; i < hi; ++i) {
         coff[i] = at;
         at += (len(i) + TB - 1) / TB;
     }
-    for (int i = tid; i < n; i += PLAN_THREADS) {
-        if (n > PLAN_SORTED) {
-            order[i] = i;
-            continue;
+    if (n <= PLAN_SORTED) {
+        const int padded = (n + 3) / 4 * 4;
+        for (int i = tid; i < padded; i += PLAN_THREADS) lens[i] = i < n ? len(i) : -1;
+        __syncthreads();
+        for (int i = tid; i < n; i += PLAN_THREADS) {
+            const int32_t l = lens[i];
+            int rank = 0;
+            for (int j = 0; j < padded; j += 4) {
+                const int4 x = *reinterpret_cast<const int4*>(lens + j);
+                rank += (x.x > l || (x.x == l && j < i)) + (x.y > l || (x.y == l && j + 1 < i)) +
+                        (x.z > l || (x.z == l && j + 2 < i)) + (x.w > l || (x.w == l && j + 3 < i));
+            }
+            order[rank] = i;
         }
-        const int32_t l = lens[i];
-        int rank = 0;
-        for (int j = 0; j < padded; j += 4) {
-            const int4 x = *reinterpret_cast<const int4*>(lens + j);
-            rank += (x.x > l || (x.x == l && j < i)) + (x.y > l || (x.y == l && j + 1 < i)) +
-                    (x.z > l || (x.z == l && j + 2 < i)) + (x.w > l || (x.w == l && j + 3 < i));
+        return;
+    }
+    // a warp owns the sequences [wlo, whi)
+    const int chunk = (n + PLAN_WARPS - 1) / PLAN_WARPS, wlo = min(n, w * chunk), whi = min(n, wlo + chunk);
+    for (int i = tid; i < PLAN_WARPS * PLAN_CLASSES; i += PLAN_THREADS) (&slot[0][0])[i] = 0;
+    __syncthreads();
+    for (int i = wlo + lane; i < whi; i += 32) atomicAdd(&slot[w][length_class(len(i))], 1);
+    __syncthreads();
+    // counts to places, longest class first, warps in order inside a class: entry 32 c' + warp, four entries per thread
+    static_assert(PLAN_WARPS * PLAN_CLASSES == 4 * PLAN_THREADS && PLAN_WARPS == 32, "four entries of the table per thread");
+    const int cls = PLAN_CLASSES - 1 - tid / 8, w0 = tid % 8 * 4;
+    int32_t cnt[4], sum = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum += cnt[j] = slot[w0 + j][cls];
+    int32_t place = plan_scan(sum, part);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        slot[w0 + j][cls] = place;
+        place += cnt[j];
+    }
+    __syncthreads();
+    for (int base = wlo; base < whi; base += 32) {
+        const int i = base + lane, c = i < whi ? length_class(len(i)) : -1;
+        const unsigned same = __match_any_sync(0xffffffffu, c);
+        const int before = __popc(same & ((1u << lane) - 1));
+        const int first = c >= 0 ? slot[w][c] : 0;
+        __syncwarp();
+        if (c >= 0) {
+            order[first + before] = i;
+            if (before == 0) slot[w][c] = first + __popc(same);
         }
-        order[rank] = i;
+        __syncwarp();
     }
 }
 
