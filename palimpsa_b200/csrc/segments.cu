@@ -29,10 +29,16 @@ __global__ void combine_fwd_kernel(const palimpsa_problem p, const palimpsa_segm
     const long long n = nh / p.H;
     const float ip = p.Ip[h];
     float4 M = make_float4(0.f, 0.f, 0.f, 0.f), J = M;
+    // From an explicit initial precision I0 the start states are D I0 + (1 - D) Ip + S, D the decay so far and S the sums from
+    // a zero start: a small I0 beside a large Ip keeps its digits, as in the walk (J + Ip with J = I0 - Ip rounds it to the
+    // grid of Ip, also where nothing decays).
+    const bool init = !in_M && p.init_mu;
+    float4 I0 = make_float4(ip, ip, ip, ip), S = M;
+    float D = 1.f;
     if (in_M) {
         M = reinterpret_cast<const float4*>(in_M)[i];
         J = reinterpret_cast<const float4*>(in_J)[i];
-    } else if (p.init_mu) {
+    } else if (init) {
         const long long e = row * p.K + 4 * c4;
         float mu[4] = {0.f, 0.f, 0.f, 0.f}, pr[4] = {ip, ip, ip, ip};
         for (int c = 0; c < 4; ++c)
@@ -41,15 +47,21 @@ __global__ void combine_fwd_kernel(const palimpsa_problem p, const palimpsa_segm
                 pr[c] = p.init_I[e + c];
             }
         M = make_float4(mu[0] * pr[0], mu[1] * pr[1], mu[2] * pr[2], mu[3] * pr[3]);
+        I0 = make_float4(pr[0], pr[1], pr[2], pr[3]);
         J = make_float4(pr[0] - ip, pr[1] - ip, pr[2] - ip, pr[3] - ip);
     }
     for (int g = 0; g < G; ++g) {
         const long long e = ((((n * G + g) * p.H + h) * p.V + v) * (long long)KP) / 4 + c4;
         reinterpret_cast<float4*>(sg.start_M)[e] = M;
-        reinterpret_cast<float4*>(sg.start_I)[e] = make_float4(J.x + ip, J.y + ip, J.z + ip, J.w + ip);
+        const float c = (1.f - D) * ip;
+        reinterpret_cast<float4*>(sg.start_I)[e] = init ? f4_axpy(D, I0, make_float4(S.x + c, S.y + c, S.z + c, S.w + c))
+                                                        : make_float4(J.x + ip, J.y + ip, J.z + ip, J.w + ip);
         const float d = sg.decay[(n * G + g) * p.H + h];
+        const float4 s = reinterpret_cast<const float4*>(sg.sum_J)[e];
         M = f4_axpy(d, M, reinterpret_cast<const float4*>(sg.sum_M)[e]);
-        J = f4_axpy(d, J, reinterpret_cast<const float4*>(sg.sum_J)[e]);
+        J = f4_axpy(d, J, s);
+        S = f4_axpy(d, S, s);
+        D *= d;
     }
     if (out_M) {
         reinterpret_cast<float4*>(out_M)[i] = M;

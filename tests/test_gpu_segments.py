@@ -153,3 +153,26 @@ def test_relay_of_a_passing_state_equals_the_full_boundary_scan(dtype):
     loc.relay(sg, inc, tot, out.data_ptr())
     torch.cuda.synchronize()
     assert orc.rel_err(out, full) <= 2e-6
+
+
+@pytest.mark.parametrize("T,dtype", [(512, torch.float32), (512, torch.float16), (2100, torch.float32)])
+def test_small_initial_precision_keeps_its_digits_across_segments(T, dtype):
+    """I0 a millionth of Ip and nothing forgotten: the boundary states have to carry I0 to float32 accuracy although
+    Ip + (I0 - Ip) would round it to 6e-8 of Ip (6 % of I0).  Tolerance: one rounding per token in the walk's sums."""
+    inp = orc.make_inputs(2, B=1, T=T, H=2, K=32, V=16, dtype=dtype)
+    inp["gt"] = torch.zeros_like(inp["gt"])
+    inp["b"] = torch.zeros_like(inp["b"]) if dtype == torch.float16 else inp["b"] * 1e-6
+    inp["v"] = torch.zeros_like(inp["v"]) if dtype == torch.float16 else inp["v"]
+    mu0, I0 = orc.make_states(4, 1, 2, 16, 32, inp["Ip"])
+    I0 = 1e-6 * (1 + torch.rand(I0.shape, generator=torch.Generator().manual_seed(5)))
+    names = ("q", "k", "v", "b", "gt", "g", "Ip")
+    from palimpsa_b200.ops import chunk_palimpsa
+    from palimpsa_b200.ops.palimpsa._core import plan_segments
+    from palimpsa_b200 import _lib as L
+    assert plan_segments(1, T, 2, 32, 16, io_dtype=L.F32 if dtype == torch.float32 else L.F16) > 1
+    o, mu, I = chunk_palimpsa(*[inp[n].to(DEV) for n in names], initial_mu_state=mu0.to(DEV), initial_I_state=I0.to(DEV),
+                              output_final_state=True)
+    ref = run_oracle(inp, mu0=mu0, I0=I0)
+    tol = T * 2 ** -24
+    assert orc.rel_err(I.cpu(), ref["final_I"]) <= tol and orc.rel_err(mu.cpu(), ref["final_mu"]) <= tol
+    assert orc.rel_err(o.cpu(), ref["o"]) <= (tol if dtype == torch.float32 else 1e-3)     # float16 output: 2^-11
