@@ -4,29 +4,25 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
-#include <mutex>
 
 #include "../../include/palimpsa_b200.h"
 
 namespace palimpsa {
 
-// Lets a kernel use `bytes` of dynamic shared memory.  The attribute stays with the kernel on a device, so it is raised
-// once per kernel, device and larger size instead of being set on every launch.
+// Lets a kernel use the `bytes` of dynamic shared memory it is about to be launched with.  The attribute belongs to the
+// kernel in one context (cudaDeviceReset, or another context on the device, starts from the default again), so it is set on
+// every launch; and always to the most a block may have beside the kernel's own static arrays, so that a thread that
+// launches with less does not take it from another that is about to launch with more.
 template <auto Kern>
 bool allow_smem(int bytes) {
-    constexpr int MAX_DEV = 64;
-    static std::atomic<int> granted[MAX_DEV];
-    static std::mutex raising;
-    int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess) return false;
-    if (dev < 0 || dev >= MAX_DEV)
-        return cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
-    if (granted[dev].load(std::memory_order_acquire) >= bytes) return true;
-    std::lock_guard<std::mutex> lock(raising);
-    if (granted[dev].load(std::memory_order_relaxed) >= bytes) return true;
-    if (cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
-    granted[dev].store(bytes, std::memory_order_release);
-    return true;
+    static std::atomic<int> most{0};  // a property of the compiled kernel, the same everywhere
+    int m = most.load(std::memory_order_relaxed);
+    if (!m) {
+        cudaFuncAttributes attr;
+        if (cudaFuncGetAttributes(&attr, Kern) != cudaSuccess) return false;
+        most.store(m = 227 * 1024 - (int)attr.sharedSizeBytes, std::memory_order_relaxed);
+    }
+    return bytes <= m && cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, m) == cudaSuccess;
 }
 
 // Enqueue the forward kernel (fwd.cu).  Parameters are assumed validated.  With `segs` every sequence is

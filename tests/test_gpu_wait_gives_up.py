@@ -64,3 +64,17 @@ def test_peer_wait_runs_out_records_its_code_and_poisons_the_buffer():
     assert flag.item() == 3 and lib.palimpsa_tensor_core_status() == 0 and bool((guarded == 1).all())
     assert lib.palimpsa_peer_wait(None, 1, 5, None, stream) == _lib.E_NULL
     assert lib.palimpsa_peer_signal(flag.data_ptr() + 4, 1, stream) == _lib.E_ALIGN   # flags are 8-byte aligned
+
+
+def test_large_shared_memory_is_granted_again_in_a_new_context():
+    """A kernel's shared-memory limit lives in one context: after cudaDeviceReset the next launch has to raise it again.  In
+    a process of its own, which ends its own context only."""
+    import subprocess
+    import sys
+    if not os.path.exists(wait_probe.LIB):
+        wait_probe.build()
+    prog = ("import ctypes\n"
+            f"f = ctypes.CDLL({wait_probe.LIB!r}).palimpsa_test_smem_grant\n"
+            "print([f(100 * 1024, 0), f(200 * 1024, 0), f(100 * 1024, 1), f(100 * 1024, 0), f(228 * 1024, 0)])\n")
+    r = subprocess.run([sys.executable, "-c", prog], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "[0, 0, 0, 0, -2]", (r.stdout, r.stderr[-500:])

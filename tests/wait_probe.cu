@@ -4,6 +4,7 @@
 // caller, records a status code, frees its TMEM and returns.  With `arrive` = 0 nobody ever arrives at the
 // barrier, so the wait runs out by construction after `limit` polls (nothing hangs and nothing faults); with
 // `arrive` = 1 one thread arrives first and the wait succeeds.
+#include "../palimpsa_b200/csrc/host.h"
 #include "../palimpsa_b200/csrc/tc_common.cuh"
 
 namespace {
@@ -37,4 +38,20 @@ __global__ void __launch_bounds__(32) wait_probe_kernel(int arrive, unsigned lim
 extern "C" int palimpsa_test_wait_probe(int arrive, unsigned limit, int* status_dev, void* cuda_stream) {
     wait_probe_kernel<<<1, 32, 0, static_cast<cudaStream_t>(cuda_stream)>>>(arrive, limit, status_dev);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// A launch with `bytes` of dynamic shared memory by way of the library's allow_smem; with `reset` the process first drops
+// its context on the device (for a process of its own).  0, or the step that failed.
+namespace {
+__global__ void smem_probe_kernel(int bytes) {
+    extern __shared__ unsigned char sm[];
+    for (int i = threadIdx.x; i < bytes; i += blockDim.x) sm[i] = (unsigned char)i;
+}
+}  // namespace
+extern "C" int palimpsa_test_smem_grant(int bytes, int reset) {
+    if (reset && cudaDeviceReset() != cudaSuccess) return -1;
+    if (!palimpsa::allow_smem<smem_probe_kernel>(bytes)) return -2;
+    smem_probe_kernel<<<1, 32, bytes>>>(bytes);
+    if (cudaGetLastError() != cudaSuccess) return -3;
+    return cudaDeviceSynchronize() == cudaSuccess ? 0 : -4;
 }

@@ -10,7 +10,8 @@ LIB = os.path.join(HERE, "libpalimpsa_wait_probe.so")
 
 
 def build(force: bool = False) -> str:
-    deps = [SRC, os.path.join(os.path.dirname(HERE), "palimpsa_b200", "csrc", "tc_common.cuh")]
+    csrc = os.path.join(os.path.dirname(HERE), "palimpsa_b200", "csrc")
+    deps = [SRC, os.path.join(csrc, "tc_common.cuh"), os.path.join(csrc, "host.h")]
     if not force and os.path.exists(LIB) and all(os.path.getmtime(LIB) >= os.path.getmtime(d) for d in deps):
         return LIB
     nvcc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "bin", "nvcc")
