@@ -411,28 +411,29 @@ BwdTuple call_bwd_op(const Tensor& d_o, const OptTensor& d_o_var, const Tensor& 
     return op.call(d_o, d_o_var, q, k, v, b, gt, g, Ip, cu, coff, ckM, ckI, scale, explicit_init, recurrent, decay);
 }
 
-// What the autograd node keeps besides the saved tensors.
-struct NodeState : torch::CustomClassHolder {
-    double scale = 1.0;
-    bool unc = false, recurrent = false, explicit_init = false, has_ckpt = true, carry_tc = true, packed = false, cut = false;
-    at::ScalarType io = at::kFloat;
-};
+// What the autograd node keeps besides the saved tensors, as one number and one set of bits: values that hash, which is
+// what compiled autograd asks of a node's state.
+enum NodeBits : int64_t { NODE_UNC = 1, NODE_RECURRENT = 2, NODE_INIT = 4, NODE_CKPT = 8, NODE_CARRY_TC = 16, NODE_PACKED = 32,
+                          NODE_CUT = 64, NODE_IO_SHIFT = 8 };
 
 // Gradients reaching the final states are ignored and initial states get none, as in the reference
 // (chunk_palimpsa_forgetting_scalar.py:522, :617-620: truncated BPTT across calls).  Gradients of the other outputs are
 // not materialised: autograd would fill a zero tensor for each checkpoint buffer (1.6 GB per step at the benchmark's size).
 variable_list node_backward(AutogradContext* ctx, const variable_list& grads, size_t num_inputs) {
     auto saved = ctx->get_saved_variables();
-    auto st = c10::static_intrusive_pointer_cast<NodeState>(ctx->saved_data["s"].toCapsule());
-    TORCH_CHECK(st->has_ckpt, "palimpsa_b200: backward needs the forward's checkpoints (forward ran with save_ckpt=False)");
-    Inputs x{saved[0], saved[1], saved[2], saved[3], saved[4], saved[5], saved[6], Tensor(), Tensor(), st->packed ? saved[7] : Tensor()};
+    const int64_t bits = ctx->saved_data["bits"].toInt();
+    const auto is = [bits](int64_t bit) { return (bits & bit) != 0; };
+    const at::ScalarType io = static_cast<at::ScalarType>(bits >> NODE_IO_SHIFT);
+    TORCH_CHECK(is(NODE_CKPT), "palimpsa_b200: backward needs the forward's checkpoints (forward ran with save_ckpt=False)");
+    Inputs x{saved[0], saved[1], saved[2], saved[3], saved[4], saved[5], saved[6], Tensor(), Tensor(), is(NODE_PACKED) ? saved[7] : Tensor()};
     BwdIn in;
-    in.d_o = grads[0].defined() ? as(grads[0], st->io) : at::zeros_like(x.v, x.v.options().dtype(st->io));
-    if (st->unc) in.d_o_var = grads[1].defined() ? as(grads[1], st->io) : at::zeros_like(in.d_o);
-    if (st->packed) in.coff = saved[8], in.order = saved[12];
+    in.d_o = grads[0].defined() ? as(grads[0], io) : at::zeros_like(x.v, x.v.options().dtype(io));
+    if (is(NODE_UNC)) in.d_o_var = grads[1].defined() ? as(grads[1], io) : at::zeros_like(in.d_o);
+    if (is(NODE_PACKED)) in.coff = saved[8], in.order = saved[12];
     in.ckM = saved[9], in.ckI = saved[10];
-    if (st->cut) in.decay = saved[11];
-    in.explicit_init = st->explicit_init, in.recurrent = st->recurrent, in.carry_tc = st->carry_tc, in.scale = st->scale;
+    if (is(NODE_CUT)) in.decay = saved[11];
+    in.explicit_init = is(NODE_INIT), in.recurrent = is(NODE_RECURRENT), in.carry_tc = is(NODE_CARRY_TC);
+    in.scale = ctx->saved_data["scale"].toDouble();
     variable_list out(num_inputs);
     // create_graph=True and traced backwards go through the registered operator
     if (at::GradMode::is_enabled() || !plain({&x.q, &x.v, &in.d_o, &in.ckM})) {
@@ -449,11 +450,11 @@ variable_list node_backward(AutogradContext* ctx, const variable_list& grads, si
 void node_save(AutogradContext* ctx, const Inputs& x, const Tensor& coff, const Tensor& order, const Tensor& ckM,
                const Tensor& ckI, const Tensor& decay, const Options& opt) {
     ctx->save_for_backward({x.q, x.k, x.v, x.b, x.gt, x.g, x.Ip, x.cu, coff, ckM, ckI, decay, order});
-    auto st = c10::make_intrusive<NodeState>();
-    st->scale = opt.scale, st->unc = opt.unc, st->recurrent = opt.recurrent, st->explicit_init = x.mu0.defined();
-    st->packed = x.cu.defined(), st->cut = opt.segments > 1;
-    st->has_ckpt = opt.save_ckpt, st->carry_tc = opt.carry_tc, st->io = x.q.scalar_type();
-    ctx->saved_data["s"] = c10::IValue::make_capsule(st);
+    const auto bit = [](bool on, int64_t b) { return on ? b : int64_t(0); };
+    ctx->saved_data["scale"] = opt.scale;
+    ctx->saved_data["bits"] = bit(opt.unc, NODE_UNC) | bit(opt.recurrent, NODE_RECURRENT) | bit(x.mu0.defined(), NODE_INIT) |
+                              bit(opt.save_ckpt, NODE_CKPT) | bit(opt.carry_tc, NODE_CARRY_TC) | bit(x.cu.defined(), NODE_PACKED) |
+                              bit(opt.segments > 1, NODE_CUT) | static_cast<int64_t>(x.q.scalar_type()) << NODE_IO_SHIFT;
     ctx->set_materialize_grads(false);
 }
 
@@ -695,11 +696,13 @@ std::vector<int64_t> with_last(const Tensor& t, int64_t H, int64_t n) {  // [...
     s[s.size() - 2] = H, s[s.size() - 1] = n;
     return s;
 }
-struct Dtypes : torch::CustomClassHolder {  // of the arguments as the caller passed them
-    std::vector<at::ScalarType> t;
-    double eps = 0;
-    bool res = false, gated = false;
-};
+// The dtypes of the arguments as the caller passed them, a byte each (a value that hashes: see the operator's node).
+int64_t pack_dtypes(std::initializer_list<at::ScalarType> ts) {
+    int64_t bits = 0, shift = 0;
+    for (at::ScalarType t : ts) bits |= static_cast<int64_t>(t) << shift, shift += 8;
+    return bits;
+}
+at::ScalarType dtype_at(int64_t bits, size_t i) { return static_cast<at::ScalarType>(bits >> (8 * i) & 0xff); }
 Tensor grad_in(const Tensor& g, at::IntArrayRef sizes, at::ScalarType dt, const at::Device& dev) {
     return g.defined() ? as(g, dt) : at::zeros(sizes, at::TensorOptions().dtype(dt).device(dev));
 }
@@ -722,12 +725,9 @@ struct PrologueFn : torch::autograd::Function<PrologueFn> {
         const at::ScalarType io = x.scalar_type();
         const at::Device dev = x.device();
         c10::cuda::CUDAGuard guard(dev);
-        auto types = c10::make_intrusive<Dtypes>();
         std::vector<Tensor> t;
-        for (const Tensor* a : {&q_raw, &k_raw, &x, &b_raw, &dt_raw, &bs_raw, &dt_bias, &b_scale}) {
-            types->t.push_back(a->scalar_type());
+        for (const Tensor* a : {&q_raw, &k_raw, &x, &b_raw, &dt_raw, &bs_raw, &dt_bias, &b_scale})
             t.push_back(as(*a, t.size() < 6 ? io : at::kFloat));
-        }
         const int64_t H = x.size(-2), K = q_raw.size(-1);
         const auto qs = with_last(x, H, K);
         Tensor q = empty(qs, io, dev), k = empty(qs, io, dev), v = empty(x.sizes(), io, dev), b = empty(x.sizes(), io, dev);
@@ -737,13 +737,15 @@ struct PrologueFn : torch::autograd::Function<PrologueFn> {
         if (a.tokens > 0)  // an empty batch has nothing to launch (and no pointers)
             check_rc(palimpsa_layer_prologue_fwd(&a, stream_of(x)), "layer prologue");
         ctx->save_for_backward(t);
-        ctx->saved_data["d"] = c10::IValue::make_capsule(types);
+        ctx->saved_data["dtypes"] = pack_dtypes({q_raw.scalar_type(), k_raw.scalar_type(), io, b_raw.scalar_type(),
+                                                 dt_raw.scalar_type(), bs_raw.scalar_type(), dt_bias.scalar_type(),
+                                                 b_scale.scalar_type()});
         ctx->set_materialize_grads(false);
         return {q, k, v, b, gt};
     }
     static variable_list backward(AutogradContext* ctx, variable_list g) {
         auto t = ctx->get_saved_variables();
-        auto types = c10::static_intrusive_pointer_cast<Dtypes>(ctx->saved_data["d"].toCapsule());
+        const int64_t types = ctx->saved_data["dtypes"].toInt();
         const Tensor& x = t[2];
         const at::ScalarType io = x.scalar_type();
         const at::Device dev = x.device();
@@ -766,7 +768,7 @@ struct PrologueFn : torch::autograd::Function<PrologueFn> {
         else
             out[6].zero_(), out[7].zero_();
         for (size_t i = 0; i < out.size(); ++i)
-            if (out[i].scalar_type() != types->t[i]) out[i] = out[i].to(types->t[i]);
+            if (out[i].scalar_type() != dtype_at(types, i)) out[i] = out[i].to(dtype_at(types, i));
         for (int i : {6, 7})
             if (out[i].sizes() != t[i].sizes()) out[i] = out[i].view(t[i].sizes());
         return out;
@@ -786,13 +788,13 @@ variable_list layer_prologue(const Tensor& q_raw, const Tensor& k_raw, const Ten
     return PrologueFn::apply(q_raw, k_raw, x, b_raw, dt_raw, bs_raw, dt_bias, b_scale);
 }
 
-palimpsa_layer_epilogue epilogue_params(const std::vector<Tensor>& t, const Dtypes& d) {  // o, x, D, weight, gate
+palimpsa_layer_epilogue epilogue_params(const std::vector<Tensor>& t, double eps, bool res, bool gated) {  // o, x, D, weight, gate
     palimpsa_layer_epilogue a{};
     a.struct_size = sizeof(a);
     a.io_dtype = io_code(t[0].scalar_type());
     a.H = (int)t[0].size(-2), a.V = (int)t[0].size(-1);
-    a.flags = (d.res ? PALIMPSA_LAYER_RESIDUAL : 0) | (d.gated ? PALIMPSA_LAYER_GATE : 0);
-    a.eps = (float)d.eps;
+    a.flags = (res ? PALIMPSA_LAYER_RESIDUAL : 0) | (gated ? PALIMPSA_LAYER_GATE : 0);
+    a.eps = (float)eps;
     a.tokens = token_count(t[0]);
     a.o = ptr(t[0]), a.x = ptr(t[1]), a.D = ptr<float>(t[2]), a.weight = ptr<float>(t[3]), a.gate = ptr(t[4]);
     return a;
@@ -802,22 +804,22 @@ struct EpilogueFn : torch::autograd::Function<EpilogueFn> {
                                  const Tensor& weight, const OptTensor& gate, double eps) {
         const at::ScalarType io = o.scalar_type();
         c10::cuda::CUDAGuard guard(o.device());
-        auto d = c10::make_intrusive<Dtypes>();
-        d->eps = eps, d->res = given(x), d->gated = given(gate);
-        d->t = {io, given(x) ? x->scalar_type() : io, given(D) ? D->scalar_type() : at::kFloat, weight.scalar_type(),
-                given(gate) ? gate->scalar_type() : io};
         std::vector<Tensor> t{as(o, io), as_opt(x, io), as_opt(D, at::kFloat), as(weight, at::kFloat), as_opt(gate, io)};
         Tensor y = empty(o.sizes(), io, o.device());
-        palimpsa_layer_epilogue a = epilogue_params(t, *d);
+        palimpsa_layer_epilogue a = epilogue_params(t, eps, given(x), given(gate));
         a.y = ptr(y);
         if (a.tokens > 0) check_rc(palimpsa_layer_epilogue_fwd(&a, stream_of(o)), "layer epilogue");
         ctx->save_for_backward(t);
-        ctx->saved_data["d"] = c10::IValue::make_capsule(d);
+        ctx->saved_data["dtypes"] = pack_dtypes({io, given(x) ? x->scalar_type() : io, given(D) ? D->scalar_type() : at::kFloat,
+                                                 weight.scalar_type(), given(gate) ? gate->scalar_type() : io});
+        ctx->saved_data["eps"] = eps;
+        ctx->saved_data["parts"] = static_cast<int64_t>((given(x) ? 1 : 0) | (given(gate) ? 2 : 0));
         return {y};
     }
     static variable_list backward(AutogradContext* ctx, variable_list g) {
         auto t = ctx->get_saved_variables();
-        auto d = c10::static_intrusive_pointer_cast<Dtypes>(ctx->saved_data["d"].toCapsule());
+        const int64_t types = ctx->saved_data["dtypes"].toInt(), parts = ctx->saved_data["parts"].toInt();
+        const bool res = (parts & 1) != 0, gated = (parts & 2) != 0;
         const Tensor& o = t[0];
         const at::ScalarType io = o.scalar_type();
         const at::Device dev = o.device();
@@ -825,9 +827,9 @@ struct EpilogueFn : torch::autograd::Function<EpilogueFn> {
         const int64_t H = o.size(-2), V = o.size(-1);
         const Tensor dy = grad_in(g[0], o.sizes(), io, dev);
         Tensor d_o = empty(o.sizes(), io, dev), dx, dD, dw = empty({V}, at::kFloat, dev), dgate;
-        if (d->res) dx = empty(o.sizes(), io, dev), dD = empty({H}, at::kFloat, dev);
-        if (d->gated) dgate = empty(o.sizes(), io, dev);
-        palimpsa_layer_epilogue a = epilogue_params(t, *d);
+        if (res) dx = empty(o.sizes(), io, dev), dD = empty({H}, at::kFloat, dev);
+        if (gated) dgate = empty(o.sizes(), io, dev);
+        palimpsa_layer_epilogue a = epilogue_params(t, ctx->saved_data["eps"].toDouble(), res, gated);
         a.dy = ptr(dy), a.d_o = ptr(d_o), a.dx = ptr(dx), a.dgate = ptr(dgate), a.dD = ptr<float>(dD), a.dweight = ptr<float>(dw);
         Tensor ws = layer_workspace(a.tokens, H, V, dev);
         a.workspace = ptr(ws), a.workspace_bytes = (size_t)ws.numel();
@@ -839,7 +841,7 @@ struct EpilogueFn : torch::autograd::Function<EpilogueFn> {
         }
         variable_list out{d_o, dx, dD, dw, dgate, Tensor()};
         for (size_t i = 0; i < 5; ++i)
-            if (out[i].defined() && out[i].scalar_type() != d->t[i]) out[i] = out[i].to(d->t[i]);
+            if (out[i].defined() && out[i].scalar_type() != dtype_at(types, i)) out[i] = out[i].to(dtype_at(types, i));
         for (int i : {2, 3})
             if (out[i].defined() && out[i].sizes() != t[i].sizes()) out[i] = out[i].view(t[i].sizes());
         return out;

@@ -239,3 +239,26 @@ def test_an_exported_program_loads_after_a_bare_import(tmp_path):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", prog], capture_output=True, text=True, cwd=root)
     assert r.returncode == 0 and "palimpsa_b200.fwd" in r.stdout, r.stderr[-1500:]
+
+
+def test_compiled_autograd_takes_the_nodes():
+    """Compiled autograd hashes a node's state; the operator's and the layer passes' hold plain numbers."""
+    import torch._dynamo.compiled_autograd as ca
+    from palimpsa_b200.layers import layer_epilogue, layer_prologue
+    from palimpsa_b200.ops import chunk_palimpsa
+
+    def step():
+        gen = torch.Generator(DEV).manual_seed(3)
+        r = lambda *s: torch.randn(*s, generator=gen, device=DEV).requires_grad_()
+        a = [r(2, 9, 2, 32), r(2, 9, 2, 32), r(2, 9, 4, 16), r(2, 9, 4, 16), r(2, 9, 4), r(2, 9, 4), r(4), r(4)]
+        w, D, g, Ip = r(16), r(4), torch.ones(4, device=DEV, requires_grad=True), torch.ones(4, device=DEV, requires_grad=True)
+        q, k, v, b, dt = layer_prologue(*a)
+        y = layer_epilogue(chunk_palimpsa(q, k, v, b, dt, g, Ip), a[2], D, w, a[3], eps=1e-4)
+        return (y ** 2).sum(), [*a, w, D, g, Ip]
+
+    loss, ref = step()
+    loss.backward()
+    loss, got = step()
+    with ca._enable(torch.compile(backend="eager")):
+        loss.backward()
+    assert all(torch.equal(x.grad, y.grad) for x, y in zip(ref, got))
