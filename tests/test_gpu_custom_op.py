@@ -262,3 +262,13 @@ def test_compiled_autograd_takes_the_nodes():
     with ca._enable(torch.compile(backend="eager")):
         loss.backward()
     assert all(torch.equal(x.grad, y.grad) for x, y in zip(ref, got))
+
+
+def test_a_profile_names_the_operators():
+    from palimpsa_b200.ops import chunk_palimpsa, decode_step
+    a = _args()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        chunk_palimpsa(*a).sum().backward()
+        decode_step(*_args(T=1, grad=False), *_state())
+    names = {e.key for e in prof.key_averages()}
+    assert {"palimpsa_b200::fwd", "palimpsa_b200::bwd", "palimpsa_b200::decode_step"} <= names
