@@ -375,6 +375,14 @@ FwdTuple fwd_cuda(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
             f(r.ckI, at::kFloat), r.coff.defined() ? r.coff.clone() : none_like(q, at::kInt), f(r.decay, at::kFloat)};
 }
 
+// palimpsa_b200.ops.palimpsa._core.carry_on_tensor_cores, for calls that come in as a registered operator (the Python
+// functions hand it over).  Those come without the interpreter lock.
+bool carry_switch() {
+    if (!Py_IsInitialized()) return true;
+    py::gil_scoped_acquire gil;
+    return py::module_::import("palimpsa_b200.ops.palimpsa._core").attr("carry_on_tensor_cores").cast<bool>();
+}
+
 BwdTuple bwd_cuda(const Tensor& d_o, const OptTensor& d_o_var, const Tensor& q, const Tensor& k, const Tensor& v,
                   const Tensor& b, const Tensor& gt, const Tensor& g, const Tensor& Ip, const OptTensor& cu_seqlens,
                   const OptTensor& chunk_offsets, const Tensor& ckpt_M, const Tensor& ckpt_I, double scale,
@@ -385,6 +393,7 @@ BwdTuple bwd_cuda(const Tensor& d_o, const OptTensor& d_o_var, const Tensor& q, 
     in.coff = dense(chunk_offsets);
     in.ckM = dense(ckpt_M), in.ckI = dense(ckpt_I), in.decay = dense(seg_decay);
     in.explicit_init = explicit_init, in.recurrent = recurrent, in.scale = scale;
+    if (in.decay.defined() && in.decay.numel() > 0) in.carry_tc = carry_switch();
     if (x.cu.defined()) {
         check_inputs(x);
         const int64_t N = x.cu.numel() - 1;
@@ -495,6 +504,7 @@ FwdTuple fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, const T
     Options opt;
     opt.scale = scale, opt.unc = uncertainty, opt.save_ckpt = save_ckpt, opt.want_final = want_final;
     opt.recurrent = recurrent, opt.segments = num_segments;
+    if (num_segments > 1) opt.carry_tc = carry_switch();
     Inputs rest;
     rest.mu0 = init_mu.value_or(Tensor()), rest.I0 = init_I.value_or(Tensor()), rest.cu = cu_seqlens.value_or(Tensor());
     auto r = OpFn::apply(q, k, v, b, gt, g, Ip, rest, opt);

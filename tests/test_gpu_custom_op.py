@@ -272,3 +272,26 @@ def test_a_profile_names_the_operators():
         decode_step(*_args(T=1, grad=False), *_state())
     names = {e.key for e in prof.key_averages()}
     assert {"palimpsa_b200::fwd", "palimpsa_b200::bwd", "palimpsa_b200::decode_step"} <= names
+
+
+def test_the_carry_switch_holds_on_the_operator_route(monkeypatch):
+    """carry_on_tensor_cores = False: the exact carried terms, whichever way the call reaches the kernels."""
+    from palimpsa_b200.ops import chunk_palimpsa
+    from palimpsa_b200.ops.palimpsa import _core
+    inp = orc.make_inputs(17, B=1, T=300, H=2, K=64, V=128, dtype=torch.bfloat16)
+    inp["gt"] = inp["gt"] * 0.05
+
+    def grads(call):
+        a = [inp[n].to(DEV).requires_grad_() for n in ("q", "k", "v", "b", "gt", "g", "Ip")]
+        return torch.autograd.grad(call(a), a, inp["do"].to(DEV))
+
+    direct = lambda a: chunk_palimpsa(*a, num_segments=3)
+    op = lambda a: _core.fwd_op(*a, None, None, None, 64 ** -0.5, False, True, False, False, 3)[0]
+    rounded = grads(direct)
+    assert all(torch.equal(x, y) for x, y in zip(rounded, grads(op)))
+    monkeypatch.setattr(_core, "carry_on_tensor_cores", False)
+    exact = grads(direct)
+    assert not torch.equal(exact[4], rounded[4])
+    assert all(torch.equal(x, y) for x, y in zip(exact, grads(op)))
+    traced = grads(lambda a: torch.compile(direct, backend="aot_eager")(a))
+    assert all(torch.equal(x, y) for x, y in zip(exact, traced))
