@@ -324,6 +324,13 @@ BwdOut bwd_impl(const Inputs& x, const BwdIn& in) {
     prm.p = make_problem(x.q, x.k, x.v, x.b, x.gt, x.g, x.Ip, x.cu, in.coff, in.order, Tensor(), Tensor(), in.scale,
                          (unc ? PALIMPSA_FLAG_UNCERTAINTY : 0) | (in.explicit_init ? PALIMPSA_FLAG_EXPLICIT_INIT : 0));
     if (in.decay.defined() && in.decay.numel() > 0) prm.p.segments = (int)in.decay.size(1);
+    Tensor plan;  // the order to start the documents in, where the forward's was not kept (the operators have no output for it)
+    if (x.cu.defined() && !in.order.defined() && seqs > 0) {
+        plan = empty({2 * seqs}, at::kInt, dev);
+        check_rc(palimpsa_varlen_plan(ptr<int32_t>(x.cu), (int)seqs, ptr<int32_t>(plan), ptr<int32_t>(plan) + seqs, st),
+                 "palimpsa packed-batch plan");
+        prm.p.seq_order = ptr<int32_t>(plan) + seqs;
+    }
     prm.d_o = ptr(in.d_o), prm.d_o_var = ptr(in.d_o_var);
     prm.ckpt_M = ptr<float>(in.ckM), prm.ckpt_I = ptr<float>(in.ckI);
     prm.dq = ptr(r.dq), prm.dk = ptr(r.dk), prm.dv = ptr(r.dv), prm.db = ptr(r.db);
@@ -394,15 +401,6 @@ BwdTuple bwd_cuda(const Tensor& d_o, const OptTensor& d_o_var, const Tensor& q, 
     in.ckM = dense(ckpt_M), in.ckI = dense(ckpt_I), in.decay = dense(seg_decay);
     in.explicit_init = explicit_init, in.recurrent = recurrent, in.scale = scale;
     if (in.decay.defined() && in.decay.numel() > 0) in.carry_tc = carry_switch();
-    if (x.cu.defined()) {
-        check_inputs(x);
-        const int64_t N = x.cu.numel() - 1;
-        c10::cuda::CUDAGuard guard(q.device());
-        Tensor plan = empty({2 * N}, at::kInt, q.device());
-        check_rc(palimpsa_varlen_plan(ptr<int32_t>(x.cu), (int)N, ptr<int32_t>(plan), ptr<int32_t>(plan) + N, stream_of(q)),
-                 "palimpsa packed-batch plan");
-        in.order = plan.narrow(0, N, N);
-    }
     BwdOut r = bwd_impl(x, in);
     return {r.dq, r.dk, r.dv, r.db, r.dgt, r.dg, r.dIp};
 }
