@@ -3,7 +3,7 @@
 
 #include <cuda_runtime.h>
 
-#include <atomic>
+#include <mutex>
 
 #include "../../include/palimpsa_b200.h"
 
@@ -11,18 +11,17 @@ namespace palimpsa {
 
 // Lets a kernel use the `bytes` of dynamic shared memory it is about to be launched with.  The attribute belongs to the
 // kernel in one context (cudaDeviceReset, or another context on the device, starts from the default again), so it is set on
-// every launch; and always to the most a block may have beside the kernel's own static arrays, so that a thread that
-// launches with less does not take it from another that is about to launch with more.
+// every launch; and never lower than before, so that a thread that launches with less does not take it from another that is
+// about to launch with more.  (Not simply to the maximum: the attribute also moves the split between shared memory and L1.)
 template <auto Kern>
 bool allow_smem(int bytes) {
-    static std::atomic<int> most{0};  // a property of the compiled kernel, the same everywhere
-    int m = most.load(std::memory_order_relaxed);
-    if (!m) {
-        cudaFuncAttributes attr;
-        if (cudaFuncGetAttributes(&attr, Kern) != cudaSuccess) return false;
-        most.store(m = 227 * 1024 - (int)attr.sharedSizeBytes, std::memory_order_relaxed);
-    }
-    return bytes <= m && cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, m) == cudaSuccess;
+    static std::mutex setting;
+    static int most = 0;
+    std::lock_guard<std::mutex> lock(setting);
+    const int limit = bytes > most ? bytes : most;
+    if (cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) return false;
+    most = limit;
+    return true;
 }
 
 // Enqueue the forward kernel (fwd.cu).  Parameters are assumed validated.  With `segs` every sequence is

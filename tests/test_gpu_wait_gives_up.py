@@ -75,6 +75,6 @@ def test_large_shared_memory_is_granted_again_in_a_new_context():
         wait_probe.build()
     prog = ("import ctypes\n"
             f"f = ctypes.CDLL({wait_probe.LIB!r}).palimpsa_test_smem_grant\n"
-            "print([f(100 * 1024, 0), f(200 * 1024, 0), f(100 * 1024, 1), f(100 * 1024, 0), f(228 * 1024, 0)])\n")
+            "print([f(100 * 1024, 0), f(200 * 1024, 0), f(100 * 1024, 1), f(100 * 1024, 0), f(228 * 1024, 0), f(8192, 0)])\n")
     r = subprocess.run([sys.executable, "-c", prog], capture_output=True, text=True, timeout=120)
-    assert r.returncode == 0 and r.stdout.strip() == "[0, 0, 0, 0, -2]", (r.stdout, r.stderr[-500:])
+    assert r.returncode == 0 and r.stdout.strip() == "[0, 0, 0, 0, -2, 0]", (r.stdout, r.stderr[-500:])
