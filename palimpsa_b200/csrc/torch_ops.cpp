@@ -115,6 +115,25 @@ int64_t segment_len(int64_t T, int64_t G) {
     return std::max<int64_t>(CI, (per + CI - 1) / CI * CI);
 }
 
+// Does cutting this problem round what crosses a boundary to bfloat16?  The summary and the carried-gradient kernels on the
+// tensor cores do (their shapes: bf16, d_v <= 128, d_k and d_v multiples of 8, padded d_k 32 to 128; the summary from 8192
+// state elements per head, the carried terms without the uncertainty output); all other passes are exact float32.
+bool boundaries_rounded(int64_t K, int64_t V, int io, bool unc) {
+    const int64_t KP = palimpsa_padded_k((int)K);
+    return io == PALIMPSA_BF16 && V <= 128 && V % 8 == 0 && K % 8 == 0 && KP >= 32 && KP <= 128 && (!unc || KP * V >= 8192);
+}
+// CTAs per sequence-head at fixed tile heights: 8 warps (4 where d_v is short), 6 at d_k = 48 and 11 or 12 at d_k = 128 by
+// which pads d_v less.  Only what is starved of CTAs at these is ever rounded: which calls keep float32 boundaries must not
+// change whenever the tile heights are tuned.
+int64_t nominal_tiles(int64_t K, int64_t V) {
+    const int64_t KP = palimpsa_padded_k((int)K), per_warp = KP <= 48 ? 8 : KP <= 96 ? 4 : 2;
+    const auto up = [V](int64_t rows) { return (V + rows - 1) / rows * rows; };
+    int64_t warps = V > 4 * per_warp ? 8 : 4;
+    if (KP == 128 && V >= 48) warps = up(22) < up(24) ? 11 : 12;
+    if (KP == 48 && warps == 8 && up(48) < up(64)) warps = 6;
+    return up(warps * per_warp) / (warps * per_warp);
+}
+
 // How many segments to cut every sequence into on one GPU (plan_segments in _core.py documents the rule).
 int64_t plan_segments(int64_t N, int64_t T, int64_t H, int64_t K, int64_t V, int64_t sms, bool backward, int io, bool unc,
                       bool packed) {
@@ -126,9 +145,12 @@ int64_t plan_segments(int64_t N, int64_t T, int64_t H, int64_t K, int64_t V, int
         const int64_t brow = palimpsa_bwd_tile_rows((int)K, (int)V, io, unc ? 1 : 0);
         TORCH_CHECK_VALUE(brow > 0, "no backward tiling for d_k = ", K, ", d_v = ", V);
         const int64_t ctas = N * H * ((V + brow - 1) / brow);
+        const bool rounded = boundaries_rounded(K, V, io, unc);
+        const int64_t nominal = N * H * nominal_tiles(K, V);
         if (packed) {
-            if (ctas >= sms) return 1;
+            if (ctas >= sms || (rounded && nominal >= sms)) return 1;
         } else {
+            if (!shorter && rounded && 10 * nominal >= 8 * ((nominal + sms - 1) / sms) * sms) return 1;
             palimpsa_problem p{};
             p.num_seqs = (int)N, p.H = (int)H, p.K = (int)K, p.V = (int)V, p.io_dtype = io;
             p.flags = unc ? PALIMPSA_FLAG_UNCERTAINTY : 0;

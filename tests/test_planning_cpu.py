@@ -29,6 +29,16 @@ def test_plan_segments():
         assert L % 16 == 0 and L * G >= T and L >= 16
 
 
+def test_bf16_boundaries_are_rounded_only_where_the_grid_is_starved():
+    """bf16 shapes whose carried terms or summaries go through the tensor cores (rounded there) stay uncut where the grid of
+    the nominal tiles fills 80 % of its waves, however the tile heights are tuned."""
+    from palimpsa_b200.ops.palimpsa._core import plan_segments
+    kw = dict(backward=True)
+    for N, K, V in ((30, 64, 128), (60, 64, 128), (40, 96, 96), (40, 80, 96), (128, 48, 48), (24, 128, 128)):
+        assert plan_segments(N, 4096, 1, K, V, **kw) == 1, (N, K, V)
+    assert all(plan_segments(n, 4096, 1, 64, 128, packed=True, **kw) == 1 for n in range(37, 50))
+
+
 def test_ramped_widths():
     from palimpsa_b200.host_pipeline import ramped_widths
     assert ramped_widths(8) == [1, 2, 2, 2, 1]
