@@ -77,7 +77,8 @@ typedef struct palimpsa_problem {
     float scale;           /* multiplies q (default of the Python wrappers: K^-0.5)            */
     int32_t segments;      /* G of a backward that runs in G segments, else 0 or 1: the backward's tile height depends on
                               how many CTAs there will be.  The same in every call of one backward, the query of its
-                              workspace among them.                                            */
+                              workspace among them; so are num_seqs, seq_len and cu_seqlens.  (A workspace smaller than
+                              the choice asks for, e.g. one sized for another batch, is run with taller tiles.)  */
     const void *q, *k, *v, *b;
     const float *gt, *g, *Ip;
     const int32_t *cu_seqlens;    /* [N+1] device, or NULL                                      */
@@ -242,13 +243,13 @@ int palimpsa_fwd_tile_rows(int K, int V);
 
 /* The same for the backward kernel, whose tile also depends on the element type (PALIMPSA_F32 / _BF16 / _F16) and on
  * whether the uncertainty output takes part (shared-memory budget): a backward launch has ceil(V / rows) x num_seqs x
- * H CTAs of up to 12 warps, usually one resident per SM, so hosts that plan a training step count waves with it.
+ * H CTAs of up to 16 warps, usually one resident per SM, so hosts that plan a training step count waves with it.
  * 0 if the shape is not supported.  No counterpart in the reference (grid (V/16) x N x H,
  * chunk_palimpsa_forgetting_scalar.py:558). */
 int palimpsa_bwd_tile_rows(int K, int V, int io_dtype, int uncertainty);
 
-/* Estimated time of the backward per token, in units of one warp's token (about 45 ns), from num_seqs, H, K, V,
- * io_dtype, flags and segments: what planners weigh an uncut backward against one in segments with.  The backward
+/* Estimated time of the backward per token of a sequence, in units of about 45 ns (a wave of CTAs of 4 warps takes 8),
+ * from num_seqs, seq_len, H, K, V, io_dtype, flags, segments and whether there are cu_seqlens: what planners weigh an uncut backward against one in segments with.  The backward
  * takes the tile height that this is smallest for; palimpsa_bwd_tile_rows() is the one of a grid of many waves.
  * 0 if the shape is not supported. */
 double palimpsa_bwd_token_cost(const palimpsa_problem *p);

@@ -23,10 +23,11 @@
 // waits taken off the compute warps count, and one scheduler had a warp less than the others (11 warps).  With every
 // warp summing and storing its share behind a split barrier: 7.42 ms a training step at B=8 T=4096 H=6 d=128, now
 // 6.79; 3.99 / 3.51 ms at H=16 d=48.
-// One CTA per SM: up to 11 warps at d_k = 128 (22-row tiles); bwd_config has the choice and its measurements.
+// One CTA per SM: up to 12 compute warps at d_k = 128 (24-row tiles); bwd_config has the choice and its measurements.
 //
 // Finishing kernels: (1) per (token, head) row: sum the row tiles, cast dq/dk, form
 // dgt = -g f df and the per-row terms of dg and dIp; (2) per head: ordered sum over rows.
+#include <atomic>
 #include <cmath>
 #include <mutex>
 
@@ -313,9 +314,23 @@ __device__ __forceinline__ void bwd_convert(const BwdArgs& a, int nthr, unsigned
 }
 
 // Threads of a CTA: W compute warps and, except in the carry-only pass, the helper warps: as many as fit beside the
-// compute warps without costing those registers (8 warps of an SM may have 255 per thread, 12 may have 168).
-__host__ __device__ constexpr int bwd_helpers(int W) { return W < 8 ? 8 - W : 12 - W; }
+// compute warps without costing those registers (8 warps of an SM may have 255 per thread, 12 may have 168, 16 128).
+__host__ __device__ constexpr int bwd_helpers(int W) { return W < 8 ? 8 - W : W < 12 ? 12 - W : 4; }
 __host__ __device__ constexpr int bwd_threads(int W, bool CO) { return 32 * (W + (CO ? 0 : bwd_helpers(W))); }
+
+// Where an even share is too little for the walk (8 warps of 12 state elements spill 200 bytes at 168 registers, 12 warps
+// of 8 the same at 128), the warpgroup of helpers gives up registers that the compute warpgroups take: {entry, compute,
+// helper} registers per thread, {0, 0, 0} = no split.  The compute warps wait for the helpers' registers, so the block must
+// have been launched with enough for all: bwd_split_fits asks the compiled kernel before the first launch.  No spills;
+// training step, ms, T = 2048 bf16 / 1024 fp32, by 8 warps of every warp summing -> 7 warps -> 8 split: 32 heads of 96x192
+// unc x2 6.82 / 7.06 / 6.39, 60 of 192x192 fp32 5.24 / 6.47 / 5.05; by 12 -> 8 -> 12 split: 17 heads of 128x192 (T = 1024)
+// 1.13 / 1.40 / 1.08, 37 of 128x96 2.28 / 2.79 / 2.14.
+struct RegSplit {
+    int entry, compute, helper;
+};
+__host__ __device__ constexpr RegSplit bwd_split(int W, int NE, bool CO) {
+    return CO ? RegSplit{0, 0, 0} : W == 8 && NE == 12 ? RegSplit{168, 208, 88} : W == 12 ? RegSplit{128, 152, 56} : RegSplit{0, 0, 0};
+}
 
 template <int RV, int NP>
 struct State {
@@ -323,10 +338,15 @@ struct State {
 };
 
 template <int RK, int KG, int RV, int W, bool UNC, bool CO>
-__global__ void __launch_bounds__(bwd_threads(W, CO)) bwd_kernel(const BwdArgs a) {
+__global__ void __launch_bounds__(bwd_threads(W, CO), bwd_split(W, RK * RV, CO).entry > 0 ? 1 : 0)
+bwd_kernel(const BwdArgs a) {
     constexpr int KP = RK * KG, VG = 32 / KG, NP = RK / 2, NE = RV * RK, KP2 = KP / 2;
     constexpr int TV = W * VG * RV, WV = W * VG, NTHR = 32 * W;
     static_assert(TV % 2 == 0, "the operand tiles are converted two rows at a time");
+    constexpr RegSplit SPLIT = bwd_split(W, NE, CO);
+    static_assert(SPLIT.entry == 0 || (W % 4 == 0 && bwd_helpers(W) == 4 &&
+                                       W * SPLIT.compute + 4 * SPLIT.helper <= (W + 4) * SPLIT.entry),
+                  "whole warpgroups on both sides, and no more registers than the block has at launch");
     constexpr int NG = TB / GR;       // groups per block
     constexpr int NR1 = GR * RV * 2;  // per-group d_v-indexed partials of a thread: (token, row, dv|db)
     constexpr int NR2 = GR * 2;       // per-group per-token scalars: (token, df|sum GI)
@@ -397,6 +417,7 @@ __global__ void __launch_bounds__(bwd_threads(W, CO)) bwd_kernel(const BwdArgs a
     }
 
     if (!CO && w >= W) {
+        if constexpr (SPLIT.entry > 0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SPLIT.helper));
         // ---- helper warps: everything a group leaves behind once its partials lie in shared memory --------------
         // dq / dk summed over the CTA's row groups and written to this row tile's partials, dv / db cast and
         // written, the per-token scalars summed over the warps.
@@ -481,6 +502,7 @@ __global__ void __launch_bounds__(bwd_threads(W, CO)) bwd_kernel(const BwdArgs a
         __syncthreads();
         return;
     }
+    if constexpr (SPLIT.entry > 0) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SPLIT.compute));
 
     // this thread's d_k columns are RK*kg .. RK*kg+RK-1: pair q covers columns RK*kg + 2q, +1
     const float2* ks2 = reinterpret_cast<const float2*>(sm + L.ks) + NP * kg;
@@ -942,22 +964,31 @@ static BwdShape bwd_shape(int KP) {
         default: return {0, 0, 0};
     }
 }
-// Compute warps a CTA may have at each tiling (launch_bwd_t instantiates these).  With the helper warps beside them up
-// to 7 leave 255 registers per thread, which 12 state elements need, and 8 to 11 leave 168, which 8 elements need.
+// Compute warps a CTA may have at each tiling (launch_bwd_t instantiates these).
 static const int* bwd_warp_choices(int KP) {
-    static const int small[] = {8, 4, 0}, w48[] = {8, 7, 6, 4, 0}, w64[] = {11, 8, 4, 0}, w96[] = {8, 7, 6, 4, 0}, wide[] = {8, 0};
-    return KP <= 32 ? small : KP == 48 ? w48 : KP == 64 || KP == 128 ? w64 : KP == 96 || KP == 192 ? w96 : wide;
+    static const int small[] = {8, 4, 0}, w64[] = {11, 8, 4, 0}, w128[] = {11, 12, 8, 4, 0}, e12[] = {8, 7, 6, 4, 0}, wide[] = {8, 0};
+    return KP <= 32 ? small : KP == 64 ? w64 : KP == 128 ? w128 : KP == 256 ? wide : e12;
+}
+// What a token costs a CTA of W compute warps (the walk, and what does not grow with the rows), in units of which 4 warps
+// take 8, fitted to steps of one to eleven whole waves at d_k = 48 to 192: 0.75 / 1.13 / 1.33 / 1.55 ms a wave at 4 / 8 / 11
+// / 12 warps of 8 elements; 0.81 / 1.11 / 1.12 / 1.32 of 4 / 6 / 7 / 8 warps of 12, at 8 warps more in segments, whose
+// state-gradient pass has no split.  With one group buffer the compute warps wait for the helpers of the last group: alone,
+// a helper makes that 1.4 times as long (7 warps, 192x192 fp32).
+static double bwd_warp_cost(int W, int KP, int NE, int kbuf, bool two_pass) {
+    double c = W == 11 ? 14 : W == 12 ? 16.5 : W + 4;
+    if (NE == 12 && KP < 192) c = W == 4 ? (two_pass ? 8.6 : 8) : W == 6 ? 10.8 : W == 7 ? 11.2 : two_pass ? 14.8 : 13.4;
+    if (NE == 12 && KP == 192) c = W == 4 ? 8.8 : W == 6 ? 11.3 : W == 7 ? 11 : two_pass ? 14.8 : 13.4;
+    return kbuf == 1 && bwd_helpers(W) == 1 ? 1.4 * c : c;
 }
 struct BwdConfig {
     BwdShape s;
     int W, TV, smem, kbuf;
     double cost;
 };
-// The choice that costs least.  A token of a CTA of W warps costs W + 4 (the walk, and what does not grow with the
-// rows; 15 % more where 12 elements per thread spill at W = 8), an SM holds one CTA, and up to three waves are whole
-// ones; a grid beyond that, or one of segments, is charged by its CTAs.  At T = 2048 bf16, ms: 16 sequence-heads of
-// 192x128 4.08 / 3.25 at W = 7 / 8 (160 and 128 CTAs), 32 of 96x192 3.04 / 3.09 / 2.41 at 8 / 7 / 6, 128 of 96x192
-// 8.95 / 8.35 / 8.41, 64 of 128x192 5.33 / 6.45 at 11 / 8; 8 of 64x64 (T = 512, fp32) 0.27 / 0.19 at 8 / 4.
+// The choice that costs least: waves of CTAs (one per SM) times the cost of a token.  CTAs of equal sequences, or of their
+// equal segments, finish together, so their waves are whole ones.  Training step at T = 2048
+// bf16, ms, by warps: 32 sequence-heads of 192x192 (T = 1500) 4.95 / 4.78 / 4.38 at 6 / 7 / 8 (4, 4, 3 waves), 64 of 128x192
+// 8.15 / 6.72 / 7.58 at 8 / 11 / 12 (6, 4, 4), 16 of 128x128 1.95 / 1.57 / 1.73 at 4 / 8 / 11 (2, 1, 1).
 static BwdConfig bwd_config(const palimpsa_problem& p) {
     BwdConfig best{};
     best.s = bwd_shape(palimpsa_padded_k(p.K));
@@ -968,6 +999,8 @@ static BwdConfig bwd_config(const palimpsa_problem& p) {
     const int es = dtype_size(p.io_dtype);
     const double units = (double)p.num_seqs * p.H;
     for (const int* w = bwd_warp_choices(KP); *w; ++w) {
+        if (*w == 12 && (units == 0 || p.cu_seqlens) && p.segments != BWD_FEWEST_TILES)
+            continue;  // pays by whole waves, which only equal sequences have
         BwdConfig c{s, *w, *w * rpw, 0, 2, 0};
         c.smem = bwd_smem_layout(KP, c.TV, s.RV * s.RK, 32 * c.W, c.W * VG, es, unc, 2).total;
         if (c.smem > 227 * 1024) {
@@ -976,11 +1009,18 @@ static BwdConfig bwd_config(const palimpsa_problem& p) {
         }
         if (c.smem > 227 * 1024) continue;
         const int tiles = (p.V + c.TV - 1) / c.TV;
-        c.cost = (units > 0 ? units : 1) * tiles / 148;
-        if (p.segments != BWD_FEWEST_TILES) {
-            if (units > 0 && p.segments <= 1 && c.cost <= 3) c.cost = ceil(c.cost);
-            c.cost *= c.W + 4;
-            if (c.W == 8 && s.RK * s.RV == 12) c.cost *= 1.15;
+        const bool cut = p.segments > 1;
+        const double cost = bwd_warp_cost(c.W, KP, s.RK * s.RV, c.kbuf, cut && !carry_tc_shape(p));
+        const double share = (units > 0 ? units : 1) * tiles / B200_SMS;  // of a wave, per segment
+        if (p.segments == BWD_FEWEST_TILES) {
+            c.cost = 1000.0 * tiles + cost;
+        } else if (p.cu_seqlens || units == 0 || p.segments == 2) {
+            // documents fill the waves up, beyond the first few; no grid given, or two segments: a share of many waves
+            c.cost = (units > 0 && !cut && share <= 3 ? ceil(share) : share) * cost;
+        } else {
+            const int G = cut ? p.segments : 1, per = ((p.seq_len + G - 1) / G + TB - 1) / TB * TB;
+            const double full = cut && per > 0 ? (double)p.seq_len / per : G;  // segments, the last one by its share
+            c.cost = (ceil(share * full) + 1e-3 * share * full) * cost / G;       // of equal waves the fuller ones
         }
         if (!best.W || c.cost < best.cost) best = c;
     }
@@ -1018,6 +1058,21 @@ BwdWorkspace bwd_workspace_layout(const palimpsa_problem& p) {
     return ws;
 }
 
+// Does the compiled kernel start with the registers its split was made for?  (Fewer, and the wait for the compute warps'
+// share would not end.)  Asked once: a property of the binary.
+template <auto Kern>
+static bool bwd_split_fits(RegSplit split) {
+    if (!split.entry) return true;
+    static std::atomic<int> regs{0};
+    int r = regs.load(std::memory_order_relaxed);
+    if (!r) {
+        cudaFuncAttributes attr;
+        if (cudaFuncGetAttributes(&attr, Kern) != cudaSuccess) return false;
+        regs.store(r = attr.numRegs, std::memory_order_relaxed);
+    }
+    return r == split.entry;
+}
+
 template <int RK, int KG, int RV, int W>
 static int launch_bwd_w(const BwdArgs& a, int tiles, int num_seg, bool carry_only, cudaStream_t stream) {
     constexpr int VG = 32 / KG, TV = W * VG * RV;
@@ -1030,6 +1085,7 @@ static int launch_bwd_w(const BwdArgs& a, int tiles, int num_seg, bool carry_onl
 #define PALIMPSA_BWD_LAUNCH(U, C)                                                                                 \
     do {                                                                                                          \
         if (!allow_smem<bwd_kernel<RK, KG, RV, W, U, C>>(L.total)) return PALIMPSA_E_LAUNCH;                        \
+        if (!bwd_split_fits<bwd_kernel<RK, KG, RV, W, U, C>>(bwd_split(W, RK * RV, C))) return PALIMPSA_E_LAUNCH;   \
         bwd_kernel<RK, KG, RV, W, U, C><<<grid, block, L.total, stream>>>(a);                                     \
     } while (0)
     if (carry_only) {
@@ -1055,6 +1111,7 @@ static int launch_bwd_t(const BwdArgs& args, int tiles, int num_seg, bool carry_
         PALIMPSA_W(6);
     }
     if constexpr (KP == 64 || KP == 128) PALIMPSA_W(11);
+    if constexpr (KP == 128) PALIMPSA_W(12);
     if constexpr (RV > 1) PALIMPSA_W(4);
 #undef PALIMPSA_W
     return PALIMPSA_E_DIM;
@@ -1125,7 +1182,7 @@ int launch_bwd(const palimpsa_bwd_params* prm, const palimpsa_segments* segs, bo
     if (rows > 0) {
         const int rpc = FIN_THREADS / (ws.KP / 4), lanes = p.H <= FIN_THREADS ? FIN_THREADS / p.H : 1;
         const long long groups = (rows + rpc - 1) / rpc, tgroups = (p.total_tokens + lanes - 1) / lanes;
-        const int col_ctas = (int)(groups < 148 * 32 ? groups : 148 * 32);
+        const int col_ctas = (int)(groups < B200_SMS * 32 ? groups : B200_SMS * 32);
         nb = (int)(tgroups < FIN_SCALAR_CTAS ? tgroups : FIN_SCALAR_CTAS);
         const uintptr_t both = reinterpret_cast<uintptr_t>(prm->dq) | reinterpret_cast<uintptr_t>(prm->dk);
         bwd_finish_rows<<<col_ctas + nb, FIN_THREADS, 0, stream>>>(

@@ -382,11 +382,14 @@ __global__ void __launch_bounds__(128) carry_tc_kernel(const CarryArgs a, const 
     if (w == 0) tc::tmem_free(tmem, 512);
 }
 
-bool carry_tc_supported(const palimpsa_problem& p) {
+bool carry_tc_shape(const palimpsa_problem& p) {
     const int KP = palimpsa_padded_k(p.K);
-    auto al = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
     return p.io_dtype == PALIMPSA_BF16 && !(p.flags & PALIMPSA_FLAG_UNCERTAINTY) && p.V <= 128 && p.V % 8 == 0 &&
-           p.K % 8 == 0 && KP >= 32 && KP <= 128 && KP % 16 == 0 && al(p.k) && al(p.v) && al(p.b);
+           p.K % 8 == 0 && KP >= 32 && KP <= 128 && KP % 16 == 0;
+}
+bool carry_tc_supported(const palimpsa_problem& p) {
+    auto al = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
+    return carry_tc_shape(p) && al(p.k) && al(p.v) && al(p.b);
 }
 
 int launch_carry_tc(const palimpsa_bwd_params* prm, const palimpsa_segments& sg, cudaStream_t stream) {

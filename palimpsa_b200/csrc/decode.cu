@@ -28,7 +28,7 @@ struct DecArgs {
     int tiles;  // row tiles per sequence-head
 };
 
-constexpr long long DEC_SMALL_WARPS = 148 * 16;  // warps that cover the device once at 4 CTAs per SM
+constexpr long long DEC_SMALL_WARPS = B200_SMS * 16;  // warps that cover the device once at 4 CTAs per SM
 
 template <int DT>
 __device__ __forceinline__ float4 ldg4(const void* base, long long idx) {  // idx: element index, multiple of 4

@@ -9,6 +9,10 @@
 
 namespace palimpsa {
 
+// SMs of the one GPU this library is built for.  Tile heights are chosen by it, on the host and without a device, so that a
+// workspace query and the launch that follows agree everywhere.
+constexpr int B200_SMS = 148;
+
 // Lets a kernel use the `bytes` of dynamic shared memory it is about to be launched with.  The attribute belongs to the
 // kernel in one context (cudaDeviceReset, or another context on the device, starts from the default again), so it is set on
 // every launch; and never lower than before, so that a thread that launches with less does not take it from another that is
@@ -48,7 +52,8 @@ int launch_summary_tc(const palimpsa_problem& p, const palimpsa_segments& segs, 
 int summary_tc_status();
 
 // Carried-gradient terms of a segmented backward on the tensor cores (carry_tc.cu).
-bool carry_tc_supported(const palimpsa_problem& p);
+bool carry_tc_shape(const palimpsa_problem& p);      // by sizes, type and flags alone
+bool carry_tc_supported(const palimpsa_problem& p);  // and by the alignment of its tensors
 int launch_carry_tc(const palimpsa_bwd_params* prm, const palimpsa_segments& segs, cudaStream_t stream);
 int carry_tc_status();
 int bwd_wait_status();  // 0, or the code of a bounded barrier wait of the backward main kernel that gave up

@@ -141,36 +141,39 @@ int64_t plan_segments(int64_t N, int64_t T, int64_t H, int64_t K, int64_t V, int
     if (shorter && (T < 256 || packed || io == PALIMPSA_BF16)) return 1;
     const int64_t rows = palimpsa_fwd_tile_rows((int)K, (int)V);
     TORCH_CHECK_VALUE(rows > 0, "d_k = ", K, " is above the supported maximum of 256");
-    if (backward) {
-        const int64_t brow = palimpsa_bwd_tile_rows((int)K, (int)V, io, unc ? 1 : 0);
-        TORCH_CHECK_VALUE(brow > 0, "no backward tiling for d_k = ", K, ", d_v = ", V);
-        const int64_t ctas = N * H * ((V + brow - 1) / brow);
-        const bool rounded = boundaries_rounded(K, V, io, unc);
-        const int64_t nominal = N * H * nominal_tiles(K, V);
-        if (packed) {
-            if (ctas >= sms || (rounded && nominal >= sms)) return 1;
-        } else {
-            if (!shorter && rounded && 10 * nominal >= 8 * ((nominal + sms - 1) / sms) * sms) return 1;
-            palimpsa_problem p{};
-            p.num_seqs = (int)N, p.H = (int)H, p.K = (int)K, p.V = (int)V, p.io_dtype = io;
-            p.flags = unc ? PALIMPSA_FLAG_UNCERTAINTY : 0;
-            const double uncut = palimpsa_bwd_token_cost(&p);
-            p.segments = 2;
-            const double cut = palimpsa_bwd_token_cost(&p);
-            if (shorter) {  // one wave of segments; a segment's backward takes its state-gradient pass first
-                const int64_t G = std::min<int64_t>(T / 64, sms / std::max<int64_t>(ctas, 1));
-                const double one_wave = cut * (double)sms / (double)std::max<int64_t>(ctas, 1);
-                return G >= 2 && (double)T * uncut > 1.6 * one_wave * (double)T / (double)G + 400 ? G : 1;
-            }
-            if (uncut <= 1.25 * cut) return 1;
+    const int64_t pieces = std::max<int64_t>(1, std::min<int64_t>(32, T / 256));
+    if (!backward) {
+        const int64_t ctas = N * H * ((V + rows - 1) / rows);
+        if (shorter) {
+            const int64_t G = std::min<int64_t>(T / 64, sms / std::max<int64_t>(ctas, 1));
+            return G >= 3 ? G : 1;
         }
-    } else if (shorter) {
-        const int64_t G = std::min<int64_t>(T / 64, sms / std::max<int64_t>(N * H * ((V + rows - 1) / rows), 1));
-        return G >= 3 ? G : 1;
-    } else if (N * H * ((V + rows - 1) / rows) >= sms) {
-        return 1;
+        return ctas >= sms ? 1 : pieces;
     }
-    return std::max<int64_t>(1, std::min<int64_t>(32, T / 256));
+    const int64_t brow = palimpsa_bwd_tile_rows((int)K, (int)V, io, unc ? 1 : 0);
+    TORCH_CHECK_VALUE(brow > 0, "no backward tiling for d_k = ", K, ", d_v = ", V);
+    const int64_t ctas = N * H * ((V + brow - 1) / brow);
+    const bool rounded = boundaries_rounded(K, V, io, unc);
+    const int64_t nominal = N * H * nominal_tiles(K, V);
+    if (packed) return ctas >= sms || (rounded && nominal >= sms) ? 1 : pieces;
+    palimpsa_problem p{};
+    p.num_seqs = (int)N, p.seq_len = (int)T, p.H = (int)H, p.K = (int)K, p.V = (int)V, p.io_dtype = io;
+    p.flags = unc ? PALIMPSA_FLAG_UNCERTAINTY : 0;
+    const double uncut = palimpsa_bwd_token_cost(&p);
+    if (shorter) {  // one wave of segments; a segment's backward takes its state-gradient pass first
+        const int64_t G = std::min<int64_t>(T / 64, sms / std::max<int64_t>(ctas, 1));
+        p.num_seqs = 0;  // per CTA of a full grid
+        const double one_wave = palimpsa_bwd_token_cost(&p) * (double)sms / (double)((V + brow - 1) / brow);
+        return G >= 2 && (double)T * uncut > 1.6 * one_wave * (double)T / (double)G + 400 ? G : 1;
+    }
+    if (rounded && 10 * nominal >= 8 * ((nominal + sms - 1) / sms) * sms) return 1;
+    if (pieces < 2) return 1;
+    p.segments = (int)pieces;
+    // How much cheaper the cut backward has to be: less where its uncut grid is one wave (that of 4 warps below 9 units, any
+    // below 15) and the forward's leaves SMs idle too, so that the summaries and the scan are paid for there.
+    const bool one = uncut < 15;
+    const double worth = rounded ? (one ? 1.05 : 1.2) : K <= 16 || uncut < 9 ? 1.2 : one ? 1.25 : 1.55;
+    return uncut > worth * palimpsa_bwd_token_cost(&p) ? pieces : 1;
 }
 
 // The [N,G,H,V,KP] boundary buffers of a segmented pass, in one allocation (returned as its owner).

@@ -97,16 +97,22 @@ def plan_segments(N: int, T: int, H: int, K: int, V: int, device=None, backward:
 
     Forward only: the forward grid has fewer CTAs than the device has SMs.  With a backward to follow
     (``backward=True``) the backward kernel decides, since it is 3/4 of the step and keeps one CTA per SM: segments
-    when its estimated time per token (``palimpsa_bwd_token_cost``: waves of CTAs times their warps, at the tile height
-    it would take) is more than 1.25 times that of a grid without idle SMs.  That is so for 72 CTAs on 148 SMs, or
-    192 = 1.3 waves that no other tile height fills better; not for 128 CTAs = 0.86 of a wave, nor 288 = 1.95 waves
-    (2 sequences x 16 heads of 96x192, bf16, T = 2048: 3.97 ms in segments, 3.23 uncut with 24-row tiles).
+    when its estimated time per token (``palimpsa_bwd_token_cost``: waves of CTAs times what their warps cost, at the
+    tile height it would take) is by enough above that of the cut grid.  How much is enough, from 270 timed steps
+    (T = 4096, 16x32 to 256x256, three types): 1.05 where the uncut grid is one wave and the boundary terms go through
+    the tensor cores (16 heads of 128x128 bf16: 3.02 ms uncut, 2.51 cut), 1.2 where it is more (54: 5.60 / 4.34; 72 of
+    64x128, ratio 1.14: 5.40 / 5.78); with the exact float32 passes, which walk twice, 1.25 and 1.55 (16 heads of 96x192,
+    1.19: 3.61 / 3.99; 64 of 128x64 float16, 1.31: 5.61 / 6.66; 54 of 64x128 float16, 1.52: 5.79 / 5.78).
+
+    bfloat16 shapes that the tensor-core passes serve round their boundary terms, so accuracy is in play there: they are
+    cut only where the grid at fixed nominal tile heights leaves a fifth of its waves idle, whatever the estimate says
+    (30 heads of 64x128 stay exact and uncut at 3.24 ms, 2.49 in segments).
 
     Below 2048 tokens only float32 and float16 are cut, down to segments of 64 tokens and to one wave of CTAs: their
-    boundary states and carried gradients are exact float32, so the results keep their accuracy, while bfloat16's
-    carried terms are rounded for the tensor cores.  A walk costs a serial chain per token and an idle GPU whatever
-    else it does: 2 sequences x 4 heads of 64x64, T = 512, forward and backward: 441 us uncut (16 CTAs), 123 in 8
-    segments; 4 x 4 heads of 31x65, T = 511, with the uncertainty output: 375 / 217 us in 4.
+    boundary states and carried gradients are exact float32, so the results keep their accuracy.  A walk costs a serial
+    chain per token and an idle GPU whatever else it does: 2 sequences x 4 heads of 64x64, T = 512, forward and backward:
+    441 us uncut (16 CTAs), 123 in 8 segments; 4 x 4 heads of 31x65, T = 511, with the uncertainty output: 375 / 217 us
+    in 4.  bfloat16 stays uncut there: its usual route would round, and the exact one has not been timed for it.
 
     ``packed``: N documents of unequal length in one row of T tokens (``cu_seqlens``).  Only N and T are known
     without a host synchronisation.  With more CTAs than SMs the documents, started longest first, fill the waves by

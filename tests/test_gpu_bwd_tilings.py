@@ -1,5 +1,5 @@
-"""Every tile height the backward may take (warps per CTA by head size, element type and grid), with one and two group
-buffers, ragged last tiles and tokens past the last whole block, against the float64 oracle."""
+"""The backward's tile heights (warps per CTA by head size, element type and grid), with one and two group buffers, ragged
+last tiles and tokens past the last whole block, against the float64 oracle."""
 import ctypes as C
 
 import pytest
@@ -11,22 +11,102 @@ from tests.gpu_util import DEV, compare, run_cuda, run_oracle, tol_for
 pytestmark = pytest.mark.gpu
 
 
+# state rows per compute warp and the warp counts a CTA may have, by padded d_k (csrc/bwd.cu)
+ROWS = {16: 8, 32: 8, 48: 8, 64: 4, 96: 4, 128: 2, 192: 2, 256: 1}
+WARPS = {16: (8, 4), 32: (8, 4), 48: (8, 7, 6, 4), 64: (11, 8, 4), 96: (8, 7, 6, 4), 128: (12, 11, 8, 4),
+         192: (8, 7, 6, 4), 256: (8,)}
+
+
+def _tiles(N, T, H, K, V, io, unc, G):
+    """Row tiles of the backward, from what its workspace holds per (token, head): 2 tiles + 1 rows of d_k and 2 (tiles + 1)
+    scalars, beside the per-head partials and six roundings to 256 bytes."""
+    from palimpsa_b200 import _lib as L
+    p = L.Problem()
+    p.num_seqs, p.seq_len, p.total_tokens, p.H, p.K, p.V = N, T, N * T, H, K, V
+    p.io_dtype, p.segments, p.flags = io, G, L.FLAG_UNCERTAINTY if unc else 0
+    rest = L.lib().palimpsa_bwd_workspace_bytes(C.byref(p)) - 2 * 296 * H * 4
+    fits = [t for t in range(1, 80)
+            if 0 <= rest - 4 * N * T * H * (L.lib().palimpsa_padded_k(K) * (2 * t + 1) + 2 * (t + 1)) <= 6 * 256]
+    assert len(fits) == 1
+    return fits[0]
+
+
+def _one_buffer(KP, W, es, unc):
+    """Two group buffers do not fit: the shared memory of a CTA, by the parts that count (operand tiles with every value
+    twice, parked states, two checkpoint stages, group partials, raw stage)."""
+    TV, NE = W * ROWS[KP], {16: 4, 48: 12, 96: 12, 192: 12}.get(KP, 8)
+    WV = TV // (1 if KP == 256 else 2)
+    raw = 16 * es * (2 * KP + (3 + unc) * ((TV + 7) // 8 * 8 + 8))
+    fixed = 16 * 4 * KP * (2 + unc) + 16 * TV * 8 * (3 + unc) + 16 * NE * 32 * W + 16 * TV * KP + raw + 600
+    return fixed + 2 * (4 * WV * 2 * KP * 4 + 2 * 16 * TV + 32 * W) > 227 * 1024
+
+
+@pytest.mark.parametrize("W,one_buffer,N,H,T,K,V,dtype,unc,G", [
+    (8, False, 15, 2, 17, 16, 129, torch.bfloat16, False, 1),
+    (4, False, 2, 1, 33, 16, 33, torch.float32, True, 1),
+    (8, False, 15, 2, 17, 32, 129, torch.float16, True, 1),
+    (4, False, 1, 2, 35, 31, 33, torch.bfloat16, False, 1),
+    (8, True, 24, 4, 17, 48, 63, torch.float32, True, 1),       # registers split between the warpgroups, as at every d_k
+    (8, True, 24, 4, 18, 48, 62, torch.bfloat16, False, 1),     # with 8 warps of 12 elements
+    (7, False, 5, 1, 80, 48, 241, torch.bfloat16, False, 5),
+    (6, False, 10, 4, 17, 48, 97, torch.bfloat16, False, 1),
+    (4, False, 1, 2, 17, 47, 33, torch.float32, True, 1),
+    (11, True, 15, 4, 17, 64, 65, torch.float32, True, 1),
+    (11, False, 15, 2, 17, 64, 129, torch.bfloat16, False, 1),
+    (8, False, 15, 2, 17, 60, 65, torch.float32, False, 1),
+    (4, False, 1, 2, 19, 64, 17, torch.float16, False, 1),
+    (8, True, 24, 4, 17, 96, 31, torch.bfloat16, False, 1),
+    (8, True, 48, 2, 5, 90, 30, torch.float32, True, 1),
+    (7, False, 5, 1, 80, 96, 121, torch.bfloat16, False, 5),
+    (6, False, 10, 4, 17, 96, 49, torch.float32, False, 1),
+    (4, False, 2, 1, 17, 96, 17, torch.bfloat16, True, 1),
+    (12, True, 25, 4, 17, 128, 23, torch.bfloat16, False, 1),   # registers split
+    (12, True, 50, 2, 18, 120, 23, torch.float32, True, 1),
+    (11, False, 15, 2, 17, 128, 67, torch.bfloat16, False, 1),  # the benchmark's tiling, ragged
+    (8, False, 15, 2, 17, 128, 33, torch.float32, True, 1),
+    (4, False, 1, 2, 17, 128, 9, torch.bfloat16, True, 1),
+    (8, True, 24, 4, 17, 192, 15, torch.float32, False, 1),
+    (8, True, 48, 2, 5, 180, 15, torch.bfloat16, True, 1),
+    (7, False, 5, 1, 64, 192, 61, torch.bfloat16, False, 4),
+    (6, False, 10, 4, 17, 192, 25, torch.float32, False, 1),
+    (4, False, 2, 1, 17, 180, 9, torch.float32, True, 1),
+    (8, True, 2, 1, 17, 256, 7, torch.float32, True, 1),
+])
+def test_every_warp_count_matches_oracle(W, one_buffer, N, H, T, K, V, dtype, unc, G):
+    """Every warp count a CTA may have, shown to be the one taken: no other gives the case's number of row tiles."""
+    from palimpsa_b200 import _lib as L
+    from palimpsa_b200.ops import chunk_palimpsa
+    KP, es = L.lib().palimpsa_padded_k(K), dtype.itemsize
+    up = lambda w: -(-V // (w * ROWS[KP]))
+    io = {torch.float32: L.F32, torch.bfloat16: L.BF16, torch.float16: L.F16}[dtype]
+    assert _tiles(N, T, H, K, V, io, unc, G) == up(W) and [up(w) for w in WARPS[KP]].count(up(W)) == 1
+    assert _one_buffer(KP, W, es, unc) == one_buffer
+    inp = orc.make_inputs(K + V, B=N, T=T, H=H, K=K, V=V, dtype=dtype)
+    a = {n: inp[n].to(DEV).requires_grad_() for n in ("q", "k", "v", "b", "gt", "g", "Ip")}
+    out = chunk_palimpsa(*a.values(), output_uncertainty=unc, num_segments=G)
+    got = dict(zip(("o", "o_var"), out)) if unc else {"o": out}
+    sum((got[n].float() * inp["d" + n].to(DEV).float()).sum() for n in got).backward()
+    got.update({"d" + n: x.grad for n, x in a.items()})
+    ref = run_oracle(inp, unc=unc)
+    compare({n: x.detach().cpu() for n, x in got.items()}, ref, tol_for(dtype), names=list(got), what=f"{W} warps, {K}x{V}")
+
+
 @pytest.mark.parametrize("N,H,T,K,V,dtype,unc", [
-    (2, 1, 33, 16, 9, torch.float32, True),       # d_k 16, 4 warps, one row past a lane group
-    (38, 4, 17, 31, 65, torch.float32, False),    # 8 warps, unaligned rows
+    (2, 1, 33, 16, 9, torch.float32, True),       # one row past a lane group
+    (38, 4, 17, 31, 65, torch.float32, False),    # unaligned rows
     (2, 2, 35, 32, 100, torch.bfloat16, True),
-    (16, 8, 17, 48, 64, torch.bfloat16, False),   # 8 warps of 12 elements
-    (16, 8, 17, 48, 56, torch.float32, True),     # 7 warps
-    (2, 2, 47, 47, 49, torch.float32, False),     # 6 or fewer, second tile of one row
-    (8, 6, 17, 64, 128, torch.bfloat16, False),   # 11 warps of two column groups
+    (16, 8, 17, 48, 64, torch.bfloat16, False),
+    (16, 8, 17, 48, 56, torch.float32, True),
+    (2, 2, 47, 47, 49, torch.float32, False),     # second tile of one row
+    (8, 6, 17, 64, 128, torch.bfloat16, False),
     (5, 1, 31, 64, 66, torch.float32, True),
-    (12, 2, 17, 96, 192, torch.bfloat16, False),  # 8 warps
-    (16, 2, 17, 90, 192, torch.float32, False),   # 6 warps, element loads
-    (32, 4, 5, 96, 196, torch.bfloat16, True),    # 7 warps, ragged last tile
-    (8, 8, 17, 128, 64, torch.float32, True),     # 8 warps, one group buffer
-    (8, 6, 17, 128, 90, torch.bfloat16, False),   # 11 warps
-    (1, 2, 49, 128, 24, torch.bfloat16, True),    # 4 warps
-    (4, 4, 17, 192, 126, torch.bfloat16, False),  # 8 warps, 126 rows
+    (12, 2, 17, 96, 192, torch.bfloat16, False),
+    (16, 2, 17, 90, 192, torch.float32, False),   # element loads
+    (32, 4, 5, 96, 196, torch.bfloat16, True),    # ragged last tile
+    (8, 8, 17, 128, 64, torch.float32, True), 
+    (8, 6, 17, 128, 90, torch.bfloat16, False),
+    (1, 2, 49, 128, 24, torch.bfloat16, True),
+    (4, 4, 17, 192, 126, torch.bfloat16, False),  # 126 rows
     (2, 1, 19, 180, 30, torch.float32, True),
     (2, 2, 18, 256, 20, torch.float32, True),
 ])

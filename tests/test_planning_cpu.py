@@ -31,12 +31,22 @@ def test_plan_segments():
 
 def test_bf16_boundaries_are_rounded_only_where_the_grid_is_starved():
     """bf16 shapes whose carried terms or summaries go through the tensor cores (rounded there) stay uncut where the grid of
-    the nominal tiles fills 80 % of its waves, however the tile heights are tuned."""
+    the nominal tiles fills 80 % of its waves, however the tile heights are tuned; the same shapes in float32 and float16,
+    and those only the exact passes serve, are cut by cost alone."""
+    from palimpsa_b200 import _lib as L
     from palimpsa_b200.ops.palimpsa._core import plan_segments
     kw = dict(backward=True)
     for N, K, V in ((30, 64, 128), (60, 64, 128), (40, 96, 96), (40, 80, 96), (128, 48, 48), (24, 128, 128)):
         assert plan_segments(N, 4096, 1, K, V, **kw) == 1, (N, K, V)
     assert all(plan_segments(n, 4096, 1, 64, 128, packed=True, **kw) == 1 for n in range(37, 50))
+    assert plan_segments(30, 4096, 1, 64, 128, io_dtype=L.F16, **kw) == 16       # exact: 3.39 ms uncut, 3.28 cut
+    # starved grids: rounded, and faster cut
+    assert plan_segments(16, 4096, 1, 128, 128, **kw) == 16                      # 3.02 ms uncut, 2.51 cut
+    assert plan_segments(32, 4096, 1, 96, 96, **kw) == 16                        # 3.56 / 3.04
+    # exact passes cost more: 16 heads of 96x192 3.54 ms uncut, 3.79 cut; 64 of 128x64 in float16 5.61 / 6.66
+    assert plan_segments(16, 4096, 1, 96, 192, **kw) == 1
+    assert plan_segments(64, 4096, 1, 128, 64, io_dtype=L.F16, **kw) == 1
+    assert plan_segments(8, 4096, 1, 96, 192, **kw) == 16                        # 2.94 / 2.17
 
 
 def test_ramped_widths():
