@@ -170,9 +170,9 @@ def native():
     with _loading:
         if _native is None:
             ext = L.torch_ops()
-            torch.library.register_fake("palimpsa_b200::fwd", _fwd_fake)
-            torch.library.register_fake("palimpsa_b200::bwd", _bwd_fake)
-            torch.library.register_fake("palimpsa_b200::decode_step", _decode_fake)
+            torch.library.register_fake("palimpsa_b200::fwd", _fwd_fake, allow_override=True)
+            torch.library.register_fake("palimpsa_b200::bwd", _bwd_fake, allow_override=True)
+            torch.library.register_fake("palimpsa_b200::decode_step", _decode_fake, allow_override=True)
             _native = ext
     return _native
 

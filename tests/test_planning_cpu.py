@@ -150,6 +150,16 @@ print([str(getattr(torch.ops.palimpsa_b200, n).default._schema).split("(")[0] fo
     assert "palimpsa_b200::fwd" in out and "palimpsa_b200::bwd" in out and "palimpsa_b200::decode_step" in out
 
 
+def test_the_module_can_be_reloaded():
+    """A reload registers the fake kernels over those that are there."""
+    assert "again" in _in_fresh_process("""
+import importlib
+from palimpsa_b200.ops.palimpsa import _core
+importlib.reload(_core)
+print("again", _core.native())
+""")
+
+
 def test_an_unbuilt_package_imports_and_says_so_at_the_first_call():
     out = _in_fresh_process("""
 import ctypes, torch
