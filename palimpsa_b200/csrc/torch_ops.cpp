@@ -3,8 +3,7 @@
 //
 // A single-token step or a short prompt keeps the GPU busy for a few microseconds, so what such a call costs is the
 // host work in front of the launch.  With the checks, ctypes structs and Python-registered operators that work took
-// 50 us for one decode step and 450 us for a small training step (the GPU was idle for most of it); here it is a few
-// microseconds plus the launches.
+// 50 us for one decode step; here it is a few microseconds plus the launches.
 //
 // Two ways in:
 //   * run(), decode_step(), layer_*(): what the Python functions call.  Plain CUDA tensors with nothing in between go
