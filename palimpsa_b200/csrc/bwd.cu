@@ -17,19 +17,24 @@
 // in registers across a thread's rows, then across the CTA's row groups through shared memory, and
 // across the CTAs of different row tiles through fp32 partial buffers in the workspace, which the
 // finishing kernel sums in a fixed order (bitwise reproducible; no atomics).
-// Helper warps do all that follows a group's partials in shared memory (sums over the row groups, casts, global
-// stores); the compute warps hand a group over through an mbarrier pair per buffer (bounded waits) and walk on.  What
-// bounds the walk is latency at 2 or 3 warps per scheduler, FP32 pipe and issue slots each half busy, so work and
-// waits taken off the compute warps count, and one scheduler had a warp less than the others (11 warps).  With every
-// warp summing and storing its share behind a split barrier: 7.42 ms a training step at B=8 T=4096 H=6 d=128, now
-// 6.79; 3.99 / 3.51 ms at H=16 d=48.
-// One CTA per SM: up to 12 compute warps at d_k = 128 (24-row tiles); bwd_config has the choice and its measurements.
+// Helper warps stage the next block (checkpoint and raw inputs by cp.async, raw inputs converted to fp32 operands in a second
+// operand stage) and do all that follows a group's partials in shared memory (sums over the row groups, casts, global
+// stores).  All hand-overs are mbarriers with bounded waits: the compute warps meet no CTA barrier and drift apart.
+// What bounds the walk is the issue rate: a packed FP32 instruction takes two issue cycles, a pair of state elements 28 per
+// token in the reverse walk and 14 in the two forward steps, and operand loads, shuffle sums and moves come on top; so it
+// pays to have 12 elements a thread (two warps per scheduler) rather than 8 (three), and to take staging off those warps.
+// Backward at B=8 T=4096 H=6 d=128: 5.21 ms with 11 warps of 8 elements that stage for themselves, 4.77 with 8 of 12 and
+// staging helpers; 2.38 / 2.13 ms at H=16 d=48, 4.71 / 4.20 at 48x96, 8.51 / 8.21 at B=4 H=16 96x192, 3.23 / 3.15 at B=2
+// T=2048 H=6 256x128, 0.39 / 0.38 at B=64 T=512 H=8 16x32.
+// One CTA per SM, beside the smallest tilings; bwd_config has the choice of the tile.
 //
 // Finishing kernels: (1) per (token, head) row: sum the row tiles, cast dq/dk, form
 // dgt = -g f df and the per-row terms of dg and dIp; (2) per head: ordered sum over rows.
 #include <atomic>
 #include <cmath>
+#include <initializer_list>
 #include <mutex>
+#include <utility>
 
 #include "host.h"
 #include "tc_common.cuh"
@@ -41,13 +46,6 @@ constexpr int GR = 4;  // tokens per register-resident group
 // 0 ok; 5 / 6: a bounded wait on the split-phase barriers of the backward's group reduction gave up
 __device__ int g_bwd_status = 0;
 
-__device__ __forceinline__ void mbar_init_n(unsigned long long* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc::smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
-    asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.shared::cta.b64 st, [%0];\n}" ::"r"(tc::smem_u32(bar)) : "memory");
-}
-
 __device__ __forceinline__ void st2(void* base, long long idx, float2 x, int dt) {  // idx even, base aligned for it
     if (dt == PALIMPSA_F32)
         *reinterpret_cast<float2*>(reinterpret_cast<float*>(base) + idx) = x;
@@ -55,12 +53,6 @@ __device__ __forceinline__ void st2(void* base, long long idx, float2 x, int dt)
         *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(base) + idx) = __floats2bfloat162_rn(x.x, x.y);
     else
         *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(base) + idx) = __floats2half2_rn(x.x, x.y);
-}
-
-// Barrier over the compute warps of a CTA (the helper warp does not take part).
-template <int N>
-__device__ __forceinline__ void bar_compute() {
-    asm volatile("bar.sync 1, %0;" ::"n"(N) : "memory");
 }
 
 struct BwdArgs {
@@ -72,7 +64,9 @@ struct BwdArgs {
     float *dq_part, *dk_part, *df_part, *dip_part;
     void *dv, *db;
     int aligned;
+    int rows;        // state rows of a tile: as many as the CTA's warps hold, or fewer
     int kbuf;        // shared-memory buffers for the per-group d_k-indexed partials: 2 where they fit, else 1
+    int opbuf;       // operand stages: 2 where they fit (the next block is converted while this one is walked), else 1
     int rows_total;  // tokens * H
     // segments (gridDim.z of them per sequence; seg_len tokens each, a multiple of 16; 0 = whole sequence)
     int seg_len;
@@ -83,9 +77,10 @@ struct BwdArgs {
 };
 
 struct BwdSmem {
-    int ks, qs, qqs, vs2, bs2, dys2, dyvs2, fc2, fn2, slots, ckb;
-    int kred, dvs, dbs, wred, fgr;  // per-group partials handed to the helper warp, kbuf buffers of each
-    int bars;                       // mbarriers: full[2], empty[2]; then the failure flag
+    int ks, qs, qqs, vb, dys2, dyvs2, fc2, fn2;  // offsets inside an operand stage; the stages come first
+    int op_stage, slots, ckb;
+    int kred, dvs, dbs, wred, fgr;  // per-group partials handed to the helper warps, kbuf buffers of each
+    int bars;                       // mbarriers: full[2], empty[2], staged[2], done[2]; then the failure flag
     int ck_stage;  // bytes of one (M, I) checkpoint stage
     int raw, rq, rk, rv, rb, rdo, rdov, rgt;
     int total;
@@ -96,10 +91,10 @@ struct BwdSmem {
 __host__ __device__ constexpr int bwd_staged_cols(int TV) { return (TV + 7) / 8 * 8 + 8; }
 
 // Shared-memory plan of one backward CTA (KP padded d_k, TV state rows, NE state elements per thread,
-// WV row groups).  Operand tiles v, b, dy are stored with every value duplicated ({x, x}) so that a
-// 64-bit load yields the register pair the packed FP32 instructions want.
+// WV row groups).  Operands v, b, dy are stored with every value duplicated ({x, x}), v and b of a row side by side, so that
+// one 128-bit load yields the two register pairs the packed FP32 instructions want.
 __host__ __device__ inline BwdSmem bwd_smem_layout(int KP, int TV, int NE, int nthr, int WV, int es, bool unc,
-                                                  int kbuf) {
+                                                  int kbuf, int opbuf) {
     BwdSmem s;
     int off = 0;
     auto take = [&](int bytes) {
@@ -110,12 +105,13 @@ __host__ __device__ inline BwdSmem bwd_smem_layout(int KP, int TV, int NE, int n
     s.ks = take(TB * KP * 4);
     s.qs = take(TB * KP * 4);
     s.qqs = unc ? take(TB * KP * 4) : 0;
-    s.vs2 = take(TB * TV * 8);
-    s.bs2 = take(TB * TV * 8);
+    s.vb = take(TB * TV * 16);
     s.dys2 = take(TB * TV * 8);
     s.dyvs2 = unc ? take(TB * TV * 8) : 0;
     s.fc2 = take(TB * 16);
     s.fn2 = take(TB * 8);
+    s.op_stage = off;
+    off *= opbuf;
     s.slots = take(2 * 2 * NE * nthr * 4);
     s.ck_stage = 2 * TV * KP * 4;
     s.ckb = take(2 * s.ck_stage);
@@ -124,7 +120,7 @@ __host__ __device__ inline BwdSmem bwd_smem_layout(int KP, int TV, int NE, int n
     s.dbs = take(kbuf * GR * TV * 4);
     s.wred = take(kbuf * (nthr / 32) * GR * 2 * 4);
     s.fgr = take(kbuf * GR * 4);
-    s.bars = take(48);
+    s.bars = take(80);
     s.raw = off;
     int r = 0;
     auto rtake = [&](int bytes) {
@@ -144,11 +140,10 @@ __host__ __device__ inline BwdSmem bwd_smem_layout(int KP, int TV, int NE, int n
     return s;
 }
 
-// Asynchronous copy of one block's checkpoint rows (M, I) into checkpoint stage `stage_idx`.
-__device__ __forceinline__ void bwd_issue_ckpt(const BwdArgs& a, int nthr, unsigned char* sm, const BwdSmem& L, int stage_idx,
-                                               int KP, int TV, long long slot, int h, int v0, int tvw) {
+// Asynchronous copy of one block's checkpoint rows (M, I) into checkpoint stage `stage_idx`, by `nthr` threads.
+__device__ __forceinline__ void bwd_issue_ckpt(const BwdArgs& a, int nthr, int tid, unsigned char* sm, const BwdSmem& L,
+                                               int stage_idx, int KP, int TV, long long slot, int h, int v0, int tvw) {
     const palimpsa_problem& p = a.p;
-    const int tid = threadIdx.x;
     unsigned char* ck = sm + L.ckb + stage_idx * L.ck_stage;
     const int cr = KP / 4;
     const long long base = ((slot * p.H + h) * (long long)p.V + v0) * KP;
@@ -159,10 +154,9 @@ __device__ __forceinline__ void bwd_issue_ckpt(const BwdArgs& a, int nthr, unsig
 }
 
 // Asynchronous copy of one block's raw inputs (aligned path only).
-__device__ __forceinline__ void bwd_issue_raw(const BwdArgs& a, int nthr, unsigned char* sm, const BwdSmem& L, int es, int KP,
-                                              int TV, long long tok0, int nt, int nt_ext, int h, int v0, int tvw) {
+__device__ __forceinline__ void bwd_issue_raw(const BwdArgs& a, int nthr, int tid, unsigned char* sm, const BwdSmem& L, int es,
+                                              int KP, int TV, long long tok0, int nt, int nt_ext, int h, int v0, int tvw) {
     const palimpsa_problem& p = a.p;
-    const int tid = threadIdx.x;
     unsigned char* stage = sm + L.raw;
     const int cq = p.K * es / 16;
     const char* gq = reinterpret_cast<const char*>(p.q);
@@ -202,18 +196,20 @@ __device__ __forceinline__ float2 ld2s(const unsigned char* base, int e) {
     return __half22float2(*reinterpret_cast<const __half2*>(base + (size_t)e * 2));
 }
 
-template <int DT, bool ALIGNED, bool UNC>
-__device__ __forceinline__ void bwd_convert(const BwdArgs& a, int nthr, unsigned char* sm, const BwdSmem& L, int KP, int TV,
-                                            long long tok0, int nt, int nt_ext, int h, int v0, float gh, float iph,
-                                            bool carry_block) {
+// One block of fp32 operands into the operand stage `op`, by `nthr` threads.
+// UNR: iterations in flight; loads from global memory want several, a warp with few registers has room for one.
+template <int DT, bool ALIGNED, bool UNC, int KP, int TV, int UNR>
+__device__ __forceinline__ void bwd_convert(const BwdArgs& a, int nthr, int tid, const unsigned char* sm, unsigned char* op,
+                                            const BwdSmem& L, long long tok0, int nt, int nt_ext, int h, int v0, int tvw,
+                                            float gh, float iph, bool carry_block) {
     const palimpsa_problem& p = a.p;
-    const int tid = threadIdx.x;
-    const int K4 = KP / 4, V4 = TV / 4;
+    constexpr int K4 = KP / 4, V2 = TV / 2;
     const unsigned char* stage = sm + L.raw;
-    float4* qs = reinterpret_cast<float4*>(sm + L.qs);
-    float4* ks = reinterpret_cast<float4*>(sm + L.ks);
-    float4* qqs = reinterpret_cast<float4*>(sm + L.qqs);
+    float4* qs = reinterpret_cast<float4*>(op + L.qs);
+    float4* ks = reinterpret_cast<float4*>(op + L.ks);
+    float4* qqs = reinterpret_cast<float4*>(op + L.qqs);
     const float sc = p.scale;
+#pragma unroll UNR
     for (int i = tid; i < TB * K4; i += nthr) {
         int t = i / K4, c4 = i - t * K4;
         float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), kv = qv;
@@ -231,66 +227,40 @@ __device__ __forceinline__ void bwd_convert(const BwdArgs& a, int nthr, unsigned
         ks[i] = kv;
         if (UNC) qqs[i] = make_float4(sc * qv.x * qv.x, sc * qv.y * qv.y, sc * qv.z * qv.z, sc * qv.w * qv.w);
     }
-    float4* vs = reinterpret_cast<float4*>(sm + L.vs2);
-    float4* bs = reinterpret_cast<float4*>(sm + L.bs2);
-    float4* dys = reinterpret_cast<float4*>(sm + L.dys2);
-    float4* dyvs = reinterpret_cast<float4*>(sm + L.dyvs2);
-    const int TVS = bwd_staged_cols(TV);
-    const int voff = ALIGNED ? v0 % (16 / dtype_size(DT)) : 0;  // tile start inside the staged superset
-    if ((TV | voff) & 3) {
-        // tile width or offset not a multiple of 4 (both are even): two values at a time
-        const int V2 = TV / 2;
-        for (int i = tid; i < TB * V2; i += nthr) {
-            const int t = i / V2, c2 = i - t * V2;
-            float2 vv = make_float2(0.f, 0.f), bv = vv, dv = vv, dvv = vv;
-            if (t < nt && v0 + c2 * 2 < p.V) {
-                if (ALIGNED) {
-                    const int e = t * TVS + voff + 2 * c2;
-                    vv = ld2s<DT>(stage + L.rv, e);
-                    bv = ld2s<DT>(stage + L.rb, e);
-                    dv = ld2s<DT>(stage + L.rdo, e);
-                    if (UNC) dvv = ld2s<DT>(stage + L.rdov, e);
-                } else {
-                    const long long row = ((tok0 + t) * p.H + h) * (long long)p.V, e = row + v0 + c2 * 2;
-                    const bool two = e + 1 < row + p.V;
-                    vv = make_float2(ld1<DT>(p.v, e), two ? ld1<DT>(p.v, e + 1) : 0.f);
-                    bv = make_float2(ld1<DT>(p.b, e), two ? ld1<DT>(p.b, e + 1) : 0.f);
-                    dv = make_float2(ld1<DT>(a.d_o, e), two ? ld1<DT>(a.d_o, e + 1) : 0.f);
-                    if (UNC) dvv = make_float2(ld1<DT>(a.d_o_var, e), two ? ld1<DT>(a.d_o_var, e + 1) : 0.f);
-                }
-            }
-            vs[i] = make_float4(vv.x, vv.x, vv.y, vv.y);
-            bs[i] = make_float4(bv.x, bv.x, bv.y, bv.y);
-            dys[i] = make_float4(dv.x, dv.x, dv.y, dv.y);
-            if (UNC) dyvs[i] = make_float4(dvv.x, dvv.x, dvv.y, dvv.y);
-        }
-    } else
-    for (int i = tid; i < TB * V4; i += nthr) {
-        int t = i / V4, c4 = i - t * V4;
-        float4 vv = make_float4(0.f, 0.f, 0.f, 0.f), bv = vv, dv = vv, dvv = vv;
-        if (t < nt && v0 + c4 * 4 < p.V) {
+    float4* vb = reinterpret_cast<float4*>(op + L.vb);
+    float4* dys = reinterpret_cast<float4*>(op + L.dys2);
+    float4* dyvs = reinterpret_cast<float4*>(op + L.dyvs2);
+    constexpr int TVS = bwd_staged_cols(TV);
+    const int voff = ALIGNED ? v0 % (16 / dtype_size(DT)) : 0;  // tile start inside the staged superset; even, as tiles are
+#pragma unroll UNR
+    for (int i = tid; i < TB * V2; i += nthr) {
+        const int t = i / V2, r = 2 * (i - t * V2);
+        float2 vv = make_float2(0.f, 0.f), bv = vv, dv = vv, dvv = vv;
+        if (t < nt && r < tvw) {
+            const bool two = r + 1 < tvw;  // the tile's last row may be the first of a pair: the second stays 0
             if (ALIGNED) {
-                const int g4 = (t * TVS + voff) / 4 + c4;  // TVS, voff multiples of 4 here
-                vv = ld4<DT>(stage + L.rv, g4);
-                bv = ld4<DT>(stage + L.rb, g4);
-                dv = ld4<DT>(stage + L.rdo, g4);
-                if (UNC) dvv = ld4<DT>(stage + L.rdov, g4);
+                const int e = t * TVS + voff + r;
+                vv = ld2s<DT>(stage + L.rv, e);
+                bv = ld2s<DT>(stage + L.rb, e);
+                dv = ld2s<DT>(stage + L.rdo, e);
+                if (UNC) dvv = ld2s<DT>(stage + L.rdov, e);
+                if (!two) vv.y = bv.y = dv.y = dvv.y = 0.f;
             } else {
-                long long row = ((tok0 + t) * p.H + h) * (long long)p.V;
-                vv = ld4_guarded<DT>(p.v, row + v0 + c4 * 4, row + p.V);
-                bv = ld4_guarded<DT>(p.b, row + v0 + c4 * 4, row + p.V);
-                dv = ld4_guarded<DT>(a.d_o, row + v0 + c4 * 4, row + p.V);
-                if (UNC) dvv = ld4_guarded<DT>(a.d_o_var, row + v0 + c4 * 4, row + p.V);
+                const long long e = ((tok0 + t) * p.H + h) * (long long)p.V + v0 + r;
+                vv = make_float2(ld1<DT>(p.v, e), two ? ld1<DT>(p.v, e + 1) : 0.f);
+                bv = make_float2(ld1<DT>(p.b, e), two ? ld1<DT>(p.b, e + 1) : 0.f);
+                dv = make_float2(ld1<DT>(a.d_o, e), two ? ld1<DT>(a.d_o, e + 1) : 0.f);
+                if (UNC) dvv = make_float2(ld1<DT>(a.d_o_var, e), two ? ld1<DT>(a.d_o_var, e + 1) : 0.f);
             }
         }
-        st_dup4(vs, i, vv);
-        st_dup4(bs, i, bv);
-        st_dup4(dys, i, dv);
-        if (UNC) st_dup4(dyvs, i, dvv);
+        vb[2 * i] = make_float4(vv.x, vv.x, bv.x, bv.x);
+        vb[2 * i + 1] = make_float4(vv.y, vv.y, bv.y, bv.y);
+        dys[i] = make_float4(dv.x, dv.x, dv.y, dv.y);
+        if (UNC) dyvs[i] = make_float4(dvv.x, dvv.x, dvv.y, dvv.y);
     }
     // per token: {f, f, c, c} with c = (1-f)*Ip, and {fn, fn}: f of the NEXT token of the sequence (0 past its end)
-    float4* fc2 = reinterpret_cast<float4*>(sm + L.fc2);
-    float2* fn2 = reinterpret_cast<float2*>(sm + L.fn2);
+    float4* fc2 = reinterpret_cast<float4*>(op + L.fc2);
+    float2* fn2 = reinterpret_cast<float2*>(op + L.fn2);
     for (int i = tid; i < TB; i += nthr) {
         float g0 = 0.f, g1 = 0.f;
         const bool has0 = i < nt, has1 = i + 1 < nt_ext;
@@ -313,23 +283,20 @@ __device__ __forceinline__ void bwd_convert(const BwdArgs& a, int nthr, unsigned
     }
 }
 
-// Threads of a CTA: W compute warps and, except in the carry-only pass, the helper warps: as many as fit beside the
-// compute warps without costing those registers (8 warps of an SM may have 255 per thread, 12 may have 168, 16 128).
-__host__ __device__ constexpr int bwd_helpers(int W) { return W < 8 ? 8 - W : W < 12 ? 12 - W : 4; }
-__host__ __device__ constexpr int bwd_threads(int W, bool CO) { return 32 * (W + (CO ? 0 : bwd_helpers(W))); }
+// Threads of a CTA: W compute warps, and helper warps: as many as fit beside the compute warps without costing those
+// registers, which are handed out per scheduler (8 warps of an SM may have 255 per thread, 12 may have 168).
+__host__ __device__ constexpr int bwd_helpers(int W) { return W == 6 ? 2 : 4; }
+__host__ __device__ constexpr int bwd_threads(int W) { return 32 * (W + bwd_helpers(W)); }
 
-// Where an even share is too little for the walk (8 warps of 12 state elements spill 200 bytes at 168 registers, 12 warps
-// of 8 the same at 128), the warpgroup of helpers gives up registers that the compute warpgroups take: {entry, compute,
-// helper} registers per thread, {0, 0, 0} = no split.  The compute warps wait for the helpers' registers, so the block must
-// have been launched with enough for all: bwd_split_fits asks the compiled kernel before the first launch.  No spills;
-// training step, ms, T = 2048 bf16 / 1024 fp32, by 8 warps of every warp summing -> 7 warps -> 8 split: 32 heads of 96x192
-// unc x2 6.82 / 7.06 / 6.39, 60 of 192x192 fp32 5.24 / 6.47 / 5.05; by 12 -> 8 -> 12 split: 17 heads of 128x192 (T = 1024)
-// 1.13 / 1.40 / 1.08, 37 of 128x96 2.28 / 2.79 / 2.14.
+// Where an even share is too little for the walk (8 warps of 12 state elements spill 200 bytes at 168 registers), the
+// warpgroup of helpers gives up registers that the compute warpgroups take: {entry, compute, helper} registers per thread,
+// {0, 0, 0} = no split.  The compute warps wait for the helpers' registers, so the block must have been launched with enough
+// for all: bwd_split_fits asks the compiled kernel before the first launch.  Three rows and the uncertainty output need 224.
 struct RegSplit {
     int entry, compute, helper;
 };
-__host__ __device__ constexpr RegSplit bwd_split(int W, int NE, bool CO) {
-    return CO ? RegSplit{0, 0, 0} : W == 8 && NE == 12 ? RegSplit{168, 208, 88} : W == 12 ? RegSplit{128, 152, 56} : RegSplit{0, 0, 0};
+__host__ __device__ constexpr RegSplit bwd_split(int W, int RV, int RK, bool unc) {
+    return W != 8 || RV * RK != 12 ? RegSplit{0, 0, 0} : unc && RV == 3 ? RegSplit{168, 224, 56} : RegSplit{168, 208, 88};
 }
 
 template <int RV, int NP>
@@ -338,13 +305,13 @@ struct State {
 };
 
 template <int RK, int KG, int RV, int W, bool UNC, bool CO>
-__global__ void __launch_bounds__(bwd_threads(W, CO), bwd_split(W, RK * RV, CO).entry > 0 ? 1 : 0)
+__global__ void __launch_bounds__(bwd_threads(W), KG == 8 && RK < 6 && W == 4 ? 2 : 1)
 bwd_kernel(const BwdArgs a) {
     constexpr int KP = RK * KG, VG = 32 / KG, NP = RK / 2, NE = RV * RK, KP2 = KP / 2;
-    constexpr int TV = W * VG * RV, WV = W * VG, NTHR = 32 * W;
+    constexpr int TV = W * VG * RV, WV = W * VG, NTHR = 32 * W, HW = bwd_helpers(W), HT = 32 * HW;
     static_assert(TV % 2 == 0, "the operand tiles are converted two rows at a time");
-    constexpr RegSplit SPLIT = bwd_split(W, NE, CO);
-    static_assert(SPLIT.entry == 0 || (W % 4 == 0 && bwd_helpers(W) == 4 &&
+    constexpr RegSplit SPLIT = bwd_split(W, RV, RK, UNC);
+    static_assert(SPLIT.entry == 0 || (W % 4 == 0 && HW == 4 &&
                                        W * SPLIT.compute + 4 * SPLIT.helper <= (W + 4) * SPLIT.entry),
                   "whole warpgroups on both sides, and no more registers than the block has at launch");
     constexpr int NG = TB / GR;       // groups per block
@@ -358,11 +325,11 @@ bwd_kernel(const BwdArgs a) {
     const int ny = blockIdx.y / p.H, h = blockIdx.y - ny * p.H;
     const int n = p.seq_order ? p.seq_order[ny] : ny;  // blocks start in grid order: a packed batch lists its longest sequences first
     const int tile = blockIdx.x;
-    const int v0 = tile * TV;
-    const int tvw = min(TV, p.V - v0);
+    const int v0 = tile * a.rows;
+    const int tvw = min(a.rows, p.V - v0);
     const int es = dtype_size(p.io_dtype);
     const int KBUF = a.kbuf;  // shared-memory buffers for the d_k-indexed partials of a token group (1 or 2)
-    const BwdSmem L = bwd_smem_layout(KP, TV, NE, NTHR, WV, es, UNC, KBUF);
+    const BwdSmem L = bwd_smem_layout(KP, TV, NE, NTHR, WV, es, UNC, KBUF, a.opbuf);
     int bos, len;
     seq_range(p, n, bos, len);
     // this CTA's segment of the sequence: tokens [s0, s1), blocks [blk0, blk1)
@@ -372,7 +339,7 @@ bwd_kernel(const BwdArgs a) {
     const long long seg_base = (((long long)n * G + g) * p.H + h) * p.V;  // row index into [N,G,H,V,KP] buffers
     if (s1 <= s0) {  // empty segment: the end-state gradient is the start-state gradient
         if (a.rloc_M) {
-            for (int i = tid; i < tvw * (KP / 4); i += bwd_threads(W, CO)) {
+            for (int i = tid; i < tvw * (KP / 4); i += bwd_threads(W)) {
                 const long long e = (seg_base + v0) * KP + (long long)i * 4;
                 float4 cm = make_float4(0.f, 0.f, 0.f, 0.f), ci = cm;
                 if (!CO && a.carry_M) {
@@ -393,66 +360,122 @@ bwd_kernel(const BwdArgs a) {
     const bool has_carry = !CO && a.carry_M != nullptr;
     const bool has_init = p.init_mu != nullptr || (p.flags & PALIMPSA_FLAG_EXPLICIT_INIT);
 
-    // Hand-over of a group's partials: full[b] (one arrival per compute warp) and empty[b] (one from the helper),
-    // buffer b = gi & (KBUF - 1).  Waits are bounded; a wait that gives up is recorded below.
+    // Hand-overs, all waits bounded (a wait that gives up is recorded below):
+    //   full[b] / empty[b]   a group's partials, buffer b = gi & (KBUF - 1): one arrival per compute / helper warp
+    //   staged[s] / done[s]  block it, s = it & 1: its operands and checkpoint lie in shared memory (one arrival per helper
+    //                        warp); the compute warps are through with it (one per compute warp)
     unsigned long long* full = reinterpret_cast<unsigned long long*>(sm + L.bars);
     unsigned long long* empty = full + 2;
-    int* fail_flag = reinterpret_cast<int*>(full + 4);
+    unsigned long long* staged = full + 4;
+    unsigned long long* done = full + 6;
+    int* fail_flag = reinterpret_cast<int*>(full + 8);
     unsigned use = 0;  // how often this thread has been through buffer KBUF - 1, the first one of a block
     int wait_fail = 0;
     float* dvs = reinterpret_cast<float*>(sm + L.dvs);
     float* dbs = reinterpret_cast<float*>(sm + L.dbs);
     float* wred = reinterpret_cast<float*>(sm + L.wred);
     float* fgr = reinterpret_cast<float*>(sm + L.fgr);
-    if (!CO) {
-        if (tid == 0) {
-            for (int b = 0; b < 2; ++b) {
-                mbar_init_n(&full[b], W);
-                mbar_init_n(&empty[b], bwd_helpers(W));
-            }
-            *fail_flag = 0;
-            tc::mbar_init_fence();
+    if (tid == 0) {
+        for (int b = 0; b < 2; ++b) {
+            mbar_init_n(&full[b], W);
+            mbar_init_n(&empty[b], HW);
+            mbar_init_n(&staged[b], HW);
+            mbar_init_n(&done[b], W);
         }
-        __syncthreads();
+        *fail_flag = 0;
+        tc::mbar_init_fence();
     }
+    __syncthreads();
 
-    if (!CO && w >= W) {
+    if (w >= W) {
         if constexpr (SPLIT.entry > 0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SPLIT.helper));
-        // ---- helper warps: everything a group leaves behind once its partials lie in shared memory --------------
-        // dq / dk summed over the CTA's row groups and written to this row tile's partials, dv / db cast and
-        // written, the per-token scalars summed over the warps.
-        constexpr int KP4 = KP / 4, HT = 32 * bwd_helpers(W);
+        // ---- helper warps ---------------------------------------------------------------------------------------
+        // In front of the walk: checkpoints and raw inputs one block ahead by cp.async, raw inputs converted to fp32
+        // operands.  Behind it, everything a group leaves once its partials lie in shared memory: dq / dk summed over
+        // the CTA's row groups and written to this row tile's partials, dv / db cast and written, the per-token scalars
+        // summed over the warps.
+        // (Every lambda is inlined: a call would need registers that a split warp does not have.)
+        constexpr int KP4 = KP / 4;
         const int ht = tid - NTHR;
-        // Two rows of dv / db in one store: d_v even (then a tile's rows are too), both buffers aligned for a pair.  The
-        // one helper beside 11 warps is what the walk waits for (64x128: 2.70 -> 2.56 ms, 128x128: 5.32 -> 5.23, B=8
-        // T=4096 H=6); beside 7 warps and fewer the rows are few and single stores are 1 % faster.
+        const int opbuf = a.opbuf;
+        auto bar_helpers = [&]() __attribute__((always_inline)) { asm volatile("bar.sync 1, %0;" ::"n"(HT) : "memory"); };
+        auto issue_ckpt = [&](int it) __attribute__((always_inline)) {
+            bwd_issue_ckpt(a, HT, ht, sm, L, it & 1, KP, TV, slot0 + blk1 - 1 - it, h, v0, tvw);
+        };
+        auto issue_raw = [&](int it) __attribute__((always_inline)) {
+            const int t0 = (blk1 - 1 - it) * TB;
+            // the step size of the token after the block too, where the sequence goes on past this segment
+            if (a.aligned)
+                bwd_issue_raw(a, HT, ht, sm, L, es, KP, TV, (long long)bos + t0, min(TB, len - t0), min(TB + 1, len - t0),
+                              h, v0, tvw);
+        };
+        auto convert = [&](int it) __attribute__((always_inline)) {
+            const int t0 = (blk1 - 1 - it) * TB, nt = min(TB, len - t0), nt_ext = min(TB + 1, len - t0);
+            const long long tok0 = (long long)bos + t0;
+            const bool cblk = has_carry && it == 0;
+            unsigned char* op = sm + (it & (opbuf - 1)) * L.op_stage;
+#define PALIMPSA_CONVERT(DT, AL) \
+    bwd_convert<DT, AL, UNC, KP, TV, (SPLIT.entry > 0 || AL ? 1 : 4)>(a, HT, ht, sm, op, L, tok0, nt, nt_ext, h, v0, tvw, gh, iph, cblk)
+            if (a.aligned) {
+                if (p.io_dtype == PALIMPSA_BF16) PALIMPSA_CONVERT(PALIMPSA_BF16, true);
+                else if (p.io_dtype == PALIMPSA_F32) PALIMPSA_CONVERT(PALIMPSA_F32, true);
+                else PALIMPSA_CONVERT(PALIMPSA_F16, true);
+            } else {
+                if (p.io_dtype == PALIMPSA_BF16) PALIMPSA_CONVERT(PALIMPSA_BF16, false);
+                else if (p.io_dtype == PALIMPSA_F32) PALIMPSA_CONVERT(PALIMPSA_F32, false);
+                else PALIMPSA_CONVERT(PALIMPSA_F16, false);
+            }
+#undef PALIMPSA_CONVERT
+        };
+        auto arrive_staged = [&](int it) __attribute__((always_inline)) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&staged[it & 1]);
+        };
+        // The raw stage is read by all helper warps: a barrier before it is converted (every lane's copies have landed)
+        // and one before it is overwritten.
+        auto convert_and_refill = [&](int it) __attribute__((always_inline)) {
+            bar_helpers();
+            convert(it);
+            bar_helpers();
+            if (it + 1 < nblk) issue_raw(it + 1);
+            cp_async_commit();
+        };
+        issue_ckpt(0);
+        issue_raw(0);
+        cp_async_commit();
+        cp_async_wait<0>();
+        convert_and_refill(0);
+        arrive_staged(0);
+
+        // Two rows of dv / db in one store: d_v even (then a tile's rows are too), both buffers aligned for a pair.
         const bool pairs = V % 2 == 0 && ((reinterpret_cast<uintptr_t>(a.dv) | reinterpret_cast<uintptr_t>(a.db)) & (2 * es - 1)) == 0;
         const float4* kred4 = reinterpret_cast<const float4*>(sm + L.kred);
         for (int it = 0; it < nblk; ++it) {
             const int t0 = (blk1 - 1 - it) * TB, nt = min(TB, len - t0);
             const long long tok0 = (long long)bos + t0;
+            const bool more = it + 1 < nblk;
 #pragma unroll 1
             for (int gi = NG - 1; gi >= 0; --gi) {
-                const int b = gi & (KBUF - 1);
-                if (!wait_fail && !tc::mbar_wait(&full[b], use & 1)) wait_fail = 5;
-                if (b == 0) ++use;
-                const int ng = min(GR, nt - gi * GR);  // tokens of the group that exist (<= 0 past the sequence end)
-                const long long trow = (tok0 + gi * GR) * p.H + h;  // (token, head) row of the group's first token
-                const size_t prow = (size_t)tile * a.rows_total + trow;
-                for (int i = ht; i < ng * 2 * KP4; i += HT) {
-                    const int j = i / (2 * KP4), which = i / KP4 - 2 * j, c4 = i % KP4;
-                    const float4* src = kred4 + ((b * GR + j) * WV * 2 + which) * KP4 + c4;
-                    float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+                if (!CO) {
+                    const int b = gi & (KBUF - 1);
+                    if (!wait_fail && !mbar_wait_idle(&full[b], use & 1)) wait_fail = 5;
+                    if (b == 0) ++use;
+                    const int ng = min(GR, nt - gi * GR);  // tokens of the group that exist (<= 0 past the sequence end)
+                    const long long trow = (tok0 + gi * GR) * p.H + h;  // (token, head) row of the group's first token
+                    const size_t prow = (size_t)tile * a.rows_total + trow;
+                    for (int i = ht; i < ng * 2 * KP4; i += HT) {
+                        const int j = i / (2 * KP4), which = i / KP4 - 2 * j, c4 = i % KP4;
+                        const float4* src = kred4 + ((b * GR + j) * WV * 2 + which) * KP4 + c4;
+                        float2 s0 = make_float2(0.f, 0.f), s1 = s0;
 #pragma unroll
-                    for (int x = 0; x < WV; ++x) {
-                        const float4 y = src[x * 2 * KP4];
-                        s0 = fadd2(s0, make_float2(y.x, y.y));
-                        s1 = fadd2(s1, make_float2(y.z, y.w));
+                        for (int x = 0; x < WV; ++x) {
+                            const float4 y = src[x * 2 * KP4];
+                            s0 = fadd2(s0, make_float2(y.x, y.y));
+                            s1 = fadd2(s1, make_float2(y.z, y.w));
+                        }
+                        reinterpret_cast<float4*>(which ? a.dk_part : a.dq_part)[(prow + (size_t)j * p.H) * KP4 + c4] =
+                            make_float4(s0.x, s0.y, s1.x, s1.y);
                     }
-                    reinterpret_cast<float4*>(which ? a.dk_part : a.dq_part)[(prow + (size_t)j * p.H) * KP4 + c4] =
-                        make_float4(s0.x, s0.y, s1.x, s1.y);
-                }
-                if constexpr (W >= 8) {
                     for (int i = ht; i < ng * (TV / 2); i += HT) {
                         const int j = i / (TV / 2), r = 2 * (i - j * (TV / 2));
                         const float2 x = *reinterpret_cast<const float2*>(dvs + b * GR * TV + 2 * i);
@@ -470,50 +493,81 @@ bwd_kernel(const BwdArgs a) {
                             }
                         }
                     }
-                } else {
-                    for (int i = ht; i < ng * TV; i += HT) {
-                        const int j = i / TV, r = i - j * TV;
-                        if (r < tvw) {
-                            const long long e = (trow + (long long)j * p.H) * V + v0 + r;
-                            st1(a.dv, e, dvs[b * GR * TV + i], p.io_dtype);
-                            st1(a.db, e, dbs[b * GR * TV + i], p.io_dtype);
-                        }
-                    }
-                }
-                if (w == W + bwd_helpers(W) - 1 && lane < ng) {
-                    float df = 0.f, s2 = 0.f;
+                    if (w == W + HW - 1 && lane < ng) {
+                        float df = 0.f, s2 = 0.f;
 #pragma unroll
-                    for (int x = 0; x < W; ++x) {
-                        const float2 y = reinterpret_cast<const float2*>(wred)[(b * W + x) * GR + lane];
-                        df += y.x;
-                        s2 += y.y;
+                        for (int x = 0; x < W; ++x) {
+                            const float2 y = reinterpret_cast<const float2*>(wred)[(b * W + x) * GR + lane];
+                            df += y.x;
+                            s2 += y.y;
+                        }
+                        const float f = fgr[b * GR + lane];
+                        float dip = (1.f - f) * s2;
+                        if (t0 + gi * GR + lane == 0 && !has_init) dip += f * s2;  // I_0 = Ip: the start-state gradient reaches Ip
+                        a.df_part[prow + (size_t)lane * p.H] = df;
+                        a.dip_part[prow + (size_t)lane * p.H] = dip;
                     }
-                    const float f = fgr[b * GR + lane];
-                    float dip = (1.f - f) * s2;
-                    if (t0 + gi * GR + lane == 0 && !has_init) dip += f * s2;  // I_0 = Ip: the start-state gradient reaches Ip
-                    a.df_part[prow + (size_t)lane * p.H] = df;
-                    a.dip_part[prow + (size_t)lane * p.H] = dip;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&empty[b]);
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&empty[b]);
+                // The next block, in steps between the groups of this one, so that no group waits for all of it.
+                if (gi == NG - 1 && more) {
+                    // its checkpoint stage was block it - 1's
+                    if (it > 0 && !wait_fail && !mbar_wait_idle(&done[(it - 1) & 1], ((it - 1) >> 1) & 1)) wait_fail = 5;
+                    issue_ckpt(it + 1);
+                    cp_async_commit();
+                    if (opbuf == 2) {
+                        cp_async_wait<1>();  // all but the checkpoint
+                        convert_and_refill(it + 1);
+                    }
+                }
+                if (gi == NG - 2 && more && opbuf == 2) {
+                    cp_async_wait<1>();  // all but the raw inputs of block it + 2
+                    arrive_staged(it + 1);
+                }
+            }
+            if (more && opbuf == 1) {  // the one operand stage is free once block `it` is done
+                if (!wait_fail && !mbar_wait_idle(&done[it & 1], (it >> 1) & 1)) wait_fail = 5;
+                cp_async_wait<0>();
+                convert_and_refill(it + 1);
+                arrive_staged(it + 1);
             }
         }
+        cp_async_wait<0>();
         if (wait_fail) *fail_flag = wait_fail;
         __syncthreads();
         return;
     }
     if constexpr (SPLIT.entry > 0) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SPLIT.compute));
 
-    // this thread's d_k columns are RK*kg .. RK*kg+RK-1: pair q covers columns RK*kg + 2q, +1
-    const float2* ks2 = reinterpret_cast<const float2*>(sm + L.ks) + NP * kg;
-    const float2* qs2 = reinterpret_cast<const float2*>(sm + L.qs) + NP * kg;
-    const float2* qqs2 = reinterpret_cast<const float2*>(sm + L.qqs) + NP * kg;
-    const float2* vs2 = reinterpret_cast<const float2*>(sm + L.vs2) + row0;
-    const float2* bs2 = reinterpret_cast<const float2*>(sm + L.bs2) + row0;
-    const float2* dys2 = reinterpret_cast<const float2*>(sm + L.dys2) + row0;
-    const float2* dyvs2 = reinterpret_cast<const float2*>(sm + L.dyvs2) + row0;
-    const float4* fc2 = reinterpret_cast<const float4*>(sm + L.fc2);
-    const float2* fn2 = reinterpret_cast<const float2*>(sm + L.fn2);
+    if (w * VG * RV >= tvw) {
+        // A warp without rows (a tile lower than the CTA, or the last one): its share of every sum is zero, written once;
+        // after that it only keeps the hand-overs going, each no earlier than the others can use it.
+        if (!CO) {
+            for (int i = lane; i < KBUF * GR * VG * 2 * KP2; i += 32) {
+                const int bj = i / (VG * 2 * KP2);
+                reinterpret_cast<float2*>(sm + L.kred)[(bj * WV + w * VG) * 2 * KP2 + i - bj * (VG * 2 * KP2)] = make_float2(0.f, 0.f);
+            }
+            for (int i = lane; i < KBUF * GR; i += 32)
+                reinterpret_cast<float2*>(wred)[((i / GR) * W + w) * GR + i % GR] = make_float2(0.f, 0.f);
+        }
+        for (int it = 0; it < nblk; ++it) {
+            if (!wait_fail && !mbar_wait_idle(&staged[it & 1], (it >> 1) & 1)) wait_fail = 6;
+            for (int gi = NG - 1; !CO && gi >= 0; --gi) {
+                const int b = gi & (KBUF - 1);
+                if (!wait_fail && !mbar_wait_idle(&empty[b], (use & 1) ^ 1)) wait_fail = 6;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[b]);
+                if (b == 0) ++use;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&done[it & 1]);
+        }
+        if (wait_fail) *fail_flag = wait_fail;
+        __syncthreads();
+        return;
+    }
+
     float4* slots4 = reinterpret_cast<float4*>(sm + L.slots) + tid;
     float2* kred2 = reinterpret_cast<float2*>(sm + L.kred);
 
@@ -533,17 +587,58 @@ bwd_kernel(const BwdArgs a) {
             }
         }
 
-    auto load_ck = [&](State<RV, NP>& s, int stage_idx) {
-        const float* ckM = reinterpret_cast<const float*>(sm + L.ckb + stage_idx * L.ck_stage);
-        const float* ckI = ckM + TV * KP;
+    // pairs of adjacent columns or rows: two 8-byte pairs go as one 16-byte access where the tiling allows it
+    auto ld_pairs = [&](const float2* base, float2 (&dst)[NP]) __attribute__((always_inline)) {
+        if constexpr (NP % 2 == 0) {
+#pragma unroll
+            for (int q = 0; q < NP; q += 2) {
+                const float4 x = *reinterpret_cast<const float4*>(base + q);
+                dst[q] = make_float2(x.x, x.y);
+                dst[q + 1] = make_float2(x.z, x.w);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < NP; ++q) dst[q] = base[q];
+        }
+    };
+    // no memory operand: the next token's operands may be loaded above it (they lie elsewhere)
+    auto st_pairs = [&](float2* base, const float2 (&src)[NP]) __attribute__((always_inline)) {
+        if constexpr (NP % 2 == 0) {
+#pragma unroll
+            for (int q = 0; q < NP; q += 2)
+                asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(tc::smem_u32(base + q)), "f"(src[q].x), "f"(src[q].y),
+                             "f"(src[q + 1].x), "f"(src[q + 1].y));
+        } else {
+#pragma unroll
+            for (int q = 0; q < NP; ++q)
+                asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(tc::smem_u32(base + q)), "f"(src[q].x), "f"(src[q].y));
+        }
+    };
+    auto ld_rows = [&](const float2* base, float2 (&dst)[RV]) __attribute__((always_inline)) {
+        if constexpr (RV % 2 == 0) {
+#pragma unroll
+            for (int r = 0; r < RV; r += 2) {
+                const float4 x = *reinterpret_cast<const float4*>(base + r);
+                dst[r] = make_float2(x.x, x.y);
+                dst[r + 1] = make_float2(x.z, x.w);
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < RV; ++r) dst[r] = base[r];
+        }
+    };
+    auto load_ck = [&](State<RV, NP>& s, int stage_idx) __attribute__((always_inline)) {
+        const float2* ckM = reinterpret_cast<const float2*>(sm + L.ckb + stage_idx * L.ck_stage) + row0 * KP2 + NP * kg;
 #pragma unroll
         for (int r = 0; r < RV; ++r) {
-            const bool ok = row0 + r < tvw;
+            ld_pairs(ckM + r * KP2, s.M[r]);
+            ld_pairs(ckM + (TV + r) * KP2, s.I[r]);
+            if (row0 + r >= tvw) {
 #pragma unroll
-            for (int q = 0; q < NP; ++q) {
-                const int e = (row0 + r) * KP + RK * kg + 2 * q;
-                s.M[r][q] = ok ? *reinterpret_cast<const float2*>(ckM + e) : make_float2(0.f, 0.f);
-                s.I[r][q] = ok ? *reinterpret_cast<const float2*>(ckI + e) : make_float2(1.f, 1.f);
+                for (int q = 0; q < NP; ++q) {
+                    s.M[r][q] = make_float2(0.f, 0.f);
+                    s.I[r][q] = make_float2(1.f, 1.f);
+                }
             }
         }
     };
@@ -566,97 +661,39 @@ bwd_kernel(const BwdArgs a) {
             for (int q = 0; q < NP; ++q)
                 sl[(r * NP + q) * NTHR] = make_float4(s.M[r][q].x, s.M[r][q].y, s.I[r][q].x, s.I[r][q].y);
     };
-    // operand loads: two adjacent 8-byte pairs come in as one 16-byte load where the tiling allows it
-    auto ld_cols = [&](const float2* base, int tl, float2 (&dst)[NP]) {
-        if constexpr (NP % 2 == 0) {
+    float f0 = 1.f;  // f of the last processed block's first token
+    for (int it = 0; it < nblk; ++it) {
+        const int st = it & 1;
+        // this block's operand stage; this thread's d_k columns are RK*kg .. RK*kg+RK-1: pair q covers columns RK*kg + 2q, +1
+        const unsigned char* op = sm + (it & (a.opbuf - 1)) * L.op_stage;
+        const float2* ks2 = reinterpret_cast<const float2*>(op + L.ks) + NP * kg;
+        const float2* qs2 = reinterpret_cast<const float2*>(op + L.qs) + NP * kg;
+        const float2* qqs2 = reinterpret_cast<const float2*>(op + L.qqs) + NP * kg;
+        const float4* vb4 = reinterpret_cast<const float4*>(op + L.vb) + row0;
+        const float2* dys2 = reinterpret_cast<const float2*>(op + L.dys2) + row0;
+        const float2* dyvs2 = reinterpret_cast<const float2*>(op + L.dyvs2) + row0;
+        const float4* fc2 = reinterpret_cast<const float4*>(op + L.fc2);
+        const float2* fn2 = reinterpret_cast<const float2*>(op + L.fn2);
+        // one forward step of the recurrence on token tl of the staged block
+        auto fstep = [&](State<RV, NP>& s, int tl) __attribute__((always_inline)) {
+            const float4 fv = fc2[tl];
+            const float2 ff = make_float2(fv.x, fv.y), cc = make_float2(fv.z, fv.w);
+            float2 kpv[NP], kk[NP];
+            ld_pairs(ks2 + tl * KP2, kpv);
 #pragma unroll
-            for (int q = 0; q < NP; q += 2) {
-                const float4 x = *reinterpret_cast<const float4*>(base + tl * KP2 + q);
-                dst[q] = make_float2(x.x, x.y);
-                dst[q + 1] = make_float2(x.z, x.w);
-            }
-        } else {
-#pragma unroll
-            for (int q = 0; q < NP; ++q) dst[q] = base[tl * KP2 + q];
-        }
-    };
-    auto ld_rows = [&](const float2* base, int tl, float2 (&dst)[RV]) {
-        if constexpr (RV % 2 == 0) {
-#pragma unroll
-            for (int r = 0; r < RV; r += 2) {
-                const float4 x = *reinterpret_cast<const float4*>(base + tl * TV + r);
-                dst[r] = make_float2(x.x, x.y);
-                dst[r + 1] = make_float2(x.z, x.w);
-            }
-        } else {
-#pragma unroll
-            for (int r = 0; r < RV; ++r) dst[r] = base[tl * TV + r];
-        }
-    };
-    // one forward step of the recurrence on token tl of the staged block
-    auto fstep = [&](State<RV, NP>& s, int tl) {
-        const float4 fv = fc2[tl];
-        const float2 ff = make_float2(fv.x, fv.y), cc = make_float2(fv.z, fv.w);
-        float2 vr[RV], br[RV], kpv[NP];
-        ld_rows(vs2, tl, vr);
-        ld_rows(bs2, tl, br);
-        ld_cols(ks2, tl, kpv);
-#pragma unroll
-        for (int q = 0; q < NP; ++q) {
-            const float2 kp = kpv[q];
-            const float2 kk = fmul2(kp, kp);
+            for (int q = 0; q < NP; ++q) kk[q] = fmul2(kpv[q], kpv[q]);
 #pragma unroll
             for (int r = 0; r < RV; ++r) {
-                s.M[r][q] = ffma2(ff, s.M[r][q], fmul2(vr[r], kp));
-                s.I[r][q] = ffma2(ff, s.I[r][q], ffma2(br[r], kk, cc));
+                const float4 x = vb4[tl * TV + r];
+                const float2 vr = make_float2(x.x, x.y), br = make_float2(x.z, x.w);
+#pragma unroll
+                for (int q = 0; q < NP; ++q) {
+                    s.M[r][q] = ffma2(ff, s.M[r][q], fmul2(vr, kpv[q]));
+                    s.I[r][q] = ffma2(ff, s.I[r][q], ffma2(br, kk[q], cc));
+                }
             }
-        }
-    };
-
-    {
-        const int c = blk1 - 1;
-        const int nt = min(TB, len - c * TB);
-        bwd_issue_ckpt(a, NTHR, sm, L, 0, KP, TV, slot0 + c, h, v0, tvw);
-        // the step size of the token after the block too, where the sequence goes on past this segment
-        if (a.aligned)
-            bwd_issue_raw(a, NTHR, sm, L, es, KP, TV, (long long)bos + c * TB, nt, min(TB + 1, len - c * TB), h, v0, tvw);
-        cp_async_commit();
-    }
-
-    for (int it = 0; it < nblk; ++it) {
-        const int c = blk1 - 1 - it;
-        const bool cblk = has_carry && it == 0;
-        const int t0 = c * TB;
-        const int nt = min(TB, len - t0);
-        const int nt_ext = min(TB + 1, len - t0);
-        const long long tok0 = (long long)bos + t0;
-        const int st = it & 1;
-        cp_async_wait<0>();
-        bar_compute<NTHR>();
-        if (a.aligned) {
-            if (p.io_dtype == PALIMPSA_BF16)
-                bwd_convert<PALIMPSA_BF16, true, UNC>(a, NTHR, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
-            else if (p.io_dtype == PALIMPSA_F32)
-                bwd_convert<PALIMPSA_F32, true, UNC>(a, NTHR, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
-            else
-                bwd_convert<PALIMPSA_F16, true, UNC>(a, NTHR, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
-        } else {
-            if (p.io_dtype == PALIMPSA_BF16)
-                bwd_convert<PALIMPSA_BF16, false, UNC>(a, NTHR, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
-            else if (p.io_dtype == PALIMPSA_F32)
-                bwd_convert<PALIMPSA_F32, false, UNC>(a, NTHR, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
-            else
-                bwd_convert<PALIMPSA_F16, false, UNC>(a, NTHR, sm, L, KP, TV, tok0, nt, nt_ext, h, v0, gh, iph, cblk);
-        }
-        bar_compute<NTHR>();
-        // the raw stage is free again: fetch the next (earlier) block while this one is processed
-        if (c > blk0) {
-            const int t0n = t0 - TB;
-            bwd_issue_ckpt(a, NTHR, sm, L, st ^ 1, KP, TV, slot0 + c - 1, h, v0, tvw);
-            if (a.aligned)
-                bwd_issue_raw(a, NTHR, sm, L, es, KP, TV, (long long)bos + t0n, TB, min(TB + 1, len - t0n), h, v0, tvw);
-            cp_async_commit();
-        }
+        };
+        if (!wait_fail && !tc::mbar_wait(&staged[st], (it >> 1) & 1)) wait_fail = 6;
 
         // Tokens past the end of the sequence (last block only) were staged as identity steps (f = 1,
         // all other operands 0): they leave the state and every gradient untouched, so the block is
@@ -690,31 +727,30 @@ bwd_kernel(const BwdArgs a) {
                 const int tl = gi * GR + j;
                 const float2 fn = fn2[tl];
                 float2 dqs[NP], Ak[NP], Bk[NP], Uk[NP];
-                float2 Sa[RV], Sb[RV], Sc[RV];  // one accumulator per row: shorter dependent chains
+                constexpr int RS = RV == 2 ? 2 : 1;  // accumulators: two shorten the dependent chains, three cost registers
+                float2 Sa[RS], Sb[RS], Sc[RS];
 #pragma unroll
-                for (int r = 0; r < RV; ++r) Sa[r] = Sb[r] = Sc[r] = make_float2(0.f, 0.f);
+                for (int r = 0; r < RS; ++r) Sa[r] = Sb[r] = Sc[r] = make_float2(0.f, 0.f);
 #pragma unroll
                 for (int q = 0; q < NP; ++q) dqs[q] = Ak[q] = Bk[q] = Uk[q] = make_float2(0.f, 0.f);
                 float2 kp[NP], kk[NP], qp[NP], qq[NP];
-                ld_cols(ks2, tl, kp);
-                ld_cols(qs2, tl, qp);
+                ld_pairs(ks2 + tl * KP2, kp);
+                ld_pairs(qs2 + tl * KP2, qp);
 #pragma unroll
                 for (int q = 0; q < NP; ++q) {
                     kk[q] = fmul2(kp[q], kp[q]);
                     qq[q] = make_float2(0.f, 0.f);
                 }
-                if (UNC) ld_cols(qqs2, tl, qq);
-                float2 vvr[RV], bvr[RV], dyr[RV], dyvr[RV];
-                ld_rows(vs2, tl, vvr);
-                ld_rows(bs2, tl, bvr);
-                ld_rows(dys2, tl, dyr);
+                if (UNC) ld_pairs(qqs2 + tl * KP2, qq);
+                float2 dyr[RV], dyvr[RV];
+                ld_rows(dys2 + tl * TV, dyr);
 #pragma unroll
                 for (int r = 0; r < RV; ++r) dyvr[r] = make_float2(0.f, 0.f);
-                if (UNC) ld_rows(dyvs2, tl, dyvr);
+                if (UNC) ld_rows(dyvs2 + tl * TV, dyvr);
 #pragma unroll
                 for (int r = 0; r < RV; ++r) {
-                    const float2 vv = vvr[r];
-                    const float2 bv = bvr[r];
+                    const float4 x = vb4[tl * TV + r];
+                    const float2 vv = make_float2(x.x, x.y), bv = make_float2(x.z, x.w);
                     const float2 dy = dyr[r];
                     const float2 dyv = dyvr[r];
                     float2 dva = make_float2(0.f, 0.f), dba = dva;
@@ -735,9 +771,9 @@ bwd_kernel(const BwdArgs a) {
                             Bk[q] = ffma2(nGI[r][q], bv, Bk[q]);
                             dva = ffma2(GM[r][q], kp[q], dva);
                             dba = ffma2(nGI[r][q], kk[q], dba);
-                            Sa[r] = ffma2(GM[r][q], P[j].M[r][q], Sa[r]);
-                            Sb[r] = ffma2(nGI[r][q], P[j].I[r][q], Sb[r]);
-                            Sc[r] = fadd2(Sc[r], nGI[r][q]);
+                            Sa[r % RS] = ffma2(GM[r][q], P[j].M[r][q], Sa[r % RS]);
+                            Sb[r % RS] = ffma2(nGI[r][q], P[j].I[r][q], Sb[r % RS]);
+                            Sc[r % RS] = fadd2(Sc[r % RS], nGI[r][q]);
                         }
                     }
                     red1[(j * RV + r) * 2 + 0] = dva.x + dva.y;
@@ -745,21 +781,22 @@ bwd_kernel(const BwdArgs a) {
                 }
                 // this row group's share of dq and dk for the token -> shared memory
                 if (!CO) {
-                    if (j == GR - 1)  // first write of the group: the helper must be done with the buffer's last contents
+                    if (j == GR - 1)  // first write of the group: the helpers must be done with the buffer's last contents
                         if (!wait_fail && !tc::mbar_wait(&empty[b], (use & 1) ^ 1)) wait_fail = 6;  // after one failure: no more waiting
                     float2* dst = kred2 + b * (GR * WV * 2 * KP2) + ((j * WV + wv) * 2) * KP2 + NP * kg;
                     const float2 sc2 = dup2(p.scale), m2 = dup2(-2.f);
 #pragma unroll
                     for (int q = 0; q < NP; ++q) {
-                        float2 dqv = fmul2(sc2, dqs[q]);
-                        if (UNC) dqv = ffma2(fmul2(dup2(2.f), qp[q]), Uk[q], dqv);
-                        dst[q] = dqv;
-                        dst[KP2 + q] = ffma2(fmul2(m2, kp[q]), Bk[q], Ak[q]);
+                        dqs[q] = fmul2(sc2, dqs[q]);
+                        if (UNC) dqs[q] = ffma2(fmul2(dup2(2.f), qp[q]), Uk[q], dqs[q]);
+                        Ak[q] = ffma2(fmul2(m2, kp[q]), Bk[q], Ak[q]);
                     }
+                    st_pairs(dst, dqs);
+                    st_pairs(dst + KP2, Ak);
                 }
                 float2 sa = Sa[0], sb = Sb[0], scv = Sc[0];
 #pragma unroll
-                for (int r = 1; r < RV; ++r) {
+                for (int r = 1; r < RS; ++r) {
                     sa = fadd2(sa, Sa[r]);
                     sb = fadd2(sb, Sb[r]);
                     scv = fadd2(scv, Sc[r]);
@@ -772,17 +809,14 @@ bwd_kernel(const BwdArgs a) {
             // d_v-indexed sums over the KG lanes of a row; per-token scalars over the whole warp
             xreduce<NR1, KG>(red1, lane);
             {
-                constexpr int REM = NR1 >= KG ? NR1 / KG : 1;
-                const int base = xreduce_index<NR1, KG>(lane);
-                const bool owner = NR1 >= KG ? true : (kg & (KG / (NR1 < KG ? NR1 : KG) - 1)) == 0;
-                if (owner) {
+                const int base = xreduce_index<NR1, KG>(lane), count = xreduce_count<NR1, KG>(lane);
 #pragma unroll
-                    for (int i = 0; i < REM; ++i) {
+                for (int i = 0; i < xreduce_most<NR1, KG>(); ++i)
+                    if (i < count) {
                         const int id = base + i;
                         const int j = id / (RV * 2), r = (id / 2) % RV, which = id & 1;
                         (which ? dbs : dvs)[(b * GR + j) * TV + row0 + r] = red1[i];
                     }
-                }
             }
             xreduce<NR2, 32>(red2, lane);
             if ((lane & (32 / NR2 - 1)) == 0) {
@@ -794,22 +828,24 @@ bwd_kernel(const BwdArgs a) {
             if (lane == 0) mbar_arrive(&full[b]);  // this warp's partials of the group are written
             if (b == 0) ++use;
         }
+        f0 = fc2[0].x;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&done[st]);
     }
 
-    if (!CO) {
-        if (wait_fail) *fail_flag = wait_fail;
-        __syncthreads();
-        if (tid == 0 && *fail_flag) {
-            // a barrier wait ran out: record it and mark this CTA's results as invalid (NaN in the decay-gradient
-            // partial of its first token, which the finishing kernels carry into dgt and dg)
-            atomicCAS(&g_bwd_status, 0, *fail_flag);
-            a.df_part[(size_t)tile * a.rows_total + (size_t)((long long)bos + s0) * p.H + h] = __int_as_float(0x7fc00000);
-        }
+    if (wait_fail) *fail_flag = wait_fail;
+    __syncthreads();
+    const bool failed = *fail_flag != 0;
+    if (tid == 0 && failed) {
+        // a barrier wait ran out: record it and mark this CTA's results as invalid (NaN in the decay-gradient
+        // partial of its first token, which the finishing kernels carry into dgt and dg; or in the state gradients below)
+        atomicCAS(&g_bwd_status, 0, *fail_flag);
+        if (!CO) a.df_part[(size_t)tile * a.rows_total + (size_t)((long long)bos + s0) * p.H + h] = __int_as_float(0x7fc00000);
     }
 
     // ---- gradient w.r.t. the segment's start state: decay the first token's totals once more ----------
     if (a.rloc_M) {
-        const float f0 = fc2[0].x;  // f of the segment's first token (operands of the last processed block)
+        if (failed) f0 = __int_as_float(0x7fc00000);
 #pragma unroll
         for (int r = 0; r < RV; ++r) {
             if (row0 + r < tvw) {
@@ -948,69 +984,84 @@ __global__ void __launch_bounds__(32) bwd_finish_heads(const float* __restrict__
 // -------------------------------------------------------------------------------------------------
 // Host side
 // -------------------------------------------------------------------------------------------------
+// Thread tilings: RK columns x KG lanes of a row, by padded d_k.
 struct BwdShape {
-    int RK, KG, RV;
+    int RK, KG;
 };
 static BwdShape bwd_shape(int KP) {
     switch (KP) {
-        case 16: return {2, 8, 2};
-        case 32: return {4, 8, 2};
-        case 48: return {6, 8, 2};
-        case 64: return {4, 16, 2};
-        case 96: return {6, 16, 2};
-        case 128: return {4, 32, 2};
-        case 192: return {6, 32, 2};
-        case 256: return {8, 32, 1};
-        default: return {0, 0, 0};
+        case 16: return {2, 8};
+        case 32: return {4, 8};
+        case 48: return {6, 8};
+        case 64: return {4, 16};
+        case 96: return {6, 16};
+        case 128: return {4, 32};
+        case 192: return {6, 32};
+        case 256: return {8, 32};
+        default: return {0, 0};
     }
 }
-// Compute warps a CTA may have at each tiling (launch_bwd_t instantiates these).
-static const int* bwd_warp_choices(int KP) {
-    static const int small[] = {8, 4, 0}, w64[] = {11, 8, 4, 0}, w128[] = {11, 12, 8, 4, 0}, e12[] = {8, 7, 6, 4, 0}, wide[] = {8, 0};
-    return KP <= 32 ? small : KP == 64 ? w64 : KP == 128 ? w128 : KP == 256 ? wide : e12;
+// Tile heights a CTA may have at each tiling, as W compute warps of RV rows a thread (launch_bwd_t instantiates these); a
+// tile lower than its warps hold leaves the last ones idle.  8 warps of 3 rows hold 24 (48 at d_k = 64) and are run with 22
+// (44) where that makes as many tiles.
+struct BwdTile {
+    int rows, RV, W;
+};
+static const BwdTile* bwd_tile_choices(int KP) {
+    static const BwdTile k16[] = {{64, 2, 8}, {32, 2, 4}, {}}, k48[] = {{64, 2, 8}, {56, 2, 8}, {48, 2, 6}, {32, 2, 4}, {}},
+                         k64[] = {{44, 3, 8}, {32, 2, 8}, {16, 2, 4}, {}},
+                         k96[] = {{32, 2, 8}, {28, 2, 8}, {24, 2, 6}, {16, 2, 4}, {}},
+                         k128[] = {{22, 3, 8}, {24, 3, 8}, {16, 2, 8}, {8, 2, 4}, {}},
+                         k192[] = {{16, 2, 8}, {14, 2, 8}, {12, 2, 6}, {8, 2, 4}, {}}, k256[] = {{8, 1, 8}, {}};
+    switch (KP) {
+        case 48: return k48;
+        case 64: return k64;
+        case 96: return k96;
+        case 128: return k128;
+        case 192: return k192;
+        case 256: return k256;
+        default: return k16;
+    }
 }
-// What a token costs a CTA of W compute warps (the walk, and what does not grow with the rows), in units of which 4 warps
-// take 8, fitted to steps of one to eleven whole waves at d_k = 48 to 192: 0.75 / 1.13 / 1.33 / 1.55 ms a wave at 4 / 8 / 11
-// / 12 warps of 8 elements; 0.81 / 1.11 / 1.12 / 1.32 of 4 / 6 / 7 / 8 warps of 12, at 8 warps more in segments, whose
-// state-gradient pass has no split.  With one group buffer the compute warps wait for the helpers of the last group: alone,
-// a helper makes that 1.4 times as long (7 warps, 192x192 fp32).
-static double bwd_warp_cost(int W, int KP, int NE, int kbuf, bool two_pass) {
-    double c = W == 11 ? 14 : W == 12 ? 16.5 : W + 4;
+// What a token costs a CTA (the walk, and what does not grow with the rows), in units of which 4 warps of 8 elements take 8.
+static double bwd_tile_cost(const BwdTile& t, int KP, int NE, int opbuf, bool two_pass) {
+    if (t.RV == 3) return t.rows % 8 ? 14 : 16.5;
+    const int W = t.rows * KP / (32 * NE);  // warps with rows
+    double c = W + 4;
     if (NE == 12 && KP < 192) c = W == 4 ? (two_pass ? 8.6 : 8) : W == 6 ? 10.8 : W == 7 ? 11.2 : two_pass ? 14.8 : 13.4;
-    if (NE == 12 && KP == 192) c = W == 4 ? 8.8 : W == 6 ? 11.3 : W == 7 ? 11 : two_pass ? 14.8 : 13.4;
-    return kbuf == 1 && bwd_helpers(W) == 1 ? 1.4 * c : c;
+    if (NE == 12 && KP == 192) c = W == 4 ? 8.8 : W == 6 ? 11.3 : W == 7 ? (opbuf == 1 ? 12 : 11) : two_pass ? 14.8 : 13.4;
+    return c;
 }
 struct BwdConfig {
     BwdShape s;
-    int W, TV, smem, kbuf;
+    BwdTile t;
+    int smem, kbuf, opbuf;
     double cost;
 };
 // The choice that costs least: waves of CTAs (one per SM) times the cost of a token.  CTAs of equal sequences, or of their
-// equal segments, finish together, so their waves are whole ones.  Training step at T = 2048
-// bf16, ms, by warps: 32 sequence-heads of 192x192 (T = 1500) 4.95 / 4.78 / 4.38 at 6 / 7 / 8 (4, 4, 3 waves), 64 of 128x192
-// 8.15 / 6.72 / 7.58 at 8 / 11 / 12 (6, 4, 4), 16 of 128x128 1.95 / 1.57 / 1.73 at 4 / 8 / 11 (2, 1, 1).
+// equal segments, finish together, so their waves are whole ones.
 static BwdConfig bwd_config(const palimpsa_problem& p) {
     BwdConfig best{};
     best.s = bwd_shape(palimpsa_padded_k(p.K));
     if (!best.s.RK) return best;
     const BwdShape s = best.s;
-    const int VG = 32 / s.KG, rpw = VG * s.RV, KP = s.RK * s.KG;
+    const int VG = 32 / s.KG, KP = s.RK * s.KG;
     const bool unc = (p.flags & PALIMPSA_FLAG_UNCERTAINTY) != 0;
     const int es = dtype_size(p.io_dtype);
     const double units = (double)p.num_seqs * p.H;
-    for (const int* w = bwd_warp_choices(KP); *w; ++w) {
-        if (*w == 12 && (units == 0 || p.cu_seqlens) && p.segments != BWD_FEWEST_TILES)
+    for (const BwdTile* t = bwd_tile_choices(KP); t->W; ++t) {
+        if (t->rows == 24 && KP == 128 && (units == 0 || p.cu_seqlens) && p.segments != BWD_FEWEST_TILES)
             continue;  // pays by whole waves, which only equal sequences have
-        BwdConfig c{s, *w, *w * rpw, 0, 2, 0};
-        c.smem = bwd_smem_layout(KP, c.TV, s.RV * s.RK, 32 * c.W, c.W * VG, es, unc, 2).total;
-        if (c.smem > 227 * 1024) {
-            c.kbuf = 1;
-            c.smem = bwd_smem_layout(KP, c.TV, s.RV * s.RK, 32 * c.W, c.W * VG, es, unc, 1).total;
+        BwdConfig c{s, *t, 0, 0, 0, 0};
+        for (const auto& bufs : {std::pair<int, int>{2, 2}, {2, 1}, {1, 2}, {1, 1}}) {
+            c.opbuf = bufs.first, c.kbuf = bufs.second;
+            c.smem = bwd_smem_layout(KP, t->W * VG * t->RV, t->RV * s.RK, 32 * t->W, t->W * VG, es, unc, c.kbuf, c.opbuf).total;
+            if (c.smem <= 227 * 1024) break;
         }
         if (c.smem > 227 * 1024) continue;
-        const int tiles = (p.V + c.TV - 1) / c.TV;
+        const int tiles = (p.V + t->rows - 1) / t->rows;
         const bool cut = p.segments > 1;
-        const double cost = bwd_warp_cost(c.W, KP, s.RK * s.RV, c.kbuf, cut && !carry_tc_shape(p));
+        const double cost = bwd_tile_cost(*t, KP, t->RV * s.RK, c.opbuf, cut && !carry_tc_shape(p));
         const double share = (units > 0 ? units : 1) * tiles / B200_SMS;  // of a wave, per segment
         if (p.segments == BWD_FEWEST_TILES) {
             c.cost = 1000.0 * tiles + cost;
@@ -1022,7 +1073,7 @@ static BwdConfig bwd_config(const palimpsa_problem& p) {
             const double full = cut && per > 0 ? (double)p.seq_len / per : G;  // segments, the last one by its share
             c.cost = (ceil(share * full) + 1e-3 * share * full) * cost / G;       // of equal waves the fuller ones
         }
-        if (!best.W || c.cost < best.cost) best = c;
+        if (!best.t.W || c.cost < best.cost) best = c;
     }
     return best;
 }
@@ -1030,8 +1081,7 @@ static BwdConfig bwd_config(const palimpsa_problem& p) {
 double bwd_token_cost(const palimpsa_problem& p) { return bwd_config(p).cost; }
 
 int bwd_tile_rows(const palimpsa_problem& p) {
-    const BwdConfig c = bwd_config(p);
-    return c.TV;  // 0: nothing fits
+    return bwd_config(p).t.rows;  // 0: nothing fits
 }
 
 BwdWorkspace bwd_workspace_layout(const palimpsa_problem& p) {
@@ -1078,14 +1128,14 @@ static int launch_bwd_w(const BwdArgs& a, int tiles, int num_seg, bool carry_onl
     constexpr int VG = 32 / KG, TV = W * VG * RV;
     const palimpsa_problem& p = a.p;
     const bool unc = (p.flags & PALIMPSA_FLAG_UNCERTAINTY) != 0;
-    const BwdSmem L = bwd_smem_layout(RK * KG, TV, RV * RK, 32 * W, W * VG, dtype_size(p.io_dtype), unc, a.kbuf);
+    const BwdSmem L = bwd_smem_layout(RK * KG, TV, RV * RK, 32 * W, W * VG, dtype_size(p.io_dtype), unc, a.kbuf, a.opbuf);
     if (L.total > 227 * 1024) return PALIMPSA_E_DIM;
     dim3 grid(tiles, p.num_seqs * p.H, num_seg);
-    dim3 block(bwd_threads(W, carry_only), 1, 1);
+    dim3 block(bwd_threads(W), 1, 1);
 #define PALIMPSA_BWD_LAUNCH(U, C)                                                                                 \
     do {                                                                                                          \
         if (!allow_smem<bwd_kernel<RK, KG, RV, W, U, C>>(L.total)) return PALIMPSA_E_LAUNCH;                        \
-        if (!bwd_split_fits<bwd_kernel<RK, KG, RV, W, U, C>>(bwd_split(W, RK * RV, C))) return PALIMPSA_E_LAUNCH;   \
+        if (!bwd_split_fits<bwd_kernel<RK, KG, RV, W, U, C>>(bwd_split(W, RV, RK, U))) return PALIMPSA_E_LAUNCH;    \
         bwd_kernel<RK, KG, RV, W, U, C><<<grid, block, L.total, stream>>>(a);                                     \
     } while (0)
     if (carry_only) {
@@ -1097,22 +1147,24 @@ static int launch_bwd_w(const BwdArgs& a, int tiles, int num_seg, bool carry_onl
     return cudaGetLastError() == cudaSuccess ? PALIMPSA_OK : PALIMPSA_E_LAUNCH;
 }
 
-template <int RK, int KG, int RV>
+template <int RK, int KG>
 static int launch_bwd_t(const BwdArgs& args, int tiles, int num_seg, bool carry_only, cudaStream_t stream) {
     const BwdConfig cfg = bwd_config(args.p);
     BwdArgs a = args;
+    a.rows = cfg.t.rows;
     a.kbuf = cfg.kbuf;
-#define PALIMPSA_W(n)                                                                                    \
-    if (cfg.W == n) return launch_bwd_w<RK, KG, RV, n>(a, tiles, num_seg, carry_only, stream)
+    a.opbuf = cfg.opbuf;
+#define PALIMPSA_W(rv, n)                                                                                \
+    if (cfg.t.W == n && cfg.t.RV == rv) return launch_bwd_w<RK, KG, rv, n>(a, tiles, num_seg, carry_only, stream)
     constexpr int KP = RK * KG;
-    PALIMPSA_W(8);
-    if constexpr (RK == 6) {
-        PALIMPSA_W(7);
-        PALIMPSA_W(6);
+    if constexpr (KP == 256) {
+        PALIMPSA_W(1, 8);
+    } else {
+        PALIMPSA_W(2, 8);
+        PALIMPSA_W(2, 4);
     }
-    if constexpr (KP == 64 || KP == 128) PALIMPSA_W(11);
-    if constexpr (KP == 128) PALIMPSA_W(12);
-    if constexpr (RV > 1) PALIMPSA_W(4);
+    if constexpr (RK == 6) PALIMPSA_W(2, 6);
+    if constexpr (KP == 64 || KP == 128) PALIMPSA_W(3, 8);
 #undef PALIMPSA_W
     return PALIMPSA_E_DIM;
 }
@@ -1165,14 +1217,14 @@ int launch_bwd(const palimpsa_bwd_params* prm, const palimpsa_segments* segs, bo
                 (a.d_o_var == nullptr || aligned16(a.d_o_var)) && ((reinterpret_cast<uintptr_t>(p.gt) & 3) == 0);
     int rc = PALIMPSA_OK;
     if (stages & 1) switch (ws.KP) {
-        case 16: rc = launch_bwd_t<2, 8, 2>(a, ws.tiles, num_seg, carry_only, stream); break;
-        case 32: rc = launch_bwd_t<4, 8, 2>(a, ws.tiles, num_seg, carry_only, stream); break;
-        case 48: rc = launch_bwd_t<6, 8, 2>(a, ws.tiles, num_seg, carry_only, stream); break;
-        case 64: rc = launch_bwd_t<4, 16, 2>(a, ws.tiles, num_seg, carry_only, stream); break;
-        case 96: rc = launch_bwd_t<6, 16, 2>(a, ws.tiles, num_seg, carry_only, stream); break;
-        case 128: rc = launch_bwd_t<4, 32, 2>(a, ws.tiles, num_seg, carry_only, stream); break;
-        case 192: rc = launch_bwd_t<6, 32, 2>(a, ws.tiles, num_seg, carry_only, stream); break;
-        case 256: rc = launch_bwd_t<8, 32, 1>(a, ws.tiles, num_seg, carry_only, stream); break;
+        case 16: rc = launch_bwd_t<2, 8>(a, ws.tiles, num_seg, carry_only, stream); break;
+        case 32: rc = launch_bwd_t<4, 8>(a, ws.tiles, num_seg, carry_only, stream); break;
+        case 48: rc = launch_bwd_t<6, 8>(a, ws.tiles, num_seg, carry_only, stream); break;
+        case 64: rc = launch_bwd_t<4, 16>(a, ws.tiles, num_seg, carry_only, stream); break;
+        case 96: rc = launch_bwd_t<6, 16>(a, ws.tiles, num_seg, carry_only, stream); break;
+        case 128: rc = launch_bwd_t<4, 32>(a, ws.tiles, num_seg, carry_only, stream); break;
+        case 192: rc = launch_bwd_t<6, 32>(a, ws.tiles, num_seg, carry_only, stream); break;
+        case 256: rc = launch_bwd_t<8, 32>(a, ws.tiles, num_seg, carry_only, stream); break;
         default: return PALIMPSA_E_DIM;
     }
     if (rc != PALIMPSA_OK) return rc;

@@ -145,14 +145,16 @@ __device__ __forceinline__ ChunkSplit chunk_split(int chunks, int nthr, int tid)
 
 // Sum N per-lane values over the L lanes that differ from this one in the low log2(L) bits
 // (L = 2^s <= 32).  "Transposed" butterfly: each step exchanges half of the remaining values, so it
-// costs N-1 (+ a few) shuffles instead of N*log2(L).  On return x[i], i < max(1, N/L), holds the sum of
-// value xreduce_index<N, L>(lane) + i.
+// costs N-1 (+ a few) shuffles instead of N*log2(L).  An odd remainder above one is padded with a zero (N itself is
+// even or one).  On return x[i], i < xreduce_count<N, L>(lane), holds the sum of value xreduce_index<N, L>(lane) + i.
 template <int N, int L>
 __device__ __forceinline__ void xreduce(float (&x)[N], int lane) {
+    static_assert(N == 1 || N % 2 == 0, "no room for the padding");
     int n = N;
 #pragma unroll
     for (int off = L / 2; off >= 1; off >>= 1) {
         if (n > 1) {
+            if (n & 1) x[n++] = 0.f;
             const int half = n / 2;
             const bool up = (lane & off) != 0;
 #pragma unroll
@@ -169,17 +171,40 @@ __device__ __forceinline__ void xreduce(float (&x)[N], int lane) {
         }
     }
 }
+// First value of this lane's share, how many of N values a lane is left with at most, and how many of them are this
+// lane's to write: none where another lane holds the same one or only padding is left.
 template <int N, int L>
 __device__ __forceinline__ int xreduce_index(int lane) {
     int idx = 0, n = N;
 #pragma unroll
     for (int off = L / 2; off >= 1; off >>= 1) {
         if (n > 1) {
-            n /= 2;
+            n = (n + 1) / 2;
             if (lane & off) idx += n;
         }
     }
     return idx;
+}
+template <int N, int L>
+__host__ __device__ constexpr int xreduce_most() {
+    int n = N;
+    for (int off = L / 2; off >= 1; off >>= 1)
+        if (n > 1) n = (n + 1) / 2;
+    return n;
+}
+template <int N, int L>
+__device__ __forceinline__ int xreduce_count(int lane) {
+    int n = N, count = N;
+#pragma unroll
+    for (int off = L / 2; off >= 1; off >>= 1) {
+        if (n > 1) {
+            n = (n + 1) / 2;
+            count = (lane & off) ? (count > n ? count - n : 0) : (count < n ? count : n);
+        } else if (lane & off) {
+            count = 0;
+        }
+    }
+    return count;
 }
 
 }  // namespace palimpsa

@@ -149,6 +149,22 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
 
 }  // namespace tc
 
+// Hand-overs between the warps of a CTA: barriers with several arrivals per phase.
+__device__ __forceinline__ void mbar_init_n(unsigned long long* bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc::smem_u32(bar)), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
+    asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.shared::cta.b64 st, [%0];\n}" ::"r"(tc::smem_u32(bar)) : "memory");
+}
+// The wait of a warp that is ahead of the others most of the time, with pauses: polling takes issue slots from them.
+__device__ __forceinline__ bool mbar_wait_idle(unsigned long long* bar, unsigned parity) {
+    for (unsigned i = 0; i < tc::SPIN_LIMIT; ++i) {
+        if (tc::mbar_wait(bar, parity, 1)) return true;
+        __nanosleep(64);
+    }
+    return false;
+}
+
 // Host side: a 2-D tensor map over a row-major bf16 matrix [rows][row_elems] of this GPU's memory, box of 64
 // elements (128 bytes) x box_rows rows, 128-byte swizzle, zero fill outside.  Returns false if the driver entry
 // point is unavailable or refuses the description (the caller then takes its non-TMA path).
