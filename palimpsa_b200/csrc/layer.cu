@@ -7,6 +7,8 @@
 // row reductions are xor-shuffles.  These kernels are HBM-bound: every input element is read once
 // (second passes over a row hit L1) and every output element written once.  Parameter gradients are
 // per-row partials in a workspace, summed by small ordered-reduction kernels (reproducible, no atomics).
+#include <initializer_list>
+
 #include "common.cuh"
 #include "host.h"
 
@@ -531,6 +533,302 @@ __global__ void __launch_bounds__(1024) layer_epilogue_reduce_kernel(const float
         sum_cols_body(w_dw, dweight, nrows, V, blockIdx.x - nh, red);
 }
 
+// ---- 16-bit rows of at most 128 elements: LPR lanes a row, 8 elements (16 bytes) a lane --------------------------
+// The kernels above give such a row a whole warp, 8 bytes a lane, and every sum over it five shuffles.  Here 32 / LPR rows
+// share a warp (LPR = 8 up to 64 elements, else 16): half or a quarter of the load and store instructions, and one shuffle
+// sequence of log2(LPR) steps serves all rows of the warp.  Both directions at B=8 T=4096 H=6 d=128 bf16: 358 -> 288 us (67 %
+// and 83 % of the copy rate).  Taken where rows are multiples of 16 bytes that start on 16-byte boundaries.
+template <int DT>
+__device__ __forceinline__ void unpack8(uint4 u, float (&f)[8]) {
+    const unsigned w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 x = DT == PALIMPSA_BF16 ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]))
+                                             : __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+        f[2 * i] = x.x;
+        f[2 * i + 1] = x.y;
+    }
+}
+template <int DT>
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+    unsigned w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (DT == PALIMPSA_BF16) {
+            const __nv_bfloat162 x = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+            w[i] = *reinterpret_cast<const unsigned*>(&x);
+        } else {
+            const __half2 x = __floats2half2_rn(f[2 * i], f[2 * i + 1]);
+            w[i] = *reinterpret_cast<const unsigned*>(&x);
+        }
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+// A lane's 16 bytes at element `off`; zeros where the lane has none.
+__device__ __forceinline__ uint4 row_ld8(const void* base, long long off, bool on) {
+    return on ? *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(base) + off) : make_uint4(0, 0, 0, 0);
+}
+template <int DT>
+__device__ __forceinline__ void row_st8(void* base, long long off, const float (&f)[8]) {
+    *reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(base) + off) = pack8<DT>(f);
+}
+template <int LPR>
+__device__ __forceinline__ float row_sum(float x) {
+#pragma unroll
+    for (int off = LPR / 2; off >= 1; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+    return x;
+}
+__device__ __forceinline__ float dot8(const float (&a)[8], const float (&b)[8]) {
+    float s = a[0] * b[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) s += a[i] * b[i];
+    return s;
+}
+
+template <int DT, int LPR>
+__global__ void __launch_bounds__(256, 4) layer_prologue_fwd16_kernel(const palimpsa_layer_prologue a, int rows) {
+    extern __shared__ float head_tab[];  // [H] softplus(b_scale)
+    constexpr int RPW = 32 / LPR;
+    const int lane = threadIdx.x & 31, e0 = 8 * (lane % LPR), sub = lane / LPR;
+    const int warp0 = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int nwarps = gridDim.x * (blockDim.x >> 5);
+    const int K = a.K, V = a.V, H = a.H, rep = a.H / a.Hq;
+    const bool onk = e0 < K, onv = e0 < V;
+    for (int h = threadIdx.x; h < H; h += blockDim.x) head_tab[h] = softplusf_(a.b_scale[h]);
+    // gt = softplus(dt_raw + dt_bias): one thread per row
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x)
+        a.gt[i] = softplusf_(ld1<DT>(a.dt_raw, i) + a.dt_bias[i % H]);
+    __syncthreads();
+    for (long long base = (long long)warp0 * RPW; base < rows; base += (long long)nwarps * RPW) {
+        const long long row = base + sub;
+        const bool ok = row < rows;
+        const int tok = (int)row / H, h = (int)row - tok * H;
+        const long long ko = ((long long)tok * a.Hq + (rep == 1 ? h : h / rep)) * K + e0, vo = row * V + e0;
+        const uint4 qu = row_ld8(a.q_raw, ko, ok && onk), ku = row_ld8(a.k_raw, ko, ok && onk);
+        const uint4 xu = row_ld8(a.x, vo, ok && onv), bu = row_ld8(a.b_raw, vo, ok && onv);
+        const float bsr = ok ? ld1<DT>(a.bs_raw, row) : 0.f;
+        float q[8], k[8];
+        unpack8<DT>(qu, q);
+        unpack8<DT>(ku, k);
+        const float rq = rsqrtf(fmaxf(row_sum<LPR>(dot8(q, q)), NORM_EPS2));
+        const float rk = rsqrtf(fmaxf(row_sum<LPR>(dot8(k, k)), NORM_EPS2));
+        if (ok && onk) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) q[i] *= rq, k[i] *= rk;
+            row_st8<DT>(a.q, row * K + e0, q);
+            row_st8<DT>(a.k, row * K + e0, k);
+        }
+        const float bs = round_io<DT>(sigmoidf_(bsr));
+        const float spb = head_tab[ok ? h : 0] * bs;
+        if (ok && onv) {
+            float x[8], b[8];
+            unpack8<DT>(xu, x);
+            unpack8<DT>(bu, b);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] *= bs, b[i] = sigmoidf_(b[i]) * spb;
+            row_st8<DT>(a.v, vo, x);
+            row_st8<DT>(a.b, vo, b);
+        }
+    }
+}
+
+template <int DT, int LPR>
+__global__ void __launch_bounds__(256, 3) layer_prologue_bwd16_kernel(const palimpsa_layer_prologue a, int qrows, float* w_dtb,
+                                                                      float* w_bsc) {
+    extern __shared__ float head_tab[];  // [2][H]: softplus(b_scale), its derivative
+    constexpr int RPW = 32 / LPR;
+    const int lane = threadIdx.x & 31, e0 = 8 * (lane % LPR), sub = lane / LPR;
+    const int warp0 = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int nwarps = gridDim.x * (blockDim.x >> 5);
+    const int K = a.K, V = a.V, H = a.H, rep = a.H / a.Hq;
+    const int rows = qrows * rep;
+    for (int h = threadIdx.x; h < H; h += blockDim.x) {
+        head_tab[h] = softplusf_(a.b_scale[h]);
+        head_tab[H + h] = softplus_grad(a.b_scale[h]);
+    }
+    // d dt_raw = dgt * softplus'(dt_raw + dt_bias): one thread per row
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
+        const float x = ld1<DT>(a.dt_raw, i) + a.dt_bias[i % H];
+        const float ddt = a.dgt[i] * (x > 20.f ? 1.f : 1.f / (1.f + expf(-x)));
+        st1(a.ddt_raw, i, ddt, DT);
+        w_dtb[i] = ddt;
+    }
+    __syncthreads();
+    for (long long base = (long long)warp0 * RPW; base < qrows; base += (long long)nwarps * RPW) {
+        const long long qrow = base + sub;
+        const bool ok = qrow < qrows, onk = ok && e0 < K, onv = ok && e0 < V;
+        const int tok = (int)qrow / a.Hq, hq = (int)qrow - tok * a.Hq;
+        const uint4 qu = row_ld8(a.q_raw, qrow * K + e0, onk), ku = row_ld8(a.k_raw, qrow * K + e0, onk);
+        float gq[8], gk[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) gq[i] = gk[i] = 0.f;
+        for (int r = 0; r < rep; ++r) {
+            const int h = hq * rep + r;
+            const long long row = (long long)tok * H + h, vo = row * V + e0;
+            // every load of this value-head row first
+            const uint4 dqu = row_ld8(a.dq, row * K + e0, onk), dku = row_ld8(a.dk, row * K + e0, onk);
+            const uint4 xu = row_ld8(a.x, vo, onv), bu = row_ld8(a.b_raw, vo, onv);
+            const uint4 dvu = row_ld8(a.dv, vo, onv), dbu = row_ld8(a.db, vo, onv);
+            const float bsf = sigmoidf_(ok ? ld1<DT>(a.bs_raw, row) : 0.f);
+            float t[8];
+            unpack8<DT>(dqu, t);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) gq[i] += t[i];
+            unpack8<DT>(dku, t);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) gk[i] += t[i];
+            const float bs = round_io<DT>(bsf);
+            const float sp = head_tab[ok ? h : 0], w = sp * bs;
+            float x[8], dv[8], b[8], db[8];
+            unpack8<DT>(xu, x);
+            unpack8<DT>(dvu, dv);
+            unpack8<DT>(bu, b);
+            unpack8<DT>(dbu, db);
+            const float dx = dot8(dv, x);
+            float dsg = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float sg = sigmoidf_(b[i]);
+                dsg += db[i] * sg;
+                dv[i] *= bs;
+                db[i] = db[i] * w * sg * (1.f - sg);
+            }
+            if (onv) {
+                row_st8<DT>(a.dx, vo, dv);
+                row_st8<DT>(a.db_raw, vo, db);
+            }
+            const float acc_bs = row_sum<LPR>(dx + sp * dsg), acc_sc = row_sum<LPR>(dsg);
+            if (ok && e0 == 0) {
+                st1(a.dbs_raw, row, acc_bs * bsf * (1.f - bsf), DT);
+                w_bsc[row] = acc_sc * bs * head_tab[H + h];
+            }
+        }
+        float q[8], k[8];
+        unpack8<DT>(qu, q);
+        unpack8<DT>(ku, k);
+        const float sq = row_sum<LPR>(dot8(q, q)), sk = row_sum<LPR>(dot8(k, k));
+        const float dq_ = row_sum<LPR>(dot8(q, gq)), dk_ = row_sum<LPR>(dot8(k, gk));
+        const float rq = rsqrtf(fmaxf(sq, NORM_EPS2)), rk = rsqrtf(fmaxf(sk, NORM_EPS2));
+        // <y, G> / n with y = x / n: the coefficient of x in the projection term (0 while the norm is clamped)
+        const float cq = sq > NORM_EPS2 ? dq_ * rq * rq : 0.f;
+        const float ck = sk > NORM_EPS2 ? dk_ * rk * rk : 0.f;
+        if (onk) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) gq[i] = (gq[i] - q[i] * cq) * rq, gk[i] = (gk[i] - k[i] * ck) * rk;
+            row_st8<DT>(a.dq_raw, qrow * K + e0, gq);
+            row_st8<DT>(a.dk_raw, qrow * K + e0, gk);
+        }
+    }
+}
+
+template <int DT, int LPR>
+__global__ void __launch_bounds__(256, 4) layer_epilogue_fwd16_kernel(const palimpsa_layer_epilogue a, int rows) {
+    constexpr int RPW = 32 / LPR;
+    const int lane = threadIdx.x & 31, e0 = 8 * (lane % LPR), sub = lane / LPR;
+    const int warp0 = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int nwarps = gridDim.x * (blockDim.x >> 5);
+    const int V = a.V, H = a.H;
+    const bool res = a.flags & PALIMPSA_LAYER_RESIDUAL, gated = a.flags & PALIMPSA_LAYER_GATE;
+    float wv[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) wv[i] = e0 + i < V ? a.weight[e0 + i] : 0.f;
+    for (long long base = (long long)warp0 * RPW; base < rows; base += (long long)nwarps * RPW) {
+        const long long row = base + sub;
+        const bool on = row < rows && e0 < V;
+        const long long o = row * V + e0;
+        const uint4 zu = row_ld8(a.o, o, on), xu = row_ld8(a.x, o, on && res), gu = row_ld8(a.gate, o, on && gated);
+        const float d = (res && row < rows) ? a.D[(int)row % H] : 0.f;
+        float z[8], x[8];
+        unpack8<DT>(zu, z);
+        unpack8<DT>(xu, x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) z[i] = x[i] * d + z[i];
+        const float rstd = rsqrtf(row_sum<LPR>(dot8(z, z)) / (float)V + a.eps);
+        if (on) {
+            unpack8<DT>(gu, x);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                z[i] = z[i] * rstd * wv[i];
+                if (gated) z[i] *= x[i] * sigmoidf_(x[i]);
+            }
+            row_st8<DT>(a.y, o, z);
+        }
+    }
+}
+
+template <int DT, int LPR>
+__global__ void __launch_bounds__(256, 3) layer_epilogue_bwd16_kernel(const palimpsa_layer_epilogue a, int rows, float* w_dD,
+                                                                      float* w_dw) {
+    constexpr int RPW = 32 / LPR;
+    __shared__ float red[8 * RPW][LPR * 8 + 1];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, e0 = 8 * (lane % LPR), sub = lane / LPR;
+    const int warp0 = blockIdx.x * 8 + wid;
+    const int nwarps = gridDim.x * 8;
+    const int V = a.V, H = a.H;
+    const bool res = a.flags & PALIMPSA_LAYER_RESIDUAL, gated = a.flags & PALIMPSA_LAYER_GATE;
+    float dw[8], wv[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) dw[i] = 0.f, wv[i] = e0 + i < V ? a.weight[e0 + i] : 0.f;
+    for (long long base = (long long)warp0 * RPW; base < rows; base += (long long)nwarps * RPW) {
+        const long long row = base + sub;
+        const bool ok = row < rows, on = ok && e0 < V;
+        const long long o = row * V + e0;
+        const uint4 zu = row_ld8(a.o, o, on), dyu = row_ld8(a.dy, o, on);
+        const uint4 xu = row_ld8(a.x, o, on && res), gu = row_ld8(a.gate, o, on && gated);
+        const float d = (res && ok) ? a.D[(int)row % H] : 0.f;
+        float z[8], x[8], dy[8];
+        unpack8<DT>(zu, z);
+        unpack8<DT>(xu, x);
+        unpack8<DT>(dyu, dy);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) z[i] = x[i] * d + z[i];
+        const float rstd = rsqrtf(row_sum<LPR>(dot8(z, z)) / (float)V + a.eps);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) z[i] *= rstd;  // xh
+        if (gated) {
+            float g[8], dg[8];
+            unpack8<DT>(gu, g);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float sg = sigmoidf_(g[i]);
+                dg[i] = dy[i] * z[i] * wv[i] * (sg + g[i] * sg * (1.f - sg));
+                dy[i] *= g[i] * sg;  // dyn
+            }
+            if (on) row_st8<DT>(a.dgate, o, dg);
+        }
+        float c1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            dw[i] += dy[i] * z[i];
+            dy[i] *= wv[i];  // dxh
+            c1 += dy[i] * z[i];
+        }
+        c1 = row_sum<LPR>(c1) / (float)V;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) dy[i] = (dy[i] - z[i] * c1) * rstd;  // dz
+        if (on) row_st8<DT>(a.d_o, o, dy);
+        if (res) {
+            const float dd = row_sum<LPR>(dot8(dy, x));
+            if (ok && e0 == 0) w_dD[row] = dd;
+            if (on) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) dy[i] *= d;
+                row_st8<DT>(a.dx, o, dy);
+            }
+        }
+    }
+    // this CTA's share of dweight: its warps' rows summed in order, one partial row per CTA
+#pragma unroll
+    for (int i = 0; i < 8; ++i) red[wid * RPW + sub][e0 + i] = dw[i];
+    __syncthreads();
+    for (int v = threadIdx.x; v < V; v += 256) {
+        float t = 0.f;
+#pragma unroll
+        for (int x = 0; x < 8 * RPW; ++x) t += red[x][v];
+        w_dw[(long long)blockIdx.x * V + v] = t;
+    }
+}
+
 }  // namespace
 
 // -------------------------------------------------------------------------------------------------
@@ -606,6 +904,13 @@ int check_epi(const palimpsa_layer_epilogue* a, bool bwd) {
         return PALIMPSA_E_WORKSPACE;
     return PALIMPSA_OK;
 }
+// Rows of n 16-bit elements, 8 to a lane: lanes a row (0: the kernels that give a row a warp).
+int row_lanes16(int dt, int n, std::initializer_list<const void*> ptrs) {
+    if (dt == PALIMPSA_F32 || n % 8 || n > 128) return 0;
+    for (const void* p : ptrs)
+        if (reinterpret_cast<uintptr_t>(p) & 15) return 0;
+    return n <= 64 ? 8 : 16;
+}
 int launched() { return cudaGetLastError() == cudaSuccess ? PALIMPSA_OK : PALIMPSA_E_LAUNCH; }
 
 // ---- dispatch on (dtype, chunks per lane, vector path) -----------------------------------------------------
@@ -664,6 +969,11 @@ unsigned epi_bwd_launch(const palimpsa_layer_epilogue& a, int rows, bool vecv, f
     return nb;
 }
 
+#define PALIMPSA_ROWS16(dt, lanes, CALL)                                                            \
+    do {                                                                                            \
+        if ((dt) == PALIMPSA_BF16) { if ((lanes) == 8) CALL(PALIMPSA_BF16, 8); else CALL(PALIMPSA_BF16, 16); } \
+        else { if ((lanes) == 8) CALL(PALIMPSA_F16, 8); else CALL(PALIMPSA_F16, 16); }              \
+    } while (0)
 #define PALIMPSA_BY_DTYPE(dt, CALL)                                   \
     do {                                                              \
         if ((dt) == PALIMPSA_BF16) { CALL(PALIMPSA_BF16); }           \
@@ -697,6 +1007,19 @@ int palimpsa_layer_prologue_fwd(const palimpsa_layer_prologue* a, void* cuda_str
     if (rows == 0) return PALIMPSA_OK;
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
     const int dt = a->io_dtype;
+    const int lk = row_lanes16(dt, a->K, {a->q_raw, a->k_raw, a->q, a->k}), lv = row_lanes16(dt, a->V, {a->x, a->b_raw, a->v, a->b});
+    if (lk && lv) {
+        const int lanes = lk > lv ? lk : lv, rpw = 32 / lanes;
+        const size_t sm = (size_t)a->H * sizeof(float);
+#define CALL16(D, N)                                                                                         \
+    do {                                                                                                     \
+        auto kern = layer_prologue_fwd16_kernel<D, N>;                                                       \
+        kern<<<row_blocks(kern, ((long long)rows + rpw - 1) / rpw, sm, 2), 256, sm, st>>>(*a, rows);         \
+    } while (0)
+        PALIMPSA_ROWS16(dt, lanes, CALL16);
+#undef CALL16
+        return launched();
+    }
     const bool veck = a->K % 4 == 0 && aligned_for(a->q_raw, dt) && aligned_for(a->k_raw, dt) && aligned_for(a->q, dt) &&
                       aligned_for(a->k, dt);
     const bool vecv = a->V % 4 == 0 && aligned_for(a->x, dt) && aligned_for(a->b_raw, dt) && aligned_for(a->v, dt) &&
@@ -726,6 +1049,19 @@ int palimpsa_layer_prologue_bwd(const palimpsa_layer_prologue* a, void* cuda_str
     float* w_bsc = w_dtb + rows;
     if (rows > 0) {
         const int dt = a->io_dtype;
+        const int lk = row_lanes16(dt, a->K, {a->q_raw, a->k_raw, a->dq, a->dk, a->dq_raw, a->dk_raw});
+        const int lv = row_lanes16(dt, a->V, {a->x, a->b_raw, a->dv, a->db, a->dx, a->db_raw});
+        if (lk && lv) {
+            const int lanes = lk > lv ? lk : lv, rpw = 32 / lanes;
+            const size_t sm = 2 * (size_t)a->H * sizeof(float);
+#define CALL16(D, N)                                                                                                       \
+    do {                                                                                                                   \
+        auto kern = layer_prologue_bwd16_kernel<D, N>;                                                                     \
+        kern<<<row_blocks(kern, ((long long)qrows + rpw - 1) / rpw, sm, 2), 256, sm, st>>>(*a, qrows, w_dtb, w_bsc);       \
+    } while (0)
+            PALIMPSA_ROWS16(dt, lanes, CALL16);
+#undef CALL16
+        } else {
         const bool veck = a->K % 4 == 0 && aligned_for(a->q_raw, dt) && aligned_for(a->k_raw, dt) &&
                           aligned_for(a->dq, dt) && aligned_for(a->dk, dt) && aligned_for(a->dq_raw, dt) &&
                           aligned_for(a->dk_raw, dt);
@@ -745,6 +1081,7 @@ int palimpsa_layer_prologue_bwd(const palimpsa_layer_prologue* a, void* cuda_str
         PALIMPSA_BY_DTYPE(dt, CALL_D);
 #undef CALL_D
 #undef CALL_V
+        }
         if (int rc = launched()) return rc;
     }
     layer_sum_heads_kernel<<<dim3(a->H, 2), 1024, 0, st>>>(w_dtb, a->d_dt_bias, w_bsc, a->d_b_scale, a->tokens, a->H);
@@ -757,6 +1094,18 @@ int palimpsa_layer_epilogue_fwd(const palimpsa_layer_epilogue* a, void* cuda_str
     if (rows == 0) return PALIMPSA_OK;
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
     const int dt = a->io_dtype;
+    const bool res = a->flags & PALIMPSA_LAYER_RESIDUAL, gated = a->flags & PALIMPSA_LAYER_GATE;
+    if (const int lanes = row_lanes16(dt, a->V, {a->o, a->y, res ? a->x : nullptr, gated ? a->gate : nullptr})) {
+        const int rpw = 32 / lanes;
+#define CALL16(D, N)                                                                                       \
+    do {                                                                                                   \
+        auto kern = layer_epilogue_fwd16_kernel<D, N>;                                                     \
+        kern<<<row_blocks(kern, ((long long)rows + rpw - 1) / rpw, 0, 2), 256, 0, st>>>(*a, rows);         \
+    } while (0)
+        PALIMPSA_ROWS16(dt, lanes, CALL16);
+#undef CALL16
+        return launched();
+    }
     const bool vecv = a->V % 4 == 0 && aligned_for(a->o, dt) && aligned_for(a->y, dt) &&
                       (!(a->flags & PALIMPSA_LAYER_RESIDUAL) || aligned_for(a->x, dt)) &&
                       (!(a->flags & PALIMPSA_LAYER_GATE) || aligned_for(a->gate, dt));
@@ -784,6 +1133,18 @@ int palimpsa_layer_epilogue_bwd(const palimpsa_layer_epilogue* a, void* cuda_str
     unsigned nb = 0;
     if (rows > 0) {
         const int dt = a->io_dtype;
+        if (const int lanes = row_lanes16(dt, a->V, {a->o, a->dy, a->d_o, res ? a->x : nullptr, res ? a->dx : nullptr,
+                                                     gated ? a->gate : nullptr, gated ? a->dgate : nullptr})) {
+            const int rpw = 32 / lanes;
+#define CALL16(D, N)                                                                               \
+    do {                                                                                           \
+        auto kern = layer_epilogue_bwd16_kernel<D, N>;                                             \
+        nb = row_blocks(kern, ((long long)rows + rpw - 1) / rpw, 0, 1, DW_CTAS);                   \
+        kern<<<nb, 256, 0, st>>>(*a, rows, w_dD, w_dw);                                            \
+    } while (0)
+            PALIMPSA_ROWS16(dt, lanes, CALL16);
+#undef CALL16
+        } else {
         const bool vecv = a->V % 4 == 0 && aligned_for(a->o, dt) && aligned_for(a->dy, dt) && aligned_for(a->d_o, dt) &&
                           (!res || (aligned_for(a->x, dt) && aligned_for(a->dx, dt))) &&
                           (!gated || (aligned_for(a->gate, dt) && aligned_for(a->dgate, dt)));
@@ -796,6 +1157,7 @@ int palimpsa_layer_epilogue_bwd(const palimpsa_layer_epilogue* a, void* cuda_str
         PALIMPSA_BY_DTYPE(dt, CALL_D);
 #undef CALL_D
 #undef CALL_V
+        }
         if (int rc = launched()) return rc;
     }
     const int nh = res ? a->H : 0;
