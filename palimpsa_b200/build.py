@@ -22,7 +22,7 @@ EXT = os.path.join(PKG, "_torch_ops" + sysconfig.get_config_var("EXT_SUFFIX"))
 EXT_STAMP = os.path.join(PKG, "_torch_ops.built_for")      # the torch version EXT was compiled and linked against
 EXT_SOURCE = os.path.join(CSRC, "torch_ops.cpp")
 HEADER = os.path.join(ROOT, "include", "palimpsa_b200.h")
-UNITS = ("abi", "fwd", "bwd", "decode", "segments", "summary_tc", "carry_tc", "layer", "peer")
+UNITS = ("abi", "fwd", "fwd_tall", "bwd", "decode", "segments", "summary_tc", "carry_tc", "layer", "peer")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--extended-lambda",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
 

@@ -197,8 +197,9 @@ int palimpsa_segment_summary(const palimpsa_problem* p, const palimpsa_segments*
 
 int palimpsa_tensor_core_status(void) {
     if (cudaDeviceSynchronize() != cudaSuccess) return -1;
-    const int a = summary_tc_status(), b = carry_tc_status(), c = bwd_wait_status(), d = peer_status();  // each clears what it read
-    return a ? a : (b ? b : (c ? c : d));
+    const int a = summary_tc_status(), b = carry_tc_status(), c = bwd_wait_status(), d = peer_status(),
+              e = fwd_wait_status();  // each clears what it read
+    return a ? a : (b ? b : (c ? c : (d ? d : e)));
 }
 
 int palimpsa_peer_wait(const void* flag, unsigned long long value, unsigned int timeout_ms, float* poison, void* cuda_stream) {

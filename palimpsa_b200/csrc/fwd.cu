@@ -23,27 +23,9 @@
 // chunk_palimpsa_fwd_kernel (chunk_palimpsa_forgetting_scalar.py:66-218) and
 // fused_palimpsa_recurrent_fwd_kernel (fused_recurrent_palimpsa.py:24-154).
 #include "common.cuh"
-#include "host.h"
+#include "fwd.h"
 
 namespace palimpsa {
-
-struct FwdArgs {
-    palimpsa_problem p;
-    void* o;
-    void* o_var;
-    float* final_mu;
-    float* final_I;
-    float* ckpt_M;
-    float* ckpt_I;
-    int aligned;  // 1: every io row is 16-byte aligned and a multiple of 16 bytes
-    // segments (gridDim.z of them per sequence; seg_len tokens each, a multiple of 16)
-    int seg_len;
-    const float* start_M;  // [N,G,H,V,KP] (M, I) at the start of every segment, or NULL
-    const float* start_I;
-    float* sum_M;          // summary mode: [N,G,H,V,KP] end state of the segment started from zero, (M, J) form
-    float* sum_J;
-    float* decay;          // summary mode: [N,G,H] product of f over the segment
-};
 
 struct FwdSmem {
     int qs, ks, qqs, vs, bs, fc, ys, yvs;  // fp32 operand / result buffers (byte offsets)
@@ -598,6 +580,11 @@ int launch_fwd(const palimpsa_fwd_params* prm, const palimpsa_segments* segs, bo
     a.aligned = ((p.K * es) % 16 == 0) && ((p.V * es) % 16 == 0) && aligned16(p.q) && aligned16(p.k) &&
                 aligned16(p.v) && aligned16(p.b) && ((reinterpret_cast<uintptr_t>(p.gt) & 3) == 0);
     const int KP = palimpsa_padded_k(p.K);
+    int elements = 0;
+#define PALIMPSA_X(RK, KG, RV, WMAX) elements = RK * RV; break
+    PALIMPSA_FWD_TILINGS(PALIMPSA_X)
+#undef PALIMPSA_X
+    if (!summary && fwd_tall_pays(p, num_seg, fwd_tile_rows(p.K, p.V), elements)) return launch_fwd_tall(a, num_seg, stream);
 #define PALIMPSA_X(RK, KG, RV, WMAX) return launch_fwd_t<RK, KG, RV, WMAX>(a, num_seg, summary, stream)
     PALIMPSA_FWD_TILINGS(PALIMPSA_X)
 #undef PALIMPSA_X

@@ -1,0 +1,558 @@
+// Forward kernel of the Palimpsa operator for tall row tiles (sm_100a): one CTA per SM.
+//
+// fwd.cu's kernel runs CTAs of at most 4 warps, several per SM, each of which converts the q and k rows of its head for
+// itself, between two CTA barriers per 16 tokens.  Here up to 12 compute warps share one tile: a block's operands are
+// converted once per SM, by helper warps, one block ahead of the walk, and the compute warps meet no barrier: they wait for
+// the staged block (an mbarrier), walk its 16 tokens with the state in registers, and hand the reduced outputs back the same
+// way.  What bounds it is the issue rate: a packed FP32 instruction takes two issue cycles (2.05 measured for FMUL2, 2.3 for
+// FFMA2 with a shared operand), so a pair of state elements takes 14 of them per token, its two reciprocals 16 of the MUFU
+// pipe, and the rest of a token (operand loads, the sums over a row's lanes) must stay small against 6 or 8 pairs.
+// Forward with checkpoints, ms, fwd.cu's kernel -> this one: B=8 T=4096 H=6 d=128 1.49 -> 1.25, H=16 d=48 1.11 -> 0.86, 48x96
+// 1.51 -> 1.21, B=4 H=16 96x192 2.62 -> 2.09; without: B=2 T=3001 H=16 96x192 1.07 -> 0.75.
+//
+//   thread layout   lane = vg*KG + kg, as in fwd.cu: RV rows x RK columns, interleaved float4 column groups.
+//   blocks          16 tokens; tokens past the end are staged as identity steps (f = 1, all else 0), so that the walk has
+//                   no conditionals.
+//   warps without rows (a tile lower than 12 warps hold) only keep the hand-overs going.
+#include <cmath>
+
+#include "common.cuh"
+#include "fwd.h"
+#include "tc_common.cuh"
+
+namespace palimpsa {
+
+// 0 ok; 8: a bounded wait of the tall-tile forward gave up
+__device__ int g_fwd_status = 0;
+
+constexpr int FT_W = 12, FT_HW = 4, FT_NTHR = 32 * FT_W, FT_HT = 32 * FT_HW;
+
+struct TallSmem {
+    int qs, ks, qqs, vb, fc, op_stage;  // offsets inside an operand stage; two stages from 0
+    int ys, yvs, y_stage;               // reduced outputs, two stages
+    int bars;                           // staged[2], done[2]; failure flag
+    int raw, rq, rk, rv, rb, rgt;
+    int total;
+};
+
+// v and b of a row lie side by side, each value twice: one 128-bit load yields both packed operands.
+__host__ __device__ inline TallSmem tall_smem_layout(int KP, int TV, int es, bool unc) {
+    TallSmem s;
+    int off = 0;
+    auto take = [&](int bytes) {
+        int o = off;
+        off += round_up(bytes, 16);
+        return o;
+    };
+    s.qs = take(TB * KP * 4);
+    s.ks = take(TB * KP * 4);
+    s.qqs = unc ? take(TB * KP * 4) : 0;
+    s.vb = take(TB * TV * 16);
+    s.fc = take(TB * 16);  // {f, f, c, c}
+    s.op_stage = off;
+    off *= 2;
+    s.ys = off;
+    s.yvs = s.ys + TB * TV * 4;
+    s.y_stage = TB * TV * 4 * (unc ? 2 : 1);
+    off += 2 * s.y_stage;
+    s.bars = take(48);
+    s.raw = off;
+    int r = 0;
+    auto rtake = [&](int bytes) {
+        int o = r;
+        r += round_up(bytes, 16);
+        return o;
+    };
+    s.rq = rtake(TB * KP * es);
+    s.rk = rtake(TB * KP * es);
+    s.rv = rtake(TB * TV * es);
+    s.rb = rtake(TB * TV * es);
+    s.rgt = rtake(TB * 4);
+    s.total = off + r;
+    return s;
+}
+
+// Asynchronous copies of one block of nt tokens by the helper warps (aligned rows only).
+__device__ __forceinline__ void tall_issue(const FwdArgs& a, int ht, unsigned char* stage, const TallSmem& L, int es, int KP,
+                                           int TV, long long tok0, int nt, int h, int v0, int tvw) {
+    const palimpsa_problem& p = a.p;
+    const int cq = p.K * es / 16, cv = tvw * es / 16;
+    const char* gq = reinterpret_cast<const char*>(p.q);
+    const char* gk = reinterpret_cast<const char*>(p.k);
+    const char* gv = reinterpret_cast<const char*>(p.v);
+    const char* gb = reinterpret_cast<const char*>(p.b);
+    for (int i = ht; i < nt; i += FT_HT) cp_async4(stage + L.rgt + i * 4, p.gt + (tok0 + i) * p.H + h);
+    for (int i = ht; i < nt * cq; i += FT_HT) {
+        const int t = i / cq, c = i - t * cq;
+        const long long src = ((tok0 + t) * p.H + h) * (long long)p.K * es + c * 16;
+        const int dst = t * KP * es + c * 16;
+        cp_async16(stage + L.rq + dst, gq + src);
+        cp_async16(stage + L.rk + dst, gk + src);
+    }
+    for (int i = ht; i < nt * cv; i += FT_HT) {
+        const int t = i / cv, c = i - t * cv;
+        const long long src = (((tok0 + t) * p.H + h) * (long long)p.V + v0) * es + c * 16;
+        const int dst = t * TV * es + c * 16;
+        cp_async16(stage + L.rv + dst, gv + src);
+        cp_async16(stage + L.rb + dst, gb + src);
+    }
+}
+
+// One block of fp32 operands, by the helper warps.  ALIGNED: from the raw stage; otherwise element by element from global
+// memory (any K, V, alignment).
+template <int DT, bool ALIGNED, bool UNC, int KP, int TV>
+__device__ __forceinline__ void tall_convert(const FwdArgs& a, int ht, const unsigned char* raw, unsigned char* op,
+                                             const TallSmem& L, long long tok0, int nt, int h, int v0, int tvw, float gh,
+                                             float iph) {
+    const palimpsa_problem& p = a.p;
+    constexpr int K4 = KP / 4, V4 = TV / 4;
+    float4* qs = reinterpret_cast<float4*>(op + L.qs);
+    float4* ks = reinterpret_cast<float4*>(op + L.ks);
+    float4* qqs = reinterpret_cast<float4*>(op + L.qqs);
+    const float sc = p.scale;
+#pragma unroll 2
+    for (int i = ht; i < TB * K4; i += FT_HT) {
+        const int t = i / K4, c4 = i - t * K4;
+        float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), kv = qv;
+        if (t < nt && c4 * 4 < p.K) {
+            if (ALIGNED) {
+                qv = ld4<DT>(raw + L.rq, i);
+                kv = ld4<DT>(raw + L.rk, i);
+            } else {
+                const long long row = ((tok0 + t) * p.H + h) * (long long)p.K;
+                qv = ld4_guarded<DT>(p.q, row + c4 * 4, row + p.K);
+                kv = ld4_guarded<DT>(p.k, row + c4 * 4, row + p.K);
+            }
+        }
+        qs[i] = make_float4(qv.x * sc, qv.y * sc, qv.z * sc, qv.w * sc);
+        ks[i] = kv;
+        if (UNC) qqs[i] = make_float4(sc * qv.x * qv.x, sc * qv.y * qv.y, sc * qv.z * qv.z, sc * qv.w * qv.w);
+    }
+    float4* vb = reinterpret_cast<float4*>(op + L.vb);
+#pragma unroll 2
+    for (int i = ht; i < TB * V4; i += FT_HT) {
+        const int t = i / V4, r = 4 * (i - t * V4);
+        if (r >= tvw) continue;  // rows past the tile belong to idle warps, or are never written out
+        float4 vv = make_float4(0.f, 0.f, 0.f, 0.f), bv = vv;
+        if (t < nt) {
+            if (ALIGNED) {
+                vv = ld4<DT>(raw + L.rv, i);
+                bv = ld4<DT>(raw + L.rb, i);
+            } else {
+                const long long row = ((tok0 + t) * p.H + h) * (long long)p.V + v0;
+                vv = ld4_guarded<DT>(p.v, row + r, row + tvw);
+                bv = ld4_guarded<DT>(p.b, row + r, row + tvw);
+            }
+        }
+        vb[4 * i] = make_float4(vv.x, vv.x, bv.x, bv.x);
+        vb[4 * i + 1] = make_float4(vv.y, vv.y, bv.y, bv.y);
+        vb[4 * i + 2] = make_float4(vv.z, vv.z, bv.z, bv.z);
+        vb[4 * i + 3] = make_float4(vv.w, vv.w, bv.w, bv.w);
+    }
+    float4* fc = reinterpret_cast<float4*>(op + L.fc);
+    for (int i = ht; i < TB; i += FT_HT) {
+        float f = 1.f, c = 0.f;
+        if (i < nt) {
+            const float gtv = ALIGNED ? reinterpret_cast<const float*>(raw + L.rgt)[i] : p.gt[(tok0 + i) * p.H + h];
+            f = expf(-gtv * gh);
+            c = (1.f - f) * iph;
+        }
+        fc[i] = make_float4(f, f, c, c);
+    }
+}
+
+// Tokens whose outputs are summed together over a row's lanes: as many as give each of the KG lanes one sum, 4 to 8.
+template <int KG, int RV, bool UNC>
+__host__ __device__ constexpr int tall_group() {
+    constexpr int g = KG / (RV * (UNC ? 2 : 1));
+    return g < 8 ? 4 : 8;
+}
+
+template <int RK, int KG, int RV, bool UNC>
+__global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdArgs a, const int rows) {
+    constexpr int KP = RK * KG, VG = 32 / KG, J4 = RK / 4, TV = FT_W * VG * RV, GF = tall_group<KG, RV, UNC>();
+    constexpr int NRED = GF * RV * (UNC ? 2 : 1);
+    static_assert(TV % 4 == 0 && TB % GF == 0, "operands are converted four rows at a time, blocks are whole groups");
+    extern __shared__ __align__(16) unsigned char sm[];
+    const palimpsa_problem& p = a.p;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int kg = lane % KG, vg = lane / KG;
+    const int row0 = (w * VG + vg) * RV;
+    const int ny = blockIdx.y / p.H, h = blockIdx.y - ny * p.H;
+    const int n = p.seq_order ? p.seq_order[ny] : ny;  // blocks start in grid order: a packed batch lists its longest sequences first
+    const int v0 = blockIdx.x * rows;
+    const int tvw = min(rows, p.V - v0);
+    const int es = dtype_size(p.io_dtype);
+    const TallSmem L = tall_smem_layout(KP, TV, es, UNC);
+    int bos, len;
+    seq_range(p, n, bos, len);
+    const float gh = p.g[h], iph = p.Ip[h];
+    const int K = p.K, V = p.V;
+    const bool vecK = (K % 4) == 0;
+    // this CTA's segment of the sequence: tokens [s0, s1)
+    const int g = blockIdx.z, G = gridDim.z;
+    const int s0 = a.seg_len > 0 ? min(len, g * a.seg_len) : 0;
+    const int s1 = a.seg_len > 0 ? min(len, s0 + a.seg_len) : len;
+    const int blk0 = s0 / TB, nblk = s1 > s0 ? (s1 + TB - 1) / TB - blk0 : 0;
+
+    // staged[s] / done[s], s = block & 1: its operands lie in shared memory (one arrival per helper warp); the compute warps
+    // are through with it and its outputs lie in shared memory (one per compute warp).  All waits are bounded.
+    unsigned long long* staged = reinterpret_cast<unsigned long long*>(sm + L.bars);
+    unsigned long long* done = staged + 2;
+    int* fail_flag = reinterpret_cast<int*>(staged + 4);
+    int wait_fail = 0;
+    if (tid == 0) {
+        for (int s = 0; s < 2; ++s) {
+            mbar_init_n(&staged[s], FT_HW);
+            mbar_init_n(&done[s], FT_W);
+        }
+        *fail_flag = 0;
+        tc::mbar_init_fence();
+    }
+    __syncthreads();
+
+    if (w >= FT_W) {
+        // ---- helper warps: operands one block ahead of the walk, outputs one block behind it ----------------------
+        const int ht = tid - FT_NTHR;
+        unsigned char* raw = sm + L.raw;
+        auto tokens = [&](int it) __attribute__((always_inline)) { return min(TB, s1 - (blk0 + it) * TB); };
+        auto token0 = [&](int it) __attribute__((always_inline)) { return (long long)bos + (blk0 + it) * TB; };
+        auto issue = [&](int it) __attribute__((always_inline)) {
+            if (a.aligned && it < nblk) tall_issue(a, ht, raw, L, es, KP, TV, token0(it), tokens(it), h, v0, tvw);
+            cp_async_commit();
+        };
+        auto bar_helpers = [&]() __attribute__((always_inline)) { asm volatile("bar.sync 1, %0;" ::"n"(FT_HT) : "memory"); };
+        auto convert = [&](int it) __attribute__((always_inline)) {
+            cp_async_wait<0>();
+            bar_helpers();  // every lane's copies have landed
+            unsigned char* op = sm + (it & 1) * L.op_stage;
+#define PALIMPSA_CONVERT(DT, AL) \
+    tall_convert<DT, AL, UNC, KP, TV>(a, ht, raw, op, L, token0(it), tokens(it), h, v0, tvw, gh, iph)
+            if (a.aligned) {
+                if (p.io_dtype == PALIMPSA_BF16) PALIMPSA_CONVERT(PALIMPSA_BF16, true);
+                else if (p.io_dtype == PALIMPSA_F32) PALIMPSA_CONVERT(PALIMPSA_F32, true);
+                else PALIMPSA_CONVERT(PALIMPSA_F16, true);
+            } else {
+                if (p.io_dtype == PALIMPSA_BF16) PALIMPSA_CONVERT(PALIMPSA_BF16, false);
+                else if (p.io_dtype == PALIMPSA_F32) PALIMPSA_CONVERT(PALIMPSA_F32, false);
+                else PALIMPSA_CONVERT(PALIMPSA_F16, false);
+            }
+#undef PALIMPSA_CONVERT
+            bar_helpers();  // the raw stage has been read
+            issue(it + 1);
+        };
+        auto arrive = [&](int it) __attribute__((always_inline)) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&staged[it & 1]);
+        };
+        auto wait_done = [&](int it) __attribute__((always_inline)) {
+            if (!wait_fail && !mbar_wait_idle(&done[it & 1], (it >> 1) & 1)) wait_fail = 8;
+        };
+        auto write_outputs = [&](int it) __attribute__((always_inline)) {
+            const float* ys = reinterpret_cast<const float*>(sm + L.ys + (it & 1) * L.y_stage);
+            const float* yvs = reinterpret_cast<const float*>(sm + L.yvs + (it & 1) * L.y_stage);
+            const long long tok0 = token0(it);
+            const int nt = tokens(it);
+            const float bad = __int_as_float(0x7fc00000);  // a wait ran out: nothing after it is valid
+            for (int i = ht; i < nt * TV; i += FT_HT) {
+                const int t = i / TV, r = i - t * TV;
+                if (r < tvw) {
+                    const long long e = ((tok0 + t) * p.H + h) * (long long)V + v0 + r;
+                    st1(a.o, e, wait_fail ? bad : ys[i], p.io_dtype);
+                    if (UNC) st1(a.o_var, e, wait_fail ? bad : yvs[i], p.io_dtype);
+                }
+            }
+        };
+        issue(0);
+        if (nblk > 0) {
+            convert(0);
+            arrive(0);
+        }
+        for (int it = 0; it < nblk; ++it) {
+            if (it > 0) wait_done(it - 1);  // frees the operand stage of block it + 1
+            if (it + 1 < nblk) convert(it + 1);
+            if (it > 0) write_outputs(it - 1);  // before the block that reuses their stage is released
+            if (it + 1 < nblk) arrive(it + 1);
+        }
+        if (nblk > 0) {
+            wait_done(nblk - 1);
+            write_outputs(nblk - 1);
+        }
+        cp_async_wait<0>();
+        if (wait_fail) *fail_flag = wait_fail;
+        __syncthreads();
+        if (ht == 0 && *fail_flag) atomicCAS(&g_fwd_status, 0, *fail_flag);
+        return;
+    }
+
+    // ---- compute warps ---------------------------------------------------------------------------------------------
+    const bool idle = w * VG * RV >= tvw;
+    const long long seg_base = (((long long)n * G + g) * p.H + h) * V;  // row index into [N,G,H,V,KP] buffers
+    const long long st_base = ((long long)n * p.H + h) * V;
+    const long long slot0 = seq_first_slot(p, n);
+    float2 M[RV][J4][2], I[RV][J4][2];
+#pragma unroll
+    for (int r = 0; r < RV; ++r) {
+        const int row = row0 + r;
+#pragma unroll
+        for (int j = 0; j < J4; ++j) {
+            const int kc = 4 * (j * KG + kg);
+            float4 m4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 i4 = make_float4(1.f, 1.f, 1.f, 1.f);
+            if (row < tvw) {
+                if (a.start_M) {
+                    const long long e = (seg_base + v0 + row) * KP + kc;
+                    m4 = *reinterpret_cast<const float4*>(a.start_M + e);
+                    i4 = *reinterpret_cast<const float4*>(a.start_I + e);
+                } else if (kc < K) {
+                    if (p.init_mu) {
+                        const long long e = (st_base + v0 + row) * K + kc;
+                        float4 mu4;
+                        if (vecK) {
+                            mu4 = *reinterpret_cast<const float4*>(p.init_mu + e);
+                            i4 = *reinterpret_cast<const float4*>(p.init_I + e);
+                        } else {
+                            const long long lim = (st_base + v0 + row + 1) * K;
+                            mu4 = ld4_guarded<PALIMPSA_F32>(p.init_mu, e, lim);
+                            i4 = ld4_guarded<PALIMPSA_F32>(p.init_I, e, lim);
+                            if (kc + 1 >= K) i4.y = 1.f;
+                            if (kc + 2 >= K) i4.z = 1.f;
+                            if (kc + 3 >= K) i4.w = 1.f;
+                        }
+                        m4 = make_float4(mu4.x * i4.x, mu4.y * i4.y, mu4.z * i4.z, mu4.w * i4.w);
+                    } else {
+                        i4 = make_float4(iph, iph, iph, iph);
+                    }
+                }
+            }
+            M[r][j][0] = make_float2(m4.x, m4.y);
+            M[r][j][1] = make_float2(m4.z, m4.w);
+            I[r][j][0] = make_float2(i4.x, i4.y);
+            I[r][j][1] = make_float2(i4.z, i4.w);
+        }
+    }
+    for (int it = 0; it < nblk; ++it) {
+        if (idle) {
+            if (!wait_fail && !mbar_wait_idle(&staged[it & 1], (it >> 1) & 1)) wait_fail = 8;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&done[it & 1]);
+            continue;
+        }
+        // ---- checkpoint: state before the first token of this block ---------------------------------------------
+        if (a.ckpt_M) {
+            const long long cbase = ((slot0 + blk0 + it) * p.H + h) * V + v0;
+#pragma unroll
+            for (int r = 0; r < RV; ++r) {
+                if (row0 + r < tvw) {
+#pragma unroll
+                    for (int j = 0; j < J4; ++j) {
+                        const long long e = (cbase + row0 + r) * KP + 4 * (j * KG + kg);
+                        *reinterpret_cast<float4*>(a.ckpt_M + e) =
+                            make_float4(M[r][j][0].x, M[r][j][0].y, M[r][j][1].x, M[r][j][1].y);
+                        *reinterpret_cast<float4*>(a.ckpt_I + e) =
+                            make_float4(I[r][j][0].x, I[r][j][0].y, I[r][j][1].x, I[r][j][1].y);
+                    }
+                }
+            }
+        }
+        const unsigned char* op = sm + (it & 1) * L.op_stage;
+        const float4* qs4 = reinterpret_cast<const float4*>(op + L.qs) + kg;
+        const float4* ks4 = reinterpret_cast<const float4*>(op + L.ks) + kg;
+        const float4* qqs4 = reinterpret_cast<const float4*>(op + L.qqs) + kg;
+        const float4* vb4 = reinterpret_cast<const float4*>(op + L.vb) + row0;
+        const float4* fc = reinterpret_cast<const float4*>(op + L.fc);
+        float* ys = reinterpret_cast<float*>(sm + L.ys + (it & 1) * L.y_stage);
+        float* yvs = reinterpret_cast<float*>(sm + L.yvs + (it & 1) * L.y_stage);
+        if (!wait_fail && !tc::mbar_wait(&staged[it & 1], (it >> 1) & 1)) {
+            wait_fail = 8;
+            M[0][0][0].x = __int_as_float(0x7fc00000);  // outputs and states from here on are not valid
+        }
+        const int end = min(TB, s1 - (blk0 + it) * TB);
+#pragma unroll 1
+        for (int tg = 0; tg < end; tg += GF) {
+            float red[NRED];
+#pragma unroll
+            for (int jt = 0; jt < GF; ++jt) {
+                const int t = tg + jt;
+                const float4 fcv = fc[t];
+                const float2 ff = make_float2(fcv.x, fcv.y), cc = make_float2(fcv.z, fcv.w);
+                float2 vr[RV], br[RV], acc[RV], accv[RV];
+#pragma unroll
+                for (int r = 0; r < RV; ++r) {
+                    const float4 x = vb4[t * TV + r];
+                    vr[r] = make_float2(x.x, x.y);
+                    br[r] = make_float2(x.z, x.w);
+                    acc[r] = accv[r] = make_float2(0.f, 0.f);
+                }
+#pragma unroll
+                for (int j = 0; j < J4; ++j) {
+                    const int idx = t * (KP / 4) + j * KG;
+                    const float4 k4 = ks4[idx], q4 = qs4[idx];
+                    float4 qq4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (UNC) qq4 = qqs4[idx];
+                    const float2 kp[2] = {make_float2(k4.x, k4.y), make_float2(k4.z, k4.w)};
+                    const float2 kkp[2] = {fmul2(kp[0], kp[0]), fmul2(kp[1], kp[1])};
+                    const float2 qp[2] = {make_float2(q4.x, q4.y), make_float2(q4.z, q4.w)};
+                    const float2 qqp[2] = {make_float2(qq4.x, qq4.y), make_float2(qq4.z, qq4.w)};
+#pragma unroll
+                    for (int r = 0; r < RV; ++r) {
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            M[r][j][e] = ffma2(ff, M[r][j][e], fmul2(vr[r], kp[e]));
+                            I[r][j][e] = ffma2(ff, I[r][j][e], ffma2(br[r], kkp[e], cc));
+                            const float2 rr = rcp2(I[r][j][e]);
+                            acc[r] = ffma2(fmul2(M[r][j][e], rr), qp[e], acc[r]);
+                            if (UNC) accv[r] = ffma2(rr, qqp[e], accv[r]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < RV; ++r) {
+                    red[(jt * RV + r) * (UNC ? 2 : 1)] = acc[r].x + acc[r].y;
+                    if (UNC) red[(jt * RV + r) * 2 + 1] = accv[r].x + accv[r].y;
+                }
+            }
+            xreduce<NRED, KG>(red, lane);
+            const int base = xreduce_index<NRED, KG>(lane), count = xreduce_count<NRED, KG>(lane);
+#pragma unroll
+            for (int i = 0; i < xreduce_most<NRED, KG>(); ++i)
+                if (i < count) {
+                    const int id = base + i, which = UNC ? (id & 1) : 0, jr = UNC ? (id >> 1) : id;
+                    const int jt = jr / RV, r = jr % RV;
+                    (which ? yvs : ys)[(tg + jt) * TV + row0 + r] = red[i];
+                }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&done[it & 1]);
+    }
+    // ---- final state in the API's (mu, I) form: written by the segment that holds the last token -----
+    if (a.final_mu && !idle && s1 == len && (s0 < len || g == 0)) {
+#pragma unroll
+        for (int r = 0; r < RV; ++r) {
+#pragma unroll
+            for (int j = 0; j < J4; ++j) {
+                const int kc = 4 * (j * KG + kg);
+                if (row0 + r < tvw && kc < K) {
+                    const float4 i4 = make_float4(I[r][j][0].x, I[r][j][0].y, I[r][j][1].x, I[r][j][1].y);
+                    const float4 mu4 = make_float4(M[r][j][0].x / i4.x, M[r][j][0].y / i4.y, M[r][j][1].x / i4.z,
+                                                   M[r][j][1].y / i4.w);
+                    const long long e = (st_base + v0 + row0 + r) * K + kc;
+                    if (vecK) {
+                        *reinterpret_cast<float4*>(a.final_mu + e) = mu4;
+                        *reinterpret_cast<float4*>(a.final_I + e) = i4;
+                    } else {
+                        const float mus[4] = {mu4.x, mu4.y, mu4.z, mu4.w};
+                        const float is[4] = {i4.x, i4.y, i4.z, i4.w};
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            if (kc + c < K) {
+                                a.final_mu[e + c] = mus[c];
+                                a.final_I[e + c] = is[c];
+                            }
+                    }
+                }
+            }
+        }
+    }
+    if (wait_fail) *fail_flag = wait_fail;
+    __syncthreads();
+}
+
+// -------------------------------------------------------------------------------------------------
+// Host side
+// -------------------------------------------------------------------------------------------------
+// The thread tilings, one per padded d_k: X(RK, KG, RV), 12 or 16 state elements a thread.
+#define PALIMPSA_TALL_TILINGS(X)       \
+    switch (KP) {                      \
+        case 48: X(12, 4, 1); break;   \
+        case 64: X(16, 4, 1); break;   \
+        case 96: X(12, 8, 1); break;   \
+        case 128: X(8, 16, 2); break;  \
+        case 192: X(12, 16, 1); break; \
+        case 256: X(16, 16, 1); break; \
+        default: break;                \
+    }
+
+struct TallPlan {
+    int rows, tiles;
+    double cost;  // per token of the longest-running SM, cycles
+};
+// Tile height: of all counts of tiles the one that costs least, waves of CTAs (one per SM) times what a token costs a CTA.
+// That is 190 cycles and 8.3 per state element on a scheduler's lanes: measured 588 with 12 warps of 16 elements (48 a
+// lane and scheduler: 48 rows of d_k = 128), 490 with 12 of 12, 455 with 8 of 16, 411 with 6 of 12.
+template <int RK, int KG, int RV>
+static TallPlan tall_plan(const palimpsa_problem& p, int num_seg) {
+    constexpr int RPW = 32 / KG * RV;
+    TallPlan best{0, 0, 0.};
+    const double units = (double)p.num_seqs * p.H * num_seg;
+    for (int n = (p.V + FT_W * RPW - 1) / (FT_W * RPW); n <= (p.V + 7) / 8; ++n) {
+        const int rows = ((p.V + n - 1) / n + 7) / 8 * 8;  // 16-byte rows of 16-bit elements
+        const int tiles = (p.V + rows - 1) / rows, warps = (rows + RPW - 1) / RPW;
+        const double share = units * tiles / B200_SMS;
+        // CTAs of equal sequences finish together; documents fill the waves up, beyond the first few
+        const double waves = p.cu_seqlens && share > 3 ? share : ceil(share);
+        const double cost = waves * (190 + 8.3 * RK * RV * ((warps + 3) / 4));
+        if (!best.rows || cost < best.cost) best = {rows, tiles, cost};
+    }
+    return best;
+}
+
+// fwd.cu's kernel by the same measure: `rows` a tile, `elements` of state a thread.  Its CTAs share an SM: up to four, a token
+// costs 300 cycles and 8.1 per element on a scheduler's lanes, 16 per element beyond 48 (260 and 10.4 where a thread has 32);
+// more run through at 13.6 per element.  Measured: 678 with 3 CTAs of 4 warps of 16, 701 and 1158 with 2 and 3 of 24, 597, 886
+// and 932 with 2, 3 and 4 of 2 warps of 32.
+static double short_cost(const palimpsa_problem& p, int num_seg, int rows, int elements) {
+    const int KP = palimpsa_padded_k(p.K), tiles = (p.V + rows - 1) / rows;
+    const double share = (double)p.num_seqs * p.H * num_seg * tiles / B200_SMS;
+    const int warps = rows * KP / (32 * elements);
+    if (share > 4) return 13.6 * warps / 4. * elements * share;
+    const double load = ceil(ceil(share) * warps / 4) * elements;  // elements on the lanes of the busiest scheduler
+    return elements >= 32 ? 260 + 10.4 * load : load <= 48 ? 300 + 8.1 * load : 16 * load;
+}
+
+bool fwd_tall_pays(const palimpsa_problem& p, int num_seg, int short_rows, int short_elements) {
+    const int KP = palimpsa_padded_k(p.K);
+    TallPlan t{0, 0, 0.};
+#define PALIMPSA_X(RK, KG, RV) t = tall_plan<RK, KG, RV>(p, num_seg)
+    PALIMPSA_TALL_TILINGS(PALIMPSA_X)
+#undef PALIMPSA_X
+    return t.rows && t.cost < 0.96 * short_cost(p, num_seg, short_rows, short_elements);
+}
+
+template <int RK, int KG, int RV>
+static int launch_tall_t(const FwdArgs& a, int num_seg, cudaStream_t stream) {
+    const palimpsa_problem& p = a.p;
+    const TallPlan t = tall_plan<RK, KG, RV>(p, num_seg);
+    const bool unc = (p.flags & PALIMPSA_FLAG_UNCERTAINTY) != 0;
+    const TallSmem L = tall_smem_layout(RK * KG, FT_W * (32 / KG) * RV, dtype_size(p.io_dtype), unc);
+    const dim3 grid(t.tiles, p.num_seqs * p.H, num_seg), block(FT_NTHR + FT_HT, 1, 1);
+    if (unc) {
+        if (!allow_smem<fwd_tall_kernel<RK, KG, RV, true>>(L.total)) return PALIMPSA_E_LAUNCH;
+        fwd_tall_kernel<RK, KG, RV, true><<<grid, block, L.total, stream>>>(a, t.rows);
+    } else {
+        if (!allow_smem<fwd_tall_kernel<RK, KG, RV, false>>(L.total)) return PALIMPSA_E_LAUNCH;
+        fwd_tall_kernel<RK, KG, RV, false><<<grid, block, L.total, stream>>>(a, t.rows);
+    }
+    return cudaGetLastError() == cudaSuccess ? PALIMPSA_OK : PALIMPSA_E_LAUNCH;
+}
+
+int launch_fwd_tall(const FwdArgs& a, int num_seg, cudaStream_t stream) {
+    const int KP = palimpsa_padded_k(a.p.K);
+#define PALIMPSA_X(RK, KG, RV) return launch_tall_t<RK, KG, RV>(a, num_seg, stream)
+    PALIMPSA_TALL_TILINGS(PALIMPSA_X)
+#undef PALIMPSA_X
+    return PALIMPSA_E_DIM;
+}
+
+int fwd_wait_status() {
+    int s = 0;
+    if (cudaDeviceSynchronize() != cudaSuccess) return -1;
+    if (cudaMemcpyFromSymbol(&s, g_fwd_status, sizeof(int)) != cudaSuccess) return -1;
+    if (s) {
+        const int zero = 0;
+        if (cudaMemcpyToSymbol(g_fwd_status, &zero, sizeof(int)) != cudaSuccess) return -1;
+    }
+    return s;
+}
+
+}  // namespace palimpsa

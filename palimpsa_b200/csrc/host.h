@@ -56,6 +56,7 @@ bool carry_tc_shape(const palimpsa_problem& p);      // by sizes, type and flags
 bool carry_tc_supported(const palimpsa_problem& p);  // and by the alignment of its tensors
 int launch_carry_tc(const palimpsa_bwd_params* prm, const palimpsa_segments& segs, cudaStream_t stream);
 int carry_tc_status();
+int fwd_wait_status();  // 0, or the code of a bounded wait of the tall-tile forward that gave up
 int bwd_wait_status();  // 0, or the code of a bounded barrier wait of the backward main kernel that gave up
 
 // Boundary scans over segments (segments.cu).
