@@ -1,4 +1,5 @@
-// Forward kernel of the Palimpsa operator (sm_100a).
+// Forward kernel of the Palimpsa operator (sm_100a): short row tiles, several CTAs per SM.  Grids of few whole waves take
+// fwd_tall.cu's kernel instead (fwd_tall_pays); segment summaries and d_k <= 32 are always here.
 //
 // One CTA owns a tile of TV state rows (d_v) x all KP state columns (padded d_k) of one
 // (sequence, head[, segment]) and walks its tokens in order with the (M, I) state pair held in
