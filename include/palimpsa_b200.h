@@ -155,7 +155,8 @@ int palimpsa_segment_summary(const palimpsa_problem *p, const palimpsa_segments 
  * kernel for tall tiles).  Every in-kernel wait of this library is bounded: a
  * kernel that gives up records the code, releases what it holds and returns.  Its results are invalid, and it
  * marks them so that the failure cannot pass unnoticed: the summary kernel writes NaN into the segment's decay
- * (every later output becomes NaN), the tall-tile forward into its outputs and states, the other two write NaN into the decay-gradient partials (dgt of the
+ * (every later output becomes NaN); the tall-tile forward into the tile's outputs, its
+ * final states and the checkpoint that a backward begins with; the other two into the decay-gradient partials (dgt of the
  * affected tokens and dg come out NaN).  Synchronises the device; reading clears the recorded code, so a
  * non-zero value belongs to the work enqueued since the previous call. */
 int palimpsa_tensor_core_status(void);

@@ -168,7 +168,7 @@ __host__ __device__ constexpr int tall_group() {
     return g < 8 ? 4 : 8;
 }
 
-template <int RK, int KG, int RV, bool UNC>
+template <int RK, int KG, int RV, bool UNC, unsigned POLLS = tc::SPIN_LIMIT>
 __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdArgs a, const int rows) {
     constexpr int KP = RK * KG, VG = 32 / KG, J4 = RK / 4, TV = FT_W * VG * RV, GF = tall_group<KG, RV, UNC>();
     constexpr int NRED = GF * RV * (UNC ? 2 : 1);
@@ -196,7 +196,9 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
     const int blk0 = s0 / TB, nblk = s1 > s0 ? (s1 + TB - 1) / TB - blk0 : 0;
 
     // staged[s] / done[s], s = block & 1: its operands lie in shared memory (one arrival per helper warp); the compute warps
-    // are through with it and its outputs lie in shared memory (one per compute warp).  All waits are bounded.
+    // are through with it and its outputs lie in shared memory (one per compute warp).  All waits are bounded (POLLS).  A
+    // warp that gives up goes on arriving, so that no other waits for it; what is computed from then on, by any warp, is not
+    // valid, and in the end all outputs and states of the tile are made NaN.
     unsigned long long* staged = reinterpret_cast<unsigned long long*>(sm + L.bars);
     unsigned long long* done = staged + 2;
     int* fail_flag = reinterpret_cast<int*>(staged + 4);
@@ -246,20 +248,19 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
             if (lane == 0) mbar_arrive(&staged[it & 1]);
         };
         auto wait_done = [&](int it) __attribute__((always_inline)) {
-            if (!wait_fail && !mbar_wait_idle(&done[it & 1], (it >> 1) & 1)) wait_fail = 8;
+            if (!wait_fail && !mbar_wait_idle(&done[it & 1], (it >> 1) & 1, POLLS)) wait_fail = 8;
         };
         auto write_outputs = [&](int it) __attribute__((always_inline)) {
             const float* ys = reinterpret_cast<const float*>(sm + L.ys + (it & 1) * L.y_stage);
             const float* yvs = reinterpret_cast<const float*>(sm + L.yvs + (it & 1) * L.y_stage);
             const long long tok0 = token0(it);
             const int nt = tokens(it);
-            const float bad = __int_as_float(0x7fc00000);  // a wait ran out: nothing after it is valid
             for (int i = ht; i < nt * TV; i += FT_HT) {
                 const int t = i / TV, r = i - t * TV;
                 if (r < tvw) {
                     const long long e = ((tok0 + t) * p.H + h) * (long long)V + v0 + r;
-                    st1(a.o, e, wait_fail ? bad : ys[i], p.io_dtype);
-                    if (UNC) st1(a.o_var, e, wait_fail ? bad : yvs[i], p.io_dtype);
+                    st1(a.o, e, ys[i], p.io_dtype);
+                    if (UNC) st1(a.o_var, e, yvs[i], p.io_dtype);
                 }
             }
         };
@@ -281,7 +282,31 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
         cp_async_wait<0>();
         if (wait_fail) *fail_flag = wait_fail;
         __syncthreads();
-        if (ht == 0 && *fail_flag) atomicCAS(&g_fwd_status, 0, *fail_flag);
+        if (*fail_flag) {
+            // somebody gave up: NaN over the tile's outputs, the final states that the compute warps have written, and the
+            // checkpoint that the backward begins with
+            if (ht == 0) atomicCAS(&g_fwd_status, 0, *fail_flag);
+            const float bad = __int_as_float(0x7fc00000);
+            for (int t = s0; t < s1; ++t)
+                for (int i = ht; i < tvw; i += FT_HT) {
+                    const long long e = (((long long)bos + t) * p.H + h) * (long long)V + v0 + i;
+                    st1(a.o, e, bad, p.io_dtype);
+                    if (UNC) st1(a.o_var, e, bad, p.io_dtype);
+                }
+            const long long state = ((long long)n * p.H + h) * V + v0;
+            const long long last = ((seq_first_slot(p, n) + blk0 + nblk - 1) * p.H + h) * V + v0;
+            for (int i = ht; i < tvw * KP; i += FT_HT) {
+                const int row = i / KP, c = i - row * KP;
+                if (a.final_mu && s1 == len && (s0 < len || g == 0) && c < K) {
+                    a.final_mu[(state + row) * K + c] = bad;
+                    a.final_I[(state + row) * K + c] = bad;
+                }
+                if (a.ckpt_M && nblk > 0) {
+                    a.ckpt_M[(last + row) * KP + c] = bad;
+                    a.ckpt_I[(last + row) * KP + c] = bad;
+                }
+            }
+        }
         return;
     }
 
@@ -333,7 +358,7 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
     }
     for (int it = 0; it < nblk; ++it) {
         if (idle) {
-            if (!wait_fail && !mbar_wait_idle(&staged[it & 1], (it >> 1) & 1)) wait_fail = 8;
+            if (!wait_fail && !mbar_wait_idle(&staged[it & 1], (it >> 1) & 1, POLLS)) wait_fail = 8;
             __syncwarp();
             if (lane == 0) mbar_arrive(&done[it & 1]);
             continue;
@@ -363,10 +388,7 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
         const float4* fc = reinterpret_cast<const float4*>(op + L.fc);
         float* ys = reinterpret_cast<float*>(sm + L.ys + (it & 1) * L.y_stage);
         float* yvs = reinterpret_cast<float*>(sm + L.yvs + (it & 1) * L.y_stage);
-        if (!wait_fail && !tc::mbar_wait(&staged[it & 1], (it >> 1) & 1)) {
-            wait_fail = 8;
-            M[0][0][0].x = __int_as_float(0x7fc00000);  // outputs and states from here on are not valid
-        }
+        if (!wait_fail && !tc::mbar_wait(&staged[it & 1], (it >> 1) & 1, POLLS)) wait_fail = 8;
         const int end = min(TB, s1 - (blk0 + it) * TB);
 #pragma unroll 1
         for (int tg = 0; tg < end; tg += GF) {
@@ -458,6 +480,7 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
     __syncthreads();
 }
 
+#ifndef PALIMPSA_TALL_KERNEL_ONLY  // a test compiles the kernel alone
 // -------------------------------------------------------------------------------------------------
 // Host side
 // -------------------------------------------------------------------------------------------------
@@ -543,6 +566,8 @@ int launch_fwd_tall(const FwdArgs& a, int num_seg, cudaStream_t stream) {
 #undef PALIMPSA_X
     return PALIMPSA_E_DIM;
 }
+
+#endif
 
 int fwd_wait_status() {
     int s = 0;

@@ -157,8 +157,8 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
     asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.shared::cta.b64 st, [%0];\n}" ::"r"(tc::smem_u32(bar)) : "memory");
 }
 // The wait of a warp that is ahead of the others most of the time, with pauses: polling takes issue slots from them.
-__device__ __forceinline__ bool mbar_wait_idle(unsigned long long* bar, unsigned parity) {
-    for (unsigned i = 0; i < tc::SPIN_LIMIT; ++i) {
+__device__ __forceinline__ bool mbar_wait_idle(unsigned long long* bar, unsigned parity, unsigned limit = tc::SPIN_LIMIT) {
+    for (unsigned i = 0; i < limit; ++i) {
         if (tc::mbar_wait(bar, parity, 1)) return true;
         __nanosleep(64);
     }

@@ -66,6 +66,44 @@ def test_peer_wait_runs_out_records_its_code_and_poisons_the_buffer():
     assert lib.palimpsa_peer_signal(flag.data_ptr() + 4, 1, stream) == _lib.E_ALIGN   # flags are 8-byte aligned
 
 
+@pytest.mark.parametrize("T,V,rows,aligned", [(45, 40, 48, 1), (16, 40, 16, 1), (45, 33, 24, 0)])
+def test_tall_forward_that_gives_up_marks_its_outputs_states_and_checkpoint(T, V, rows, aligned):
+    """The tall-tile forward's kernel from the test-only library.  With a poll limit of 0 every wait gives up: the code is
+    recorded, and all outputs, the final states and the checkpoint that a backward begins with are NaN in every row, idle warps
+    and ragged tiles included.  With the product's limit the same launch matches the oracle."""
+    from palimpsa_b200 import _lib as L
+    from palimpsa_b200.ops.palimpsa import _core
+    if not os.path.exists(wait_probe.LIB):
+        wait_probe.build()
+    lib = C.CDLL(wait_probe.LIB)
+    run = lib.palimpsa_test_tall_forward
+    run.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]
+    N, H, K = 2, 2, 128
+    inp = orc.make_inputs(T, B=N, T=T, H=H, K=K, V=V)
+    a = [inp[n].to("cuda:0") for n in ("q", "k", "v", "b", "gt", "g", "Ip")]
+    prm = L.FwdParams()
+    prm.struct_size, prm.p = C.sizeof(L.FwdParams), _core._problem(*a, None, None, None, None, K ** -0.5, L.FLAG_UNCERTAINTY)
+    slots = N * -(-T // 16)
+    out = {"o": torch.empty_like(a[2]), "o_var": torch.empty_like(a[2])}
+    out.update({n: torch.empty(N, H, V, K, device="cuda:0") for n in ("final_mu", "final_I")})
+    out.update({n: torch.empty(slots, H, V, K, device="cuda:0") for n in ("ckpt_M", "ckpt_I")})
+    for n, x in out.items():
+        setattr(prm, n, x.data_ptr())
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for give_up in (1, 0):
+        for x in out.values():
+            x.zero_()
+        assert run(C.addressof(prm), rows, give_up, aligned, stream) == 0
+        assert lib.palimpsa_test_tall_status() == (8 if give_up else 0)
+        assert lib.palimpsa_test_tall_status() == 0                         # reading cleared it
+        last = [n * (slots // N) + slots // N - 1 for n in range(N)]
+        marked = [out[n] for n in ("o", "o_var", "final_mu", "final_I")] + [out[n][last] for n in ("ckpt_M", "ckpt_I")]
+        assert all(bool((x.isnan() if give_up else x.isfinite()).all()) for x in marked)
+    ref = run_oracle(inp, unc=True)
+    got = {n: out[n].cpu() for n in ("o", "o_var", "final_mu", "final_I")}
+    compare(got, ref, TOL_FP32, names=[*got], what="product's poll limit")
+
+
 def test_large_shared_memory_is_granted_again_in_a_new_context():
     """A kernel's shared-memory limit lives in one context: after cudaDeviceReset the next launch has to raise it again.  In
     a process of its own, which ends its own context only."""

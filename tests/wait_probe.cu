@@ -55,3 +55,32 @@ extern "C" int palimpsa_test_smem_grant(int bytes, int reset) {
     if (cudaGetLastError() != cudaSuccess) return -3;
     return cudaDeviceSynchronize() == cudaSuccess ? 0 : -4;
 }
+
+// The tall-tile forward's kernel, one tiling (97 <= d_k <= 128, tiles of `rows` rows), with the product's poll limit or one of 0.
+// With 0 every wait gives up at once, by construction; all accesses stay inside the buffers of an ordinary launch, and nothing
+// waits for anything but the CTA barriers that all threads reach.
+#define PALIMPSA_TALL_KERNEL_ONLY
+#include "../palimpsa_b200/csrc/fwd_tall.cu"
+
+namespace {
+template <unsigned POLLS>
+int launch_tall(const palimpsa::FwdArgs& a, int rows, cudaStream_t stream) {
+    using namespace palimpsa;
+    const TallSmem L = tall_smem_layout(128, FT_W * 2 * 2, dtype_size(a.p.io_dtype), true);
+    const dim3 grid((a.p.V + rows - 1) / rows, a.p.num_seqs * a.p.H, 1);
+    if (!allow_smem<fwd_tall_kernel<8, 16, 2, true, POLLS>>(L.total)) return -2;
+    fwd_tall_kernel<8, 16, 2, true, POLLS><<<grid, FT_NTHR + FT_HT, L.total, stream>>>(a, rows);
+    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+}  // namespace
+extern "C" int palimpsa_test_tall_forward(const palimpsa_fwd_params* prm, int rows, int give_up, int aligned, void* cuda_stream) {
+    palimpsa::FwdArgs a{};
+    a.p = prm->p;
+    a.o = prm->o, a.o_var = prm->o_var, a.final_mu = prm->final_mu, a.final_I = prm->final_I;
+    a.ckpt_M = prm->ckpt_M, a.ckpt_I = prm->ckpt_I;
+    a.aligned = aligned;
+    if (a.p.K <= 96 || a.p.K > 128 || rows > palimpsa::FT_W * 2 * 2 || rows % 8 || !a.o_var) return -4;
+    cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+    return give_up ? launch_tall<0>(a, rows, stream) : launch_tall<palimpsa::tc::SPIN_LIMIT>(a, rows, stream);
+}
+extern "C" int palimpsa_test_tall_status(void) { return palimpsa::fwd_wait_status(); }
