@@ -237,13 +237,14 @@ const char *palimpsa_last_error_string(int code);
 /* K rounded up to the kernels' tile width (16, 32, 48, 64, 96, 128, 192 or 256); 0 if K > 256. */
 int palimpsa_padded_k(int K);
 
-/* State rows (d_v) that one CTA of the forward kernel owns at head dimensions (K, V); 0 if d_k is not
- * supported.  A forward launch has ceil(V / rows) x num_seqs x H CTAs (times the segment count): hosts use it
- * to decide whether a problem fills the GPU or should be cut into segments.  No counterpart in the reference,
- * whose grid is fixed at (V/16) x N x H programs (chunk_palimpsa_forgetting_scalar.py:478). */
+/* State rows (d_v) of a tile of the forward kernel for short tiles at head dimensions (K, V); 0 if d_k is not supported.
+ * A nominal height: planners count ceil(V / rows) x num_seqs x H with it (times the segment count) to judge whether a
+ * problem fills the GPU or should be cut into segments; the grid that a call launches may have taller tiles
+ * (palimpsa_fwd_plan).  No counterpart in the reference, whose grid is fixed at (V/16) x N x H programs
+ * (chunk_palimpsa_forgetting_scalar.py:478). */
 int palimpsa_fwd_tile_rows(int K, int V);
 
-/* The same for the backward kernel, whose tile also depends on the element type (PALIMPSA_F32 / _BF16 / _F16) and on
+/* The rows that one CTA of the backward kernel owns; its tile also depends on the element type (PALIMPSA_F32 / _BF16 / _F16) and on
  * whether the uncertainty output takes part (shared-memory budget): a backward launch has ceil(V / rows) x num_seqs x
  * H CTAs of up to 16 warps, usually one resident per SM, so hosts that plan a training step count waves with it.
  * 0 if the shape is not supported.  No counterpart in the reference (grid (V/16) x N x H,
@@ -255,6 +256,11 @@ int palimpsa_bwd_tile_rows(int K, int V, int io_dtype, int uncertainty);
  * takes the tile height that this is smallest for; palimpsa_bwd_tile_rows() is the one of a grid of many waves.
  * 0 if the shape is not supported. */
 double palimpsa_bwd_token_cost(const palimpsa_problem *p);
+
+/* What a launch takes for a problem of these sizes (num_seqs, seq_len, total_tokens, H, K, V, io_dtype, flags, segments, and
+ * whether there are cu_seqlens; no pointer is followed): the forward {1 for the kernel for tall tiles, else 0; rows of a
+ * tile}.  For diagnostics and tests. */
+int palimpsa_fwd_plan(const palimpsa_problem *p, int32_t *plan);
 
 /* Copies n <= 8 device buffers (src[i] -> dst[i], bytes[i]; not overlapping) in one launch: the token inputs of a
  * replayed decode step. */

@@ -128,6 +128,17 @@ double palimpsa_bwd_token_cost(const palimpsa_problem* p) {
     return bwd_token_cost(*p);
 }
 
+static bool plannable(const palimpsa_problem* p) {
+    return p && p->K > 0 && p->V > 0 && p->K <= PALIMPSA_MAX_K && p->num_seqs > 0 && p->H > 0 &&
+           (p->io_dtype == PALIMPSA_F32 || p->io_dtype == PALIMPSA_BF16 || p->io_dtype == PALIMPSA_F16);
+}
+int palimpsa_fwd_plan(const palimpsa_problem* p, int32_t* plan) {
+    if (!plan) return PALIMPSA_E_NULL;
+    if (!plannable(p)) return PALIMPSA_E_DIM;
+    fwd_plan(*p, plan);
+    return PALIMPSA_OK;
+}
+
 int palimpsa_fwd_tile_rows(int K, int V) {
     if (K <= 0 || V <= 0 || K > PALIMPSA_MAX_K) return 0;
     return fwd_tile_rows(K, V);

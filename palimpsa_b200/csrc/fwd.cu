@@ -552,6 +552,21 @@ int fwd_tile_rows(int K, int V) {
     return 0;
 }
 
+static bool takes_tall(const palimpsa_problem& p, int num_seg) {
+    const int KP = palimpsa_padded_k(p.K);
+    int elements = 0;
+#define PALIMPSA_X(RK, KG, RV, WMAX) elements = RK * RV; break
+    PALIMPSA_FWD_TILINGS(PALIMPSA_X)
+#undef PALIMPSA_X
+    return fwd_tall_pays(p, num_seg, fwd_tile_rows(p.K, p.V), elements);
+}
+
+void fwd_plan(const palimpsa_problem& p, int32_t* plan) {
+    const int num_seg = p.segments > 1 ? p.segments : 1;
+    plan[0] = takes_tall(p, num_seg);
+    plan[1] = plan[0] ? fwd_tall_rows(p, num_seg) : fwd_tile_rows(p.K, p.V);
+}
+
 static bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; }
 
 int launch_fwd(const palimpsa_fwd_params* prm, const palimpsa_segments* segs, bool summary, cudaStream_t stream) {
@@ -581,11 +596,7 @@ int launch_fwd(const palimpsa_fwd_params* prm, const palimpsa_segments* segs, bo
     a.aligned = ((p.K * es) % 16 == 0) && ((p.V * es) % 16 == 0) && aligned16(p.q) && aligned16(p.k) &&
                 aligned16(p.v) && aligned16(p.b) && ((reinterpret_cast<uintptr_t>(p.gt) & 3) == 0);
     const int KP = palimpsa_padded_k(p.K);
-    int elements = 0;
-#define PALIMPSA_X(RK, KG, RV, WMAX) elements = RK * RV; break
-    PALIMPSA_FWD_TILINGS(PALIMPSA_X)
-#undef PALIMPSA_X
-    if (!summary && fwd_tall_pays(p, num_seg, fwd_tile_rows(p.K, p.V), elements)) return launch_fwd_tall(a, num_seg, stream);
+    if (!summary && takes_tall(p, num_seg)) return launch_fwd_tall(a, num_seg, stream);
 #define PALIMPSA_X(RK, KG, RV, WMAX) return launch_fwd_t<RK, KG, RV, WMAX>(a, num_seg, summary, stream)
     PALIMPSA_FWD_TILINGS(PALIMPSA_X)
 #undef PALIMPSA_X

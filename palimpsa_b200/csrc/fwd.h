@@ -26,6 +26,7 @@ struct FwdArgs {
 // Is the tall-tile kernel the faster one for this call (fwd_tall.cu)?  `short_rows`, `short_elements`: the other kernel's tile
 // height and state elements per thread.
 bool fwd_tall_pays(const palimpsa_problem& p, int num_seg, int short_rows, int short_elements);
+int fwd_tall_rows(const palimpsa_problem& p, int num_seg);
 int launch_fwd_tall(const FwdArgs& a, int num_seg, cudaStream_t stream);
 
 }  // namespace palimpsa

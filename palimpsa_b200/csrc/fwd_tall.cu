@@ -520,26 +520,44 @@ static TallPlan tall_plan(const palimpsa_problem& p, int num_seg) {
     return best;
 }
 
-// fwd.cu's kernel by the same measure: `rows` a tile, `elements` of state a thread.  Its CTAs share an SM: up to four, a token
-// costs 300 cycles and 8.1 per element on a scheduler's lanes, 16 per element beyond 48 (260 and 10.4 where a thread has 32);
-// more run through at 13.6 per element.  Measured: 678 with 3 CTAs of 4 warps of 16, 701 and 1158 with 2 and 3 of 24, 597, 886
-// and 932 with 2, 3 and 4 of 2 warps of 32.
+// fwd.cu's kernel by the same measure: `rows` a tile, `elements` of state a thread, n of its CTAs on an SM.  Measured, 4 warps:
+// 367, 497, 666 and 859 with 1 to 4 CTAs of 16 elements; 494, 701, 1158 and 1350 of 24; 597, 886 and 932 with 2, 3 and 4 of 2
+// warps of 32; more run through at 13.6 per element.  The uncertainty output costs 16 elements 1.17, 1.2 and, from three CTAs on,
+// 1.4 times that, more elements 1.05, 1.17 and 1.2 times, the tall tiles 1.25 times.
 static double short_cost(const palimpsa_problem& p, int num_seg, int rows, int elements) {
     const int KP = palimpsa_padded_k(p.K), tiles = (p.V + rows - 1) / rows;
-    const double share = (double)p.num_seqs * p.H * num_seg * tiles / B200_SMS;
+    const double share = (double)p.num_seqs * p.H * num_seg * tiles / B200_SMS, n = ceil(share);
     const int warps = rows * KP / (32 * elements);
-    if (share > 4) return 13.6 * warps / 4. * elements * share;
-    const double load = ceil(ceil(share) * warps / 4) * elements;  // elements on the lanes of the busiest scheduler
-    return elements >= 32 ? 260 + 10.4 * load : load <= 48 ? 300 + 8.1 * load : 16 * load;
+    const bool few = elements <= 16;
+    const double unc = !(p.flags & PALIMPSA_FLAG_UNCERTAINTY) ? 1
+                       : n <= 1                               ? (few ? 1.17 : 1.05)
+                       : n <= 2                               ? (few ? 1.2 : 1.17)
+                                                              : (few ? 1.4 : 1.2);
+    if (share > 4) return unc * 13.6 * warps / 4. * elements * share;
+    const double load = ceil(n * warps / 4) * elements;  // elements on the lanes of the busiest scheduler
+    if (elements >= 32) return unc * (260 + 10.4 * load);
+    if (load > 48) return unc * (n < 4 ? 16 : 13.8) * load;
+    return unc * (elements > 16 ? 300 + 8.1 * load : 235 + 8.4 * load);
 }
 
+// Taken where a CTA's tokens make up for what it costs to start: 1300 cycles beside fwd.cu's kernel at 4 warps of 16 elements
+// (its other tilings start no sooner), and 9500 for every wave after the first, since CTAs that fill an SM do not overlap.
+// Device time, us, fwd.cu's kernel against this one, 128x128 bf16: 2 heads, T = 16 / 48 / 64 / 256 5.9 / 12.1 / 15.1 / 51.5
+// against 6.4 / 11.9 / 14.6 / 44.7; 64 heads (two waves) 11.2 / 25.0 / 32.7 / 118 against 15.0 / 30.7 / 38.1 / 125; 12 heads with the
+// uncertainty output, T = 64 / 256 20.6 / 62.7 against 21.7 / 59.4.  The estimates are good for about 4 %: below that it stays
+// with the kernel that shares an SM.
 bool fwd_tall_pays(const palimpsa_problem& p, int num_seg, int short_rows, int short_elements) {
     const int KP = palimpsa_padded_k(p.K);
     TallPlan t{0, 0, 0.};
 #define PALIMPSA_X(RK, KG, RV) t = tall_plan<RK, KG, RV>(p, num_seg)
     PALIMPSA_TALL_TILINGS(PALIMPSA_X)
 #undef PALIMPSA_X
-    return t.rows && t.cost < 0.96 * short_cost(p, num_seg, short_rows, short_elements);
+    if (!t.rows) return false;
+    const double units = (double)p.num_seqs * p.H * num_seg, waves = ceil(units * t.tiles / B200_SMS);
+    const double tokens = units > 0 ? (double)p.total_tokens * p.H / units : 0;
+    const double start = (short_elements <= 16 ? 1300 : 0) + (waves > 1 ? 9500 * (waves - 1) : 0);
+    const double cost = t.cost * (p.flags & PALIMPSA_FLAG_UNCERTAINTY ? 1.25 : 1);
+    return start + cost * tokens < 0.96 * short_cost(p, num_seg, short_rows, short_elements) * tokens;
 }
 
 template <int RK, int KG, int RV>
@@ -557,6 +575,14 @@ static int launch_tall_t(const FwdArgs& a, int num_seg, cudaStream_t stream) {
         fwd_tall_kernel<RK, KG, RV, false><<<grid, block, L.total, stream>>>(a, t.rows);
     }
     return cudaGetLastError() == cudaSuccess ? PALIMPSA_OK : PALIMPSA_E_LAUNCH;
+}
+
+int fwd_tall_rows(const palimpsa_problem& p, int num_seg) {
+    const int KP = palimpsa_padded_k(p.K);
+#define PALIMPSA_X(RK, KG, RV) return tall_plan<RK, KG, RV>(p, num_seg).rows
+    PALIMPSA_TALL_TILINGS(PALIMPSA_X)
+#undef PALIMPSA_X
+    return 0;
 }
 
 int launch_fwd_tall(const FwdArgs& a, int num_seg, cudaStream_t stream) {

@@ -247,7 +247,7 @@ def test_missing_library_is_a_loud_error(monkeypatch, tmp_path):
 
 
 def test_forward_tile_rows_from_the_library():
-    """Pure host function of the C ABI: rows of one forward CTA per head shape (what plan_segments counts CTAs with)."""
+    """Pure host function of the C ABI: nominal rows of one forward CTA per head shape (what plan_segments counts CTAs with)."""
     from palimpsa_b200 import _lib
     lib = _lib.lib()
     assert lib.palimpsa_fwd_tile_rows(128, 128) == 16
@@ -262,3 +262,17 @@ def test_forward_tile_rows_from_the_library():
     assert lib.palimpsa_bwd_tile_rows(300, 64, _lib.BF16, 0) == 0
     assert lib.palimpsa_bwd_tile_rows(64, 64, 99, 0) == 0             # unknown element type
     assert lib.palimpsa_last_error_string(_lib.E_SYMBOL).startswith(b"the library's own scratch array")
+
+
+def test_the_forward_takes_tall_tiles_where_they_pay():
+    """Not for the few tokens that do not make up for filling an SM with one CTA, nor where a second wave has to start."""
+    import torch
+    from tests.helpers import fwd_plan
+    bf = torch.bfloat16
+    assert [fwd_plan(1, T, 12, 128, 128, bf)[0] for T in (1, 16, 32, 64, 512)] == [0, 0, 0, 1, 1]
+    assert [fwd_plan(1, T, 12, 128, 128, bf, unc=True)[0] for T in (64, 256)] == [0, 1]
+    assert [fwd_plan(4, T, 16, 128, 128, bf)[0] for T in (16, 64, 256, 4096)] == [0, 0, 0, 0]    # 64 heads: two waves
+    assert [fwd_plan(4, T, 16, 48, 96, bf)[0] for T in (2, 37, 4096)] == [1, 1, 1]
+    assert fwd_plan(8, 4096, 6, 128, 128, bf) == (1, 48) and fwd_plan(2, 3001, 16, 96, 192, bf) == (1, 48)
+    assert fwd_plan(8, 0, 6, 128, 128, bf)[0] == 0
+    assert fwd_plan(40, 40 * 20, 6, 128, 128, bf, packed=True)[0] == 0
