@@ -244,9 +244,9 @@ int palimpsa_padded_k(int K);
  * (chunk_palimpsa_forgetting_scalar.py:478). */
 int palimpsa_fwd_tile_rows(int K, int V);
 
-/* The rows that one CTA of the backward kernel owns; its tile also depends on the element type (PALIMPSA_F32 / _BF16 / _F16) and on
- * whether the uncertainty output takes part (shared-memory budget): a backward launch has ceil(V / rows) x num_seqs x
- * H CTAs of up to 16 warps, usually one resident per SM, so hosts that plan a training step count waves with it.
+/* State rows (d_v) that one CTA of the backward kernel owns in a grid of many waves, by element type (PALIMPSA_F32 / _BF16 /
+ * _F16) and whether the uncertainty output takes part: such a backward launches ceil(V / rows) x num_seqs x H CTAs of up to
+ * 12 warps, usually one resident per SM, so hosts that plan a training step count waves with it.
  * 0 if the shape is not supported.  No counterpart in the reference (grid (V/16) x N x H,
  * chunk_palimpsa_forgetting_scalar.py:558). */
 int palimpsa_bwd_tile_rows(int K, int V, int io_dtype, int uncertainty);
@@ -259,8 +259,9 @@ double palimpsa_bwd_token_cost(const palimpsa_problem *p);
 
 /* What a launch takes for a problem of these sizes (num_seqs, seq_len, total_tokens, H, K, V, io_dtype, flags, segments, and
  * whether there are cu_seqlens; no pointer is followed): the forward {1 for the kernel for tall tiles, else 0; rows of a
- * tile}.  For diagnostics and tests. */
+ * tile}, the backward {rows of a tile; compute warps of a CTA; buffers for a group's partials}.  For diagnostics and tests. */
 int palimpsa_fwd_plan(const palimpsa_problem *p, int32_t *plan);
+int palimpsa_bwd_plan(const palimpsa_problem *p, int32_t *plan);
 
 /* Copies n <= 8 device buffers (src[i] -> dst[i], bytes[i]; not overlapping) in one launch: the token inputs of a
  * replayed decode step. */

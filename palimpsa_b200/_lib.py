@@ -99,6 +99,7 @@ SYMBOLS = {
     "palimpsa_bwd_tile_rows": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int]),
     "palimpsa_bwd_token_cost": (C.c_double, [C.POINTER(Problem)]),
     "palimpsa_fwd_plan": (C.c_int, [C.POINTER(Problem), C.POINTER(C.c_int32)]),
+    "palimpsa_bwd_plan": (C.c_int, [C.POINTER(Problem), C.POINTER(C.c_int32)]),
     "palimpsa_peer_wait": (C.c_int, [C.c_void_p, C.c_uint64, C.c_uint32, C.c_void_p, C.c_void_p]),
     "palimpsa_peer_signal": (C.c_int, [C.c_void_p, C.c_uint64, C.c_void_p]),
     "palimpsa_ckpt_slots": (C.c_longlong, [C.POINTER(Problem)]),

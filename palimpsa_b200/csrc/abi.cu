@@ -138,6 +138,12 @@ int palimpsa_fwd_plan(const palimpsa_problem* p, int32_t* plan) {
     fwd_plan(*p, plan);
     return PALIMPSA_OK;
 }
+int palimpsa_bwd_plan(const palimpsa_problem* p, int32_t* plan) {
+    if (!plan) return PALIMPSA_E_NULL;
+    if (!plannable(p)) return PALIMPSA_E_DIM;
+    bwd_plan(*p, plan);
+    return PALIMPSA_OK;
+}
 
 int palimpsa_fwd_tile_rows(int K, int V) {
     if (K <= 0 || V <= 0 || K > PALIMPSA_MAX_K) return 0;

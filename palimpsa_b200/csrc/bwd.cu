@@ -2,13 +2,13 @@
 //
 // Main kernel: one CTA owns TV state rows x all KP columns of one (sequence, head) and walks the
 // sequence's 16-token blocks from the last to the first.  Per block it
-//   1. takes the block's start state (M, I) from the checkpoint the forward saved (prefetched into
-//      shared memory one block ahead with cp.async, together with the block's raw inputs),
+//   1. takes the block's start state (M, I) from the checkpoint the forward saved, which lies in
+//      shared memory beside the block's operands (the helper warps brought both one block ahead),
 //   2. sweeps forward once, parking the state at the start of each 4-token group (thread-private
 //      slots in shared memory),
 //   3. per group, last first: recomputes the 4 per-token states into registers, then walks the
 //      tokens in reverse, carrying the state gradients (GM, -GI) in registers:
-//          h    = dy*q_s / I            GM = f_next*GM + h          -GI = f_next*(-GI) + h*mu (+var)
+//          h    = dy*q_s / I            GM = f_next*GM + h          -GI = f_next*(-GI) + h*mu (+ dy_var*(q/I)^2)
 //          dq  += dy*mu   dk += GM*v + 2k*GI*b   dv += GM*k   db += GI*k^2
 //          df   = <GM, M_prev> + <GI, I_prev - Ip>
 //      (the algebra of chunk_palimpsa_bwd_kernel, chunk_palimpsa_forgetting_scalar.py:343-434,
@@ -17,15 +17,18 @@
 // in registers across a thread's rows, then across the CTA's row groups through shared memory, and
 // across the CTAs of different row tiles through fp32 partial buffers in the workspace, which the
 // finishing kernel sums in a fixed order (bitwise reproducible; no atomics).
-// Helper warps stage the next block (checkpoint and raw inputs by cp.async, raw inputs converted to fp32 operands in a second
-// operand stage) and do all that follows a group's partials in shared memory (sums over the row groups, casts, global
-// stores).  All hand-overs are mbarriers with bounded waits: the compute warps meet no CTA barrier and drift apart.
+// Helper warps stage the next block (checkpoint by cp.async; inputs through registers, where they wait while a group is summed,
+// into fp32 operands of a second operand stage) and do all that follows a group's partials in shared memory (sums over the row
+// groups, casts, global stores).  All hand-overs are mbarriers with bounded waits: the compute warps meet no CTA barrier and
+// drift apart.
 // What bounds the walk is the issue rate: a packed FP32 instruction takes two issue cycles, a pair of state elements 28 per
 // token in the reverse walk and 14 in the two forward steps, and operand loads, shuffle sums and moves come on top; so it
 // pays to have 12 elements a thread (two warps per scheduler) rather than 8 (three), and to take staging off those warps.
-// Backward at B=8 T=4096 H=6 d=128: 5.21 ms with 11 warps of 8 elements that stage for themselves, 4.77 with 8 of 12 and
-// staging helpers; 2.38 / 2.13 ms at H=16 d=48, 4.71 / 4.20 at 48x96, 8.51 / 8.21 at B=4 H=16 96x192, 3.23 / 3.15 at B=2
-// T=2048 H=6 256x128, 0.39 / 0.38 at B=64 T=512 H=8 16x32.
+// Through registers, because a copy in shared memory to convert from costs 10 to 37 KB, for want of which some shapes had one
+// operand stage or one group buffer, and because rows that start at any offset can only be loaded one by one, which four warps
+// do not get done between two groups.  One wave of 148 CTAs, T = 512, converted from shared memory -> through registers, us:
+// 128x88 bf16 296 -> 291, 48x48 268 -> 269, 48x48 float32 with the uncertainty output 379 -> 305, 96x32 436 -> 375, 192x12 407 ->
+// 269, 256x8 426 -> 363; rows at any offset: 127x87 363 -> 296, 95x23 411 -> 269, 47x47 415 -> 277, 15x63 238 -> 165.
 // One CTA per SM, beside the smallest tilings; bwd_config has the choice of the tile.
 //
 // Finishing kernels: (1) per (token, head) row: sum the row tiles, cast dq/dk, form
@@ -63,10 +66,9 @@ struct BwdArgs {
     const float* ckpt_I;
     float *dq_part, *dk_part, *df_part, *dip_part;
     void *dv, *db;
-    int aligned;
+    int vec_k, vec_v;  // four columns of q and k, two rows of v, b and the output gradients come in one load: else one by one
     int rows;        // state rows of a tile: as many as the CTA's warps hold, or fewer
     int kbuf;        // shared-memory buffers for the per-group d_k-indexed partials: 2 where they fit, else 1
-    int opbuf;       // operand stages: 2 where they fit (the next block is converted while this one is walked), else 1
     int rows_total;  // tokens * H
     // segments (gridDim.z of them per sequence; seg_len tokens each, a multiple of 16; 0 = whole sequence)
     int seg_len;
@@ -77,24 +79,18 @@ struct BwdArgs {
 };
 
 struct BwdSmem {
-    int ks, qs, qqs, vb, dys2, dyvs2, fc2, fn2;  // offsets inside an operand stage; the stages come first
+    int ks, qs, vb, dys2, dyvs2, fc2, fn2;  // offsets inside an operand stage; the two stages come first
     int op_stage, slots, ckb;
     int kred, dvs, dbs, wred, fgr;  // per-group partials handed to the helper warps, kbuf buffers of each
     int bars;                       // mbarriers: full[2], empty[2], staged[2], done[2]; then the failure flag
     int ck_stage;  // bytes of one (M, I) checkpoint stage
-    int raw, rq, rk, rv, rb, rdo, rdov, rgt;
     int total;
 };
 
-// Columns per token of the raw d_v-indexed staging tiles: the row tile widened to 16-byte boundaries of the
-// global rows on both sides (a tile of 22 rows does not start on one).
-__host__ __device__ constexpr int bwd_staged_cols(int TV) { return (TV + 7) / 8 * 8 + 8; }
-
-// Shared-memory plan of one backward CTA (KP padded d_k, TV state rows, NE state elements per thread,
-// WV row groups).  Operands v, b, dy are stored with every value duplicated ({x, x}), v and b of a row side by side, so that
-// one 128-bit load yields the two register pairs the packed FP32 instructions want.
-__host__ __device__ inline BwdSmem bwd_smem_layout(int KP, int TV, int NE, int nthr, int WV, int es, bool unc,
-                                                  int kbuf, int opbuf) {
+// Shared-memory plan of one backward CTA (KP padded d_k, NE state elements per thread, W compute warps that hold TV state rows
+// in WV row groups).  Operands v, b, dy are stored with every value duplicated ({x, x}), v and b of a row side by side, so
+// that one 128-bit load yields the two register pairs the packed FP32 instructions want.
+__host__ __device__ inline BwdSmem bwd_smem_layout(int KP, int TV, int NE, int W, int WV, bool unc, int kbuf) {
     BwdSmem s;
     int off = 0;
     auto take = [&](int bytes) {
@@ -104,39 +100,23 @@ __host__ __device__ inline BwdSmem bwd_smem_layout(int KP, int TV, int NE, int n
     };
     s.ks = take(TB * KP * 4);
     s.qs = take(TB * KP * 4);
-    s.qqs = unc ? take(TB * KP * 4) : 0;
     s.vb = take(TB * TV * 16);
     s.dys2 = take(TB * TV * 8);
     s.dyvs2 = unc ? take(TB * TV * 8) : 0;
     s.fc2 = take(TB * 16);
     s.fn2 = take(TB * 8);
     s.op_stage = off;
-    off *= opbuf;
-    s.slots = take(2 * 2 * NE * nthr * 4);
+    off *= 2;
+    s.slots = take(2 * 2 * NE * 32 * W * 4);
     s.ck_stage = 2 * TV * KP * 4;
     s.ckb = take(2 * s.ck_stage);
     s.kred = take(kbuf * GR * WV * 2 * KP * 4);  // kbuf = 2 group buffers where they fit (host's choice), else 1
     s.dvs = take(kbuf * GR * TV * 4);
     s.dbs = take(kbuf * GR * TV * 4);
-    s.wred = take(kbuf * (nthr / 32) * GR * 2 * 4);
+    s.wred = take(kbuf * W * GR * 2 * 4);
     s.fgr = take(kbuf * GR * 4);
     s.bars = take(80);
-    s.raw = off;
-    int r = 0;
-    auto rtake = [&](int bytes) {
-        int o = r;
-        r += round_up(bytes, 16);
-        return o;
-    };
-    const int TVS = bwd_staged_cols(TV);
-    s.rq = rtake(TB * KP * es);
-    s.rk = rtake(TB * KP * es);
-    s.rv = rtake(TB * TVS * es);
-    s.rb = rtake(TB * TVS * es);
-    s.rdo = rtake(TB * TVS * es);
-    s.rdov = unc ? rtake(TB * TVS * es) : 0;
-    s.rgt = rtake((TB + 1) * 4);
-    s.total = off + r;
+    s.total = off;
     return s;
 }
 
@@ -153,133 +133,143 @@ __device__ __forceinline__ void bwd_issue_ckpt(const BwdArgs& a, int nthr, int t
     }
 }
 
-// Asynchronous copy of one block's raw inputs (aligned path only).
-__device__ __forceinline__ void bwd_issue_raw(const BwdArgs& a, int nthr, int tid, unsigned char* sm, const BwdSmem& L, int es,
-                                              int KP, int TV, long long tok0, int nt, int nt_ext, int h, int v0, int tvw) {
-    const palimpsa_problem& p = a.p;
-    unsigned char* stage = sm + L.raw;
-    const int cq = p.K * es / 16;
-    const char* gq = reinterpret_cast<const char*>(p.q);
-    const char* gk = reinterpret_cast<const char*>(p.k);
-    for (int i = tid; i < nt * cq; i += nthr) {
-        int t = i / cq, c = i - t * cq;
-        long long src = ((tok0 + t) * p.H + h) * (long long)p.K * es + c * 16;
-        int dst = t * KP * es + c * 16;
-        cp_async16(stage + L.rq + dst, gq + src);
-        cp_async16(stage + L.rk + dst, gk + src);
-    }
-    // the aligned superset [va, va + span) of the tile's columns [v0, v0 + tvw); d_v*es is a multiple of 16 on
-    // this path, so the superset stays inside the row
-    const int ea = 16 / es, va = v0 / ea * ea, span = (v0 - va + tvw + ea - 1) / ea * ea;
-    const int cv = span * es / 16, TVS = bwd_staged_cols(TV);
-    const char* gv = reinterpret_cast<const char*>(p.v);
-    const char* gb = reinterpret_cast<const char*>(p.b);
-    const char* gdo = reinterpret_cast<const char*>(a.d_o);
-    const char* gdov = reinterpret_cast<const char*>(a.d_o_var);
-    for (int i = tid; i < nt * cv; i += nthr) {
-        int t = i / cv, c = i - t * cv;
-        long long src = (((tok0 + t) * p.H + h) * (long long)p.V + va) * es + c * 16;
-        int dst = t * TVS * es + c * 16;
-        cp_async16(stage + L.rv + dst, gv + src);
-        cp_async16(stage + L.rb + dst, gb + src);
-        cp_async16(stage + L.rdo + dst, gdo + src);
-        if (gdov) cp_async16(stage + L.rdov + dst, gdov + src);
-    }
-    for (int i = tid; i < nt_ext; i += nthr) cp_async4(stage + L.rgt + i * 4, p.gt + (tok0 + i) * p.H + h);
-}
+// A thread's share of TS tokens of a block on its way from global memory to the operand stage: loaded as it lies there, and
+// converted when it is stored.  Between the two the helper warps wait for a group and sum it, so that neither the loads'
+// latency nor, where rows start at any offset, the many single loads are in anybody's way.
+template <int KP, int TV, int TS, int NTH, bool UNC>
+struct BwdStaging {
+    static constexpr int F0 = NTH > 64 ? NTH - 64 : 0;  // the threads of the step sizes: neither the first nor the last warp's
+    static constexpr int K4 = KP / 4, V2 = TV / 2, NQ = (TS * K4 + NTH - 1) / NTH, NV = (TS * V2 + NTH - 1) / NTH;
+    unsigned q[NQ][4], k[NQ][4];                // 4 columns: packed 16-bit pairs in [0], [1] where they came in one load
+    unsigned v[NV][2], b[NV][2], o[NV][2], ov[NV][2];  // 2 rows: a packed 16-bit pair in [0]
+    float g0, g1;                               // step sizes of a token and the next
+};
 
-// Two consecutive staged values starting at the even element index e (shared memory).
+// N consecutive elements of ES bytes at element e, the first n of them (the others 0).
+template <int ES, int N>
+__device__ __forceinline__ void ld_words(unsigned (&w)[N], const void* base, long long e, int n, bool vec) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = 0;
+    if (vec) {
+        if (n > 0) {
+            const char* p = reinterpret_cast<const char*>(base) + e * ES;
+            if constexpr (ES * N == 16) {
+                const uint4 x = *reinterpret_cast<const uint4*>(p);
+                w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w;
+            } else if constexpr (ES * N == 8) {
+                const uint2 x = *reinterpret_cast<const uint2*>(p);
+                w[0] = x.x, w[1] = x.y;
+            } else {
+                w[0] = *reinterpret_cast<const unsigned*>(p);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (i < n)
+                w[i] = ES == 4 ? reinterpret_cast<const unsigned*>(base)[e + i] : reinterpret_cast<const unsigned short*>(base)[e + i];
+    }
+}
 template <int DT>
-__device__ __forceinline__ float2 ld2s(const unsigned char* base, int e) {
-    if (DT == PALIMPSA_F32) return *reinterpret_cast<const float2*>(base + (size_t)e * 4);
-    if (DT == PALIMPSA_BF16) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(base + (size_t)e * 2));
-    return __half22float2(*reinterpret_cast<const __half2*>(base + (size_t)e * 2));
+__device__ __forceinline__ float word_value(unsigned w) {  // of a single element
+    if (DT == PALIMPSA_F32) return __uint_as_float(w);
+    if (DT == PALIMPSA_BF16) return __uint_as_float(w << 16);
+    return __half2float(__ushort_as_half((unsigned short)w));
+}
+template <int DT, int N>
+__device__ __forceinline__ void word_values(const unsigned (&w)[N], float (&x)[N], bool vec) {
+    if (DT != PALIMPSA_F32 && vec) {
+#pragma unroll
+        for (int i = 0; i < N; i += 2) {
+            x[i] = word_value<DT>(w[i / 2] & 0xffffu);
+            x[i + 1] = word_value<DT>(w[i / 2] >> 16);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) x[i] = word_value<DT>(w[i]);
+    }
 }
 
-// One block of fp32 operands into the operand stage `op`, by `nthr` threads.
-// UNR: iterations in flight; loads from global memory want several, a warp with few registers has room for one.
-template <int DT, bool ALIGNED, bool UNC, int KP, int TV, int UNR>
-__device__ __forceinline__ void bwd_convert(const BwdArgs& a, int nthr, int tid, const unsigned char* sm, unsigned char* op,
-                                            const BwdSmem& L, long long tok0, int nt, int nt_ext, int h, int v0, int tvw,
-                                            float gh, float iph, bool carry_block) {
+// Tokens [ts, ts + TS) of the block of nt tokens that starts at token tok0 (nt_ext: with the token after it, where the
+// sequence goes on), by NTH threads.
+template <int ES, int KP, int TV, int TS, int NTH, bool UNC>
+__device__ __forceinline__ void bwd_load(BwdStaging<KP, TV, TS, NTH, UNC>& s, const BwdArgs& a, int tid, long long tok0, int ts,
+                                         int nt, int nt_ext, int h, int v0, int tvw) {
+    using S = BwdStaging<KP, TV, TS, NTH, UNC>;
     const palimpsa_problem& p = a.p;
-    constexpr int K4 = KP / 4, V2 = TV / 2;
-    const unsigned char* stage = sm + L.raw;
-    float4* qs = reinterpret_cast<float4*>(op + L.qs);
-    float4* ks = reinterpret_cast<float4*>(op + L.ks);
-    float4* qqs = reinterpret_cast<float4*>(op + L.qqs);
-    const float sc = p.scale;
-#pragma unroll UNR
-    for (int i = tid; i < TB * K4; i += nthr) {
-        int t = i / K4, c4 = i - t * K4;
-        float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), kv = qv;
-        if (t < nt && c4 * 4 < p.K) {
-            if (ALIGNED) {
-                qv = ld4<DT>(stage + L.rq, i);
-                kv = ld4<DT>(stage + L.rk, i);
-            } else {
-                long long row = ((tok0 + t) * p.H + h) * (long long)p.K;
-                qv = ld4_guarded<DT>(p.q, row + c4 * 4, row + p.K);
-                kv = ld4_guarded<DT>(p.k, row + c4 * 4, row + p.K);
-            }
-        }
-        qs[i] = make_float4(qv.x * sc, qv.y * sc, qv.z * sc, qv.w * sc);
-        ks[i] = kv;
-        if (UNC) qqs[i] = make_float4(sc * qv.x * qv.x, sc * qv.y * qv.y, sc * qv.z * qv.z, sc * qv.w * qv.w);
+#pragma unroll
+    for (int x = 0; x < S::NQ; ++x) {
+        const int i = tid + x * NTH, t = ts + i / S::K4, c = 4 * (i % S::K4);
+        const long long row = ((tok0 + t) * p.H + h) * (long long)p.K + c;
+        const int n = t < nt && i < TS * S::K4 ? p.K - c : 0;
+        ld_words<ES>(s.q[x], p.q, row, n, a.vec_k);
+        ld_words<ES>(s.k[x], p.k, row, n, a.vec_k);
     }
-    float4* vb = reinterpret_cast<float4*>(op + L.vb);
-    float4* dys = reinterpret_cast<float4*>(op + L.dys2);
-    float4* dyvs = reinterpret_cast<float4*>(op + L.dyvs2);
-    constexpr int TVS = bwd_staged_cols(TV);
-    const int voff = ALIGNED ? v0 % (16 / dtype_size(DT)) : 0;  // tile start inside the staged superset; even, as tiles are
-#pragma unroll UNR
-    for (int i = tid; i < TB * V2; i += nthr) {
-        const int t = i / V2, r = 2 * (i - t * V2);
-        float2 vv = make_float2(0.f, 0.f), bv = vv, dv = vv, dvv = vv;
-        if (t < nt && r < tvw) {
-            const bool two = r + 1 < tvw;  // the tile's last row may be the first of a pair: the second stays 0
-            if (ALIGNED) {
-                const int e = t * TVS + voff + r;
-                vv = ld2s<DT>(stage + L.rv, e);
-                bv = ld2s<DT>(stage + L.rb, e);
-                dv = ld2s<DT>(stage + L.rdo, e);
-                if (UNC) dvv = ld2s<DT>(stage + L.rdov, e);
-                if (!two) vv.y = bv.y = dv.y = dvv.y = 0.f;
-            } else {
-                const long long e = ((tok0 + t) * p.H + h) * (long long)p.V + v0 + r;
-                vv = make_float2(ld1<DT>(p.v, e), two ? ld1<DT>(p.v, e + 1) : 0.f);
-                bv = make_float2(ld1<DT>(p.b, e), two ? ld1<DT>(p.b, e + 1) : 0.f);
-                dv = make_float2(ld1<DT>(a.d_o, e), two ? ld1<DT>(a.d_o, e + 1) : 0.f);
-                if (UNC) dvv = make_float2(ld1<DT>(a.d_o_var, e), two ? ld1<DT>(a.d_o_var, e + 1) : 0.f);
-            }
+#pragma unroll
+    for (int x = 0; x < S::NV; ++x) {
+        const int i = tid + x * NTH, t = ts + i / S::V2, r = 2 * (i % S::V2);
+        const long long row = ((tok0 + t) * p.H + h) * (long long)p.V + v0 + r;
+        const int n = t < nt && i < TS * S::V2 ? tvw - r : 0;
+        ld_words<ES>(s.v[x], p.v, row, n, a.vec_v);
+        ld_words<ES>(s.b[x], p.b, row, n, a.vec_v);
+        ld_words<ES>(s.o[x], a.d_o, row, n, a.vec_v);
+        if (UNC) ld_words<ES>(s.ov[x], a.d_o_var, row, n, a.vec_v);
+    }
+    const int j = tid - S::F0, t = ts + j;
+    const bool on = j >= 0 && j < TS;
+    s.g0 = on && t < nt ? p.gt[(tok0 + t) * p.H + h] : 0.f;
+    s.g1 = on && t + 1 < nt_ext ? p.gt[(tok0 + t + 1) * p.H + h] : 0.f;
+}
+
+// What bwd_load brought, as fp32 operands into the operand stage `op`.
+template <int DT, int KP, int TV, int TS, int NTH, bool UNC>
+__device__ __forceinline__ void bwd_store(const BwdStaging<KP, TV, TS, NTH, UNC>& s, const BwdArgs& a, int tid, unsigned char* op,
+                                          const BwdSmem& L, int ts, int nt, int nt_ext, float gh, float iph, bool carry_block) {
+    using S = BwdStaging<KP, TV, TS, NTH, UNC>;
+    float4* qs = reinterpret_cast<float4*>(op + L.qs) + ts * S::K4;
+    float4* ks = reinterpret_cast<float4*>(op + L.ks) + ts * S::K4;
+    // The scale goes with q; with the uncertainty output, which wants q and q squared, with the output gradients instead.
+    const float sq = UNC ? 1.f : a.p.scale, so = UNC ? a.p.scale : 1.f;
+#pragma unroll
+    for (int x = 0; x < S::NQ; ++x) {
+        const int i = tid + x * NTH;
+        if (i >= TS * S::K4) break;
+        float q[4], k[4];
+        word_values<DT>(s.q[x], q, a.vec_k);
+        word_values<DT>(s.k[x], k, a.vec_k);
+        qs[i] = make_float4(q[0] * sq, q[1] * sq, q[2] * sq, q[3] * sq);
+        ks[i] = make_float4(k[0], k[1], k[2], k[3]);
+    }
+    float4* vb = reinterpret_cast<float4*>(op + L.vb) + ts * TV;
+    float4* dys = reinterpret_cast<float4*>(op + L.dys2) + ts * S::V2;
+    float4* dyvs = reinterpret_cast<float4*>(op + L.dyvs2) + ts * S::V2;
+#pragma unroll
+    for (int x = 0; x < S::NV; ++x) {
+        const int i = tid + x * NTH;
+        if (i >= TS * S::V2) break;
+        float v[2], b[2], o[2];
+        word_values<DT>(s.v[x], v, a.vec_v);
+        word_values<DT>(s.b[x], b, a.vec_v);
+        word_values<DT>(s.o[x], o, a.vec_v);
+        vb[2 * i] = make_float4(v[0], v[0], b[0], b[0]);
+        vb[2 * i + 1] = make_float4(v[1], v[1], b[1], b[1]);
+        dys[i] = make_float4(o[0] * so, o[0] * so, o[1] * so, o[1] * so);
+        if (UNC) {
+            word_values<DT>(s.ov[x], o, a.vec_v);
+            dyvs[i] = make_float4(o[0] * so, o[0] * so, o[1] * so, o[1] * so);
         }
-        vb[2 * i] = make_float4(vv.x, vv.x, bv.x, bv.x);
-        vb[2 * i + 1] = make_float4(vv.y, vv.y, bv.y, bv.y);
-        dys[i] = make_float4(dv.x, dv.x, dv.y, dv.y);
-        if (UNC) dyvs[i] = make_float4(dvv.x, dvv.x, dvv.y, dvv.y);
     }
     // per token: {f, f, c, c} with c = (1-f)*Ip, and {fn, fn}: f of the NEXT token of the sequence (0 past its end)
-    float4* fc2 = reinterpret_cast<float4*>(op + L.fc2);
-    float2* fn2 = reinterpret_cast<float2*>(op + L.fn2);
-    for (int i = tid; i < TB; i += nthr) {
-        float g0 = 0.f, g1 = 0.f;
-        const bool has0 = i < nt, has1 = i + 1 < nt_ext;
-        if (ALIGNED) {
-            const float* rg = reinterpret_cast<const float*>(stage + L.rgt);
-            if (has0) g0 = rg[i];
-            if (has1) g1 = rg[i + 1];
-        } else {
-            if (has0) g0 = p.gt[(tok0 + i) * p.H + h];
-            if (has1) g1 = p.gt[(tok0 + i + 1) * p.H + h];
-        }
-        const float f = expf(-g0 * gh);
-        float fn = has1 ? expf(-g1 * gh) : 0.f;
+    if (tid >= S::F0 && tid < S::F0 + TS) {
+        const int t = ts + tid - S::F0;
+        const float f = expf(-s.g0 * gh);
+        float fn = t + 1 < nt_ext ? expf(-s.g1 * gh) : 0.f;
         // Last block of a segment whose end-state gradient is supplied: that gradient is already expressed
         // at the boundary, so the last real token (and any identity padding after it) passes it on undecayed.
-        if (carry_block && i >= nt - 1) fn = 1.f;
+        if (carry_block && t >= nt - 1) fn = 1.f;
         const float c = (1.f - f) * iph;
-        fc2[i] = make_float4(f, f, c, c);
-        fn2[i] = make_float2(fn, fn);
+        reinterpret_cast<float4*>(op + L.fc2)[t] = make_float4(f, f, c, c);
+        reinterpret_cast<float2*>(op + L.fn2)[t] = make_float2(fn, fn);
     }
 }
 
@@ -299,13 +289,29 @@ __host__ __device__ constexpr RegSplit bwd_split(int W, int RV, int RK, bool unc
     return W != 8 || RV * RK != 12 ? RegSplit{0, 0, 0} : unc && RV == 3 ? RegSplit{168, 224, 56} : RegSplit{168, 208, 88};
 }
 
+// CTAs of an SM that the registers have to do for: two of the smallest tilings.  At d_k = 32 that spills 36 bytes: 148 / 296 / 740
+// CTAs of 32x32, T = 512, take 175 / 268 / 658 us, with one 148 / 289 / 715; with the uncertainty output it would spill 192:
+// 205 / 340 / 831 us against 164 / 320 / 792.
+__host__ __device__ constexpr int bwd_min_ctas(int RK, int KG, int W, bool unc) {
+    return KG == 8 && W == 4 && (RK == 2 || (RK == 4 && !unc)) ? 2 : 1;
+}
+
+// Tokens of a block that the helper warps carry through registers at a time (BwdStaging): the whole block where they have the
+// registers, since every step costs a helper its address and type branches again.
+__host__ __device__ constexpr int bwd_step_tokens(int KP, int TV, int HT, bool unc, RegSplit split) {
+    const int room = split.entry > 0 ? split.helper - 54 : 72;
+    for (int ts = TB; ts > 4; ts /= 2)
+        if ((ts * KP / 4 + HT - 1) / HT * 8 + (ts * TV / 2 + HT - 1) / HT * (unc ? 8 : 6) <= room) return ts;
+    return 4;
+}
+
 template <int RV, int NP>
 struct State {
     float2 M[RV][NP], I[RV][NP];
 };
 
 template <int RK, int KG, int RV, int W, bool UNC, bool CO>
-__global__ void __launch_bounds__(bwd_threads(W), KG == 8 && RK < 6 && W == 4 ? 2 : 1)
+__global__ void __launch_bounds__(bwd_threads(W), bwd_min_ctas(RK, KG, W, UNC))
 bwd_kernel(const BwdArgs a) {
     constexpr int KP = RK * KG, VG = 32 / KG, NP = RK / 2, NE = RV * RK, KP2 = KP / 2;
     constexpr int TV = W * VG * RV, WV = W * VG, NTHR = 32 * W, HW = bwd_helpers(W), HT = 32 * HW;
@@ -329,7 +335,7 @@ bwd_kernel(const BwdArgs a) {
     const int tvw = min(a.rows, p.V - v0);
     const int es = dtype_size(p.io_dtype);
     const int KBUF = a.kbuf;  // shared-memory buffers for the d_k-indexed partials of a token group (1 or 2)
-    const BwdSmem L = bwd_smem_layout(KP, TV, NE, NTHR, WV, es, UNC, KBUF, a.opbuf);
+    const BwdSmem L = bwd_smem_layout(KP, TV, NE, W, WV, UNC, KBUF);
     int bos, len;
     seq_range(p, n, bos, len);
     // this CTA's segment of the sequence: tokens [s0, s1), blocks [blk0, blk1)
@@ -385,67 +391,46 @@ bwd_kernel(const BwdArgs a) {
         *fail_flag = 0;
         tc::mbar_init_fence();
     }
+    // the block that is walked first, by all threads
+    auto tok0_of = [&](int it) __attribute__((always_inline)) { return (long long)bos + (blk1 - 1 - it) * TB; };
+    auto load = [&](auto& s, int id, int it, int ts) __attribute__((always_inline)) {
+        const int left = len - (blk1 - 1 - it) * TB, nt = min(TB, left), nt_ext = min(TB + 1, left);
+        if (es == 4) bwd_load<4>(s, a, id, tok0_of(it), ts, nt, nt_ext, h, v0, tvw);
+        else bwd_load<2>(s, a, id, tok0_of(it), ts, nt, nt_ext, h, v0, tvw);
+    };
+    auto store = [&](const auto& s, int id, int it, int ts) __attribute__((always_inline)) {
+        const int left = len - (blk1 - 1 - it) * TB, nt = min(TB, left), nt_ext = min(TB + 1, left);
+        const bool cblk = has_carry && it == 0;
+        unsigned char* op = sm + (it & 1) * L.op_stage;
+        if (p.io_dtype == PALIMPSA_BF16) bwd_store<PALIMPSA_BF16>(s, a, id, op, L, ts, nt, nt_ext, gh, iph, cblk);
+        else if (p.io_dtype == PALIMPSA_F32) bwd_store<PALIMPSA_F32>(s, a, id, op, L, ts, nt, nt_ext, gh, iph, cblk);
+        else bwd_store<PALIMPSA_F16>(s, a, id, op, L, ts, nt, nt_ext, gh, iph, cblk);
+    };
+    bwd_issue_ckpt(a, bwd_threads(W), tid, sm, L, 0, KP, TV, slot0 + blk1 - 1, h, v0, tvw);
+    cp_async_commit();
+    {
+        BwdStaging<KP, TV, TB, bwd_threads(W), UNC> s;
+        load(s, tid, 0, 0);
+        store(s, tid, 0, 0);
+    }
+    cp_async_wait<0>();
     __syncthreads();
 
-    if (w >= W) {
-        if constexpr (SPLIT.entry > 0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SPLIT.helper));
+    // (inlined, as every lambda in it: a call would need registers that a split warp does not have)
+    auto help = [&](const int ht) __attribute__((always_inline)) {
         // ---- helper warps ---------------------------------------------------------------------------------------
-        // In front of the walk: checkpoints and raw inputs one block ahead by cp.async, raw inputs converted to fp32
-        // operands.  Behind it, everything a group leaves once its partials lie in shared memory: dq / dk summed over
-        // the CTA's row groups and written to this row tile's partials, dv / db cast and written, the per-token scalars
-        // summed over the warps.
-        // (Every lambda is inlined: a call would need registers that a split warp does not have.)
-        constexpr int KP4 = KP / 4;
-        const int ht = tid - NTHR;
-        const int opbuf = a.opbuf;
-        auto bar_helpers = [&]() __attribute__((always_inline)) { asm volatile("bar.sync 1, %0;" ::"n"(HT) : "memory"); };
-        auto issue_ckpt = [&](int it) __attribute__((always_inline)) {
-            bwd_issue_ckpt(a, HT, ht, sm, L, it & 1, KP, TV, slot0 + blk1 - 1 - it, h, v0, tvw);
-        };
-        auto issue_raw = [&](int it) __attribute__((always_inline)) {
-            const int t0 = (blk1 - 1 - it) * TB;
-            // the step size of the token after the block too, where the sequence goes on past this segment
-            if (a.aligned)
-                bwd_issue_raw(a, HT, ht, sm, L, es, KP, TV, (long long)bos + t0, min(TB, len - t0), min(TB + 1, len - t0),
-                              h, v0, tvw);
-        };
-        auto convert = [&](int it) __attribute__((always_inline)) {
-            const int t0 = (blk1 - 1 - it) * TB, nt = min(TB, len - t0), nt_ext = min(TB + 1, len - t0);
-            const long long tok0 = (long long)bos + t0;
-            const bool cblk = has_carry && it == 0;
-            unsigned char* op = sm + (it & (opbuf - 1)) * L.op_stage;
-#define PALIMPSA_CONVERT(DT, AL) \
-    bwd_convert<DT, AL, UNC, KP, TV, (SPLIT.entry > 0 || AL ? 1 : 4)>(a, HT, ht, sm, op, L, tok0, nt, nt_ext, h, v0, tvw, gh, iph, cblk)
-            if (a.aligned) {
-                if (p.io_dtype == PALIMPSA_BF16) PALIMPSA_CONVERT(PALIMPSA_BF16, true);
-                else if (p.io_dtype == PALIMPSA_F32) PALIMPSA_CONVERT(PALIMPSA_F32, true);
-                else PALIMPSA_CONVERT(PALIMPSA_F16, true);
-            } else {
-                if (p.io_dtype == PALIMPSA_BF16) PALIMPSA_CONVERT(PALIMPSA_BF16, false);
-                else if (p.io_dtype == PALIMPSA_F32) PALIMPSA_CONVERT(PALIMPSA_F32, false);
-                else PALIMPSA_CONVERT(PALIMPSA_F16, false);
-            }
-#undef PALIMPSA_CONVERT
-        };
+        // In front of the walk: the next block's checkpoint by cp.async, its inputs TS tokens at a time through registers into
+        // the other operand stage.  Behind it, everything a group leaves once its partials lie in shared memory: dq / dk
+        // summed over the CTA's row groups and written to this row tile's partials, dv / db cast and written, the per-token
+        // scalars summed over the warps.
+        constexpr int KP4 = KP / 4, TS = bwd_step_tokens(KP, TV, HT, UNC, SPLIT);
+        BwdStaging<KP, TV, TS, HT, UNC> next;
         auto arrive_staged = [&](int it) __attribute__((always_inline)) {
             __syncwarp();
             if (lane == 0) mbar_arrive(&staged[it & 1]);
         };
-        // The raw stage is read by all helper warps: a barrier before it is converted (every lane's copies have landed)
-        // and one before it is overwritten.
-        auto convert_and_refill = [&](int it) __attribute__((always_inline)) {
-            bar_helpers();
-            convert(it);
-            bar_helpers();
-            if (it + 1 < nblk) issue_raw(it + 1);
-            cp_async_commit();
-        };
-        issue_ckpt(0);
-        issue_raw(0);
-        cp_async_commit();
-        cp_async_wait<0>();
-        convert_and_refill(0);
         arrive_staged(0);
+        if (nblk > 1) load(next, ht, 1, 0);
 
         // Two rows of dv / db in one store: d_v even (then a tile's rows are too), both buffers aligned for a pair.
         const bool pairs = V % 2 == 0 && ((reinterpret_cast<uintptr_t>(a.dv) | reinterpret_cast<uintptr_t>(a.db)) & (2 * es - 1)) == 0;
@@ -454,8 +439,24 @@ bwd_kernel(const BwdArgs a) {
             const int t0 = (blk1 - 1 - it) * TB, nt = min(TB, len - t0);
             const long long tok0 = (long long)bos + t0;
             const bool more = it + 1 < nblk;
+            int ts = 0;
 #pragma unroll 1
             for (int gi = NG - 1; gi >= 0; --gi) {
+                // While a group is walked: a step of the next block, and the loads of the step after it.
+                if (more && ts < TB) {
+                    if (ts == 0) {  // the stages were block it - 1's
+                        if (it > 0 && !wait_fail && !mbar_wait_idle(&done[(it - 1) & 1], ((it - 1) >> 1) & 1)) wait_fail = 5;
+                        bwd_issue_ckpt(a, HT, ht, sm, L, (it + 1) & 1, KP, TV, slot0 + blk1 - 2 - it, h, v0, tvw);
+                        cp_async_commit();
+                    }
+                    store(next, ht, it + 1, ts);
+                    ts += TS;
+                    if (ts < TB || it + 2 < nblk) load(next, ht, it + (ts < TB ? 1 : 2), ts < TB ? ts : 0);
+                }
+                if (more && gi == (TS < 8 ? 0 : 1)) {  // as early as can be: warps that are ahead wait for it
+                    cp_async_wait<0>();
+                    arrive_staged(it + 1);
+                }
                 if (!CO) {
                     const int b = gi & (KBUF - 1);
                     if (!wait_fail && !mbar_wait_idle(&full[b], use & 1)) wait_fail = 5;
@@ -493,7 +494,7 @@ bwd_kernel(const BwdArgs a) {
                             }
                         }
                     }
-                    if (w == W + HW - 1 && lane < ng) {
+                    if (ht >= HT - 32 && lane < ng) {
                         float df = 0.f, s2 = 0.f;
 #pragma unroll
                         for (int x = 0; x < W; ++x) {
@@ -510,353 +511,339 @@ bwd_kernel(const BwdArgs a) {
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&empty[b]);
                 }
-                // The next block, in steps between the groups of this one, so that no group waits for all of it.
-                if (gi == NG - 1 && more) {
-                    // its checkpoint stage was block it - 1's
-                    if (it > 0 && !wait_fail && !mbar_wait_idle(&done[(it - 1) & 1], ((it - 1) >> 1) & 1)) wait_fail = 5;
-                    issue_ckpt(it + 1);
-                    cp_async_commit();
-                    if (opbuf == 2) {
-                        cp_async_wait<1>();  // all but the checkpoint
-                        convert_and_refill(it + 1);
-                    }
-                }
-                if (gi == NG - 2 && more && opbuf == 2) {
-                    cp_async_wait<1>();  // all but the raw inputs of block it + 2
-                    arrive_staged(it + 1);
-                }
-            }
-            if (more && opbuf == 1) {  // the one operand stage is free once block `it` is done
-                if (!wait_fail && !mbar_wait_idle(&done[it & 1], (it >> 1) & 1)) wait_fail = 5;
-                cp_async_wait<0>();
-                convert_and_refill(it + 1);
-                arrive_staged(it + 1);
             }
         }
         cp_async_wait<0>();
         if (wait_fail) *fail_flag = wait_fail;
         __syncthreads();
-        return;
-    }
-    if constexpr (SPLIT.entry > 0) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SPLIT.compute));
-
-    if (w * VG * RV >= tvw) {
-        // A warp without rows (a tile lower than the CTA, or the last one): its share of every sum is zero, written once;
-        // after that it only keeps the hand-overs going, each no earlier than the others can use it.
-        if (!CO) {
-            for (int i = lane; i < KBUF * GR * VG * 2 * KP2; i += 32) {
-                const int bj = i / (VG * 2 * KP2);
-                reinterpret_cast<float2*>(sm + L.kred)[(bj * WV + w * VG) * 2 * KP2 + i - bj * (VG * 2 * KP2)] = make_float2(0.f, 0.f);
-            }
-            for (int i = lane; i < KBUF * GR; i += 32)
-                reinterpret_cast<float2*>(wred)[((i / GR) * W + w) * GR + i % GR] = make_float2(0.f, 0.f);
-        }
-        for (int it = 0; it < nblk; ++it) {
-            if (!wait_fail && !mbar_wait_idle(&staged[it & 1], (it >> 1) & 1)) wait_fail = 6;
-            for (int gi = NG - 1; !CO && gi >= 0; --gi) {
-                const int b = gi & (KBUF - 1);
-                if (!wait_fail && !mbar_wait_idle(&empty[b], (use & 1) ^ 1)) wait_fail = 6;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full[b]);
-                if (b == 0) ++use;
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&done[it & 1]);
-        }
-        if (wait_fail) *fail_flag = wait_fail;
-        __syncthreads();
-        return;
-    }
-
-    float4* slots4 = reinterpret_cast<float4*>(sm + L.slots) + tid;
-    float2* kred2 = reinterpret_cast<float2*>(sm + L.kred);
-
-    // running state gradients: GM = dL/dM_t, nGI = -dL/dI_t of the earliest token processed so far
-    float2 GM[RV][NP], nGI[RV][NP];
-#pragma unroll
-    for (int r = 0; r < RV; ++r)
-#pragma unroll
-        for (int q = 0; q < NP; ++q) {
-            GM[r][q] = nGI[r][q] = make_float2(0.f, 0.f);
-            if (has_carry && row0 + r < tvw) {
-                const long long e = (seg_base + v0 + row0 + r) * KP + RK * kg + 2 * q;
-                const float2 cm = *reinterpret_cast<const float2*>(a.carry_M + e);
-                const float2 ci = *reinterpret_cast<const float2*>(a.carry_I + e);
-                GM[r][q] = cm;
-                nGI[r][q] = make_float2(-ci.x, -ci.y);
-            }
-        }
-
-    // pairs of adjacent columns or rows: two 8-byte pairs go as one 16-byte access where the tiling allows it
-    auto ld_pairs = [&](const float2* base, float2 (&dst)[NP]) __attribute__((always_inline)) {
-        if constexpr (NP % 2 == 0) {
-#pragma unroll
-            for (int q = 0; q < NP; q += 2) {
-                const float4 x = *reinterpret_cast<const float4*>(base + q);
-                dst[q] = make_float2(x.x, x.y);
-                dst[q + 1] = make_float2(x.z, x.w);
-            }
-        } else {
-#pragma unroll
-            for (int q = 0; q < NP; ++q) dst[q] = base[q];
-        }
     };
-    // no memory operand: the next token's operands may be loaded above it (they lie elsewhere)
-    auto st_pairs = [&](float2* base, const float2 (&src)[NP]) __attribute__((always_inline)) {
-        if constexpr (NP % 2 == 0) {
-#pragma unroll
-            for (int q = 0; q < NP; q += 2)
-                asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(tc::smem_u32(base + q)), "f"(src[q].x), "f"(src[q].y),
-                             "f"(src[q + 1].x), "f"(src[q + 1].y));
-        } else {
-#pragma unroll
-            for (int q = 0; q < NP; ++q)
-                asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(tc::smem_u32(base + q)), "f"(src[q].x), "f"(src[q].y));
-        }
-    };
-    auto ld_rows = [&](const float2* base, float2 (&dst)[RV]) __attribute__((always_inline)) {
-        if constexpr (RV % 2 == 0) {
-#pragma unroll
-            for (int r = 0; r < RV; r += 2) {
-                const float4 x = *reinterpret_cast<const float4*>(base + r);
-                dst[r] = make_float2(x.x, x.y);
-                dst[r + 1] = make_float2(x.z, x.w);
-            }
-        } else {
-#pragma unroll
-            for (int r = 0; r < RV; ++r) dst[r] = base[r];
-        }
-    };
-    auto load_ck = [&](State<RV, NP>& s, int stage_idx) __attribute__((always_inline)) {
-        const float2* ckM = reinterpret_cast<const float2*>(sm + L.ckb + stage_idx * L.ck_stage) + row0 * KP2 + NP * kg;
-#pragma unroll
-        for (int r = 0; r < RV; ++r) {
-            ld_pairs(ckM + r * KP2, s.M[r]);
-            ld_pairs(ckM + (TV + r) * KP2, s.I[r]);
-            if (row0 + r >= tvw) {
-#pragma unroll
-                for (int q = 0; q < NP; ++q) {
-                    s.M[r][q] = make_float2(0.f, 0.f);
-                    s.I[r][q] = make_float2(1.f, 1.f);
+    // ---- compute warps -------------------------------------------------------------------------------------------------
+    auto walk = [&]() __attribute__((always_inline)) {
+        if (w * VG * RV >= tvw) {
+            // A warp without rows (a tile lower than the CTA, or the last one): its share of every sum is zero, written once;
+            // after that it only keeps the hand-overs going, each no earlier than the others can use it.
+            if (!CO) {
+                for (int i = lane; i < KBUF * GR * VG * 2 * KP2; i += 32) {
+                    const int bj = i / (VG * 2 * KP2);
+                    reinterpret_cast<float2*>(sm + L.kred)[(bj * WV + w * VG) * 2 * KP2 + i - bj * (VG * 2 * KP2)] = make_float2(0.f, 0.f);
                 }
+                for (int i = lane; i < KBUF * GR; i += 32)
+                    reinterpret_cast<float2*>(wred)[((i / GR) * W + w) * GR + i % GR] = make_float2(0.f, 0.f);
             }
+            for (int it = 0; it < nblk; ++it) {
+                if (!wait_fail && !mbar_wait_idle(&staged[it & 1], (it >> 1) & 1)) wait_fail = 6;
+                for (int gi = NG - 1; !CO && gi >= 0; --gi) {
+                    const int b = gi & (KBUF - 1);
+                    if (!wait_fail && !mbar_wait_idle(&empty[b], (use & 1) ^ 1)) wait_fail = 6;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&full[b]);
+                    if (b == 0) ++use;
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&done[it & 1]);
+            }
+            if (wait_fail) *fail_flag = wait_fail;
+            __syncthreads();
+            return;
         }
-    };
-    auto load_slot = [&](State<RV, NP>& s, int slot) {
-        const float4* sl = slots4 + slot * (NE / 2) * NTHR;
+
+        float4* slots4 = reinterpret_cast<float4*>(sm + L.slots) + tid;
+        float2* kred2 = reinterpret_cast<float2*>(sm + L.kred);
+
+        // running state gradients: GM = dL/dM_t, nGI = -dL/dI_t of the earliest token processed so far
+        float2 GM[RV][NP], nGI[RV][NP];
 #pragma unroll
         for (int r = 0; r < RV; ++r)
 #pragma unroll
             for (int q = 0; q < NP; ++q) {
-                const float4 x = sl[(r * NP + q) * NTHR];
-                s.M[r][q] = make_float2(x.x, x.y);
-                s.I[r][q] = make_float2(x.z, x.w);
+                GM[r][q] = nGI[r][q] = make_float2(0.f, 0.f);
+                if (has_carry && row0 + r < tvw) {
+                    const long long e = (seg_base + v0 + row0 + r) * KP + RK * kg + 2 * q;
+                    const float2 cm = *reinterpret_cast<const float2*>(a.carry_M + e);
+                    const float2 ci = *reinterpret_cast<const float2*>(a.carry_I + e);
+                    GM[r][q] = cm;
+                    nGI[r][q] = make_float2(-ci.x, -ci.y);
+                }
             }
-    };
-    auto store_slot = [&](const State<RV, NP>& s, int slot) {
-        float4* sl = slots4 + slot * (NE / 2) * NTHR;
+
+        // pairs of adjacent columns or rows: two 8-byte pairs go as one 16-byte access where the tiling allows it
+        auto ld_pairs = [&](const float2* base, float2 (&dst)[NP]) __attribute__((always_inline)) {
+            if constexpr (NP % 2 == 0) {
 #pragma unroll
-        for (int r = 0; r < RV; ++r)
+                for (int q = 0; q < NP; q += 2) {
+                    const float4 x = *reinterpret_cast<const float4*>(base + q);
+                    dst[q] = make_float2(x.x, x.y);
+                    dst[q + 1] = make_float2(x.z, x.w);
+                }
+            } else {
 #pragma unroll
-            for (int q = 0; q < NP; ++q)
-                sl[(r * NP + q) * NTHR] = make_float4(s.M[r][q].x, s.M[r][q].y, s.I[r][q].x, s.I[r][q].y);
-    };
-    float f0 = 1.f;  // f of the last processed block's first token
-    for (int it = 0; it < nblk; ++it) {
-        const int st = it & 1;
-        // this block's operand stage; this thread's d_k columns are RK*kg .. RK*kg+RK-1: pair q covers columns RK*kg + 2q, +1
-        const unsigned char* op = sm + (it & (a.opbuf - 1)) * L.op_stage;
-        const float2* ks2 = reinterpret_cast<const float2*>(op + L.ks) + NP * kg;
-        const float2* qs2 = reinterpret_cast<const float2*>(op + L.qs) + NP * kg;
-        const float2* qqs2 = reinterpret_cast<const float2*>(op + L.qqs) + NP * kg;
-        const float4* vb4 = reinterpret_cast<const float4*>(op + L.vb) + row0;
-        const float2* dys2 = reinterpret_cast<const float2*>(op + L.dys2) + row0;
-        const float2* dyvs2 = reinterpret_cast<const float2*>(op + L.dyvs2) + row0;
-        const float4* fc2 = reinterpret_cast<const float4*>(op + L.fc2);
-        const float2* fn2 = reinterpret_cast<const float2*>(op + L.fn2);
-        // one forward step of the recurrence on token tl of the staged block
-        auto fstep = [&](State<RV, NP>& s, int tl) __attribute__((always_inline)) {
-            const float4 fv = fc2[tl];
-            const float2 ff = make_float2(fv.x, fv.y), cc = make_float2(fv.z, fv.w);
-            float2 kpv[NP], kk[NP];
-            ld_pairs(ks2 + tl * KP2, kpv);
+                for (int q = 0; q < NP; ++q) dst[q] = base[q];
+            }
+        };
+        // no memory operand: the next token's operands may be loaded above it (they lie elsewhere)
+        auto st_pairs = [&](float2* base, const float2 (&src)[NP]) __attribute__((always_inline)) {
+            if constexpr (NP % 2 == 0) {
 #pragma unroll
-            for (int q = 0; q < NP; ++q) kk[q] = fmul2(kpv[q], kpv[q]);
+                for (int q = 0; q < NP; q += 2)
+                    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(tc::smem_u32(base + q)), "f"(src[q].x), "f"(src[q].y),
+                                 "f"(src[q + 1].x), "f"(src[q + 1].y));
+            } else {
+#pragma unroll
+                for (int q = 0; q < NP; ++q)
+                    asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(tc::smem_u32(base + q)), "f"(src[q].x), "f"(src[q].y));
+            }
+        };
+        auto ld_rows = [&](const float2* base, float2 (&dst)[RV]) __attribute__((always_inline)) {
+            if constexpr (RV % 2 == 0) {
+#pragma unroll
+                for (int r = 0; r < RV; r += 2) {
+                    const float4 x = *reinterpret_cast<const float4*>(base + r);
+                    dst[r] = make_float2(x.x, x.y);
+                    dst[r + 1] = make_float2(x.z, x.w);
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < RV; ++r) dst[r] = base[r];
+            }
+        };
+        auto load_ck = [&](State<RV, NP>& s, int stage_idx) __attribute__((always_inline)) {
+            const float2* ckM = reinterpret_cast<const float2*>(sm + L.ckb + stage_idx * L.ck_stage) + row0 * KP2 + NP * kg;
 #pragma unroll
             for (int r = 0; r < RV; ++r) {
-                const float4 x = vb4[tl * TV + r];
-                const float2 vr = make_float2(x.x, x.y), br = make_float2(x.z, x.w);
+                ld_pairs(ckM + r * KP2, s.M[r]);
+                ld_pairs(ckM + (TV + r) * KP2, s.I[r]);
+                if (row0 + r >= tvw) {
 #pragma unroll
-                for (int q = 0; q < NP; ++q) {
-                    s.M[r][q] = ffma2(ff, s.M[r][q], fmul2(vr, kpv[q]));
-                    s.I[r][q] = ffma2(ff, s.I[r][q], ffma2(br, kk[q], cc));
+                    for (int q = 0; q < NP; ++q) {
+                        s.M[r][q] = make_float2(0.f, 0.f);
+                        s.I[r][q] = make_float2(1.f, 1.f);
+                    }
                 }
             }
         };
-        if (!wait_fail && !tc::mbar_wait(&staged[st], (it >> 1) & 1)) wait_fail = 6;
-
-        // Tokens past the end of the sequence (last block only) were staged as identity steps (f = 1,
-        // all other operands 0): they leave the state and every gradient untouched, so the block is
-        // always processed as NG full groups with no per-token conditionals.
-        // ---- forward sweep: park the start states of groups 1 .. NG-2, keep the last group's in registers
-        State<RV, NP> P[GR + 1];
-        load_ck(P[0], st);
-#pragma unroll 1
-        for (int g = 0; g < NG - 1; ++g) {
+        auto load_slot = [&](State<RV, NP>& s, int slot) {
+            const float4* sl = slots4 + slot * (NE / 2) * NTHR;
 #pragma unroll
-            for (int j = 0; j < GR; ++j) fstep(P[0], g * GR + j);
-            if (g < NG - 2) store_slot(P[0], g);
-        }
-
-#pragma unroll 1
-        for (int gi = NG - 1; gi >= 0; --gi) {
-            if (gi == 0)
-                load_ck(P[0], st);
-            else if (gi < NG - 1)
-                load_slot(P[0], gi - 1);
-#pragma unroll
-            for (int j = 0; j < GR; ++j) {
-                P[j + 1] = P[j];
-                fstep(P[j + 1], gi * GR + j);
-            }
-            const int b = gi & (KBUF - 1);
-            float red1[NR1], red2[NR2];
-            // ---- reverse walk over the group ----------------------------------------------------
-#pragma unroll
-            for (int j = GR - 1; j >= 0; --j) {
-                const int tl = gi * GR + j;
-                const float2 fn = fn2[tl];
-                float2 dqs[NP], Ak[NP], Bk[NP], Uk[NP];
-                constexpr int RS = RV == 2 ? 2 : 1;  // accumulators: two shorten the dependent chains, three cost registers
-                float2 Sa[RS], Sb[RS], Sc[RS];
-#pragma unroll
-                for (int r = 0; r < RS; ++r) Sa[r] = Sb[r] = Sc[r] = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int q = 0; q < NP; ++q) dqs[q] = Ak[q] = Bk[q] = Uk[q] = make_float2(0.f, 0.f);
-                float2 kp[NP], kk[NP], qp[NP], qq[NP];
-                ld_pairs(ks2 + tl * KP2, kp);
-                ld_pairs(qs2 + tl * KP2, qp);
+            for (int r = 0; r < RV; ++r)
 #pragma unroll
                 for (int q = 0; q < NP; ++q) {
-                    kk[q] = fmul2(kp[q], kp[q]);
-                    qq[q] = make_float2(0.f, 0.f);
+                    const float4 x = sl[(r * NP + q) * NTHR];
+                    s.M[r][q] = make_float2(x.x, x.y);
+                    s.I[r][q] = make_float2(x.z, x.w);
                 }
-                if (UNC) ld_pairs(qqs2 + tl * KP2, qq);
-                float2 dyr[RV], dyvr[RV];
-                ld_rows(dys2 + tl * TV, dyr);
+        };
+        auto store_slot = [&](const State<RV, NP>& s, int slot) {
+            float4* sl = slots4 + slot * (NE / 2) * NTHR;
 #pragma unroll
-                for (int r = 0; r < RV; ++r) dyvr[r] = make_float2(0.f, 0.f);
-                if (UNC) ld_rows(dyvs2 + tl * TV, dyvr);
+            for (int r = 0; r < RV; ++r)
+#pragma unroll
+                for (int q = 0; q < NP; ++q)
+                    sl[(r * NP + q) * NTHR] = make_float4(s.M[r][q].x, s.M[r][q].y, s.I[r][q].x, s.I[r][q].y);
+        };
+        float f0 = 1.f;  // f of the last processed block's first token
+        for (int it = 0; it < nblk; ++it) {
+            const int st = it & 1;
+            // this block's operand stage; this thread's d_k columns are RK*kg .. RK*kg+RK-1: pair q covers columns RK*kg + 2q, +1
+            const unsigned char* op = sm + st * L.op_stage;
+            const float2* ks2 = reinterpret_cast<const float2*>(op + L.ks) + NP * kg;
+            const float2* qs2 = reinterpret_cast<const float2*>(op + L.qs) + NP * kg;
+            const float4* vb4 = reinterpret_cast<const float4*>(op + L.vb) + row0;
+            const float2* dys2 = reinterpret_cast<const float2*>(op + L.dys2) + row0;
+            const float2* dyvs2 = reinterpret_cast<const float2*>(op + L.dyvs2) + row0;
+            const float4* fc2 = reinterpret_cast<const float4*>(op + L.fc2);
+            const float2* fn2 = reinterpret_cast<const float2*>(op + L.fn2);
+            // one forward step of the recurrence on token tl of the staged block
+            auto fstep = [&](State<RV, NP>& s, int tl) __attribute__((always_inline)) {
+                const float4 fv = fc2[tl];
+                const float2 ff = make_float2(fv.x, fv.y), cc = make_float2(fv.z, fv.w);
+                float2 kpv[NP], kk[NP];
+                ld_pairs(ks2 + tl * KP2, kpv);
+#pragma unroll
+                for (int q = 0; q < NP; ++q) kk[q] = fmul2(kpv[q], kpv[q]);
 #pragma unroll
                 for (int r = 0; r < RV; ++r) {
                     const float4 x = vb4[tl * TV + r];
-                    const float2 vv = make_float2(x.x, x.y), bv = make_float2(x.z, x.w);
-                    const float2 dy = dyr[r];
-                    const float2 dyv = dyvr[r];
-                    float2 dva = make_float2(0.f, 0.f), dba = dva;
+                    const float2 vr = make_float2(x.x, x.y), br = make_float2(x.z, x.w);
 #pragma unroll
                     for (int q = 0; q < NP; ++q) {
-                        const float2 Mt = P[j + 1].M[r][q], It = P[j + 1].I[r][q];
-                        const float2 rr = rcp2(It);
-                        const float2 mu = fmul2(Mt, rr);
-                        const float2 hh = fmul2(fmul2(dy, qp[q]), rr);
-                        GM[r][q] = ffma2(fn, GM[r][q], hh);
-                        float2 hm = fmul2(hh, mu);
-                        if (UNC) hm = ffma2(fmul2(dyv, qq[q]), fmul2(rr, rr), hm);
-                        nGI[r][q] = ffma2(fn, nGI[r][q], hm);
-                        if (!CO) {
-                            dqs[q] = ffma2(dy, mu, dqs[q]);
-                            if (UNC) Uk[q] = ffma2(dyv, rr, Uk[q]);
-                            Ak[q] = ffma2(GM[r][q], vv, Ak[q]);
-                            Bk[q] = ffma2(nGI[r][q], bv, Bk[q]);
-                            dva = ffma2(GM[r][q], kp[q], dva);
-                            dba = ffma2(nGI[r][q], kk[q], dba);
-                            Sa[r % RS] = ffma2(GM[r][q], P[j].M[r][q], Sa[r % RS]);
-                            Sb[r % RS] = ffma2(nGI[r][q], P[j].I[r][q], Sb[r % RS]);
-                            Sc[r % RS] = fadd2(Sc[r % RS], nGI[r][q]);
+                        s.M[r][q] = ffma2(ff, s.M[r][q], fmul2(vr, kpv[q]));
+                        s.I[r][q] = ffma2(ff, s.I[r][q], ffma2(br, kk[q], cc));
+                    }
+                }
+            };
+            if (!wait_fail && !tc::mbar_wait(&staged[st], (it >> 1) & 1)) wait_fail = 6;
+
+            // Tokens past the end of the sequence (last block only) were staged as identity steps (f = 1,
+            // all other operands 0): they leave the state and every gradient untouched, so the block is
+            // always processed as NG full groups with no per-token conditionals.
+            // ---- forward sweep: park the start states of groups 1 .. NG-2, keep the last group's in registers
+            State<RV, NP> P[GR + 1];
+            load_ck(P[0], st);
+#pragma unroll 1
+            for (int g = 0; g < NG - 1; ++g) {
+#pragma unroll
+                for (int j = 0; j < GR; ++j) fstep(P[0], g * GR + j);
+                if (g < NG - 2) store_slot(P[0], g);
+            }
+
+#pragma unroll 1
+            for (int gi = NG - 1; gi >= 0; --gi) {
+                if (gi == 0)
+                    load_ck(P[0], st);
+                else if (gi < NG - 1)
+                    load_slot(P[0], gi - 1);
+#pragma unroll
+                for (int j = 0; j < GR; ++j) {
+                    P[j + 1] = P[j];
+                    fstep(P[j + 1], gi * GR + j);
+                }
+                const int b = gi & (KBUF - 1);
+                float red1[NR1], red2[NR2];
+                // ---- reverse walk over the group ----------------------------------------------------
+#pragma unroll
+                for (int j = GR - 1; j >= 0; --j) {
+                    const int tl = gi * GR + j;
+                    const float2 fn = fn2[tl];
+                    float2 dqs[NP], Ak[NP], Bk[NP], Uk[NP];
+                    constexpr int RS = RV == 2 ? 2 : 1;  // accumulators: two shorten the dependent chains, three cost registers
+                    float2 Sa[RS], Sb[RS], Sc[RS];
+#pragma unroll
+                    for (int r = 0; r < RS; ++r) Sa[r] = Sb[r] = Sc[r] = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int q = 0; q < NP; ++q) dqs[q] = Ak[q] = Bk[q] = Uk[q] = make_float2(0.f, 0.f);
+                    float2 kp[NP], kk[NP], qp[NP];
+                    ld_pairs(ks2 + tl * KP2, kp);
+                    ld_pairs(qs2 + tl * KP2, qp);
+#pragma unroll
+                    for (int q = 0; q < NP; ++q) kk[q] = fmul2(kp[q], kp[q]);
+                    float2 dyr[RV], dyvr[RV];
+                    ld_rows(dys2 + tl * TV, dyr);
+#pragma unroll
+                    for (int r = 0; r < RV; ++r) dyvr[r] = make_float2(0.f, 0.f);
+                    if (UNC) ld_rows(dyvs2 + tl * TV, dyvr);
+#pragma unroll
+                    for (int r = 0; r < RV; ++r) {
+                        const float4 x = vb4[tl * TV + r];
+                        const float2 vv = make_float2(x.x, x.y), bv = make_float2(x.z, x.w);
+                        const float2 dy = dyr[r];
+                        const float2 dyv = dyvr[r];
+                        float2 dva = make_float2(0.f, 0.f), dba = dva;
+#pragma unroll
+                        for (int q = 0; q < NP; ++q) {
+                            const float2 Mt = P[j + 1].M[r][q], It = P[j + 1].I[r][q];
+                            const float2 rr = rcp2(It);
+                            const float2 mu = fmul2(Mt, rr);
+                            const float2 qr = UNC ? fmul2(qp[q], rr) : make_float2(0.f, 0.f);
+                        const float2 hh = UNC ? fmul2(dy, qr) : fmul2(fmul2(dy, qp[q]), rr);
+                            GM[r][q] = ffma2(fn, GM[r][q], hh);
+                            float2 hm = fmul2(hh, mu);
+                            if (UNC) hm = ffma2(fmul2(dyv, qr), qr, hm);
+                            nGI[r][q] = ffma2(fn, nGI[r][q], hm);
+                            if (!CO) {
+                                dqs[q] = ffma2(dy, mu, dqs[q]);
+                                if (UNC) Uk[q] = ffma2(dyv, rr, Uk[q]);
+                                Ak[q] = ffma2(GM[r][q], vv, Ak[q]);
+                                Bk[q] = ffma2(nGI[r][q], bv, Bk[q]);
+                                dva = ffma2(GM[r][q], kp[q], dva);
+                                dba = ffma2(nGI[r][q], kk[q], dba);
+                                Sa[r % RS] = ffma2(GM[r][q], P[j].M[r][q], Sa[r % RS]);
+                                Sb[r % RS] = ffma2(nGI[r][q], P[j].I[r][q], Sb[r % RS]);
+                                Sc[r % RS] = fadd2(Sc[r % RS], nGI[r][q]);
+                            }
                         }
+                        red1[(j * RV + r) * 2 + 0] = dva.x + dva.y;
+                        red1[(j * RV + r) * 2 + 1] = -(dba.x + dba.y);
                     }
-                    red1[(j * RV + r) * 2 + 0] = dva.x + dva.y;
-                    red1[(j * RV + r) * 2 + 1] = -(dba.x + dba.y);
+                    // this row group's share of dq and dk for the token -> shared memory
+                    if (!CO) {
+                        if (j == GR - 1)  // first write of the group: the helpers must be done with the buffer's last contents
+                            if (!wait_fail && !tc::mbar_wait(&empty[b], (use & 1) ^ 1)) wait_fail = 6;  // after one failure: no more waiting
+                        float2* dst = kred2 + b * (GR * WV * 2 * KP2) + ((j * WV + wv) * 2) * KP2 + NP * kg;
+                        const float2 sc2 = dup2(p.scale), m2 = dup2(-2.f);
+#pragma unroll
+                        for (int q = 0; q < NP; ++q) {
+                            dqs[q] = UNC ? ffma2(fmul2(dup2(2.f), qp[q]), Uk[q], dqs[q]) : fmul2(sc2, dqs[q]);
+                            Ak[q] = ffma2(fmul2(m2, kp[q]), Bk[q], Ak[q]);
+                        }
+                        st_pairs(dst, dqs);
+                        st_pairs(dst + KP2, Ak);
+                    }
+                    float2 sa = Sa[0], sb = Sb[0], scv = Sc[0];
+#pragma unroll
+                    for (int r = 1; r < RS; ++r) {
+                        sa = fadd2(sa, Sa[r]);
+                        sb = fadd2(sb, Sb[r]);
+                        scv = fadd2(scv, Sc[r]);
+                    }
+                    const float sc_ = scv.x + scv.y;
+                    red2[j * 2 + 0] = (sa.x + sa.y) - (sb.x + sb.y) + iph * sc_;
+                    red2[j * 2 + 1] = -sc_;
                 }
-                // this row group's share of dq and dk for the token -> shared memory
-                if (!CO) {
-                    if (j == GR - 1)  // first write of the group: the helpers must be done with the buffer's last contents
-                        if (!wait_fail && !tc::mbar_wait(&empty[b], (use & 1) ^ 1)) wait_fail = 6;  // after one failure: no more waiting
-                    float2* dst = kred2 + b * (GR * WV * 2 * KP2) + ((j * WV + wv) * 2) * KP2 + NP * kg;
-                    const float2 sc2 = dup2(p.scale), m2 = dup2(-2.f);
+                if (CO) continue;  // carry-only pass: nothing but the state gradients is wanted
+                // d_v-indexed sums over the KG lanes of a row; per-token scalars over the whole warp
+                xreduce<NR1, KG>(red1, lane);
+                {
+                    const int base = xreduce_index<NR1, KG>(lane), count = xreduce_count<NR1, KG>(lane);
+#pragma unroll
+                    for (int i = 0; i < xreduce_most<NR1, KG>(); ++i)
+                        if (i < count) {
+                            const int id = base + i;
+                            const int j = id / (RV * 2), r = (id / 2) % RV, which = id & 1;
+                            (which ? dbs : dvs)[(b * GR + j) * TV + row0 + r] = red1[i];
+                        }
+                }
+                xreduce<NR2, 32>(red2, lane);
+                if ((lane & (32 / NR2 - 1)) == 0) {
+                    const int id = xreduce_index<NR2, 32>(lane);
+                    wred[((b * W + w) * GR + (id >> 1)) * 2 + (id & 1)] = red2[0];
+                }
+                if (tid < GR) fgr[b * GR + tid] = fc2[gi * GR + tid].x;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[b]);  // this warp's partials of the group are written
+                if (b == 0) ++use;
+            }
+            f0 = fc2[0].x;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&done[st]);
+        }
+
+        if (wait_fail) *fail_flag = wait_fail;
+        __syncthreads();
+        const bool failed = *fail_flag != 0;
+        if (tid == 0 && failed) {
+            // a barrier wait ran out: record it and mark this CTA's results as invalid (NaN in the decay-gradient
+            // partial of its first token, which the finishing kernels carry into dgt and dg; or in the state gradients below)
+            atomicCAS(&g_bwd_status, 0, *fail_flag);
+            if (!CO) a.df_part[(size_t)tile * a.rows_total + (size_t)((long long)bos + s0) * p.H + h] = __int_as_float(0x7fc00000);
+        }
+
+        // ---- gradient w.r.t. the segment's start state: decay the first token's totals once more ----------
+        if (a.rloc_M) {
+            if (failed) f0 = __int_as_float(0x7fc00000);
+#pragma unroll
+            for (int r = 0; r < RV; ++r) {
+                if (row0 + r < tvw) {
 #pragma unroll
                     for (int q = 0; q < NP; ++q) {
-                        dqs[q] = fmul2(sc2, dqs[q]);
-                        if (UNC) dqs[q] = ffma2(fmul2(dup2(2.f), qp[q]), Uk[q], dqs[q]);
-                        Ak[q] = ffma2(fmul2(m2, kp[q]), Bk[q], Ak[q]);
+                        const long long e = (seg_base + v0 + row0 + r) * KP + RK * kg + 2 * q;
+                        *reinterpret_cast<float2*>(a.rloc_M + e) = make_float2(f0 * GM[r][q].x, f0 * GM[r][q].y);
+                        *reinterpret_cast<float2*>(a.rloc_I + e) = make_float2(-f0 * nGI[r][q].x, -f0 * nGI[r][q].y);
                     }
-                    st_pairs(dst, dqs);
-                    st_pairs(dst + KP2, Ak);
-                }
-                float2 sa = Sa[0], sb = Sb[0], scv = Sc[0];
-#pragma unroll
-                for (int r = 1; r < RS; ++r) {
-                    sa = fadd2(sa, Sa[r]);
-                    sb = fadd2(sb, Sb[r]);
-                    scv = fadd2(scv, Sc[r]);
-                }
-                const float sc_ = scv.x + scv.y;
-                red2[j * 2 + 0] = (sa.x + sa.y) - (sb.x + sb.y) + iph * sc_;
-                red2[j * 2 + 1] = -sc_;
-            }
-            if (CO) continue;  // carry-only pass: nothing but the state gradients is wanted
-            // d_v-indexed sums over the KG lanes of a row; per-token scalars over the whole warp
-            xreduce<NR1, KG>(red1, lane);
-            {
-                const int base = xreduce_index<NR1, KG>(lane), count = xreduce_count<NR1, KG>(lane);
-#pragma unroll
-                for (int i = 0; i < xreduce_most<NR1, KG>(); ++i)
-                    if (i < count) {
-                        const int id = base + i;
-                        const int j = id / (RV * 2), r = (id / 2) % RV, which = id & 1;
-                        (which ? dbs : dvs)[(b * GR + j) * TV + row0 + r] = red1[i];
-                    }
-            }
-            xreduce<NR2, 32>(red2, lane);
-            if ((lane & (32 / NR2 - 1)) == 0) {
-                const int id = xreduce_index<NR2, 32>(lane);
-                wred[((b * W + w) * GR + (id >> 1)) * 2 + (id & 1)] = red2[0];
-            }
-            if (tid < GR) fgr[b * GR + tid] = fc2[gi * GR + tid].x;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&full[b]);  // this warp's partials of the group are written
-            if (b == 0) ++use;
-        }
-        f0 = fc2[0].x;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&done[st]);
-    }
-
-    if (wait_fail) *fail_flag = wait_fail;
-    __syncthreads();
-    const bool failed = *fail_flag != 0;
-    if (tid == 0 && failed) {
-        // a barrier wait ran out: record it and mark this CTA's results as invalid (NaN in the decay-gradient
-        // partial of its first token, which the finishing kernels carry into dgt and dg; or in the state gradients below)
-        atomicCAS(&g_bwd_status, 0, *fail_flag);
-        if (!CO) a.df_part[(size_t)tile * a.rows_total + (size_t)((long long)bos + s0) * p.H + h] = __int_as_float(0x7fc00000);
-    }
-
-    // ---- gradient w.r.t. the segment's start state: decay the first token's totals once more ----------
-    if (a.rloc_M) {
-        if (failed) f0 = __int_as_float(0x7fc00000);
-#pragma unroll
-        for (int r = 0; r < RV; ++r) {
-            if (row0 + r < tvw) {
-#pragma unroll
-                for (int q = 0; q < NP; ++q) {
-                    const long long e = (seg_base + v0 + row0 + r) * KP + RK * kg + 2 * q;
-                    *reinterpret_cast<float2*>(a.rloc_M + e) = make_float2(f0 * GM[r][q].x, f0 * GM[r][q].y);
-                    *reinterpret_cast<float2*>(a.rloc_I + e) = make_float2(-f0 * nGI[r][q].x, -f0 * nGI[r][q].y);
                 }
             }
         }
+    };
+    // The roles in two orders, for the register allocation that comes of it: with the uncertainty output and 6 or 4 warps of 12
+    // elements the walk takes 302 us a wave (48x48, T = 512) with its code first and 319 with the helpers' first.
+    if (UNC && w < W) {
+        if constexpr (SPLIT.entry > 0) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SPLIT.compute));
+        walk();
+    } else if (UNC || w >= W) {
+        if constexpr (SPLIT.entry > 0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SPLIT.helper));
+        help(tid - NTHR);
+    } else {
+        if constexpr (SPLIT.entry > 0) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SPLIT.compute));
+        walk();
     }
 }
 
@@ -1002,17 +989,16 @@ static BwdShape bwd_shape(int KP) {
     }
 }
 // Tile heights a CTA may have at each tiling, as W compute warps of RV rows a thread (launch_bwd_t instantiates these); a
-// tile lower than its warps hold leaves the last ones idle.  8 warps of 3 rows hold 24 (48 at d_k = 64) and are run with 22
-// (44) where that makes as many tiles.
+// tile lower than its warps hold leaves the last ones idle.  8 warps of 3 rows hold 24 (48 at d_k = 64): 22 (44) rows cost them
+// the same and come first, for the tiles of a d_v that both cut into as many.
 struct BwdTile {
     int rows, RV, W;
 };
 static const BwdTile* bwd_tile_choices(int KP) {
-    static const BwdTile k16[] = {{64, 2, 8}, {32, 2, 4}, {}}, k48[] = {{64, 2, 8}, {56, 2, 8}, {48, 2, 6}, {32, 2, 4}, {}},
-                         k64[] = {{44, 3, 8}, {32, 2, 8}, {16, 2, 4}, {}},
-                         k96[] = {{32, 2, 8}, {28, 2, 8}, {24, 2, 6}, {16, 2, 4}, {}},
+    static const BwdTile k16[] = {{64, 2, 8}, {32, 2, 4}, {}}, k48[] = {{64, 2, 8}, {48, 2, 6}, {32, 2, 4}, {}},
+                         k64[] = {{44, 3, 8}, {32, 2, 8}, {16, 2, 4}, {}}, k96[] = {{32, 2, 8}, {24, 2, 6}, {16, 2, 4}, {}},
                          k128[] = {{22, 3, 8}, {24, 3, 8}, {16, 2, 8}, {8, 2, 4}, {}},
-                         k192[] = {{16, 2, 8}, {14, 2, 8}, {12, 2, 6}, {8, 2, 4}, {}}, k256[] = {{8, 1, 8}, {}};
+                         k192[] = {{16, 2, 8}, {12, 2, 6}, {8, 2, 4}, {}}, k256[] = {{8, 1, 8}, {}};
     switch (KP) {
         case 48: return k48;
         case 64: return k64;
@@ -1023,19 +1009,19 @@ static const BwdTile* bwd_tile_choices(int KP) {
         default: return k16;
     }
 }
-// What a token costs a CTA (the walk, and what does not grow with the rows), in units of which 4 warps of 8 elements take 8.
-static double bwd_tile_cost(const BwdTile& t, int KP, int NE, int opbuf, bool two_pass) {
-    if (t.RV == 3) return t.rows % 8 ? 14 : 16.5;
-    const int W = t.rows * KP / (32 * NE);  // warps with rows
-    double c = W + 4;
-    if (NE == 12 && KP < 192) c = W == 4 ? (two_pass ? 8.6 : 8) : W == 6 ? 10.8 : W == 7 ? 11.2 : two_pass ? 14.8 : 13.4;
-    if (NE == 12 && KP == 192) c = W == 4 ? 8.8 : W == 6 ? 11.3 : W == 7 ? (opbuf == 1 ? 12 : 11) : two_pass ? 14.8 : 13.4;
-    return c;
+// What a token costs a CTA (the walk, and what does not grow with the rows), in units of which 4 warps take 8.  One wave, T =
+// 512, bf16 and float32 alike within 3 %, us at 4 / 6 / 8 warps (8 of 3 rows): d_k = 48 196 / 268 / 342, 96 193 / 261 / 337, 192
+// 197 / 268 / 355, 64 151 / - / 230 (285), 128 148 / - / 226 (290), 32 173 / - / 229, 16 113 / - / 162, 256 - / - / 357.  With
+// the uncertainty output 213 / 305 / 374, 213 / 292 / 374, 216 / 283 / 387, 159 / - / 247 (342), 160 / - / 246 (328), 159 / - / 253,
+// 121 / - / 173, - / - / 370.  The state-gradient pass of exact segments takes 0.45 to 0.55 of that at every height.
+static double bwd_tile_cost(const BwdTile& t, int KP, int NE, bool unc) {
+    if (t.RV == 3) return KP == 64 ? (unc ? 17.2 : 15.1) : unc ? 16.4 : 15.7;
+    return t.W == 4 ? 8 : t.W == 6 ? 11 : NE == 12 ? 14.2 : 12;
 }
 struct BwdConfig {
     BwdShape s;
     BwdTile t;
-    int smem, kbuf, opbuf;
+    int smem, kbuf;
     double cost;
 };
 // The choice that costs least: waves of CTAs (one per SM) times the cost of a token.  CTAs of equal sequences, or of their
@@ -1047,21 +1033,17 @@ static BwdConfig bwd_config(const palimpsa_problem& p) {
     const BwdShape s = best.s;
     const int VG = 32 / s.KG, KP = s.RK * s.KG;
     const bool unc = (p.flags & PALIMPSA_FLAG_UNCERTAINTY) != 0;
-    const int es = dtype_size(p.io_dtype);
     const double units = (double)p.num_seqs * p.H;
     for (const BwdTile* t = bwd_tile_choices(KP); t->W; ++t) {
-        if (t->rows == 24 && KP == 128 && (units == 0 || p.cu_seqlens) && p.segments != BWD_FEWEST_TILES)
-            continue;  // pays by whole waves, which only equal sequences have
-        BwdConfig c{s, *t, 0, 0, 0, 0};
-        for (const auto& bufs : {std::pair<int, int>{2, 2}, {2, 1}, {1, 2}, {1, 1}}) {
-            c.opbuf = bufs.first, c.kbuf = bufs.second;
-            c.smem = bwd_smem_layout(KP, t->W * VG * t->RV, t->RV * s.RK, 32 * t->W, t->W * VG, es, unc, c.kbuf, c.opbuf).total;
-            if (c.smem <= 227 * 1024) break;
+        BwdConfig c{s, *t, 0, 0, 0};
+        for (c.kbuf = 2;; c.kbuf = 1) {
+            c.smem = bwd_smem_layout(KP, t->W * VG * t->RV, t->RV * s.RK, t->W, t->W * VG, unc, c.kbuf).total;
+            if (c.kbuf == 1 || c.smem <= 227 * 1024) break;
         }
         if (c.smem > 227 * 1024) continue;
         const int tiles = (p.V + t->rows - 1) / t->rows;
         const bool cut = p.segments > 1;
-        const double cost = bwd_tile_cost(*t, KP, t->RV * s.RK, c.opbuf, cut && !carry_tc_shape(p));
+        const double cost = bwd_tile_cost(*t, KP, t->RV * s.RK, unc);
         const double share = (units > 0 ? units : 1) * tiles / B200_SMS;  // of a wave, per segment
         if (p.segments == BWD_FEWEST_TILES) {
             c.cost = 1000.0 * tiles + cost;
@@ -1082,6 +1064,11 @@ double bwd_token_cost(const palimpsa_problem& p) { return bwd_config(p).cost; }
 
 int bwd_tile_rows(const palimpsa_problem& p) {
     return bwd_config(p).t.rows;  // 0: nothing fits
+}
+
+void bwd_plan(const palimpsa_problem& p, int32_t* plan) {
+    const BwdConfig c = bwd_config(p);
+    plan[0] = c.t.rows, plan[1] = c.t.W, plan[2] = c.kbuf;
 }
 
 BwdWorkspace bwd_workspace_layout(const palimpsa_problem& p) {
@@ -1128,7 +1115,7 @@ static int launch_bwd_w(const BwdArgs& a, int tiles, int num_seg, bool carry_onl
     constexpr int VG = 32 / KG, TV = W * VG * RV;
     const palimpsa_problem& p = a.p;
     const bool unc = (p.flags & PALIMPSA_FLAG_UNCERTAINTY) != 0;
-    const BwdSmem L = bwd_smem_layout(RK * KG, TV, RV * RK, 32 * W, W * VG, dtype_size(p.io_dtype), unc, a.kbuf, a.opbuf);
+    const BwdSmem L = bwd_smem_layout(RK * KG, TV, RV * RK, W, W * VG, unc, a.kbuf);
     if (L.total > 227 * 1024) return PALIMPSA_E_DIM;
     dim3 grid(tiles, p.num_seqs * p.H, num_seg);
     dim3 block(bwd_threads(W), 1, 1);
@@ -1153,7 +1140,6 @@ static int launch_bwd_t(const BwdArgs& args, int tiles, int num_seg, bool carry_
     BwdArgs a = args;
     a.rows = cfg.t.rows;
     a.kbuf = cfg.kbuf;
-    a.opbuf = cfg.opbuf;
 #define PALIMPSA_W(rv, n)                                                                                \
     if (cfg.t.W == n && cfg.t.RV == rv) return launch_bwd_w<RK, KG, rv, n>(a, tiles, num_seg, carry_only, stream)
     constexpr int KP = RK * KG;
@@ -1179,8 +1165,6 @@ int bwd_wait_status() {
     }
     return s;
 }
-
-static bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; }
 
 int launch_bwd(const palimpsa_bwd_params* prm, const palimpsa_segments* segs, bool carry_only, cudaStream_t stream,
                int stages) {
@@ -1212,9 +1196,13 @@ int launch_bwd(const palimpsa_bwd_params* prm, const palimpsa_segments* segs, bo
     a.db = prm->db;
     a.rows_total = p.total_tokens * p.H;
     const int es = dtype_size(p.io_dtype);
-    a.aligned = ((p.K * es) % 16 == 0) && ((p.V * es) % 16 == 0) && aligned16(p.q) && aligned16(p.k) &&
-                aligned16(p.v) && aligned16(p.b) && aligned16(prm->d_o) &&
-                (a.d_o_var == nullptr || aligned16(a.d_o_var)) && ((reinterpret_cast<uintptr_t>(p.gt) & 3) == 0);
+    const auto starts_on = [](std::initializer_list<const void*> ptrs, int bytes) {
+        for (const void* x : ptrs)
+            if (reinterpret_cast<uintptr_t>(x) & (bytes - 1)) return false;
+        return true;
+    };
+    a.vec_k = p.K % 4 == 0 && starts_on({p.q, p.k}, 4 * es);
+    a.vec_v = p.V % 2 == 0 && starts_on({p.v, p.b, a.d_o, a.d_o_var}, 2 * es);  // tiles start on even rows
     int rc = PALIMPSA_OK;
     if (stages & 1) switch (ws.KP) {
         case 16: rc = launch_bwd_t<2, 8>(a, ws.tiles, num_seg, carry_only, stream); break;

@@ -59,8 +59,9 @@ int carry_tc_status();
 int fwd_wait_status();  // 0, or the code of a bounded wait of the tall-tile forward that gave up
 int bwd_wait_status();  // 0, or the code of a bounded barrier wait of the backward main kernel that gave up
 
-// What a launch of these sizes takes: {1 for the tall-tile kernel, rows of a tile}.
+// What a launch of these sizes takes: {1 for the tall-tile kernel, rows of a tile}; {rows, compute warps, group buffers}.
 void fwd_plan(const palimpsa_problem& p, int32_t* plan);
+void bwd_plan(const palimpsa_problem& p, int32_t* plan);
 
 // Boundary scans over segments (segments.cu).
 int launch_combine_fwd(const palimpsa_problem& p, const palimpsa_segments& segs, const float* in_M, const float* in_J,

@@ -171,7 +171,7 @@ int64_t plan_segments(int64_t N, int64_t T, int64_t H, int64_t K, int64_t V, int
     // How much cheaper the cut backward has to be: less where its uncut grid is one wave (that of 4 warps below 9 units, any
     // below 15) and the forward's leaves SMs idle too, so that the summaries and the scan are paid for there.
     const bool one = uncut < 15;
-    const double worth = rounded ? (one ? 1.05 : 1.2) : K <= 16 || uncut < 9 ? 1.2 : one ? 1.25 : 1.55;
+    const double worth = rounded ? (one ? 1.05 : 1.15) : K <= 16 || uncut < 9 ? 1.2 : one ? 1.25 : 1.55;
     return uncut > worth * palimpsa_bwd_token_cost(&p) ? pieces : 1;
 }
 

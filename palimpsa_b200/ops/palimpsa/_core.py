@@ -100,8 +100,9 @@ def plan_segments(N: int, T: int, H: int, K: int, V: int, device=None, backward:
     when its estimated time per token (``palimpsa_bwd_token_cost``: waves of CTAs times what their warps cost, at the
     tile height it would take) is by enough above that of the cut grid.  How much is enough, from 270 timed steps
     (T = 4096, 16x32 to 256x256, three types): 1.05 where the uncut grid is one wave and the boundary terms go through
-    the tensor cores (16 heads of 128x128 bf16: 3.02 ms uncut, 2.51 cut), 1.2 where it is more (54: 5.60 / 4.34; 72 of
-    64x128, ratio 1.14: 5.40 / 5.78); with the exact float32 passes, which walk twice, 1.25 and 1.55 (16 heads of 96x192,
+    the tensor cores (16 heads of 128x128 bf16: 3.02 ms uncut, 2.51 cut), 1.15 where it is more (54: 5.60 / 4.34; 72 of
+    64x128, ratio 1.14: 5.40 / 5.78; of the present kernels 32 of 128x128, T = 18793, 1.19: 20.5 / 19.5; 36, T = 4931,
+    1.06: 5.54 / 6.09); with the exact float32 passes, which walk twice, 1.25 and 1.55 (16 heads of 96x192,
     1.19: 3.61 / 3.99; 64 of 128x64 float16, 1.31: 5.61 / 6.66; 54 of 64x128 float16, 1.52: 5.79 / 5.78).
 
     bfloat16 shapes that the tensor-core passes serve round their boundary terms, so accuracy is in play there: they are

@@ -40,3 +40,8 @@ def _plan(which, N, T, H, K, V, dtype, unc, segments, packed, n):
 def fwd_plan(N, T, H, K, V, dtype=torch.float32, unc=False, segments=0, packed=False):
     """(1 for the forward kernel for tall tiles, rows of a tile); T of a packed batch is that of all its documents."""
     return _plan("palimpsa_fwd_plan", N, T, H, K, V, dtype, unc, segments, packed, 2)
+
+
+def bwd_plan(N, T, H, K, V, dtype=torch.float32, unc=False, segments=0, packed=False):
+    """(rows of a tile, compute warps, group buffers) of the backward."""
+    return _plan("palimpsa_bwd_plan", N, T, H, K, V, dtype, unc, segments, packed, 3)

@@ -1,5 +1,5 @@
 """The backward's staged blocks: sequences of several blocks (both operand stages and both barrier phases in use), a ragged
-last block, warps without rows in the last tile, rows staged pair by pair at every offset of a tile, and the state-gradient
+last block, warps without rows in the last tile, steps of 4, 8 and 16 tokens, and the state-gradient
 pass of exact segments, against the float64 oracle."""
 import pytest
 import torch
@@ -14,8 +14,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("N,H,T,K,V,dtype,unc", [
     (1, 2, 83, 128, 128, torch.bfloat16, False),   # 3 rows a thread, tiles of 22 rows starting at every even offset
     (25, 4, 67, 128, 24, torch.bfloat16, False),   # tiles of 24
-    (2, 2, 81, 128, 67, torch.float32, True),      # odd rows; one operand stage
-    (2, 2, 66, 64, 90, torch.float16, False),      # 44 rows, then 46 in a tile that holds 48
+    (2, 2, 81, 128, 67, torch.float32, True),      # odd rows
+    (2, 2, 66, 64, 90, torch.float16, False),      # tiles of 44 rows and one of 2
     (2, 2, 97, 48, 57, torch.bfloat16, False),     # a second tile of one row: all but one warp without rows
     (2, 2, 70, 96, 97, torch.bfloat16, True),
     (2, 2, 65, 31, 65, torch.float32, True),       # element loads

@@ -1,5 +1,5 @@
-"""The backward's tile heights (warps per CTA by head size, element type and grid), with one and two group buffers, ragged
-last tiles and tokens past the last whole block, against the float64 oracle."""
+"""The backward's tile heights (rows and warps of a CTA by head size, element type and grid), with one and two group buffers,
+ragged last tiles, tokens past the last whole block and rows that start at any offset, against the float64 oracle."""
 import ctypes as C
 
 import pytest
@@ -7,14 +7,9 @@ import torch
 
 from oracle import palimpsa_oracle as orc
 from tests.gpu_util import DEV, compare, run_cuda, run_oracle, tol_for
+from tests.helpers import bwd_plan
 
 pytestmark = pytest.mark.gpu
-
-
-# state rows per compute warp and the warp counts a CTA may have, by padded d_k (csrc/bwd.cu)
-ROWS = {16: 8, 32: 8, 48: 8, 64: 4, 96: 4, 128: 2, 192: 2, 256: 1}
-WARPS = {16: (8, 4), 32: (8, 4), 48: (8, 7, 6, 4), 64: (11, 8, 4), 96: (8, 7, 6, 4), 128: (12, 11, 8, 4),
-         192: (8, 7, 6, 4), 256: (8,)}
 
 
 def _tiles(N, T, H, K, V, io, unc, G):
@@ -31,56 +26,46 @@ def _tiles(N, T, H, K, V, io, unc, G):
     return fits[0]
 
 
-def _one_buffer(KP, W, es, unc):
-    """Two group buffers do not fit: the shared memory of a CTA, by the parts that count (operand tiles with every value
-    twice, parked states, two checkpoint stages, group partials, raw stage)."""
-    TV, NE = W * ROWS[KP], {16: 4, 48: 12, 96: 12, 192: 12}.get(KP, 8)
-    WV = TV // (1 if KP == 256 else 2)
-    raw = 16 * es * (2 * KP + (3 + unc) * ((TV + 7) // 8 * 8 + 8))
-    fixed = 16 * 4 * KP * (2 + unc) + 16 * TV * 8 * (3 + unc) + 16 * NE * 32 * W + 16 * TV * KP + raw + 600
-    return fixed + 2 * (4 * WV * 2 * KP * 4 + 2 * 16 * TV + 32 * W) > 227 * 1024
-
-
-@pytest.mark.parametrize("W,one_buffer,N,H,T,K,V,dtype,unc,G", [
-    (8, False, 15, 2, 17, 16, 129, torch.bfloat16, False, 1),
-    (4, False, 2, 1, 33, 16, 33, torch.float32, True, 1),
-    (8, False, 15, 2, 17, 32, 129, torch.float16, True, 1),
-    (4, False, 1, 2, 35, 31, 33, torch.bfloat16, False, 1),
-    (8, True, 24, 4, 17, 48, 63, torch.float32, True, 1),       # registers split between the warpgroups, as at every d_k
-    (8, True, 24, 4, 18, 48, 62, torch.bfloat16, False, 1),     # with 8 warps of 12 elements
-    (7, False, 5, 1, 80, 48, 241, torch.bfloat16, False, 5),
-    (6, False, 10, 4, 17, 48, 97, torch.bfloat16, False, 1),
-    (4, False, 1, 2, 17, 47, 33, torch.float32, True, 1),
-    (11, True, 15, 4, 17, 64, 65, torch.float32, True, 1),
-    (11, False, 15, 2, 17, 64, 129, torch.bfloat16, False, 1),
-    (8, False, 15, 2, 17, 60, 65, torch.float32, False, 1),
-    (4, False, 1, 2, 19, 64, 17, torch.float16, False, 1),
-    (8, True, 24, 4, 17, 96, 31, torch.bfloat16, False, 1),
-    (8, True, 48, 2, 5, 90, 30, torch.float32, True, 1),
-    (7, False, 5, 1, 80, 96, 121, torch.bfloat16, False, 5),
-    (6, False, 10, 4, 17, 96, 49, torch.float32, False, 1),
-    (4, False, 2, 1, 17, 96, 17, torch.bfloat16, True, 1),
-    (12, True, 25, 4, 17, 128, 23, torch.bfloat16, False, 1),   # registers split
-    (12, True, 50, 2, 18, 120, 23, torch.float32, True, 1),
-    (11, False, 15, 2, 17, 128, 67, torch.bfloat16, False, 1),  # the benchmark's tiling, ragged
-    (8, False, 15, 2, 17, 128, 33, torch.float32, True, 1),
-    (4, False, 1, 2, 17, 128, 9, torch.bfloat16, True, 1),
-    (8, True, 24, 4, 17, 192, 15, torch.float32, False, 1),
-    (8, True, 48, 2, 5, 180, 15, torch.bfloat16, True, 1),
-    (7, False, 5, 1, 64, 192, 61, torch.bfloat16, False, 4),
-    (6, False, 10, 4, 17, 192, 25, torch.float32, False, 1),
-    (4, False, 2, 1, 17, 180, 9, torch.float32, True, 1),
-    (8, True, 2, 1, 17, 256, 7, torch.float32, True, 1),
+@pytest.mark.parametrize("rows,warps,buffers,N,H,T,K,V,dtype,unc,G", [
+    (64, 8, 2, 15, 2, 17, 16, 129, torch.bfloat16, False, 1),
+    (32, 4, 2, 2, 1, 33, 16, 33, torch.float32, True, 1),
+    (64, 8, 2, 15, 2, 17, 32, 129, torch.float16, True, 1),
+    (32, 4, 2, 1, 2, 35, 31, 33, torch.bfloat16, False, 1),
+    (64, 8, 1, 24, 4, 17, 48, 63, torch.float32, True, 1),       # registers split between the warpgroups, as at every d_k
+    (64, 8, 1, 24, 4, 18, 48, 62, torch.bfloat16, False, 1),     # with 8 warps of 12 elements
+    (64, 8, 1, 5, 1, 80, 48, 241, torch.float32, False, 5),      # the state-gradient pass of exact segments too
+    (48, 6, 2, 10, 4, 17, 48, 97, torch.bfloat16, False, 1),
+    (48, 6, 2, 10, 4, 17, 48, 97, torch.bfloat16, True, 1),
+    (32, 4, 2, 1, 2, 17, 47, 33, torch.float32, True, 1),
+    (44, 8, 1, 15, 4, 17, 64, 65, torch.float32, True, 1),
+    (44, 8, 2, 15, 2, 17, 64, 129, torch.bfloat16, False, 1),
+    (32, 8, 2, 15, 2, 17, 60, 65, torch.float32, False, 1),
+    (16, 4, 2, 1, 2, 19, 64, 17, torch.float16, False, 1),
+    (32, 8, 1, 24, 4, 17, 96, 31, torch.bfloat16, False, 1),
+    (32, 8, 1, 48, 2, 5, 90, 30, torch.float32, True, 1),
+    (32, 8, 1, 5, 1, 80, 96, 121, torch.float32, True, 5),
+    (24, 6, 2, 10, 4, 17, 96, 49, torch.float32, False, 1),
+    (16, 4, 2, 2, 1, 17, 96, 17, torch.bfloat16, True, 1),
+    (24, 8, 2, 25, 4, 17, 128, 23, torch.bfloat16, False, 1),    # registers split
+    (24, 8, 2, 50, 2, 18, 120, 23, torch.float32, True, 1),
+    (22, 8, 2, 24, 2, 17, 128, 110, torch.float32, True, 1),
+    (24, 8, 2, 15, 2, 17, 128, 67, torch.bfloat16, False, 1),
+    (16, 8, 2, 15, 2, 17, 128, 33, torch.float32, True, 1),
+    (8, 4, 2, 1, 2, 17, 128, 9, torch.bfloat16, True, 1),
+    (16, 8, 1, 24, 4, 17, 192, 15, torch.float32, False, 1),
+    (16, 8, 1, 48, 2, 5, 180, 15, torch.bfloat16, True, 1),
+    (12, 6, 2, 5, 1, 64, 192, 61, torch.bfloat16, False, 4),
+    (12, 6, 2, 10, 4, 17, 192, 25, torch.float32, True, 1),
+    (8, 4, 2, 2, 1, 17, 180, 9, torch.float32, True, 1),
+    (8, 8, 1, 2, 1, 17, 256, 7, torch.float32, True, 1),
 ])
-def test_every_warp_count_matches_oracle(W, one_buffer, N, H, T, K, V, dtype, unc, G):
-    """Every warp count a CTA may have, shown to be the one taken: no other gives the case's number of row tiles."""
+def test_every_tile_matches_oracle(rows, warps, buffers, N, H, T, K, V, dtype, unc, G):
+    """Every tile a CTA may have, with the group buffers that fit beside it, as the library says that it takes them."""
     from palimpsa_b200 import _lib as L
     from palimpsa_b200.ops import chunk_palimpsa
-    KP, es = L.lib().palimpsa_padded_k(K), dtype.itemsize
-    up = lambda w: -(-V // (w * ROWS[KP]))
     io = {torch.float32: L.F32, torch.bfloat16: L.BF16, torch.float16: L.F16}[dtype]
-    assert _tiles(N, T, H, K, V, io, unc, G) == up(W) and [up(w) for w in WARPS[KP]].count(up(W)) == 1
-    assert _one_buffer(KP, W, es, unc) == one_buffer
+    assert bwd_plan(N, T, H, K, V, dtype, unc, G) == (rows, warps, buffers)
+    assert _tiles(N, T, H, K, V, io, unc, G) == -(-V // rows)
     inp = orc.make_inputs(K + V, B=N, T=T, H=H, K=K, V=V, dtype=dtype)
     a = {n: inp[n].to(DEV).requires_grad_() for n in ("q", "k", "v", "b", "gt", "g", "Ip")}
     out = chunk_palimpsa(*a.values(), output_uncertainty=unc, num_segments=G)
@@ -88,7 +73,40 @@ def test_every_warp_count_matches_oracle(W, one_buffer, N, H, T, K, V, dtype, un
     sum((got[n].float() * inp["d" + n].to(DEV).float()).sum() for n in got).backward()
     got.update({"d" + n: x.grad for n, x in a.items()})
     ref = run_oracle(inp, unc=unc)
-    compare({n: x.detach().cpu() for n, x in got.items()}, ref, tol_for(dtype), names=list(got), what=f"{W} warps, {K}x{V}")
+    compare({n: x.detach().cpu() for n, x in got.items()}, ref, tol_for(dtype), names=list(got), what=f"{rows} rows, {K}x{V}")
+
+
+@pytest.mark.parametrize("K,V,dtype,unc,off", [
+    (47, 65, torch.bfloat16, False, 0),   # odd rows of 16-bit values: every second one starts between two words
+    (95, 23, torch.float16, True, 1),
+    (127, 45, torch.float32, False, 0),
+    (64, 66, torch.bfloat16, False, 1),   # whole rows of vectors, on buffers that do not start on one
+    (48, 48, torch.bfloat16, True, 2),
+    (128, 24, torch.float32, False, 1),
+    (60, 50, torch.bfloat16, False, 4),   # rows of words, but not of 16 bytes
+    (20, 34, torch.float32, True, 3),
+    (189, 13, torch.bfloat16, True, 3),
+    (255, 9, torch.float16, False, 7),
+])
+def test_rows_at_any_offset(K, V, dtype, unc, off):
+    """Inputs that start `off` elements into their buffers give what the same values give at the front of theirs, to the bit."""
+    from palimpsa_b200.ops import chunk_palimpsa
+    N, T, H = 2, 37, 2
+    inp = orc.make_inputs(K * V, B=N, T=T, H=H, K=K, V=V, dtype=dtype)
+    res = []
+    for shift in (0, off):
+        def place(x):
+            buf = torch.empty(x.numel() + shift, dtype=x.dtype, device=DEV)
+            buf[shift:] = x.flatten().to(DEV)
+            return buf[shift:].view(x.shape)
+        a = {n: (place(inp[n]) if n in "qkvb" else inp[n].to(DEV)).requires_grad_() for n in ("q", "k", "v", "b", "gt", "g", "Ip")}
+        out = chunk_palimpsa(*a.values(), output_uncertainty=unc, num_segments=1)
+        out = list(out) if unc else [out]
+        grads = torch.autograd.grad(out, list(a.values()), [place(inp[n]) for n in ("do", "do_var")[:len(out)]])
+        res.append([x.detach().cpu() for x in (*out, *grads)])
+    assert all(torch.equal(x, y) for x, y in zip(*res))
+    names = ["o", "o_var"][:len(out)] + ["d" + n for n in a]
+    compare(dict(zip(names, res[1])), run_oracle(inp, unc=unc), tol_for(dtype), names=names, what=f"{K}x{V} +{off}")
 
 
 @pytest.mark.parametrize("N,H,T,K,V,dtype,unc", [

@@ -255,7 +255,7 @@ def test_forward_tile_rows_from_the_library():
     assert lib.palimpsa_fwd_tile_rows(64, 8) == 16         # short d_v: one warp instead of two, half the tile
     assert lib.palimpsa_fwd_tile_rows(300, 64) == 0        # d_k above the supported maximum
     assert lib.palimpsa_fwd_tile_rows(48, 48) == 48        # three warps: no idle rows at the 170M model's heads
-    assert lib.palimpsa_bwd_tile_rows(128, 128, _lib.BF16, 0) == 22   # 11 warps x 2 rows: 6 tiles = 132 rows
+    assert lib.palimpsa_bwd_tile_rows(128, 128, _lib.BF16, 0) == 22   # 22 of the 24 rows of 8 warps x 3: 6 tiles = 132 rows
     assert lib.palimpsa_bwd_tile_rows(48, 48, _lib.BF16, 0) == 48     # 6 warps x 8 rows
     assert lib.palimpsa_bwd_tile_rows(48, 96, _lib.BF16, 0) == 48
     assert lib.palimpsa_bwd_tile_rows(64, 64, _lib.BF16, 0) == 32
@@ -276,3 +276,32 @@ def test_the_forward_takes_tall_tiles_where_they_pay():
     assert fwd_plan(8, 4096, 6, 128, 128, bf) == (1, 48) and fwd_plan(2, 3001, 16, 96, 192, bf) == (1, 48)
     assert fwd_plan(8, 0, 6, 128, 128, bf)[0] == 0
     assert fwd_plan(40, 40 * 20, 6, 128, 128, bf, packed=True)[0] == 0
+
+
+def test_backward_tiles_by_what_they_cost():
+    import torch
+    from tests.helpers import bwd_plan
+    bf = torch.bfloat16
+    assert bwd_plan(8, 4096, 6, 128, 128, bf) == (22, 8, 2)
+    assert bwd_plan(8, 4096, 16, 48, 48, bf) == (48, 6, 2)
+    assert bwd_plan(17, 699, 12, 96, 192, bf) == (32, 8, 1)           # 9 waves of 6 tiles
+    assert bwd_plan(14, 27244, 16, 96, 192, bf, packed=True)[0] == 32
+    assert bwd_plan(50, 32768, 6, 128, 72, bf, packed=True)[0] == 24   # 3 tiles for packed rows too
+    # as many rows in shared memory whatever the element type; the tallest tile of every d_k serves as the least scratch
+    for K in (16, 32, 48, 64, 96, 128, 192, 256):
+        for unc in (False, True):
+            plans = {bwd_plan(64, 2048, 8, K, 192, dt, unc) for dt in (torch.float32, bf, torch.float16)}
+            assert len(plans) == 1
+
+
+def test_plans_are_refused_for_what_no_launch_takes():
+    import ctypes as C
+    from palimpsa_b200 import _lib as L
+    lib, plan, p = L.lib(), (C.c_int32 * 3)(), L.Problem()
+    for fn in (lib.palimpsa_fwd_plan, lib.palimpsa_bwd_plan):
+        p.num_seqs, p.seq_len, p.total_tokens, p.H, p.K, p.V, p.io_dtype = 1, 64, 64, 2, 300, 64, L.F32
+        assert fn(C.byref(p), plan) != 0
+        p.K = 64
+        assert fn(C.byref(p), plan) == 0 and fn(C.byref(p), None) == L.E_NULL and fn(None, plan) != 0
+        p.num_seqs = 0
+        assert fn(C.byref(p), plan) != 0
