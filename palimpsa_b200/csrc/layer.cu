@@ -1062,23 +1062,23 @@ int palimpsa_layer_prologue_bwd(const palimpsa_layer_prologue* a, void* cuda_str
             PALIMPSA_ROWS16(dt, lanes, CALL16);
 #undef CALL16
         } else {
-        const bool veck = a->K % 4 == 0 && aligned_for(a->q_raw, dt) && aligned_for(a->k_raw, dt) &&
-                          aligned_for(a->dq, dt) && aligned_for(a->dk, dt) && aligned_for(a->dq_raw, dt) &&
-                          aligned_for(a->dk_raw, dt);
-        const bool vecv = a->V % 4 == 0 && aligned_for(a->x, dt) && aligned_for(a->b_raw, dt) && aligned_for(a->dv, dt) &&
-                          aligned_for(a->db, dt) && aligned_for(a->dx, dt) && aligned_for(a->db_raw, dt);
-        const int nck = (a->K + 127) / 128, ncv = (a->V + 127) / 128;
+            const bool veck = a->K % 4 == 0 && aligned_for(a->q_raw, dt) && aligned_for(a->k_raw, dt) &&
+                              aligned_for(a->dq, dt) && aligned_for(a->dk, dt) && aligned_for(a->dq_raw, dt) &&
+                              aligned_for(a->dk_raw, dt);
+            const bool vecv = a->V % 4 == 0 && aligned_for(a->x, dt) && aligned_for(a->b_raw, dt) && aligned_for(a->dv, dt) &&
+                              aligned_for(a->db, dt) && aligned_for(a->dx, dt) && aligned_for(a->db_raw, dt);
+            const int nck = (a->K + 127) / 128, ncv = (a->V + 127) / 128;
 #define CALL_V(NV)                                                                                \
-    do {                                                                                          \
-        if (nck <= 1) pro_bwd_launch<DTX, 1, NV>(*a, qrows, veck, vecv, w_dtb, w_bsc, st);        \
-        else pro_bwd_launch<DTX, 2, NV>(*a, qrows, veck, vecv, w_dtb, w_bsc, st);                 \
-    } while (0)
+        do {                                                                                          \
+            if (nck <= 1) pro_bwd_launch<DTX, 1, NV>(*a, qrows, veck, vecv, w_dtb, w_bsc, st);        \
+            else pro_bwd_launch<DTX, 2, NV>(*a, qrows, veck, vecv, w_dtb, w_bsc, st);                 \
+        } while (0)
 #define CALL_D(D)                      \
-    do {                               \
-        constexpr int DTX = D;         \
-        PALIMPSA_BY_NCV(ncv, CALL_V);  \
-    } while (0)
-        PALIMPSA_BY_DTYPE(dt, CALL_D);
+        do {                               \
+            constexpr int DTX = D;         \
+            PALIMPSA_BY_NCV(ncv, CALL_V);  \
+        } while (0)
+            PALIMPSA_BY_DTYPE(dt, CALL_D);
 #undef CALL_D
 #undef CALL_V
         }
@@ -1145,16 +1145,16 @@ int palimpsa_layer_epilogue_bwd(const palimpsa_layer_epilogue* a, void* cuda_str
             PALIMPSA_ROWS16(dt, lanes, CALL16);
 #undef CALL16
         } else {
-        const bool vecv = a->V % 4 == 0 && aligned_for(a->o, dt) && aligned_for(a->dy, dt) && aligned_for(a->d_o, dt) &&
-                          (!res || (aligned_for(a->x, dt) && aligned_for(a->dx, dt))) &&
-                          (!gated || (aligned_for(a->gate, dt) && aligned_for(a->dgate, dt)));
+            const bool vecv = a->V % 4 == 0 && aligned_for(a->o, dt) && aligned_for(a->dy, dt) && aligned_for(a->d_o, dt) &&
+                              (!res || (aligned_for(a->x, dt) && aligned_for(a->dx, dt))) &&
+                              (!gated || (aligned_for(a->gate, dt) && aligned_for(a->dgate, dt)));
 #define CALL_V(NV) nb = epi_bwd_launch<DTX, NV>(*a, rows, vecv, w_dD, w_dw, st)
 #define CALL_D(D)                     \
-    do {                              \
-        constexpr int DTX = D;        \
-        PALIMPSA_BY_NCV(nc, CALL_V);  \
-    } while (0)
-        PALIMPSA_BY_DTYPE(dt, CALL_D);
+        do {                              \
+            constexpr int DTX = D;        \
+            PALIMPSA_BY_NCV(nc, CALL_V);  \
+        } while (0)
+            PALIMPSA_BY_DTYPE(dt, CALL_D);
 #undef CALL_D
 #undef CALL_V
         }
