@@ -8,11 +8,15 @@
 //      slots in shared memory),
 //   3. per group, last first: recomputes the 4 per-token states into registers, then walks the
 //      tokens in reverse, carrying the state gradients (GM, -GI) in registers:
-//          h    = dy*q_s / I            GM = f_next*GM + h          -GI = f_next*(-GI) + h*mu (+ dy_var*(q/I)^2)
-//          dq  += dy*mu   dk += GM*v + 2k*GI*b   dv += GM*k   db += GI*k^2
-//          df   = <GM, M_prev> + <GI, I_prev - Ip>
-//      (the algebra of chunk_palimpsa_bwd_kernel, chunk_palimpsa_forgetting_scalar.py:343-434,
-//      with the previous state carried forward instead of rebuilt by a division, :409-410).
+//          r    = 1 / (B + Z)           mu = M*r                    h = dy*q_s * r
+//          GM  += h                     -GI += h*mu (+ dy_var/F * (q*r)^2)
+//          dq  += dy*mu   dk += GM*v/F + 2k*GI*b/F   dv/F += GM*k   db/F += GI*k^2
+//          f*df = <GM, M_prev> + <GI, B_prev - Ip>
+//      all in the scaled form in which neither the state nor its gradient decays from token to token (block_scale in
+//      common.cuh; GM, GI are the gradients of the scaled M and B): the algebra of chunk_palimpsa_bwd_kernel,
+//      chunk_palimpsa_forgetting_scalar.py:343-434, divided by F, with the previous state carried forward instead of rebuilt
+//      by a division, :409-410.  A block in which a token scales the state it finds takes a second copy of the walk, which
+//      also scales the gradients behind that token.
 // Reductions: over d_k (dv, db) by xor-shuffles inside the lanes of a row; over d_v (dq, dk) first
 // in registers across a thread's rows, then across the CTA's row groups through shared memory, and
 // across the CTAs of different row tiles through fp32 partial buffers in the workspace, which the
@@ -22,7 +26,10 @@
 // groups, casts, global stores).  All hand-overs are mbarriers with bounded waits: the compute warps meet no CTA barrier and
 // drift apart.
 // What bounds the walk is the issue rate: a packed FP32 instruction takes two issue cycles, a pair of state elements 28 per
-// token in the reverse walk and 14 in the two forward steps, and operand loads, shuffle sums and moves come on top; so it
+// token in the reverse walk and 7 in the two forward steps (14 before the scaled form), and operand loads, shuffle sums and moves
+// come on top.  The scaled form, with the first term of every sum as a product instead of an FMA on a zero, took the backward at
+// B=8 T=4096 H=6 d=128 from 4.75 to 4.31 ms, at H=16 48x48 from 2.15 to 1.98 and at B=4 T=2048 H=16 96x192 from 4.06 to 3.84; as a
+// branch per group instead of per block it was 4.63 and 2.11 (moves of the gradients where the two copies meet).  So it
 // pays to have 12 elements a thread (two warps per scheduler) rather than 8 (three), and to take staging off those warps.
 // Through registers, because a copy in shared memory to convert from costs 10 to 37 KB, for want of which some shapes had one
 // operand stage or one group buffer, and because rows that start at any offset can only be loaded one by one, which four warps
@@ -37,6 +44,7 @@
 #include <cmath>
 #include <initializer_list>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 
 #include "host.h"
@@ -79,7 +87,7 @@ struct BwdArgs {
 };
 
 struct BwdSmem {
-    int ks, qs, vb, dys2, dyvs2, fc2, fn2;  // offsets inside an operand stage; the two stages come first
+    int ks, qs, vb, dys2, dyvs2, fc2, zz2, fi2, blk;  // offsets inside an operand stage; the two stages come first
     int op_stage, slots, ckb;
     int kred, dvs, dbs, wred, fgr;  // per-group partials handed to the helper warps, kbuf buffers of each
     int bars;                       // mbarriers: full[2], empty[2], staged[2], done[2]; then the failure flag
@@ -103,8 +111,10 @@ __host__ __device__ inline BwdSmem bwd_smem_layout(int KP, int TV, int NE, int W
     s.vb = take(TB * TV * 16);
     s.dys2 = take(TB * TV * 8);
     s.dyvs2 = unc ? take(TB * TV * 8) : 0;
-    s.fc2 = take(TB * 16);
-    s.fn2 = take(TB * 8);
+    s.fc2 = take(TB * 16);  // {s, s, c, c}
+    s.zz2 = take(TB * 8);   // {Z, Z}
+    s.fi2 = take(TB * 8);   // {f, 1 / F}
+    s.blk = take(16);       // F at the block's end, BlockScale::special
     s.op_stage = off;
     off *= 2;
     s.slots = take(2 * 2 * NE * 32 * W * 4);
@@ -114,7 +124,7 @@ __host__ __device__ inline BwdSmem bwd_smem_layout(int KP, int TV, int NE, int W
     s.dvs = take(kbuf * GR * TV * 4);
     s.dbs = take(kbuf * GR * TV * 4);
     s.wred = take(kbuf * W * GR * 2 * 4);
-    s.fgr = take(kbuf * GR * 4);
+    s.fgr = take(kbuf * GR * 8);
     s.bars = take(80);
     s.total = off;
     return s;
@@ -138,11 +148,12 @@ __device__ __forceinline__ void bwd_issue_ckpt(const BwdArgs& a, int nthr, int t
 // latency nor, where rows start at any offset, the many single loads are in anybody's way.
 template <int KP, int TV, int TS, int NTH, bool UNC>
 struct BwdStaging {
-    static constexpr int F0 = NTH > 64 ? NTH - 64 : 0;  // the threads of the step sizes: neither the first nor the last warp's
+    static constexpr int F0 = NTH > 64 ? NTH - 64 : 0;  // the threads that write a block's scalars: neither the first nor the last warp's
     static constexpr int K4 = KP / 4, V2 = TV / 2, NQ = (TS * K4 + NTH - 1) / NTH, NV = (TS * V2 + NTH - 1) / NTH;
     unsigned q[NQ][4], k[NQ][4];                // 4 columns: packed 16-bit pairs in [0], [1] where they came in one load
     unsigned v[NV][2], b[NV][2], o[NV][2], ov[NV][2];  // 2 rows: a packed 16-bit pair in [0]
-    float g0, g1;                               // step sizes of a token and the next
+    float gt;                                   // step size of token lane & 15 of the block
+    float inv;                                  // and 1 / F of that token, once its first step has been stored
 };
 
 // N consecutive elements of ES bytes at element e, the first n of them (the others 0).
@@ -190,11 +201,10 @@ __device__ __forceinline__ void word_values(const unsigned (&w)[N], float (&x)[N
     }
 }
 
-// Tokens [ts, ts + TS) of the block of nt tokens that starts at token tok0 (nt_ext: with the token after it, where the
-// sequence goes on), by NTH threads.
+// Tokens [ts, ts + TS) of the block of nt tokens that starts at token tok0, by NTH threads.
 template <int ES, int KP, int TV, int TS, int NTH, bool UNC>
 __device__ __forceinline__ void bwd_load(BwdStaging<KP, TV, TS, NTH, UNC>& s, const BwdArgs& a, int tid, long long tok0, int ts,
-                                         int nt, int nt_ext, int h, int v0, int tvw) {
+                                         int nt, int h, int v0, int tvw) {
     using S = BwdStaging<KP, TV, TS, NTH, UNC>;
     const palimpsa_problem& p = a.p;
 #pragma unroll
@@ -215,17 +225,29 @@ __device__ __forceinline__ void bwd_load(BwdStaging<KP, TV, TS, NTH, UNC>& s, co
         ld_words<ES>(s.o[x], a.d_o, row, n, a.vec_v);
         if (UNC) ld_words<ES>(s.ov[x], a.d_o_var, row, n, a.vec_v);
     }
-    const int j = tid - S::F0, t = ts + j;
-    const bool on = j >= 0 && j < TS;
-    s.g0 = on && t < nt ? p.gt[(tok0 + t) * p.H + h] : 0.f;
-    s.g1 = on && t + 1 < nt_ext ? p.gt[(tok0 + t + 1) * p.H + h] : 0.f;
+    if (ts == 0) {
+        const int t = tid & (TB - 1);
+        s.gt = t < nt ? p.gt[(tok0 + t) * p.H + h] : 0.f;
+    }
 }
 
-// What bwd_load brought, as fp32 operands into the operand stage `op`.
+// What bwd_load brought, as fp32 operands into the operand stage `op`: v, b and the uncertainty's gradient divided by F
+// (block_scale).  By whole warps, each of which finds the block's scalars for itself.
 template <int DT, int KP, int TV, int TS, int NTH, bool UNC>
-__device__ __forceinline__ void bwd_store(const BwdStaging<KP, TV, TS, NTH, UNC>& s, const BwdArgs& a, int tid, unsigned char* op,
-                                          const BwdSmem& L, int ts, int nt, int nt_ext, float gh, float iph, bool carry_block) {
+__device__ __forceinline__ void bwd_store(BwdStaging<KP, TV, TS, NTH, UNC>& s, const BwdArgs& a, int tid, unsigned char* op,
+                                          const BwdSmem& L, int ts, int nt, float gh, float iph) {
     using S = BwdStaging<KP, TV, TS, NTH, UNC>;
+    if (ts == 0) {
+        const int lane = tid & 31, t = lane & (TB - 1);
+        const BlockScale b = block_scale(s.gt, t < nt, gh, iph, lane);
+        s.inv = b.inv;
+        if (tid >= S::F0 && tid < S::F0 + TB) {
+            reinterpret_cast<float4*>(op + L.fc2)[t] = make_float4(b.s, b.s, b.c, b.c);
+            reinterpret_cast<float2*>(op + L.zz2)[t] = make_float2(b.z, b.z);
+            reinterpret_cast<float2*>(op + L.fi2)[t] = make_float2(b.f, b.inv);
+            if (t == 0) *reinterpret_cast<float2*>(op + L.blk) = make_float2(b.end, __uint_as_float(b.special));
+        }
+    }
     float4* qs = reinterpret_cast<float4*>(op + L.qs) + ts * S::K4;
     float4* ks = reinterpret_cast<float4*>(op + L.ks) + ts * S::K4;
     // The scale goes with q; with the uncertainty output, which wants q and q squared, with the output gradients instead.
@@ -246,30 +268,21 @@ __device__ __forceinline__ void bwd_store(const BwdStaging<KP, TV, TS, NTH, UNC>
 #pragma unroll
     for (int x = 0; x < S::NV; ++x) {
         const int i = tid + x * NTH;
+        const float inv = __shfl_sync(0xffffffffu, s.inv, (ts + i / S::V2) & (TB - 1));
         if (i >= TS * S::V2) break;
         float v[2], b[2], o[2];
         word_values<DT>(s.v[x], v, a.vec_v);
         word_values<DT>(s.b[x], b, a.vec_v);
         word_values<DT>(s.o[x], o, a.vec_v);
+        v[0] *= inv, v[1] *= inv, b[0] *= inv, b[1] *= inv;
         vb[2 * i] = make_float4(v[0], v[0], b[0], b[0]);
         vb[2 * i + 1] = make_float4(v[1], v[1], b[1], b[1]);
         dys[i] = make_float4(o[0] * so, o[0] * so, o[1] * so, o[1] * so);
         if (UNC) {
             word_values<DT>(s.ov[x], o, a.vec_v);
-            dyvs[i] = make_float4(o[0] * so, o[0] * so, o[1] * so, o[1] * so);
+            o[0] *= so * inv, o[1] *= so * inv;
+            dyvs[i] = make_float4(o[0], o[0], o[1], o[1]);
         }
-    }
-    // per token: {f, f, c, c} with c = (1-f)*Ip, and {fn, fn}: f of the NEXT token of the sequence (0 past its end)
-    if (tid >= S::F0 && tid < S::F0 + TS) {
-        const int t = ts + tid - S::F0;
-        const float f = expf(-s.g0 * gh);
-        float fn = t + 1 < nt_ext ? expf(-s.g1 * gh) : 0.f;
-        // Last block of a segment whose end-state gradient is supplied: that gradient is already expressed
-        // at the boundary, so the last real token (and any identity padding after it) passes it on undecayed.
-        if (carry_block && t >= nt - 1) fn = 1.f;
-        const float c = (1.f - f) * iph;
-        reinterpret_cast<float4*>(op + L.fc2)[t] = make_float4(f, f, c, c);
-        reinterpret_cast<float2*>(op + L.fn2)[t] = make_float2(fn, fn);
     }
 }
 
@@ -281,12 +294,13 @@ __host__ __device__ constexpr int bwd_threads(int W) { return 32 * (W + bwd_help
 // Where an even share is too little for the walk (8 warps of 12 state elements spill 200 bytes at 168 registers), the
 // warpgroup of helpers gives up registers that the compute warpgroups take: {entry, compute, helper} registers per thread,
 // {0, 0, 0} = no split.  The compute warps wait for the helpers' registers, so the block must have been launched with enough
-// for all: bwd_split_fits asks the compiled kernel before the first launch.  Three rows and the uncertainty output need 224.
+// for all: bwd_split_fits asks the compiled kernel before the first launch.
+// (With the uncertainty output 224 and 56 registers: 2.67 ms at B=8 T=2048 H=6 d=128, with 208 and 88 2.46.)
 struct RegSplit {
     int entry, compute, helper;
 };
-__host__ __device__ constexpr RegSplit bwd_split(int W, int RV, int RK, bool unc) {
-    return W != 8 || RV * RK != 12 ? RegSplit{0, 0, 0} : unc && RV == 3 ? RegSplit{168, 224, 56} : RegSplit{168, 208, 88};
+__host__ __device__ constexpr RegSplit bwd_split(int W, int RV, int RK) {
+    return W == 8 && RV * RK == 12 ? RegSplit{168, 208, 88} : RegSplit{0, 0, 0};
 }
 
 // CTAs of an SM that the registers have to do for: two of the smallest tilings.  At d_k = 32 that spills 36 bytes: 148 / 296 / 740
@@ -316,7 +330,7 @@ bwd_kernel(const BwdArgs a) {
     constexpr int KP = RK * KG, VG = 32 / KG, NP = RK / 2, NE = RV * RK, KP2 = KP / 2;
     constexpr int TV = W * VG * RV, WV = W * VG, NTHR = 32 * W, HW = bwd_helpers(W), HT = 32 * HW;
     static_assert(TV % 2 == 0, "the operand tiles are converted two rows at a time");
-    constexpr RegSplit SPLIT = bwd_split(W, RV, RK, UNC);
+    constexpr RegSplit SPLIT = bwd_split(W, RV, RK);
     static_assert(SPLIT.entry == 0 || (W % 4 == 0 && HW == 4 &&
                                        W * SPLIT.compute + 4 * SPLIT.helper <= (W + 4) * SPLIT.entry),
                   "whole warpgroups on both sides, and no more registers than the block has at launch");
@@ -380,7 +394,7 @@ bwd_kernel(const BwdArgs a) {
     float* dvs = reinterpret_cast<float*>(sm + L.dvs);
     float* dbs = reinterpret_cast<float*>(sm + L.dbs);
     float* wred = reinterpret_cast<float*>(sm + L.wred);
-    float* fgr = reinterpret_cast<float*>(sm + L.fgr);
+    float2* fgr = reinterpret_cast<float2*>(sm + L.fgr);  // {f, 1 / F}
     if (tid == 0) {
         for (int b = 0; b < 2; ++b) {
             mbar_init_n(&full[b], W);
@@ -394,17 +408,16 @@ bwd_kernel(const BwdArgs a) {
     // the block that is walked first, by all threads
     auto tok0_of = [&](int it) __attribute__((always_inline)) { return (long long)bos + (blk1 - 1 - it) * TB; };
     auto load = [&](auto& s, int id, int it, int ts) __attribute__((always_inline)) {
-        const int left = len - (blk1 - 1 - it) * TB, nt = min(TB, left), nt_ext = min(TB + 1, left);
-        if (es == 4) bwd_load<4>(s, a, id, tok0_of(it), ts, nt, nt_ext, h, v0, tvw);
-        else bwd_load<2>(s, a, id, tok0_of(it), ts, nt, nt_ext, h, v0, tvw);
+        const int nt = min(TB, len - (blk1 - 1 - it) * TB);
+        if (es == 4) bwd_load<4>(s, a, id, tok0_of(it), ts, nt, h, v0, tvw);
+        else bwd_load<2>(s, a, id, tok0_of(it), ts, nt, h, v0, tvw);
     };
-    auto store = [&](const auto& s, int id, int it, int ts) __attribute__((always_inline)) {
-        const int left = len - (blk1 - 1 - it) * TB, nt = min(TB, left), nt_ext = min(TB + 1, left);
-        const bool cblk = has_carry && it == 0;
+    auto store = [&](auto& s, int id, int it, int ts) __attribute__((always_inline)) {
+        const int nt = min(TB, len - (blk1 - 1 - it) * TB);
         unsigned char* op = sm + (it & 1) * L.op_stage;
-        if (p.io_dtype == PALIMPSA_BF16) bwd_store<PALIMPSA_BF16>(s, a, id, op, L, ts, nt, nt_ext, gh, iph, cblk);
-        else if (p.io_dtype == PALIMPSA_F32) bwd_store<PALIMPSA_F32>(s, a, id, op, L, ts, nt, nt_ext, gh, iph, cblk);
-        else bwd_store<PALIMPSA_F16>(s, a, id, op, L, ts, nt, nt_ext, gh, iph, cblk);
+        if (p.io_dtype == PALIMPSA_BF16) bwd_store<PALIMPSA_BF16>(s, a, id, op, L, ts, nt, gh, iph);
+        else if (p.io_dtype == PALIMPSA_F32) bwd_store<PALIMPSA_F32>(s, a, id, op, L, ts, nt, gh, iph);
+        else bwd_store<PALIMPSA_F16>(s, a, id, op, L, ts, nt, gh, iph);
     };
     bwd_issue_ckpt(a, bwd_threads(W), tid, sm, L, 0, KP, TV, slot0 + blk1 - 1, h, v0, tvw);
     cp_async_commit();
@@ -474,13 +487,19 @@ bwd_kernel(const BwdArgs a) {
                             s0 = fadd2(s0, make_float2(y.x, y.y));
                             s1 = fadd2(s1, make_float2(y.z, y.w));
                         }
+                        if (!UNC) {
+                            const float2 m = dup2(which ? 1.f : p.scale);
+                            s0 = fmul2(m, s0);
+                            s1 = fmul2(m, s1);
+                        }
                         reinterpret_cast<float4*>(which ? a.dk_part : a.dq_part)[(prow + (size_t)j * p.H) * KP4 + c4] =
                             make_float4(s0.x, s0.y, s1.x, s1.y);
                     }
                     for (int i = ht; i < ng * (TV / 2); i += HT) {
                         const int j = i / (TV / 2), r = 2 * (i - j * (TV / 2));
-                        const float2 x = *reinterpret_cast<const float2*>(dvs + b * GR * TV + 2 * i);
-                        const float2 y = *reinterpret_cast<const float2*>(dbs + b * GR * TV + 2 * i);
+                        const float2 inv = dup2(fgr[b * GR + j].y);
+                        const float2 x = fmul2(inv, *reinterpret_cast<const float2*>(dvs + b * GR * TV + 2 * i));
+                        const float2 y = fmul2(make_float2(-inv.x, -inv.y), *reinterpret_cast<const float2*>(dbs + b * GR * TV + 2 * i));
                         const long long e = (trow + (long long)j * p.H) * V + v0 + r;
                         if (pairs && r < tvw) {
                             st2(a.dv, e, x, p.io_dtype);
@@ -502,9 +521,10 @@ bwd_kernel(const BwdArgs a) {
                             df += y.x;
                             s2 += y.y;
                         }
-                        const float f = fgr[b * GR + lane];
-                        float dip = (1.f - f) * s2;
-                        if (t0 + gi * GR + lane == 0 && !has_init) dip += f * s2;  // I_0 = Ip: the start-state gradient reaches Ip
+                        const float2 fi = fgr[b * GR + lane];
+                        s2 *= -fi.y;
+                        float dip = (1.f - fi.x) * s2;
+                        if (t0 + gi * GR + lane == 0 && !has_init) dip += fi.x * s2;  // I_0 = Ip: the start-state gradient reaches Ip
                         a.df_part[prow + (size_t)lane * p.H] = df;
                         a.dip_part[prow + (size_t)lane * p.H] = dip;
                     }
@@ -640,7 +660,6 @@ bwd_kernel(const BwdArgs a) {
                 for (int q = 0; q < NP; ++q)
                     sl[(r * NP + q) * NTHR] = make_float4(s.M[r][q].x, s.M[r][q].y, s.I[r][q].x, s.I[r][q].y);
         };
-        float f0 = 1.f;  // f of the last processed block's first token
         for (int it = 0; it < nblk; ++it) {
             const int st = it & 1;
             // this block's operand stage; this thread's d_k columns are RK*kg .. RK*kg+RK-1: pair q covers columns RK*kg + 2q, +1
@@ -651,10 +670,11 @@ bwd_kernel(const BwdArgs a) {
             const float2* dys2 = reinterpret_cast<const float2*>(op + L.dys2) + row0;
             const float2* dyvs2 = reinterpret_cast<const float2*>(op + L.dyvs2) + row0;
             const float4* fc2 = reinterpret_cast<const float4*>(op + L.fc2);
-            const float2* fn2 = reinterpret_cast<const float2*>(op + L.fn2);
-            // one forward step of the recurrence on token tl of the staged block
-            auto fstep = [&](State<RV, NP>& s, int tl) __attribute__((always_inline)) {
-                const float4 fv = fc2[tl];
+            const float2* zz2 = reinterpret_cast<const float2*>(op + L.zz2);
+            // one forward step of the recurrence on token tl of the staged block: P to s; `scaled`: its s may differ from 1
+            auto fstep = [&](auto scaled, const State<RV, NP>& from, State<RV, NP>& s, int tl) __attribute__((always_inline)) {
+                constexpr bool SCALED = decltype(scaled)::value;
+                const float4 fv = SCALED ? fc2[tl] : make_float4(1.f, 1.f, 0.f, 0.f);
                 const float2 ff = make_float2(fv.x, fv.y), cc = make_float2(fv.z, fv.w);
                 float2 kpv[NP], kk[NP];
                 ld_pairs(ks2 + tl * KP2, kpv);
@@ -666,8 +686,8 @@ bwd_kernel(const BwdArgs a) {
                     const float2 vr = make_float2(x.x, x.y), br = make_float2(x.z, x.w);
 #pragma unroll
                     for (int q = 0; q < NP; ++q) {
-                        s.M[r][q] = ffma2(ff, s.M[r][q], fmul2(vr, kpv[q]));
-                        s.I[r][q] = ffma2(ff, s.I[r][q], ffma2(br, kk[q], cc));
+                        s.M[r][q] = SCALED ? ffma2(ff, from.M[r][q], fmul2(vr, kpv[q])) : ffma2(vr, kpv[q], from.M[r][q]);
+                        s.I[r][q] = SCALED ? ffma2(ff, from.I[r][q], ffma2(br, kk[q], cc)) : ffma2(br, kk[q], from.I[r][q]);
                     }
                 }
             };
@@ -676,133 +696,149 @@ bwd_kernel(const BwdArgs a) {
             // Tokens past the end of the sequence (last block only) were staged as identity steps (f = 1,
             // all other operands 0): they leave the state and every gradient untouched, so the block is
             // always processed as NG full groups with no per-token conditionals.
-            // ---- forward sweep: park the start states of groups 1 .. NG-2, keep the last group's in registers
-            State<RV, NP> P[GR + 1];
-            load_ck(P[0], st);
+            const float2 blk = *reinterpret_cast<const float2*>(op + L.blk);
+            const unsigned special = __float_as_uint(blk.y);
+            auto block = [&](auto scaled) __attribute__((always_inline)) {
+                constexpr bool SCALED = decltype(scaled)::value;
+                // ---- forward sweep: park the start states of groups 1 .. NG-2, keep the last group's in registers
+                State<RV, NP> P[GR + 1];
+                load_ck(P[0], st);
 #pragma unroll 1
-            for (int g = 0; g < NG - 1; ++g) {
+                for (int g = 0; g < NG - 1; ++g) {
 #pragma unroll
-                for (int j = 0; j < GR; ++j) fstep(P[0], g * GR + j);
-                if (g < NG - 2) store_slot(P[0], g);
-            }
+                    for (int j = 0; j < GR; ++j) fstep(scaled, P[0], P[0], g * GR + j);
+                    if (g < NG - 2) store_slot(P[0], g);
+                }
+                // the gradients of the block's end state become those of the last window's scaled state
+#pragma unroll
+                for (int r = 0; r < RV; ++r)
+#pragma unroll
+                    for (int q = 0; q < NP; ++q) {
+                        GM[r][q] = fmul2(dup2(blk.x), GM[r][q]);
+                        nGI[r][q] = fmul2(dup2(blk.x), nGI[r][q]);
+                    }
 
+                // Per group: the states of its four tokens from P[0] on, then the reverse walk over them.  With SCALED, a token may have
+                // scaled the state it found, by s, and so does the gradient on its way back.
 #pragma unroll 1
-            for (int gi = NG - 1; gi >= 0; --gi) {
-                if (gi == 0)
-                    load_ck(P[0], st);
-                else if (gi < NG - 1)
-                    load_slot(P[0], gi - 1);
+                for (int gi = NG - 1; gi >= 0; --gi) {
+                    if (gi == 0)
+                        load_ck(P[0], st);
+                    else if (gi < NG - 1)
+                        load_slot(P[0], gi - 1);
+                    const int b = gi & (KBUF - 1);
+                    float red1[NR1], red2[NR2];
 #pragma unroll
-                for (int j = 0; j < GR; ++j) {
-                    P[j + 1] = P[j];
-                    fstep(P[j + 1], gi * GR + j);
-                }
-                const int b = gi & (KBUF - 1);
-                float red1[NR1], red2[NR2];
-                // ---- reverse walk over the group ----------------------------------------------------
+                    for (int j = 0; j < GR; ++j) fstep(scaled, P[j], P[j + 1], gi * GR + j);
 #pragma unroll
-                for (int j = GR - 1; j >= 0; --j) {
-                    const int tl = gi * GR + j;
-                    const float2 fn = fn2[tl];
-                    float2 dqs[NP], Ak[NP], Bk[NP], Uk[NP];
-                    constexpr int RS = RV == 2 ? 2 : 1;  // accumulators: two shorten the dependent chains, three cost registers
-                    float2 Sa[RS], Sb[RS], Sc[RS];
+                    for (int j = GR - 1; j >= 0; --j) {
+                        const int tl = gi * GR + j;
+                        const float2 z = zz2[tl];
+                        const float s = SCALED ? fc2[tl].x : 1.f;
+                        float2 dqs[NP], Ak[NP], Bk[NP], Uk[NP];
+                        constexpr int RS = RV == 2 ? 2 : 1;  // accumulators: two shorten the dependent chains, three cost registers
+                        float2 Sa[RS], Sb[RS], Sc[RS];
 #pragma unroll
-                    for (int r = 0; r < RS; ++r) Sa[r] = Sb[r] = Sc[r] = make_float2(0.f, 0.f);
+                        for (int r = 0; r < RS; ++r) Sa[r] = Sb[r] = Sc[r] = make_float2(0.f, 0.f);
+                        auto add = [](bool first, float2& sum, float2 x, float2 y) __attribute__((always_inline)) { sum = first ? fmul2(x, y) : ffma2(x, y, sum); };
+                        float2 kp[NP], kk[NP], qp[NP];
+                        ld_pairs(ks2 + tl * KP2, kp);
+                        ld_pairs(qs2 + tl * KP2, qp);
 #pragma unroll
-                    for (int q = 0; q < NP; ++q) dqs[q] = Ak[q] = Bk[q] = Uk[q] = make_float2(0.f, 0.f);
-                    float2 kp[NP], kk[NP], qp[NP];
-                    ld_pairs(ks2 + tl * KP2, kp);
-                    ld_pairs(qs2 + tl * KP2, qp);
+                        for (int q = 0; q < NP; ++q) kk[q] = fmul2(kp[q], kp[q]);
+                        float2 dyr[RV], dyvr[RV];
+                        ld_rows(dys2 + tl * TV, dyr);
 #pragma unroll
-                    for (int q = 0; q < NP; ++q) kk[q] = fmul2(kp[q], kp[q]);
-                    float2 dyr[RV], dyvr[RV];
-                    ld_rows(dys2 + tl * TV, dyr);
+                        for (int r = 0; r < RV; ++r) dyvr[r] = make_float2(0.f, 0.f);
+                        if (UNC) ld_rows(dyvs2 + tl * TV, dyvr);
 #pragma unroll
-                    for (int r = 0; r < RV; ++r) dyvr[r] = make_float2(0.f, 0.f);
-                    if (UNC) ld_rows(dyvs2 + tl * TV, dyvr);
+                        for (int r = 0; r < RV; ++r) {
+                            const float4 x = vb4[tl * TV + r];
+                            const float2 vv = make_float2(x.x, x.y), bv = make_float2(x.z, x.w);
+                            const float2 dy = dyr[r];
+                            const float2 dyv = dyvr[r];
+                            float2 dva, dba;
 #pragma unroll
-                    for (int r = 0; r < RV; ++r) {
-                        const float4 x = vb4[tl * TV + r];
-                        const float2 vv = make_float2(x.x, x.y), bv = make_float2(x.z, x.w);
-                        const float2 dy = dyr[r];
-                        const float2 dyv = dyvr[r];
-                        float2 dva = make_float2(0.f, 0.f), dba = dva;
-#pragma unroll
-                        for (int q = 0; q < NP; ++q) {
-                            const float2 Mt = P[j + 1].M[r][q], It = P[j + 1].I[r][q];
-                            const float2 rr = rcp2(It);
-                            const float2 mu = fmul2(Mt, rr);
-                            const float2 qr = UNC ? fmul2(qp[q], rr) : make_float2(0.f, 0.f);
-                        const float2 hh = UNC ? fmul2(dy, qr) : fmul2(fmul2(dy, qp[q]), rr);
-                            GM[r][q] = ffma2(fn, GM[r][q], hh);
-                            float2 hm = fmul2(hh, mu);
-                            if (UNC) hm = ffma2(fmul2(dyv, qr), qr, hm);
-                            nGI[r][q] = ffma2(fn, nGI[r][q], hm);
-                            if (!CO) {
-                                dqs[q] = ffma2(dy, mu, dqs[q]);
-                                if (UNC) Uk[q] = ffma2(dyv, rr, Uk[q]);
-                                Ak[q] = ffma2(GM[r][q], vv, Ak[q]);
-                                Bk[q] = ffma2(nGI[r][q], bv, Bk[q]);
-                                dva = ffma2(GM[r][q], kp[q], dva);
-                                dba = ffma2(nGI[r][q], kk[q], dba);
-                                Sa[r % RS] = ffma2(GM[r][q], P[j].M[r][q], Sa[r % RS]);
-                                Sb[r % RS] = ffma2(nGI[r][q], P[j].I[r][q], Sb[r % RS]);
-                                Sc[r % RS] = fadd2(Sc[r % RS], nGI[r][q]);
+                            for (int q = 0; q < NP; ++q) {
+                                const float2 rr = rcp2(fadd2(P[j + 1].I[r][q], z));
+                                const float2 mu = fmul2(P[j + 1].M[r][q], rr);
+                                const float2 qr = UNC ? fmul2(qp[q], rr) : make_float2(0.f, 0.f);
+                                const float2 hh = UNC ? fmul2(dy, qr) : fmul2(fmul2(dy, qp[q]), rr);
+                                GM[r][q] = fadd2(GM[r][q], hh);
+                                nGI[r][q] = ffma2(hh, mu, nGI[r][q]);
+                                if (UNC) nGI[r][q] = ffma2(fmul2(dyv, qr), qr, nGI[r][q]);
+                                if (!CO) {
+                                    add(r == 0, dqs[q], dy, mu);
+                                    if (UNC) add(r == 0, Uk[q], dyv, rr);
+                                    add(r == 0, Ak[q], GM[r][q], vv);
+                                    add(r == 0, Bk[q], nGI[r][q], bv);
+                                    add(q == 0, dva, GM[r][q], kp[q]);
+                                    add(q == 0, dba, nGI[r][q], kk[q]);
+                                    add(r < RS && q == 0, Sa[r % RS], GM[r][q], P[j].M[r][q]);
+                                    add(r < RS && q == 0, Sb[r % RS], nGI[r][q], P[j].I[r][q]);
+                                    Sc[r % RS] = r < RS && q == 0 ? nGI[r][q] : fadd2(Sc[r % RS], nGI[r][q]);
+                                }
+                                if (SCALED) {
+                                    GM[r][q] = fmul2(dup2(s), GM[r][q]);
+                                    nGI[r][q] = fmul2(dup2(s), nGI[r][q]);
+                                }
                             }
+                            red1[(j * RV + r) * 2 + 0] = dva.x + dva.y;
+                            red1[(j * RV + r) * 2 + 1] = dba.x + dba.y;  // of -GI, as the sum below: the helpers turn the sign
                         }
-                        red1[(j * RV + r) * 2 + 0] = dva.x + dva.y;
-                        red1[(j * RV + r) * 2 + 1] = -(dba.x + dba.y);
-                    }
-                    // this row group's share of dq and dk for the token -> shared memory
-                    if (!CO) {
-                        if (j == GR - 1)  // first write of the group: the helpers must be done with the buffer's last contents
-                            if (!wait_fail && !tc::mbar_wait(&empty[b], (use & 1) ^ 1)) wait_fail = 6;  // after one failure: no more waiting
-                        float2* dst = kred2 + b * (GR * WV * 2 * KP2) + ((j * WV + wv) * 2) * KP2 + NP * kg;
-                        const float2 sc2 = dup2(p.scale), m2 = dup2(-2.f);
+                        // this row group's share of dq (the helpers multiply it by the scale) and dk for the token -> shared memory
+                        if (!CO) {
+                            if (j == GR - 1)  // first write of the group: the helpers must be done with the buffer's last contents
+                                if (!wait_fail && !tc::mbar_wait(&empty[b], (use & 1) ^ 1)) wait_fail = 6;  // after one failure: no more waiting
+                            float2* dst = kred2 + b * (GR * WV * 2 * KP2) + ((j * WV + wv) * 2) * KP2 + NP * kg;
+                            const float2 m2 = dup2(-2.f);
 #pragma unroll
-                        for (int q = 0; q < NP; ++q) {
-                            dqs[q] = UNC ? ffma2(fmul2(dup2(2.f), qp[q]), Uk[q], dqs[q]) : fmul2(sc2, dqs[q]);
-                            Ak[q] = ffma2(fmul2(m2, kp[q]), Bk[q], Ak[q]);
+                            for (int q = 0; q < NP; ++q) {
+                                if (UNC) dqs[q] = ffma2(fmul2(dup2(2.f), qp[q]), Uk[q], dqs[q]);
+                                Ak[q] = ffma2(fmul2(m2, kp[q]), Bk[q], Ak[q]);
+                            }
+                            st_pairs(dst, dqs);
+                            st_pairs(dst + KP2, Ak);
                         }
-                        st_pairs(dst, dqs);
-                        st_pairs(dst + KP2, Ak);
-                    }
-                    float2 sa = Sa[0], sb = Sb[0], scv = Sc[0];
+                        float2 sa = Sa[0], sb = Sb[0], scv = Sc[0];
 #pragma unroll
-                    for (int r = 1; r < RS; ++r) {
-                        sa = fadd2(sa, Sa[r]);
-                        sb = fadd2(sb, Sb[r]);
-                        scv = fadd2(scv, Sc[r]);
-                    }
-                    const float sc_ = scv.x + scv.y;
-                    red2[j * 2 + 0] = (sa.x + sa.y) - (sb.x + sb.y) + iph * sc_;
-                    red2[j * 2 + 1] = -sc_;
-                }
-                if (CO) continue;  // carry-only pass: nothing but the state gradients is wanted
-                // d_v-indexed sums over the KG lanes of a row; per-token scalars over the whole warp
-                xreduce<NR1, KG>(red1, lane);
-                {
-                    const int base = xreduce_index<NR1, KG>(lane), count = xreduce_count<NR1, KG>(lane);
-#pragma unroll
-                    for (int i = 0; i < xreduce_most<NR1, KG>(); ++i)
-                        if (i < count) {
-                            const int id = base + i;
-                            const int j = id / (RV * 2), r = (id / 2) % RV, which = id & 1;
-                            (which ? dbs : dvs)[(b * GR + j) * TV + row0 + r] = red1[i];
+                        for (int r = 1; r < RS; ++r) {
+                            sa = fadd2(sa, Sa[r]);
+                            sb = fadd2(sb, Sb[r]);
+                            scv = fadd2(scv, Sc[r]);
                         }
+                        const float sc_ = scv.x + scv.y;
+                        const float fdf = (sa.x + sa.y) - (sb.x + sb.y) + iph * sc_;
+                        red2[j * 2 + 0] = SCALED ? s * fdf : fdf;
+                        red2[j * 2 + 1] = sc_;
+                    }
+                    if (!CO) {  // a carry-only pass wants nothing but the state gradients
+                        // d_v-indexed sums over the KG lanes of a row; per-token scalars over the whole warp
+                        xreduce<NR1, KG>(red1, lane);
+                        {
+                            const int base = xreduce_index<NR1, KG>(lane), count = xreduce_count<NR1, KG>(lane);
+#pragma unroll
+                            for (int i = 0; i < xreduce_most<NR1, KG>(); ++i)
+                                if (i < count) {
+                                    const int id = base + i;
+                                    const int j = id / (RV * 2), r = (id / 2) % RV, which = id & 1;
+                                    (which ? dbs : dvs)[(b * GR + j) * TV + row0 + r] = red1[i];
+                                }
+                        }
+                        xreduce<NR2, 32>(red2, lane);
+                        if ((lane & (32 / NR2 - 1)) == 0) {
+                            const int id = xreduce_index<NR2, 32>(lane);
+                            wred[((b * W + w) * GR + (id >> 1)) * 2 + (id & 1)] = red2[0];
+                        }
+                        if (tid < GR) fgr[b * GR + tid] = reinterpret_cast<const float2*>(op + L.fi2)[gi * GR + tid];
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&full[b]);  // this warp's partials of the group are written
+                        if (b == 0) ++use;
+                    }
                 }
-                xreduce<NR2, 32>(red2, lane);
-                if ((lane & (32 / NR2 - 1)) == 0) {
-                    const int id = xreduce_index<NR2, 32>(lane);
-                    wred[((b * W + w) * GR + (id >> 1)) * 2 + (id & 1)] = red2[0];
-                }
-                if (tid < GR) fgr[b * GR + tid] = fc2[gi * GR + tid].x;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full[b]);  // this warp's partials of the group are written
-                if (b == 0) ++use;
-            }
-            f0 = fc2[0].x;
+            };
+            if (special) block(std::true_type{});
+            else block(std::false_type{});
             __syncwarp();
             if (lane == 0) mbar_arrive(&done[st]);
         }
@@ -817,17 +853,17 @@ bwd_kernel(const BwdArgs a) {
             if (!CO) a.df_part[(size_t)tile * a.rows_total + (size_t)((long long)bos + s0) * p.H + h] = __int_as_float(0x7fc00000);
         }
 
-        // ---- gradient w.r.t. the segment's start state: decay the first token's totals once more ----------
+        // ---- gradient w.r.t. the segment's start state: that of the first window's ------------------------------
         if (a.rloc_M) {
-            if (failed) f0 = __int_as_float(0x7fc00000);
+            const float bad = failed ? __int_as_float(0x7fc00000) : 1.f;
 #pragma unroll
             for (int r = 0; r < RV; ++r) {
                 if (row0 + r < tvw) {
 #pragma unroll
                     for (int q = 0; q < NP; ++q) {
                         const long long e = (seg_base + v0 + row0 + r) * KP + RK * kg + 2 * q;
-                        *reinterpret_cast<float2*>(a.rloc_M + e) = make_float2(f0 * GM[r][q].x, f0 * GM[r][q].y);
-                        *reinterpret_cast<float2*>(a.rloc_I + e) = make_float2(-f0 * nGI[r][q].x, -f0 * nGI[r][q].y);
+                        *reinterpret_cast<float2*>(a.rloc_M + e) = make_float2(bad * GM[r][q].x, bad * GM[r][q].y);
+                        *reinterpret_cast<float2*>(a.rloc_I + e) = make_float2(-bad * nGI[r][q].x, -bad * nGI[r][q].y);
                     }
                 }
             }
@@ -848,13 +884,14 @@ bwd_kernel(const BwdArgs a) {
 }
 
 // ---- finishing kernel 1 ----------------------------------------------------------------------------------
-// CTAs [0, col_ctas): dq, dk = the row tiles' partials summed in tile order and cast.  A thread owns four consecutive
+// CTAs from nb on: dq, dk = the row tiles' partials summed in tile order and cast.  A thread owns four consecutive
 // columns of a row (16-byte loads, all tiles' loads independent); as many whole rows as fit share a CTA, so that no
-// lane idles whatever d_k is.  The other CTAs: the per-token scalars of a strided share of the tokens, thread = (token
+// lane idles whatever d_k is.  The first nb CTAs: the per-token scalars of a strided share of the tokens, thread = (token
 // lane, head): df and dIp terms summed over the tiles, dgt written, dg and dIp terms accumulated per head and reduced over
-// the CTA's token lanes in a fixed order.  HBM-bound: 8 (KP tiles + 1) bytes read per (token, head), and K io values written
+// the CTA's token lanes in a fixed order, in 64 bits: dg sums terms of both signs that may cancel to a few thousandths of what
+// they add up to, and float sums left it off by 1.1e-5 where 64-bit ones leave 0.4e-5.  HBM-bound: 8 (KP tiles + 1) bytes read per (token, head), and K io values written
 // twice.  With one warp per row, 48-column rows kept 12 of 32 lanes busy: 336 us at B=8 T=4096 H=16 d_k=d_v=48.
-constexpr int FIN_THREADS = 256, FIN_SCALAR_CTAS = 296;
+constexpr int FIN_THREADS = 256, FIN_SCALAR_CTAS = 148;
 
 __device__ __forceinline__ void st4(void* base, long long idx, float4 x, int dt) {  // idx a multiple of 4, base aligned for it
     if (dt == PALIMPSA_F32) {
@@ -875,13 +912,14 @@ __device__ __forceinline__ void st4(void* base, long long idx, float4 x, int dt)
 __global__ void __launch_bounds__(FIN_THREADS)
 bwd_finish_rows(const palimpsa_problem p, const float* __restrict__ dq_part, const float* __restrict__ dk_part,
                 const float* __restrict__ df_part, const float* __restrict__ dip_part, void* dq, void* dk, float* dgt,
-                float* w_dg, float* w_dip, int tiles, int tiles_k, int KP, long long rows, int vec, int col_ctas) {
+                double* w_dg, double* w_dip, int tiles, int tiles_k, int KP, long long rows, int vec, int nb) {
     const int tid = threadIdx.x;
-    if ((int)blockIdx.x < col_ctas) {
+    if ((int)blockIdx.x >= nb) {
+        const int col_ctas = gridDim.x - nb;
         const int KP4 = KP / 4, rpc = FIN_THREADS / KP4, r = tid / KP4, c4 = tid - r * KP4, kc = 4 * c4;
         if (r >= rpc || kc >= p.K) return;
         const size_t step = (size_t)rows * KP4;
-        for (long long row = (long long)blockIdx.x * rpc + r; row < rows; row += (long long)col_ctas * rpc) {
+        for (long long row = (long long)(blockIdx.x - nb) * rpc + r; row < rows; row += (long long)col_ctas * rpc) {
             const float4* pq = reinterpret_cast<const float4*>(dq_part) + (size_t)row * KP4 + c4;
             const float4* pk = reinterpret_cast<const float4*>(dk_part) + (size_t)row * KP4 + c4;
             float4 sq = make_float4(0.f, 0.f, 0.f, 0.f), sk = sq;
@@ -910,26 +948,25 @@ bwd_finish_rows(const palimpsa_problem p, const float* __restrict__ dq_part, con
         }
         return;
     }
-    __shared__ float red[2][FIN_THREADS];
-    const int b = blockIdx.x - col_ctas, nb = gridDim.x - col_ctas, H = p.H;
+    __shared__ double red[2][FIN_THREADS];
+    const int b = blockIdx.x, H = p.H;
     const long long tokens = rows / H;
     const int lanes = H <= FIN_THREADS ? FIN_THREADS / H : 1;  // token lanes
     for (int h0 = 0; h0 < H; h0 += FIN_THREADS) {              // one turn unless there are more heads than threads
         const int lane = H <= FIN_THREADS ? tid / H : 0, h = h0 + (H <= FIN_THREADS ? tid - lane * H : tid);
-        float a0 = 0.f, a1 = 0.f;
+        double a0 = 0., a1 = 0.;
         if (lane < lanes && h < H) {
             const float gh = p.g[h];
             for (long long tok = (long long)b * lanes + lane; tok < tokens; tok += (long long)nb * lanes) {
                 const long long row = tok * H + h;
-                float df = 0.f, dip = 0.f;
+                double df = 0., dip = 0.;
 #pragma unroll 4
                 for (int t = 0; t < tiles_k; ++t) {
                     df += df_part[(size_t)t * rows + row];
                     dip += dip_part[(size_t)t * rows + row];
                 }
-                const float gtv = p.gt[row], fdf = expf(-gtv * gh) * df;
-                dgt[row] = -gh * fdf;
-                a0 -= gtv * fdf;
+                dgt[row] = -gh * (float)df;
+                a0 -= p.gt[row] * df;
                 a1 += dip;
             }
         }
@@ -949,10 +986,10 @@ bwd_finish_rows(const palimpsa_problem p, const float* __restrict__ dq_part, con
 }
 
 // ---- finishing kernel 2: one warp per head, ordered sum over the scalar CTAs' partials -------------------------
-__global__ void __launch_bounds__(32) bwd_finish_heads(const float* __restrict__ w_dg, const float* __restrict__ w_dip,
+__global__ void __launch_bounds__(32) bwd_finish_heads(const double* __restrict__ w_dg, const double* __restrict__ w_dip,
                                                        float* dg, float* dIp, int nb, int H) {
     const int h = blockIdx.x, lane = threadIdx.x;
-    float a0 = 0.f, a1 = 0.f;
+    double a0 = 0., a1 = 0.;
     for (int b = lane; b < nb; b += 32) {
         a0 += w_dg[(size_t)b * H + h];
         a1 += w_dip[(size_t)b * H + h];
@@ -963,8 +1000,8 @@ __global__ void __launch_bounds__(32) bwd_finish_heads(const float* __restrict__
         a1 += __shfl_xor_sync(0xffffffffu, a1, off);
     }
     if (lane == 0) {
-        dg[h] = a0;
-        dIp[h] = a1;
+        dg[h] = (float)a0;
+        dIp[h] = (float)a1;
     }
 }
 
@@ -1089,8 +1126,8 @@ BwdWorkspace bwd_workspace_layout(const palimpsa_problem& p) {
     ws.dk_part = take((size_t)(ws.tiles + 1) * rows * ws.KP * 4);
     ws.df_part = take((size_t)(ws.tiles + 1) * rows * 4);
     ws.dip_part = take((size_t)(ws.tiles + 1) * rows * 4);
-    ws.w_dg = take((size_t)FIN_SCALAR_CTAS * p.H * 4);
-    ws.w_dip = take((size_t)FIN_SCALAR_CTAS * p.H * 4);
+    ws.w_dg = take((size_t)FIN_SCALAR_CTAS * p.H * 8);
+    ws.w_dip = take((size_t)FIN_SCALAR_CTAS * p.H * 8);
     ws.total = off;
     return ws;
 }
@@ -1122,7 +1159,7 @@ static int launch_bwd_w(const BwdArgs& a, int tiles, int num_seg, bool carry_onl
 #define PALIMPSA_BWD_LAUNCH(U, C)                                                                                 \
     do {                                                                                                          \
         if (!allow_smem<bwd_kernel<RK, KG, RV, W, U, C>>(L.total)) return PALIMPSA_E_LAUNCH;                        \
-        if (!bwd_split_fits<bwd_kernel<RK, KG, RV, W, U, C>>(bwd_split(W, RV, RK, U))) return PALIMPSA_E_LAUNCH;    \
+        if (!bwd_split_fits<bwd_kernel<RK, KG, RV, W, U, C>>(bwd_split(W, RV, RK))) return PALIMPSA_E_LAUNCH;    \
         bwd_kernel<RK, KG, RV, W, U, C><<<grid, block, L.total, stream>>>(a);                                     \
     } while (0)
     if (carry_only) {
@@ -1227,12 +1264,12 @@ int launch_bwd(const palimpsa_bwd_params* prm, const palimpsa_segments* segs, bo
         const uintptr_t both = reinterpret_cast<uintptr_t>(prm->dq) | reinterpret_cast<uintptr_t>(prm->dk);
         bwd_finish_rows<<<col_ctas + nb, FIN_THREADS, 0, stream>>>(
             p, a.dq_part, a.dk_part, a.df_part, a.dip_part, prm->dq, prm->dk, prm->dgt,
-            reinterpret_cast<float*>(base + ws.w_dg), reinterpret_cast<float*>(base + ws.w_dip), ws.tiles,
-            ws.tiles + ((stages & 4) ? 1 : 0), ws.KP, rows, p.K % 4 == 0 && (both & (4 * es - 1)) == 0, col_ctas);
+            reinterpret_cast<double*>(base + ws.w_dg), reinterpret_cast<double*>(base + ws.w_dip), ws.tiles,
+            ws.tiles + ((stages & 4) ? 1 : 0), ws.KP, rows, p.K % 4 == 0 && (both & (4 * es - 1)) == 0, nb);
         if (cudaGetLastError() != cudaSuccess) return PALIMPSA_E_LAUNCH;
     }
-    bwd_finish_heads<<<p.H, 32, 0, stream>>>(reinterpret_cast<float*>(base + ws.w_dg),
-                                             reinterpret_cast<float*>(base + ws.w_dip), prm->dg, prm->dIp, nb, p.H);
+    bwd_finish_heads<<<p.H, 32, 0, stream>>>(reinterpret_cast<double*>(base + ws.w_dg),
+                                             reinterpret_cast<double*>(base + ws.w_dip), prm->dg, prm->dIp, nb, p.H);
     return cudaGetLastError() == cudaSuccess ? PALIMPSA_OK : PALIMPSA_E_LAUNCH;
 }
 

@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(128) carry_tc_kernel(const CarryArgs a, const 
         const float c_t = lane == 0 ? c_ws : fmaf(Fp, c_ws, Wp);
         if (tid == 127) cnext_s = fmaf(F, c_ws, Wc);
         if (live) {
-            a.df_x[row] = status == 0 ? a_t * c_t : __int_as_float(0x7fc00000);  // a wait ran out: mark dgt / dg invalid
+            a.df_x[row] = status == 0 ? expf(lf) * a_t * c_t : __int_as_float(0x7fc00000);  // a wait ran out: mark dgt / dg invalid
             float dip = (1.f - f_t) * a_t * SRI;
             if (t0 + tid == 0 && !has_init) dip += f_t * a_t * SRI;
             a.dip_x[row] = dip;

@@ -143,6 +143,76 @@ __device__ __forceinline__ ChunkSplit chunk_split(int chunks, int nthr, int tid)
     return s;
 }
 
+// ---------------------------------------------------------------------------------------------
+// The recurrence without its decay.  Inside a window of tokens over which F_t is the product of the decays f, the scaled
+// state M' = M / F, B' = (I - (1 - F) Ip) / F obeys
+//     M'_t = M'_{t-1} + (v_t / F_t) k_t^T        B'_t = B'_{t-1} + (b_t / F_t) (k_t^2)^T
+//     I_t / F_t = B'_t + Z_t,  Z_t = (1 - F_t) Ip / F_t          mu_t = M'_t / (B'_t + Z_t)
+// -- one packed FMA per pair of state elements instead of a multiply and an FMA for M and two FMAs for I.  B' starts from the
+// true I of the window's start and only positive terms join it, so a small I beside a large Ip keeps its bits.  Every
+// rounding is relative to the value it rounds, as before; F only has to stay in the range of a float, for which a window ends
+// when F would fall below SCALE_LO (gradients of that window's end are held multiplied by F).  A block of 16 tokens is one window unless its decays are faster than that: then a new one
+// begins in front of a group of 4 tokens, and a group that leaves the range by itself (or has an f above 1) is walked token by
+// token in unscaled form (F = 1).  A token that begins a window or is walked by itself first scales the state it finds, by s:
+//     M' <- s M'        B' <- s B' + (1 - s) Ip
+// (s = F at the window's end, times f_t for a token by itself; s = 1 elsewhere: the state is left alone.)
+// ---------------------------------------------------------------------------------------------
+constexpr float SCALE_LO = 0x1p-64f;
+
+struct BlockScale {
+    float f;           // decay of this lane's token (1 past the end)
+    float inv;         // 1 / F_t
+    float z;           // Z_t
+    float s, c;        // scale of the state in front of the token, and (1 - s) Ip
+    float end;         // F at the end of the block, by which its last window ends (the same for the whole block)
+    unsigned special;  // bit t: token t has s != 1 (the same for the whole block)
+};
+// By a whole warp: lanes 0 to 15 hold the tokens of one block, lanes 16 to 31 those of another, or the same again.
+__device__ __forceinline__ BlockScale block_scale(float gt, bool live, float gh, float iph, int lane) {
+    static_assert(TB == 16, "two blocks in a warp");
+    BlockScale b;
+    const int t = lane & 15, j = t & 3, half = lane & 16;
+    b.f = live ? expf(-gt * gh) : 1.f;
+    float x = b.f;  // product over the group up to this token
+    const float y1 = __shfl_up_sync(0xffffffffu, x, 1, 4);
+    if (j >= 1) x *= y1;
+    const float y2 = __shfl_up_sync(0xffffffffu, x, 2, 4);
+    if (j >= 2) x *= y2;
+    float grp[TB / 4], F = x;
+#pragma unroll
+    for (int q = 0; q < TB / 4; ++q) grp[q] = __shfl_sync(0xffffffffu, x, 4 * q + 3, 16);
+    if (t >= 4) F = x * (t < 8 ? grp[0] : t < 12 ? grp[0] * grp[1] : grp[0] * grp[1] * grp[2]);
+    b.s = 1.f;
+    b.special = 0;
+    const unsigned many = __ballot_sync(0xffffffffu, !(F >= SCALE_LO && b.f <= 1.f));
+    if (many) {  // more than one window, in one of the two blocks at least
+        const unsigned out = __ballot_sync(0xffffffffu, !(x >= SCALE_LO && b.f <= 1.f)) >> half;
+        float cum = 1.f, base = 1.f, s = 1.f;
+        bool alone = false;
+#pragma unroll
+        for (int q = 0; q < TB / 4; ++q) {
+            const float next = cum * grp[q];
+            const bool slow = (out >> (4 * q)) & 15u, fresh = slow || !(next >= SCALE_LO);
+            if ((t >> 2) == q) {
+                alone = slow;
+                base = fresh ? 1.f : cum;
+                s = fresh && j == 0 ? cum : 1.f;
+            }
+            cum = slow ? 1.f : fresh ? grp[q] : next;
+        }
+        if ((many >> half) & 0xffffu) {  // a block's scalars depend on nothing but the block
+            b.s = alone ? s * b.f : s;
+            F = alone ? 1.f : base * x;
+        }
+        b.special = (__ballot_sync(0xffffffffu, b.s != 1.f) >> half) & 0xffffu;
+    }
+    b.inv = __frcp_rn(F);
+    b.z = (1.f - F) * iph * b.inv;
+    b.c = (1.f - b.s) * iph;
+    b.end = __shfl_sync(0xffffffffu, F, 15, 16);
+    return b;
+}
+
 // Sum N per-lane values over the L lanes that differ from this one in the low log2(L) bits
 // (L = 2^s <= 32).  "Transposed" butterfly: each step exchanges half of the remaining values, so it
 // costs N-1 (+ a few) shuffles instead of N*log2(L).  An odd remainder above one is padded with a zero (N itself is

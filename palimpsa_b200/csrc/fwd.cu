@@ -3,8 +3,8 @@
 //
 // One CTA owns a tile of TV state rows (d_v) x all KP state columns (padded d_k) of one
 // (sequence, head[, segment]) and walks its tokens in order with the (M, I) state pair held in
-// registers for the whole walk.  Work per state element and token: 6 packed-FP32 lane ops and one
-// MUFU reciprocal -- the kernel is bound by the MUFU pipe, not by HBM.
+// registers for the whole walk, in the scaled form that needs no decay per token (block_scale in common.cuh).  Work per state
+// element and token: 5 packed-FP32 lane ops and one MUFU reciprocal -- the kernel is bound by the MUFU pipe, not by HBM.
 //
 //   thread layout   lane = vg*KG + kg.  A thread owns RV rows x RK columns; the KG lanes of a row
 //                   group own interleaved float4 column groups (column = 4*(j*KG+kg)+i), so that
@@ -12,8 +12,8 @@
 //                   Tile shapes are template parameters: every index in the hot loop is a constant.
 //   staging         blocks of 16 tokens: cp.async (16 B) into a raw double buffer one block ahead,
 //                   then one cooperative pass converts to fp32 operands (q*scale, k; v, b as
-//                   duplicated pairs; {f, f, c, c} with f = exp(-gt*g), c = (1-f)*Ip) shared by every
-//                   thread of the CTA.  k*k is formed in registers.
+//                   duplicated pairs, divided by F) shared by every thread of the CTA.  k*k is formed in
+//                   registers.  The scalars of 8 blocks are worked out together (fwd_scalars).
 //   reduction       o[v] = sum_k: in-thread over RK, then one transposed butterfly per 4 tokens over
 //                   the KG lanes of the row group.
 //   checkpoints     optional (M, I) store at the start of every 16-token block (for backward).
@@ -28,10 +28,15 @@
 
 namespace palimpsa {
 
+// Blocks whose scalars (block_scale) are worked out at a time: what they depend on each other for takes some 300 cycles, which
+// every block would add to the two barriers around its conversion (T = 23, 4 sequences of 4 heads of 128x128: 10.3 -> 10.8 us).
+constexpr int FWD_AHEAD = 8;
+
 struct FwdSmem {
-    int qs, ks, qqs, vs, bs, fc, ys, yvs;  // fp32 operand / result buffers (byte offsets)
+    int qs, ks, qqs, vs, bs, ys, yvs;           // fp32 operand / result buffers (byte offsets)
+    int fc, zz, inv, fs, blk;                   // scalars of FWD_AHEAD blocks
     int raw;                                    // two raw stages follow each other from here
-    int rq, rk, rv, rb, rgt, raw_stage;         // offsets inside a stage, stage size
+    int rq, rk, rv, rb, raw_stage;              // offsets inside a stage, stage size
     int total;
 };
 
@@ -48,7 +53,11 @@ __host__ __device__ inline FwdSmem fwd_smem_layout(int KP, int TV, int es, bool 
     s.qqs = unc ? take(TB * KP * 4) : 0;
     s.vs = take(TB * TV * 8);   // every value stored twice: {v, v}
     s.bs = take(TB * TV * 8);
-    s.fc = take(TB * 16);       // {f, f, c, c}
+    s.fc = take(FWD_AHEAD * TB * 16);   // {s, s, c, c}
+    s.zz = take(FWD_AHEAD * TB * 8);    // {Z, Z}
+    s.inv = take(FWD_AHEAD * TB * 4);   // 1 / F
+    s.fs = take(FWD_AHEAD * TB * 4);    // f
+    s.blk = take(FWD_AHEAD * 16);       // F at the block's end, (1 - F) Ip, BlockScale::special
     s.ys = take(TB * TV * 4);
     s.yvs = unc ? take(TB * TV * 4) : 0;
     s.raw = off;
@@ -62,7 +71,6 @@ __host__ __device__ inline FwdSmem fwd_smem_layout(int KP, int TV, int es, bool 
     s.rk = rtake(TB * KP * es);
     s.rv = rtake(TB * TV * es);
     s.rb = rtake(TB * TV * es);
-    s.rgt = rtake(TB * 4);
     s.raw_stage = r;
     s.total = off + 2 * r;
     return s;
@@ -112,15 +120,55 @@ __device__ __forceinline__ void fwd_issue(const FwdArgs& a, unsigned char* stage
             cp_async16(stage + L.rb + dst, gb + src);
         }
     }
-    for (int i = tid; i < nt; i += nthr) cp_async4(stage + L.rgt + i * 4, p.gt + (tok0 + i) * p.H + h);
 }
 
-// Convert one block to fp32 operands.  ALIGNED: read the raw stage; otherwise read global memory
+// Step sizes of FWD_AHEAD blocks from the one at tok0, of which nt tokens are left, in the registers of NTHR threads.
+template <int NTHR>
+struct FwdSteps {
+    float gt[(FWD_AHEAD * TB + NTHR - 1) / NTHR];
+};
+template <int NTHR>
+__device__ __forceinline__ void fwd_load_steps(FwdSteps<NTHR>& s, const FwdArgs& a, long long tok0, int nt, int h) {
+#pragma unroll
+    for (int x = 0; x < (int)(sizeof(s.gt) / 4); ++x) {
+        const int i = threadIdx.x + x * NTHR;
+        s.gt[x] = i < FWD_AHEAD * TB && i < nt ? a.p.gt[(tok0 + i) * a.p.H + h] : 0.f;
+    }
+}
+
+// Their scalars, two blocks a warp; at d_k = 16 every token by itself (SCALED = false): one warp does this for its 32 rows there,
+// which takes longer than what it saves (B=27 T=1016 H=6 16x32: 244 us unscaled, 255 scaled).
+template <bool SCALED, int NTHR>
+__device__ __forceinline__ void fwd_scalars(const FwdSteps<NTHR>& s, unsigned char* sm, const FwdSmem& L, int nt, float gh, float iph) {
+#pragma unroll
+    for (int x = 0; x < (int)(sizeof(s.gt) / 4); ++x) {
+        const int i = threadIdx.x + x * NTHR;
+        if (i >= FWD_AHEAD * TB || i >= round_up(nt, 32)) break;
+        BlockScale b;
+        if (SCALED) {
+            b = block_scale(s.gt[x], i < nt, gh, iph, i & 31);
+        } else {
+            b.f = b.s = i < nt ? expf(-s.gt[x] * gh) : 1.f;
+            b.c = (1.f - b.s) * iph;
+            b.z = 0.f;
+            b.inv = b.end = 1.f;
+            b.special = 0xffffu;
+        }
+        reinterpret_cast<float4*>(sm + L.fc)[i] = make_float4(b.s, b.s, b.c, b.c);
+        reinterpret_cast<float2*>(sm + L.zz)[i] = make_float2(b.z, b.z);
+        reinterpret_cast<float*>(sm + L.inv)[i] = b.inv;
+        reinterpret_cast<float*>(sm + L.fs)[i] = b.f;
+        if (i % TB == 0)
+            reinterpret_cast<float4*>(sm + L.blk)[i / TB] = make_float4(b.end, (1.f - b.end) * iph, __uint_as_float(b.special), 0.f);
+    }
+}
+
+// Convert one block to fp32 operands (v and b as v / F and b / F, with 1 / F of its tokens in `inv`).  ALIGNED: read the raw stage; otherwise read global memory
 // element by element (any K, V, alignment).
 template <int DT, bool ALIGNED, bool UNC>
 __device__ __forceinline__ void fwd_convert(const FwdArgs& a, unsigned char* sm, const unsigned char* stage,
                                             const FwdSmem& L, int KP, int TV, long long tok0, int nt, int h, int v0,
-                                            float gh, float iph) {
+                                            const float* inv) {
     const palimpsa_problem& p = a.p;
     const int nthr = blockDim.x, tid = threadIdx.x;
     const int K4 = KP / 4, V4 = TV / 4;
@@ -143,7 +191,10 @@ __device__ __forceinline__ void fwd_convert(const FwdArgs& a, unsigned char* sm,
         }
         qs[i] = make_float4(qv.x * sc, qv.y * sc, qv.z * sc, qv.w * sc);
         ks[i] = kv;
-        if (UNC) qqs[i] = make_float4(sc * qv.x * qv.x, sc * qv.y * qv.y, sc * qv.z * qv.z, sc * qv.w * qv.w);
+        if (UNC) {
+            const float scv = sc * inv[t];
+            qqs[i] = make_float4(scv * qv.x * qv.x, scv * qv.y * qv.y, scv * qv.z * qv.z, scv * qv.w * qv.w);
+        }
     }
     float4* vs = reinterpret_cast<float4*>(sm + L.vs);
     float4* bs = reinterpret_cast<float4*>(sm + L.bs);
@@ -160,33 +211,26 @@ __device__ __forceinline__ void fwd_convert(const FwdArgs& a, unsigned char* sm,
                 bv = ld4_guarded<DT>(p.b, row + v0 + c4 * 4, row + p.V);
             }
         }
-        st_dup4(vs, i, vv);
-        st_dup4(bs, i, bv);
-    }
-    float4* fc = reinterpret_cast<float4*>(sm + L.fc);
-    for (int i = tid; i < TB; i += nthr) {
-        float gtv = 0.f;
-        if (i < nt) gtv = ALIGNED ? reinterpret_cast<const float*>(stage + L.rgt)[i] : p.gt[(tok0 + i) * p.H + h];
-        float f = expf(-gtv * gh);
-        const float c = (1.f - f) * iph;
-        fc[i] = make_float4(f, f, c, c);
+        const float m = inv[t];
+        st_dup4(vs, i, make_float4(vv.x * m, vv.y * m, vv.z * m, vv.w * m));
+        st_dup4(bs, i, make_float4(bv.x * m, bv.y * m, bv.z * m, bv.w * m));
     }
 }
 
-// The recurrence over G consecutive tokens (no bounds checks: the caller only passes full groups),
-// followed by one batched reduction of the G*RV (x2 with uncertainty) output partials over the KG lanes
+// The recurrence over G consecutive tokens, some of which scale the state first if SCALED (no bounds checks: the caller only
+// passes full groups), followed by one batched reduction of the G*RV (x2 with uncertainty) output partials over the KG lanes
 // of the row group.  Kept free of conditionals on purpose: the state arrays M, I are updated in place.
-template <int RK, int KG, int RV, int TV, bool UNC, bool SUM, int G>
+template <int RK, int KG, int RV, int TV, bool UNC, bool SUM, int G, bool SCALED>
 __device__ __forceinline__ void fwd_group(float2 (&M)[RV][RK / 4][2], float2 (&I)[RV][RK / 4][2], const float4* ks4,
                                           const float4* qs4, const float4* qqs4, const float2* vs2, const float2* bs2,
-                                          const float4* fc, float* ys, float* yvs, int tg, int kg, int row0, int lane) {
+                                          const float4* fc, const float2* zz, float* ys, float* yvs, int tg, int kg, int row0, int lane) {
     constexpr int KP = RK * KG, J4 = RK / 4, NRED = G * RV * (UNC ? 2 : 1);
     float red[NRED];
 #pragma unroll
     for (int jt = 0; jt < G; ++jt) {
         const int t = tg + jt;
-        const float4 fcv = fc[t];
-        const float2 ff = make_float2(fcv.x, fcv.y), cc = make_float2(fcv.z, fcv.w);
+        const float4 fcv = SCALED ? fc[t] : make_float4(1.f, 1.f, 0.f, 0.f);
+        const float2 ff = make_float2(fcv.x, fcv.y), cc = make_float2(fcv.z, fcv.w), z = SUM ? make_float2(0.f, 0.f) : zz[t];
         float2 vr[RV], br[RV], acc[RV], accv[RV];
         if constexpr (RV % 2 == 0) {  // two adjacent duplicated pairs come in as one 16-byte load (row0 and TV are even)
 #pragma unroll
@@ -221,12 +265,11 @@ __device__ __forceinline__ void fwd_group(float2 (&M)[RV][RK / 4][2], float2 (&I
             for (int r = 0; r < RV; ++r) {
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    M[r][j][e] = ffma2(ff, M[r][j][e], fmul2(vr[r], kp[e]));
-                    if (SUM) {  // J = f*J + b k^2: no prior term, no output
-                        I[r][j][e] = ffma2(ff, I[r][j][e], fmul2(br[r], kkp[e]));
-                    } else {
-                        I[r][j][e] = ffma2(ff, I[r][j][e], ffma2(br[r], kkp[e], cc));
-                        const float2 rr = rcp2(I[r][j][e]);
+                    M[r][j][e] = SCALED ? ffma2(ff, M[r][j][e], fmul2(vr[r], kp[e])) : ffma2(vr[r], kp[e], M[r][j][e]);
+                    // summaries: J = f*J + b k^2, no prior term (Ip = 0, so c = 0) and no output
+                    I[r][j][e] = SCALED ? ffma2(ff, I[r][j][e], ffma2(br[r], kkp[e], cc)) : ffma2(br[r], kkp[e], I[r][j][e]);
+                    if (!SUM) {
+                        const float2 rr = rcp2(KP == 16 ? I[r][j][e] : fadd2(I[r][j][e], z));
                         acc[r] = ffma2(fmul2(M[r][j][e], rr), qp[e], acc[r]);
                         if (UNC) accv[r] = ffma2(rr, qqp[e], accv[r]);
                     }
@@ -279,7 +322,7 @@ __global__ void __launch_bounds__(32 * W, fwd_small_tile<RK, KG, RV, UNC> ? 4 : 
     const FwdSmem L = fwd_smem_layout(KP, TV, es, UNC);
     int bos, len;
     seq_range(p, n, bos, len);
-    const float gh = p.g[h], iph = p.Ip[h];
+    const float gh = p.g[h], iph = SUM ? 0.f : p.Ip[h];
     const int K = p.K, V = p.V;
     const bool vecK = (K % 4) == 0;
     // this CTA's segment of the sequence: tokens [s0, s1)
@@ -287,6 +330,9 @@ __global__ void __launch_bounds__(32 * W, fwd_small_tile<RK, KG, RV, UNC> ? 4 : 
     const int s0 = a.seg_len > 0 ? min(len, g * a.seg_len) : 0;
     const int s1 = a.seg_len > 0 ? min(len, s0 + a.seg_len) : len;
     const long long seg_base = (((long long)n * G + g) * p.H + h) * V;  // row index into [N,G,H,V,KP] buffers
+
+    FwdSteps<NTHR> steps;  // first, so that they are here before the rows: what is made of them takes some 300 cycles
+    fwd_load_steps(steps, a, (long long)bos + s0, s1 - s0, h);
 
     // ---- state registers ------------------------------------------------------------------
     float2 M[RV][J4][2], I[RV][J4][2];
@@ -342,7 +388,6 @@ __global__ void __launch_bounds__(32 * W, fwd_small_tile<RK, KG, RV, UNC> ? 4 : 
     const float4* qqs4 = reinterpret_cast<const float4*>(sm + L.qqs);
     const float2* vs2 = reinterpret_cast<const float2*>(sm + L.vs) + row0;
     const float2* bs2 = reinterpret_cast<const float2*>(sm + L.bs) + row0;
-    const float4* fc = reinterpret_cast<const float4*>(sm + L.fc);
     float* ys = reinterpret_cast<float*>(sm + L.ys);
     float* yvs = reinterpret_cast<float*>(sm + L.yvs);
     unsigned char* raw = sm + L.raw;
@@ -355,7 +400,15 @@ __global__ void __launch_bounds__(32 * W, fwd_small_tile<RK, KG, RV, UNC> ? 4 : 
     }
 
     for (int blk = blk0; blk < nblk; ++blk) {
-        const int t0 = blk * TB;
+        const int t0 = blk * TB, ahead = (blk - blk0) % FWD_AHEAD;
+        if (ahead == 0) {  // the scalars before these have been used: a barrier ago
+            fwd_scalars<(KP > 16)>(steps, sm, L, s1 - t0, gh, iph);
+            fwd_load_steps(steps, a, (long long)bos + t0 + FWD_AHEAD * TB, s1 - t0 - FWD_AHEAD * TB, h);
+        }
+        const float4* fc = reinterpret_cast<const float4*>(sm + L.fc) + ahead * TB;
+        const float2* zz = reinterpret_cast<const float2*>(sm + L.zz) + ahead * TB;
+        const float* inv = reinterpret_cast<const float*>(sm + L.inv) + ahead * TB;
+        const float* fs = reinterpret_cast<const float*>(sm + L.fs) + ahead * TB;
         const int nt = min(TB, s1 - t0);
         const long long tok0 = (long long)bos + t0;
         unsigned char* stage = raw + (blk & 1) * L.raw_stage;
@@ -372,23 +425,23 @@ __global__ void __launch_bounds__(32 * W, fwd_small_tile<RK, KG, RV, UNC> ? 4 : 
         __syncthreads();
         if (a.aligned) {
             if (p.io_dtype == PALIMPSA_BF16)
-                fwd_convert<PALIMPSA_BF16, true, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, gh, iph);
+                fwd_convert<PALIMPSA_BF16, true, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, inv);
             else if (p.io_dtype == PALIMPSA_F32)
-                fwd_convert<PALIMPSA_F32, true, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, gh, iph);
+                fwd_convert<PALIMPSA_F32, true, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, inv);
             else
-                fwd_convert<PALIMPSA_F16, true, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, gh, iph);
+                fwd_convert<PALIMPSA_F16, true, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, inv);
         } else {
             if (p.io_dtype == PALIMPSA_BF16)
-                fwd_convert<PALIMPSA_BF16, false, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, gh, iph);
+                fwd_convert<PALIMPSA_BF16, false, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, inv);
             else if (p.io_dtype == PALIMPSA_F32)
-                fwd_convert<PALIMPSA_F32, false, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, gh, iph);
+                fwd_convert<PALIMPSA_F32, false, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, inv);
             else
-                fwd_convert<PALIMPSA_F16, false, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, gh, iph);
+                fwd_convert<PALIMPSA_F16, false, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, inv);
         }
         __syncthreads();
 
         if (SUM && tid == 0)
-            for (int t = 0; t < nt; ++t) Pdecay *= fc[t].x;
+            for (int t = 0; t < nt; ++t) Pdecay *= fs[t];
         // ---- checkpoint: state before the first token of this block ---------------------------
         if (!SUM && a.ckpt_M) {
             const long long cbase = ((slot0 + blk) * p.H + h) * V;
@@ -409,13 +462,30 @@ __global__ void __launch_bounds__(32 * W, fwd_small_tile<RK, KG, RV, UNC> ? 4 : 
         }
 
         // ---- the recurrence: full groups of GF tokens, then the remaining tokens one by one --------
+        const float4 blk_end = reinterpret_cast<const float4*>(sm + L.blk)[ahead];
+        const unsigned special = __float_as_uint(blk_end.z);
         int tg = 0;
+#define PALIMPSA_GROUP(G)                                                                                                            \
+    do {                                                                                                                             \
+        if (KP == 16 || ((special >> tg) & ((1u << G) - 1u)))                                                                        \
+            fwd_group<RK, KG, RV, TV, UNC, SUM, G, true>(M, I, ks4, qs4, qqs4, vs2, bs2, fc, zz, ys, yvs, tg, kg, row0, lane);       \
+        else                                                                                                                         \
+            fwd_group<RK, KG, RV, TV, UNC, SUM, G, false>(M, I, ks4, qs4, qqs4, vs2, bs2, fc, zz, ys, yvs, tg, kg, row0, lane);      \
+    } while (0)
 #pragma unroll 1
-        for (; tg + GF <= nt; tg += GF)
-            fwd_group<RK, KG, RV, TV, UNC, SUM, GF>(M, I, ks4, qs4, qqs4, vs2, bs2, fc, ys, yvs, tg, kg, row0, lane);
+        for (; tg + GF <= nt; tg += GF) PALIMPSA_GROUP(GF);
 #pragma unroll 1
-        for (; tg < nt; ++tg)
-            fwd_group<RK, KG, RV, TV, UNC, SUM, 1>(M, I, ks4, qs4, qqs4, vs2, bs2, fc, ys, yvs, tg, kg, row0, lane);
+        for (; tg < nt; ++tg) PALIMPSA_GROUP(1);
+#undef PALIMPSA_GROUP
+#pragma unroll
+        for (int r = 0; r < RV; ++r)
+#pragma unroll
+            for (int j = 0; j < J4; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    M[r][j][e] = fmul2(dup2(blk_end.x), M[r][j][e]);
+                    I[r][j][e] = ffma2(dup2(blk_end.x), I[r][j][e], dup2(blk_end.y));
+                }
         __syncthreads();
 
         // ---- write the block's outputs -----------------------------------------------------------

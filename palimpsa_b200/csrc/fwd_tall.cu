@@ -5,16 +5,18 @@
 // converted once per SM, by helper warps, one block ahead of the walk, and the compute warps meet no barrier: they wait for
 // the staged block (an mbarrier), walk its 16 tokens with the state in registers, and hand the reduced outputs back the same
 // way.  What bounds it is the issue rate: a packed FP32 instruction takes two issue cycles (2.05 measured for FMUL2, 2.3 for
-// FFMA2 with a shared operand), so a pair of state elements takes 14 of them per token, its two reciprocals 16 of the MUFU
+// FFMA2 with a shared operand), so a pair of state elements takes 11 of them per token, its two reciprocals 16 of the MUFU
 // pipe, and the rest of a token (operand loads, the sums over a row's lanes) must stay small against 6 or 8 pairs.
-// Forward with checkpoints, ms, fwd.cu's kernel -> this one: B=8 T=4096 H=6 d=128 1.49 -> 1.25, H=16 d=48 1.11 -> 0.86, 48x96
-// 1.51 -> 1.21, B=4 H=16 96x192 2.62 -> 2.09; without: B=2 T=3001 H=16 96x192 1.07 -> 0.75.
+// Forward with checkpoints, ms, fwd.cu's kernel -> this one with the decay in every step -> in the scaled form (block_scale in
+// common.cuh; 5 packed operations a pair instead of 6): B=8 T=4096 H=6 d=128 1.49 -> 1.26 -> 1.16, H=16 d=48 1.11 -> 0.84 -> 0.81,
+// B=4 H=16 96x192 2.62 -> 2.05 -> 1.94; without: B=2 T=3001 H=16 96x192 1.07 -> 0.73 -> 0.68.
 //
 //   thread layout   lane = vg*KG + kg, as in fwd.cu: RV rows x RK columns, interleaved float4 column groups.
 //   blocks          16 tokens; tokens past the end are staged as identity steps (f = 1, all else 0), so that the walk has
-//                   no conditionals.
+//                   no conditionals.  Groups in which a token scales the state take a second copy of the walk.
 //   warps without rows (a tile lower than 12 warps hold) only keep the hand-overs going.
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 #include "fwd.h"
@@ -28,10 +30,10 @@ __device__ int g_fwd_status = 0;
 constexpr int FT_W = 12, FT_HW = 4, FT_NTHR = 32 * FT_W, FT_HT = 32 * FT_HW;
 
 struct TallSmem {
-    int qs, ks, qqs, vb, fc, op_stage;  // offsets inside an operand stage; two stages from 0
+    int qs, ks, qqs, vb, fc, zz, blk, op_stage;  // offsets inside an operand stage; two stages from 0
     int ys, yvs, y_stage;               // reduced outputs, two stages
     int bars;                           // staged[2], done[2]; failure flag
-    int raw, rq, rk, rv, rb, rgt;
+    int raw, rq, rk, rv, rb;
     int total;
 };
 
@@ -48,7 +50,9 @@ __host__ __device__ inline TallSmem tall_smem_layout(int KP, int TV, int es, boo
     s.ks = take(TB * KP * 4);
     s.qqs = unc ? take(TB * KP * 4) : 0;
     s.vb = take(TB * TV * 16);
-    s.fc = take(TB * 16);  // {f, f, c, c}
+    s.fc = take(TB * 16);  // {s, s, c, c}
+    s.zz = take(TB * 8);   // {Z, Z}
+    s.blk = take(16);      // F at the block's end, (1 - F) Ip, BlockScale::special
     s.op_stage = off;
     off *= 2;
     s.ys = off;
@@ -67,7 +71,6 @@ __host__ __device__ inline TallSmem tall_smem_layout(int KP, int TV, int es, boo
     s.rk = rtake(TB * KP * es);
     s.rv = rtake(TB * TV * es);
     s.rb = rtake(TB * TV * es);
-    s.rgt = rtake(TB * 4);
     s.total = off + r;
     return s;
 }
@@ -81,7 +84,6 @@ __device__ __forceinline__ void tall_issue(const FwdArgs& a, int ht, unsigned ch
     const char* gk = reinterpret_cast<const char*>(p.k);
     const char* gv = reinterpret_cast<const char*>(p.v);
     const char* gb = reinterpret_cast<const char*>(p.b);
-    for (int i = ht; i < nt; i += FT_HT) cp_async4(stage + L.rgt + i * 4, p.gt + (tok0 + i) * p.H + h);
     for (int i = ht; i < nt * cq; i += FT_HT) {
         const int t = i / cq, c = i - t * cq;
         const long long src = ((tok0 + t) * p.H + h) * (long long)p.K * es + c * 16;
@@ -98,21 +100,29 @@ __device__ __forceinline__ void tall_issue(const FwdArgs& a, int ht, unsigned ch
     }
 }
 
-// One block of fp32 operands, by the helper warps.  ALIGNED: from the raw stage; otherwise element by element from global
-// memory (any K, V, alignment).
+// One block of fp32 operands (v and b as v / F and b / F: block_scale), by the helper warps.  ALIGNED: from the raw stage;
+// otherwise element by element from global memory (any K, V, alignment).
 template <int DT, bool ALIGNED, bool UNC, int KP, int TV>
 __device__ __forceinline__ void tall_convert(const FwdArgs& a, int ht, const unsigned char* raw, unsigned char* op,
-                                             const TallSmem& L, long long tok0, int nt, int h, int v0, int tvw, float gh,
-                                             float iph) {
+                                             const TallSmem& L, long long tok0, int nt, int h, int v0, int tvw, float iph,
+                                             const BlockScale& bs) {
     const palimpsa_problem& p = a.p;
     constexpr int K4 = KP / 4, V4 = TV / 4;
     float4* qs = reinterpret_cast<float4*>(op + L.qs);
     float4* ks = reinterpret_cast<float4*>(op + L.ks);
     float4* qqs = reinterpret_cast<float4*>(op + L.qqs);
+    if (ht < TB) {
+        reinterpret_cast<float4*>(op + L.fc)[ht] = make_float4(bs.s, bs.s, bs.c, bs.c);
+        reinterpret_cast<float2*>(op + L.zz)[ht] = make_float2(bs.z, bs.z);
+        if (ht == 0)
+            *reinterpret_cast<float4*>(op + L.blk) = make_float4(bs.end, (1.f - bs.end) * iph, __uint_as_float(bs.special), 0.f);
+    }
     const float sc = p.scale;
 #pragma unroll 2
-    for (int i = ht; i < TB * K4; i += FT_HT) {
-        const int t = i / K4, c4 = i - t * K4;
+    for (int i0 = 0; i0 < TB * K4; i0 += FT_HT) {
+        const int i = i0 + ht, t = i / K4, c4 = i - t * K4;
+        const float scv = UNC ? sc * __shfl_sync(0xffffffffu, bs.inv, t & 15) : 0.f;
+        if (i >= TB * K4) break;
         float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), kv = qv;
         if (t < nt && c4 * 4 < p.K) {
             if (ALIGNED) {
@@ -126,13 +136,14 @@ __device__ __forceinline__ void tall_convert(const FwdArgs& a, int ht, const uns
         }
         qs[i] = make_float4(qv.x * sc, qv.y * sc, qv.z * sc, qv.w * sc);
         ks[i] = kv;
-        if (UNC) qqs[i] = make_float4(sc * qv.x * qv.x, sc * qv.y * qv.y, sc * qv.z * qv.z, sc * qv.w * qv.w);
+        if (UNC) qqs[i] = make_float4(scv * qv.x * qv.x, scv * qv.y * qv.y, scv * qv.z * qv.z, scv * qv.w * qv.w);
     }
     float4* vb = reinterpret_cast<float4*>(op + L.vb);
 #pragma unroll 2
-    for (int i = ht; i < TB * V4; i += FT_HT) {
-        const int t = i / V4, r = 4 * (i - t * V4);
-        if (r >= tvw) continue;  // rows past the tile belong to idle warps, or are never written out
+    for (int i0 = 0; i0 < TB * V4; i0 += FT_HT) {
+        const int i = i0 + ht, t = i / V4, r = 4 * (i - t * V4);
+        const float inv = __shfl_sync(0xffffffffu, bs.inv, t & 15);
+        if (i >= TB * V4 || r >= tvw) continue;  // rows past the tile belong to idle warps, or are never written out
         float4 vv = make_float4(0.f, 0.f, 0.f, 0.f), bv = vv;
         if (t < nt) {
             if (ALIGNED) {
@@ -144,20 +155,12 @@ __device__ __forceinline__ void tall_convert(const FwdArgs& a, int ht, const uns
                 bv = ld4_guarded<DT>(p.b, row + r, row + tvw);
             }
         }
+        vv = make_float4(vv.x * inv, vv.y * inv, vv.z * inv, vv.w * inv);
+        bv = make_float4(bv.x * inv, bv.y * inv, bv.z * inv, bv.w * inv);
         vb[4 * i] = make_float4(vv.x, vv.x, bv.x, bv.x);
         vb[4 * i + 1] = make_float4(vv.y, vv.y, bv.y, bv.y);
         vb[4 * i + 2] = make_float4(vv.z, vv.z, bv.z, bv.z);
         vb[4 * i + 3] = make_float4(vv.w, vv.w, bv.w, bv.w);
-    }
-    float4* fc = reinterpret_cast<float4*>(op + L.fc);
-    for (int i = ht; i < TB; i += FT_HT) {
-        float f = 1.f, c = 0.f;
-        if (i < nt) {
-            const float gtv = ALIGNED ? reinterpret_cast<const float*>(raw + L.rgt)[i] : p.gt[(tok0 + i) * p.H + h];
-            f = expf(-gtv * gh);
-            c = (1.f - f) * iph;
-        }
-        fc[i] = make_float4(f, f, c, c);
     }
 }
 
@@ -224,12 +227,24 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
             cp_async_commit();
         };
         auto bar_helpers = [&]() __attribute__((always_inline)) { asm volatile("bar.sync 1, %0;" ::"n"(FT_HT) : "memory"); };
+        float gt = 0.f;  // step size of token lane & 15 of the block that is converted next
+        auto load_gt = [&](int it) __attribute__((always_inline)) {
+            if (it < nblk && (lane & 15) < tokens(it)) gt = p.gt[(token0(it) + (lane & 15)) * p.H + h];
+        };
+        // and that block's scalars: before the wait for the walk, or after it where 16 elements a thread leave no registers to keep
+        // them (B=8 T=4096 H=6 d=128: 1.13 after, 1.16 before; B=2 T=3001 H=16 96x192 0.70 after, 0.68 before)
+        constexpr bool EARLY = RK * RV < 16;
+        BlockScale bs;
+        auto scale = [&](int it) __attribute__((always_inline)) {  // while the rows arrive, or the walk goes on
+            bs = block_scale(gt, (lane & 15) < tokens(it), gh, iph, lane);
+            load_gt(it + 1);
+        };
         auto convert = [&](int it) __attribute__((always_inline)) {
             cp_async_wait<0>();
             bar_helpers();  // every lane's copies have landed
             unsigned char* op = sm + (it & 1) * L.op_stage;
 #define PALIMPSA_CONVERT(DT, AL) \
-    tall_convert<DT, AL, UNC, KP, TV>(a, ht, raw, op, L, token0(it), tokens(it), h, v0, tvw, gh, iph)
+    tall_convert<DT, AL, UNC, KP, TV>(a, ht, raw, op, L, token0(it), tokens(it), h, v0, tvw, iph, bs)
             if (a.aligned) {
                 if (p.io_dtype == PALIMPSA_BF16) PALIMPSA_CONVERT(PALIMPSA_BF16, true);
                 else if (p.io_dtype == PALIMPSA_F32) PALIMPSA_CONVERT(PALIMPSA_F32, true);
@@ -265,15 +280,22 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
             }
         };
         issue(0);
+        load_gt(0);
         if (nblk > 0) {
+            scale(0);
             convert(0);
             arrive(0);
+            if (EARLY) scale(1);
         }
         for (int it = 0; it < nblk; ++it) {
             if (it > 0) wait_done(it - 1);  // frees the operand stage of block it + 1
+            if (!EARLY && it + 1 < nblk) scale(it + 1);
             if (it + 1 < nblk) convert(it + 1);
             if (it > 0) write_outputs(it - 1);  // before the block that reuses their stage is released
-            if (it + 1 < nblk) arrive(it + 1);
+            if (it + 1 < nblk) {
+                arrive(it + 1);
+                if (EARLY) scale(it + 2);
+            }
         }
         if (nblk > 0) {
             wait_done(nblk - 1);
@@ -386,18 +408,21 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
         const float4* qqs4 = reinterpret_cast<const float4*>(op + L.qqs) + kg;
         const float4* vb4 = reinterpret_cast<const float4*>(op + L.vb) + row0;
         const float4* fc = reinterpret_cast<const float4*>(op + L.fc);
+        const float2* zz = reinterpret_cast<const float2*>(op + L.zz);
         float* ys = reinterpret_cast<float*>(sm + L.ys + (it & 1) * L.y_stage);
         float* yvs = reinterpret_cast<float*>(sm + L.yvs + (it & 1) * L.y_stage);
         if (!wait_fail && !tc::mbar_wait(&staged[it & 1], (it >> 1) & 1, POLLS)) wait_fail = 8;
         const int end = min(TB, s1 - (blk0 + it) * TB);
-#pragma unroll 1
-        for (int tg = 0; tg < end; tg += GF) {
-            float red[NRED];
+        const float4 blk = *reinterpret_cast<const float4*>(op + L.blk);
+        const unsigned special = __float_as_uint(blk.z);
+        // GF tokens from tg on; `scaled`: some of them scale the state first
+        auto group = [&](auto scaled, int tg, auto& red) __attribute__((always_inline)) {
+            constexpr bool SCALED = decltype(scaled)::value;
 #pragma unroll
             for (int jt = 0; jt < GF; ++jt) {
                 const int t = tg + jt;
-                const float4 fcv = fc[t];
-                const float2 ff = make_float2(fcv.x, fcv.y), cc = make_float2(fcv.z, fcv.w);
+                const float4 fcv = SCALED ? fc[t] : make_float4(1.f, 1.f, 0.f, 0.f);
+                const float2 ff = make_float2(fcv.x, fcv.y), cc = make_float2(fcv.z, fcv.w), z = zz[t];
                 float2 vr[RV], br[RV], acc[RV], accv[RV];
 #pragma unroll
                 for (int r = 0; r < RV; ++r) {
@@ -420,9 +445,9 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
                     for (int r = 0; r < RV; ++r) {
 #pragma unroll
                         for (int e = 0; e < 2; ++e) {
-                            M[r][j][e] = ffma2(ff, M[r][j][e], fmul2(vr[r], kp[e]));
-                            I[r][j][e] = ffma2(ff, I[r][j][e], ffma2(br[r], kkp[e], cc));
-                            const float2 rr = rcp2(I[r][j][e]);
+                            M[r][j][e] = SCALED ? ffma2(ff, M[r][j][e], fmul2(vr[r], kp[e])) : ffma2(vr[r], kp[e], M[r][j][e]);
+                            I[r][j][e] = SCALED ? ffma2(ff, I[r][j][e], ffma2(br[r], kkp[e], cc)) : ffma2(br[r], kkp[e], I[r][j][e]);
+                            const float2 rr = rcp2(fadd2(I[r][j][e], z));
                             acc[r] = ffma2(fmul2(M[r][j][e], rr), qp[e], acc[r]);
                             if (UNC) accv[r] = ffma2(rr, qqp[e], accv[r]);
                         }
@@ -434,6 +459,12 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
                     if (UNC) red[(jt * RV + r) * 2 + 1] = accv[r].x + accv[r].y;
                 }
             }
+        };
+#pragma unroll 1
+        for (int tg = 0; tg < end; tg += GF) {
+            float red[NRED];
+            if ((special >> tg) & ((1u << GF) - 1u)) group(std::true_type{}, tg, red);
+            else group(std::false_type{}, tg, red);
             xreduce<NRED, KG>(red, lane);
             const int base = xreduce_index<NRED, KG>(lane), count = xreduce_count<NRED, KG>(lane);
 #pragma unroll
@@ -444,6 +475,15 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
                     (which ? yvs : ys)[(tg + jt) * TV + row0 + r] = red[i];
                 }
         }
+#pragma unroll
+        for (int r = 0; r < RV; ++r)
+#pragma unroll
+            for (int j = 0; j < J4; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    M[r][j][e] = fmul2(dup2(blk.x), M[r][j][e]);
+                    I[r][j][e] = ffma2(dup2(blk.x), I[r][j][e], dup2(blk.y));
+                }
         __syncwarp();
         if (lane == 0) mbar_arrive(&done[it & 1]);
     }

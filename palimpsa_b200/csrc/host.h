@@ -98,7 +98,7 @@ double bwd_token_cost(const palimpsa_problem& p);  // estimated time per token o
 struct BwdWorkspace {
     size_t dq_part, dk_part;    // float [tiles][tokens*H][KP]   (dk, df, dip: tiles + 1 slots)
     size_t df_part, dip_part;   // float [tiles][tokens*H]
-    size_t w_dg, w_dip;         // float [scalar CTAs of the finishing kernel][H]
+    size_t w_dg, w_dip;         // double [scalar CTAs of the finishing kernel][H]
     size_t total;
     int tiles, KP;
 };
