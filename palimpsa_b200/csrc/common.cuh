@@ -72,6 +72,22 @@ __device__ __forceinline__ float4 ld4(const void* base, int idx4) {
     }
 }
 
+// N (2 or 4) consecutive floats in one access, as pairs.
+template <int N>
+__device__ __forceinline__ void ld_cols(const float* p, float2 (&x)[N / 2]) {
+    if constexpr (N == 4) {
+        const float4 y = *reinterpret_cast<const float4*>(p);
+        x[0] = make_float2(y.x, y.y), x[1] = make_float2(y.z, y.w);
+    } else {
+        x[0] = *reinterpret_cast<const float2*>(p);
+    }
+}
+template <int N>
+__device__ __forceinline__ void st_cols(float* p, const float2 (&x)[N / 2]) {
+    if constexpr (N == 4) *reinterpret_cast<float4*>(p) = make_float4(x[0].x, x[0].y, x[1].x, x[1].y);
+    else *reinterpret_cast<float2*>(p) = x[0];
+}
+
 // One value from global memory, any alignment.
 template <int DT>
 __device__ __forceinline__ float ld1(const void* base, long long idx) {

@@ -217,6 +217,11 @@ __device__ __forceinline__ void fwd_convert(const FwdArgs& a, unsigned char* sm,
     }
 }
 
+// Sums of a row that a lane keeps: two where two lanes of the tall kernel's tiling have its columns between them (RK = 12: either
+// half of its groups of four columns; RK = 16: every second group) and add their sums first, so that both kernels add up a row in
+// the same order.
+__host__ __device__ constexpr int fwd_sums(int RK) { return RK >= 12 ? 2 : 1; }
+
 // The recurrence over G consecutive tokens, some of which scale the state first if SCALED (no bounds checks: the caller only
 // passes full groups), followed by one batched reduction of the G*RV (x2 with uncertainty) output partials over the KG lanes
 // of the row group.  Kept free of conditionals on purpose: the state arrays M, I are updated in place.
@@ -224,14 +229,14 @@ template <int RK, int KG, int RV, int TV, bool UNC, bool SUM, int G, bool SCALED
 __device__ __forceinline__ void fwd_group(float2 (&M)[RV][RK / 4][2], float2 (&I)[RV][RK / 4][2], const float4* ks4,
                                           const float4* qs4, const float4* qqs4, const float2* vs2, const float2* bs2,
                                           const float4* fc, const float2* zz, float* ys, float* yvs, int tg, int kg, int row0, int lane) {
-    constexpr int KP = RK * KG, J4 = RK / 4, NRED = G * RV * (UNC ? 2 : 1);
+    constexpr int KP = RK * KG, J4 = RK / 4, NA = fwd_sums(RK), NRED = G * RV * (UNC ? 2 : 1);
     float red[NRED];
 #pragma unroll
     for (int jt = 0; jt < G; ++jt) {
         const int t = tg + jt;
         const float4 fcv = SCALED ? fc[t] : make_float4(1.f, 1.f, 0.f, 0.f);
         const float2 ff = make_float2(fcv.x, fcv.y), cc = make_float2(fcv.z, fcv.w), z = SUM ? make_float2(0.f, 0.f) : zz[t];
-        float2 vr[RV], br[RV], acc[RV], accv[RV];
+        float2 vr[RV], br[RV], acc[RV][NA], accv[RV][NA];
         if constexpr (RV % 2 == 0) {  // two adjacent duplicated pairs come in as one 16-byte load (row0 and TV are even)
 #pragma unroll
             for (int r = 0; r < RV; r += 2) {
@@ -250,7 +255,9 @@ __device__ __forceinline__ void fwd_group(float2 (&M)[RV][RK / 4][2], float2 (&I
             }
         }
 #pragma unroll
-        for (int r = 0; r < RV; ++r) acc[r] = accv[r] = make_float2(0.f, 0.f);
+        for (int r = 0; r < RV; ++r)
+#pragma unroll
+            for (int e = 0; e < NA; ++e) acc[r][e] = accv[r][e] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int j = 0; j < J4; ++j) {
             const int idx = t * (KP / 4) + j * KG + kg;
@@ -270,16 +277,21 @@ __device__ __forceinline__ void fwd_group(float2 (&M)[RV][RK / 4][2], float2 (&I
                     I[r][j][e] = SCALED ? ffma2(ff, I[r][j][e], ffma2(br[r], kkp[e], cc)) : ffma2(br[r], kkp[e], I[r][j][e]);
                     if (!SUM) {
                         const float2 rr = rcp2(KP == 16 ? I[r][j][e] : fadd2(I[r][j][e], z));
-                        acc[r] = ffma2(fmul2(M[r][j][e], rr), qp[e], acc[r]);
-                        if (UNC) accv[r] = ffma2(rr, qqp[e], accv[r]);
+                        acc[r][RK == 16 ? j % NA : e % NA] = ffma2(fmul2(M[r][j][e], rr), qp[e], acc[r][RK == 16 ? j % NA : e % NA]);
+                        if (UNC) accv[r][RK == 16 ? j % NA : e % NA] = ffma2(rr, qqp[e], accv[r][RK == 16 ? j % NA : e % NA]);
                     }
                 }
             }
         }
 #pragma unroll
         for (int r = 0; r < RV; ++r) {
-            red[(jt * RV + r) * (UNC ? 2 : 1)] = acc[r].x + acc[r].y;
-            if (UNC) red[(jt * RV + r) * 2 + 1] = accv[r].x + accv[r].y;
+            float y = acc[r][0].x + acc[r][0].y, yv = accv[r][0].x + accv[r][0].y;
+            if (NA == 2) {
+                y += acc[r][NA - 1].x + acc[r][NA - 1].y;
+                yv += accv[r][NA - 1].x + accv[r][NA - 1].y;
+            }
+            red[(jt * RV + r) * (UNC ? 2 : 1)] = y;
+            if (UNC) red[(jt * RV + r) * 2 + 1] = yv;
         }
     }
     if (SUM) return;

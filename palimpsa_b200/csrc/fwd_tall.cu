@@ -8,10 +8,14 @@
 // FFMA2 with a shared operand), so a pair of state elements takes 11 of them per token, its two reciprocals 16 of the MUFU
 // pipe, and the rest of a token (operand loads, the sums over a row's lanes) must stay small against 6 or 8 pairs.
 // Forward with checkpoints, ms, fwd.cu's kernel -> this one with the decay in every step -> in the scaled form (block_scale in
-// common.cuh; 5 packed operations a pair instead of 6): B=8 T=4096 H=6 d=128 1.49 -> 1.26 -> 1.16, H=16 d=48 1.11 -> 0.84 -> 0.81,
-// B=4 H=16 96x192 2.62 -> 2.05 -> 1.94; without: B=2 T=3001 H=16 96x192 1.07 -> 0.73 -> 0.68.
+// common.cuh; 5 packed operations a pair instead of 6) -> with 2 rows of 6 or 8 columns a thread where it had one row of 12 or 16
+// (d_k other than 128: half the operand loads and squares of k per element, for one more value to sum over the lanes): B=8 T=4096
+// H=6 d=128 1.49 -> 1.26 -> 1.16, H=16 d=48 1.11 -> 0.84 -> 0.81 -> 0.71 (1 row of 6 there: launch_tall_t), B=4 T=2048 H=16 96x192
+// 1.31 -> 1.03 -> 0.97 -> 0.95, with the uncertainty output 1.31 -> 1.31 -> 1.15; without checkpoints: B=2 T=3001 H=16 96x192
+// 1.07 -> 0.73 -> 0.68 -> 0.66, B=4 T=2048 H=6 256x128 0.64 -> 0.59 -> 0.57.
 //
-//   thread layout   lane = vg*KG + kg, as in fwd.cu: RV rows x RK columns, interleaved float4 column groups.
+//   thread layout   lane = vg*KG + kg, as in fwd.cu: RV rows x RK columns, interleaved float4 column groups, or halves of them
+//                   where a lane has 6 columns.
 //   blocks          16 tokens; tokens past the end are staged as identity steps (f = 1, all else 0), so that the walk has
 //                   no conditionals.  Groups in which a token scales the state take a second copy of the walk.
 //   warps without rows (a tile lower than 12 warps hold) only keep the hand-overs going.
@@ -173,13 +177,17 @@ __host__ __device__ constexpr int tall_group() {
 
 template <int RK, int KG, int RV, bool UNC, unsigned POLLS = tc::SPIN_LIMIT>
 __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdArgs a, const int rows) {
-    constexpr int KP = RK * KG, VG = 32 / KG, J4 = RK / 4, TV = FT_W * VG * RV, GF = tall_group<KG, RV, UNC>();
+    constexpr int KP = RK * KG, VG = 32 / KG, CW = RK % 4 ? 2 : 4, J = RK / CW, E = CW / 2, TV = FT_W * VG * RV, GF = tall_group<KG, RV, UNC>();
     constexpr int NRED = GF * RV * (UNC ? 2 : 1);
-    static_assert(TV % 4 == 0 && TB % GF == 0, "operands are converted four rows at a time, blocks are whole groups");
+    static_assert(TV % 8 == 0 && TB % GF == 0, "raw rows of 16-bit values start on 16 bytes, blocks are whole groups");
     extern __shared__ __align__(16) unsigned char sm[];
     const palimpsa_problem& p = a.p;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int kg = lane % KG, vg = lane / KG;
+    // Columns of a lane: groups of four, every KG-th; with two columns a group the lanes of the upper half have the second half of
+    // the groups of those of the lower.
+    constexpr int GS = CW == 4 ? 4 * KG : 2 * KG;  // from one group of a lane to its next
+    const int col0 = CW == 4 ? 4 * kg : 4 * (kg % (KG / 2)) + 2 * (kg / (KG / 2));
     const int row0 = (w * VG + vg) * RV;
     const int ny = blockIdx.y / p.H, h = blockIdx.y - ny * p.H;
     const int n = p.seq_order ? p.seq_order[ny] : ny;  // blocks start in grid order: a packed batch lists its longest sequences first
@@ -337,45 +345,45 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
     const long long seg_base = (((long long)n * G + g) * p.H + h) * V;  // row index into [N,G,H,V,KP] buffers
     const long long st_base = ((long long)n * p.H + h) * V;
     const long long slot0 = seq_first_slot(p, n);
-    float2 M[RV][J4][2], I[RV][J4][2];
+    float2 M[RV][J][E], I[RV][J][E];  // columns col0 + j*GS + 2e, + 1
 #pragma unroll
     for (int r = 0; r < RV; ++r) {
         const int row = row0 + r;
 #pragma unroll
-        for (int j = 0; j < J4; ++j) {
-            const int kc = 4 * (j * KG + kg);
-            float4 m4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            float4 i4 = make_float4(1.f, 1.f, 1.f, 1.f);
+        for (int j = 0; j < J; ++j) {
+            const int kc = col0 + j * GS;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                M[r][j][e] = make_float2(0.f, 0.f);
+                I[r][j][e] = make_float2(1.f, 1.f);
+            }
             if (row < tvw) {
                 if (a.start_M) {
                     const long long e = (seg_base + v0 + row) * KP + kc;
-                    m4 = *reinterpret_cast<const float4*>(a.start_M + e);
-                    i4 = *reinterpret_cast<const float4*>(a.start_I + e);
+                    ld_cols<CW>(a.start_M + e, M[r][j]);
+                    ld_cols<CW>(a.start_I + e, I[r][j]);
                 } else if (kc < K) {
                     if (p.init_mu) {
                         const long long e = (st_base + v0 + row) * K + kc;
-                        float4 mu4;
                         if (vecK) {
-                            mu4 = *reinterpret_cast<const float4*>(p.init_mu + e);
-                            i4 = *reinterpret_cast<const float4*>(p.init_I + e);
+                            ld_cols<CW>(p.init_mu + e, M[r][j]);
+                            ld_cols<CW>(p.init_I + e, I[r][j]);
                         } else {
-                            const long long lim = (st_base + v0 + row + 1) * K;
-                            mu4 = ld4_guarded<PALIMPSA_F32>(p.init_mu, e, lim);
-                            i4 = ld4_guarded<PALIMPSA_F32>(p.init_I, e, lim);
-                            if (kc + 1 >= K) i4.y = 1.f;
-                            if (kc + 2 >= K) i4.z = 1.f;
-                            if (kc + 3 >= K) i4.w = 1.f;
+#pragma unroll
+                            for (int c = 0; c < CW; ++c)
+                                if (kc + c < K) {
+                                    (c & 1 ? M[r][j][c / 2].y : M[r][j][c / 2].x) = p.init_mu[e + c];
+                                    (c & 1 ? I[r][j][c / 2].y : I[r][j][c / 2].x) = p.init_I[e + c];
+                                }
                         }
-                        m4 = make_float4(mu4.x * i4.x, mu4.y * i4.y, mu4.z * i4.z, mu4.w * i4.w);
+#pragma unroll
+                        for (int c = 0; c < E; ++c) M[r][j][c] = fmul2(M[r][j][c], I[r][j][c]);
                     } else {
-                        i4 = make_float4(iph, iph, iph, iph);
+#pragma unroll
+                        for (int c = 0; c < E; ++c) I[r][j][c] = dup2(iph);
                     }
                 }
             }
-            M[r][j][0] = make_float2(m4.x, m4.y);
-            M[r][j][1] = make_float2(m4.z, m4.w);
-            I[r][j][0] = make_float2(i4.x, i4.y);
-            I[r][j][1] = make_float2(i4.z, i4.w);
         }
     }
     for (int it = 0; it < nblk; ++it) {
@@ -392,20 +400,18 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
             for (int r = 0; r < RV; ++r) {
                 if (row0 + r < tvw) {
 #pragma unroll
-                    for (int j = 0; j < J4; ++j) {
-                        const long long e = (cbase + row0 + r) * KP + 4 * (j * KG + kg);
-                        *reinterpret_cast<float4*>(a.ckpt_M + e) =
-                            make_float4(M[r][j][0].x, M[r][j][0].y, M[r][j][1].x, M[r][j][1].y);
-                        *reinterpret_cast<float4*>(a.ckpt_I + e) =
-                            make_float4(I[r][j][0].x, I[r][j][0].y, I[r][j][1].x, I[r][j][1].y);
+                    for (int j = 0; j < J; ++j) {
+                        const long long e = (cbase + row0 + r) * KP + col0 + j * GS;
+                        st_cols<CW>(a.ckpt_M + e, M[r][j]);
+                        st_cols<CW>(a.ckpt_I + e, I[r][j]);
                     }
                 }
             }
         }
         const unsigned char* op = sm + (it & 1) * L.op_stage;
-        const float4* qs4 = reinterpret_cast<const float4*>(op + L.qs) + kg;
-        const float4* ks4 = reinterpret_cast<const float4*>(op + L.ks) + kg;
-        const float4* qqs4 = reinterpret_cast<const float4*>(op + L.qqs) + kg;
+        const float* qs = reinterpret_cast<const float*>(op + L.qs) + col0;
+        const float* ks = reinterpret_cast<const float*>(op + L.ks) + col0;
+        const float* qqs = reinterpret_cast<const float*>(op + L.qqs) + col0;
         const float4* vb4 = reinterpret_cast<const float4*>(op + L.vb) + row0;
         const float4* fc = reinterpret_cast<const float4*>(op + L.fc);
         const float2* zz = reinterpret_cast<const float2*>(op + L.zz);
@@ -432,19 +438,18 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
                     acc[r] = accv[r] = make_float2(0.f, 0.f);
                 }
 #pragma unroll
-                for (int j = 0; j < J4; ++j) {
-                    const int idx = t * (KP / 4) + j * KG;
-                    const float4 k4 = ks4[idx], q4 = qs4[idx];
-                    float4 qq4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (UNC) qq4 = qqs4[idx];
-                    const float2 kp[2] = {make_float2(k4.x, k4.y), make_float2(k4.z, k4.w)};
-                    const float2 kkp[2] = {fmul2(kp[0], kp[0]), fmul2(kp[1], kp[1])};
-                    const float2 qp[2] = {make_float2(q4.x, q4.y), make_float2(q4.z, q4.w)};
-                    const float2 qqp[2] = {make_float2(qq4.x, qq4.y), make_float2(qq4.z, qq4.w)};
+                for (int j = 0; j < J; ++j) {
+                    const int idx = t * KP + j * GS;
+                    float2 kp[E], kkp[E], qp[E], qqp[E];
+                    ld_cols<CW>(ks + idx, kp);
+                    ld_cols<CW>(qs + idx, qp);
+                    if (UNC) ld_cols<CW>(qqs + idx, qqp);
+#pragma unroll
+                    for (int e = 0; e < E; ++e) kkp[e] = fmul2(kp[e], kp[e]);
 #pragma unroll
                     for (int r = 0; r < RV; ++r) {
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) {
+                        for (int e = 0; e < E; ++e) {
                             M[r][j][e] = SCALED ? ffma2(ff, M[r][j][e], fmul2(vr[r], kp[e])) : ffma2(vr[r], kp[e], M[r][j][e]);
                             I[r][j][e] = SCALED ? ffma2(ff, I[r][j][e], ffma2(br[r], kkp[e], cc)) : ffma2(br[r], kkp[e], I[r][j][e]);
                             const float2 rr = rcp2(fadd2(I[r][j][e], z));
@@ -478,9 +483,9 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
 #pragma unroll
         for (int r = 0; r < RV; ++r)
 #pragma unroll
-            for (int j = 0; j < J4; ++j)
+            for (int j = 0; j < J; ++j)
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
+                for (int e = 0; e < E; ++e) {
                     M[r][j][e] = fmul2(dup2(blk.x), M[r][j][e]);
                     I[r][j][e] = ffma2(dup2(blk.x), I[r][j][e], dup2(blk.y));
                 }
@@ -492,24 +497,22 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
 #pragma unroll
         for (int r = 0; r < RV; ++r) {
 #pragma unroll
-            for (int j = 0; j < J4; ++j) {
-                const int kc = 4 * (j * KG + kg);
+            for (int j = 0; j < J; ++j) {
+                const int kc = col0 + j * GS;
                 if (row0 + r < tvw && kc < K) {
-                    const float4 i4 = make_float4(I[r][j][0].x, I[r][j][0].y, I[r][j][1].x, I[r][j][1].y);
-                    const float4 mu4 = make_float4(M[r][j][0].x / i4.x, M[r][j][0].y / i4.y, M[r][j][1].x / i4.z,
-                                                   M[r][j][1].y / i4.w);
+                    float2 mu[E];
+#pragma unroll
+                    for (int e = 0; e < E; ++e) mu[e] = make_float2(M[r][j][e].x / I[r][j][e].x, M[r][j][e].y / I[r][j][e].y);
                     const long long e = (st_base + v0 + row0 + r) * K + kc;
                     if (vecK) {
-                        *reinterpret_cast<float4*>(a.final_mu + e) = mu4;
-                        *reinterpret_cast<float4*>(a.final_I + e) = i4;
+                        st_cols<CW>(a.final_mu + e, mu);
+                        st_cols<CW>(a.final_I + e, I[r][j]);
                     } else {
-                        const float mus[4] = {mu4.x, mu4.y, mu4.z, mu4.w};
-                        const float is[4] = {i4.x, i4.y, i4.z, i4.w};
 #pragma unroll
-                        for (int c = 0; c < 4; ++c)
+                        for (int c = 0; c < CW; ++c)
                             if (kc + c < K) {
-                                a.final_mu[e + c] = mus[c];
-                                a.final_I[e + c] = is[c];
+                                a.final_mu[e + c] = c & 1 ? mu[c / 2].y : mu[c / 2].x;
+                                a.final_I[e + c] = c & 1 ? I[r][j][c / 2].y : I[r][j][c / 2].x;
                             }
                     }
                 }
@@ -524,15 +527,16 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
 // -------------------------------------------------------------------------------------------------
 // Host side
 // -------------------------------------------------------------------------------------------------
-// The thread tilings, one per padded d_k: X(RK, KG, RV), 12 or 16 state elements a thread.
+// The thread tilings, one per padded d_k: X(RK, KG, RV), 12 or 16 state elements a thread.  The sums of a row add up in
+// the same order as with fwd.cu's tiling at that d_k.
 #define PALIMPSA_TALL_TILINGS(X)       \
     switch (KP) {                      \
-        case 48: X(12, 4, 1); break;   \
-        case 64: X(16, 4, 1); break;   \
-        case 96: X(12, 8, 1); break;   \
+        case 48: X(6, 8, 2); break;    \
+        case 64: X(8, 8, 2);  break;   \
+        case 96: X(6, 16, 2); break;   \
         case 128: X(8, 16, 2); break;  \
-        case 192: X(12, 16, 1); break; \
-        case 256: X(16, 16, 1); break; \
+        case 192: X(6, 32, 2);  break; \
+        case 256: X(8, 32, 2);  break; \
         default: break;                \
     }
 
@@ -601,9 +605,8 @@ bool fwd_tall_pays(const palimpsa_problem& p, int num_seg, int short_rows, int s
 }
 
 template <int RK, int KG, int RV>
-static int launch_tall_t(const FwdArgs& a, int num_seg, cudaStream_t stream) {
+static int launch_tall_k(const FwdArgs& a, const TallPlan& t, int num_seg, cudaStream_t stream) {
     const palimpsa_problem& p = a.p;
-    const TallPlan t = tall_plan<RK, KG, RV>(p, num_seg);
     const bool unc = (p.flags & PALIMPSA_FLAG_UNCERTAINTY) != 0;
     const TallSmem L = tall_smem_layout(RK * KG, FT_W * (32 / KG) * RV, dtype_size(p.io_dtype), unc);
     const dim3 grid(t.tiles, p.num_seqs * p.H, num_seg), block(FT_NTHR + FT_HT, 1, 1);
@@ -615,6 +618,16 @@ static int launch_tall_t(const FwdArgs& a, int num_seg, cudaStream_t stream) {
         fwd_tall_kernel<RK, KG, RV, false><<<grid, block, L.total, stream>>>(a, t.rows);
     }
     return cudaGetLastError() == cudaSuccess ? PALIMPSA_OK : PALIMPSA_E_LAUNCH;
+}
+
+// Tiles of up to 12 warps of one row a thread (48 rows at d_k = 48) fill half of the warps or less with two: with one all have rows,
+// and each scheduler has as many.  B=8 T=4096 H=16 48x48 (48 rows: 6 warps or 12): 0.81 -> 0.71 ms; T=37 of 4 sequences 12.0 -> 10.2 us.
+template <int RK, int KG, int RV>
+static int launch_tall_t(const FwdArgs& a, int num_seg, cudaStream_t stream) {
+    const TallPlan t = tall_plan<RK, KG, RV>(a.p, num_seg);
+    if constexpr (RK == 6 && FT_W * (32 / KG) % 8 == 0)  // whole 16-byte chunks of 16-bit rows
+        if (t.rows <= FT_W * (32 / KG)) return launch_tall_k<RK, KG, 1>(a, t, num_seg, stream);
+    return launch_tall_k<RK, KG, RV>(a, t, num_seg, stream);
 }
 
 int fwd_tall_rows(const palimpsa_problem& p, int num_seg) {
