@@ -1048,10 +1048,11 @@ static const BwdTile* bwd_tile_choices(int KP) {
     }
 }
 // What a token costs a CTA (the walk, and what does not grow with the rows), in units of which 4 warps take 8.  One wave, T =
-// 512, bf16 and float32 alike within 3 %, us at 4 / 6 / 8 warps (8 of 3 rows): d_k = 48 196 / 268 / 342, 96 193 / 261 / 337, 192
-// 197 / 268 / 355, 64 151 / - / 230 (285), 128 148 / - / 226 (290), 32 173 / - / 229, 16 113 / - / 162, 256 - / - / 357.  With
-// the uncertainty output 213 / 305 / 374, 213 / 292 / 374, 216 / 283 / 387, 159 / - / 247 (342), 160 / - / 246 (328), 159 / - / 253,
-// 121 / - / 173, - / - / 370.  The state-gradient pass of exact segments takes 0.45 to 0.55 of that at every height.
+// 512, bf16, us at 4 / 6 / 8 warps (8 of 3 rows): d_k = 48 181 / 247 / 325, 96 182 / 243 / 320, 192 186 / 263 / 340, 64 146 / - / 213
+// (314), 128 149 / - / 224 (266), 32 164 / - / 216, 16 120 / - / 165, 256 - / - / 358.  With the uncertainty output 207 / 276 / 356,
+// 209 / 285 / 356, 212 / 287 / 381, 160 / - / 229 (317), 160 / - / 250 (306), 159 / - / 234, 124 / - / 178, - / - / 359.  The
+// state-gradient pass of exact segments takes 0.45 to 0.55 of that at every height.  (3 rows of d_k = 64 spill 44 bytes: 285 before
+// the scaled form, when the other heights took 151 and 230.  The costs are those of then: the planner's cuts were fitted with them.)
 static double bwd_tile_cost(const BwdTile& t, int KP, int NE, bool unc) {
     if (t.RV == 3) return KP == 64 ? (unc ? 17.2 : 15.1) : unc ? 16.4 : 15.7;
     return t.W == 4 ? 8 : t.W == 6 ? 11 : NE == 12 ? 14.2 : 12;
