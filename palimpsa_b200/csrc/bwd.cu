@@ -973,12 +973,15 @@ bwd_finish_rows(const palimpsa_problem p, const float* __restrict__ dq_part, con
         }
         red[0][tid] = a0;
         red[1][tid] = a1;
-        __syncthreads();
-        if (lane == 0 && h < H) {
-            for (int l = 1; l < lanes; ++l) {
-                a0 += red[0][l * H + h];
-                a1 += red[1][l * H + h];
+        for (int n = lanes; n > 1; n = (n + 1) / 2) {  // lanes of the upper half join those of the lower
+            const int upper = lane + (n + 1) / 2;
+            __syncthreads();
+            if (upper < n && h < H) {
+                red[0][tid] = a0 += red[0][upper * H + h];
+                red[1][tid] = a1 += red[1][upper * H + h];
             }
+        }
+        if (lane == 0 && h < H) {
             w_dg[(size_t)b * H + h] = a0;
             w_dip[(size_t)b * H + h] = a1;
         }
