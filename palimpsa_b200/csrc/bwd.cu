@@ -153,7 +153,7 @@ struct BwdStaging {
     unsigned q[NQ][4], k[NQ][4];                // 4 columns: packed 16-bit pairs in [0], [1] where they came in one load
     unsigned v[NV][2], b[NV][2], o[NV][2], ov[NV][2];  // 2 rows: a packed 16-bit pair in [0]
     float gt;                                   // step size of token lane & 15 of the block
-    float inv;                                  // and 1 / F of that token, once its first step has been stored
+    BlockScale sc;                              // and what bwd_scale has made of the block's
 };
 
 // N consecutive elements of ES bytes at element e, the first n of them (the others 0).
@@ -231,22 +231,24 @@ __device__ __forceinline__ void bwd_load(BwdStaging<KP, TV, TS, NTH, UNC>& s, co
     }
 }
 
+// The scalars of a block of nt tokens.  By whole warps, each for itself; between the block's first load and its first store.
+template <int KP, int TV, int TS, int NTH, bool UNC>
+__device__ __forceinline__ void bwd_scale(BwdStaging<KP, TV, TS, NTH, UNC>& s, int tid, int nt, float gh, float iph) {
+    s.sc = block_scale<true>(s.gt, (tid & (TB - 1)) < nt, gh, iph, tid & 31);
+}
+
 // What bwd_load brought, as fp32 operands into the operand stage `op`: v, b and the uncertainty's gradient divided by F
-// (block_scale).  By whole warps, each of which finds the block's scalars for itself.
+// (block_scale).  By whole warps.
 template <int DT, int KP, int TV, int TS, int NTH, bool UNC>
 __device__ __forceinline__ void bwd_store(BwdStaging<KP, TV, TS, NTH, UNC>& s, const BwdArgs& a, int tid, unsigned char* op,
-                                          const BwdSmem& L, int ts, int nt, float gh, float iph) {
+                                          const BwdSmem& L, int ts) {
     using S = BwdStaging<KP, TV, TS, NTH, UNC>;
-    if (ts == 0) {
-        const int lane = tid & 31, t = lane & (TB - 1);
-        const BlockScale b = block_scale(s.gt, t < nt, gh, iph, lane);
-        s.inv = b.inv;
-        if (tid >= S::F0 && tid < S::F0 + TB) {
-            reinterpret_cast<float4*>(op + L.fc2)[t] = make_float4(b.s, b.s, b.c, b.c);
-            reinterpret_cast<float2*>(op + L.zz2)[t] = make_float2(b.z, b.z);
-            reinterpret_cast<float2*>(op + L.fi2)[t] = make_float2(b.f, b.inv);
-            if (t == 0) *reinterpret_cast<float2*>(op + L.blk) = make_float2(b.end, __uint_as_float(b.special));
-        }
+    if (ts == 0 && tid >= S::F0 && tid < S::F0 + TB) {
+        const int t = tid & (TB - 1);
+        reinterpret_cast<float4*>(op + L.fc2)[t] = make_float4(s.sc.s, s.sc.s, s.sc.c, s.sc.c);
+        reinterpret_cast<float2*>(op + L.zz2)[t] = make_float2(s.sc.z, s.sc.z);
+        reinterpret_cast<float2*>(op + L.fi2)[t] = make_float2(s.sc.f, s.sc.w);
+        if (t == 0) *reinterpret_cast<float2*>(op + L.blk) = make_float2(s.sc.end, __uint_as_float(s.sc.special));
     }
     float4* qs = reinterpret_cast<float4*>(op + L.qs) + ts * S::K4;
     float4* ks = reinterpret_cast<float4*>(op + L.ks) + ts * S::K4;
@@ -268,7 +270,7 @@ __device__ __forceinline__ void bwd_store(BwdStaging<KP, TV, TS, NTH, UNC>& s, c
 #pragma unroll
     for (int x = 0; x < S::NV; ++x) {
         const int i = tid + x * NTH;
-        const float inv = __shfl_sync(0xffffffffu, s.inv, (ts + i / S::V2) & (TB - 1));
+        const float inv = __shfl_sync(0xffffffffu, s.sc.w, (ts + i / S::V2) & (TB - 1));
         if (i >= TS * S::V2) break;
         float v[2], b[2], o[2];
         word_values<DT>(s.v[x], v, a.vec_v);
@@ -413,18 +415,21 @@ bwd_kernel(const BwdArgs a) {
         if (es == 4) bwd_load<4>(s, a, id, tok0_of(it), ts, nt, h, v0, tvw);
         else bwd_load<2>(s, a, id, tok0_of(it), ts, nt, h, v0, tvw);
     };
+    auto scale = [&](auto& s, int id, int it) __attribute__((always_inline)) {
+        bwd_scale(s, id, min(TB, len - (blk1 - 1 - it) * TB), gh, iph);
+    };
     auto store = [&](auto& s, int id, int it, int ts) __attribute__((always_inline)) {
-        const int nt = min(TB, len - (blk1 - 1 - it) * TB);
         unsigned char* op = sm + (it & 1) * L.op_stage;
-        if (p.io_dtype == PALIMPSA_BF16) bwd_store<PALIMPSA_BF16>(s, a, id, op, L, ts, nt, gh, iph);
-        else if (p.io_dtype == PALIMPSA_F32) bwd_store<PALIMPSA_F32>(s, a, id, op, L, ts, nt, gh, iph);
-        else bwd_store<PALIMPSA_F16>(s, a, id, op, L, ts, nt, gh, iph);
+        if (p.io_dtype == PALIMPSA_BF16) bwd_store<PALIMPSA_BF16>(s, a, id, op, L, ts);
+        else if (p.io_dtype == PALIMPSA_F32) bwd_store<PALIMPSA_F32>(s, a, id, op, L, ts);
+        else bwd_store<PALIMPSA_F16>(s, a, id, op, L, ts);
     };
     bwd_issue_ckpt(a, bwd_threads(W), tid, sm, L, 0, KP, TV, slot0 + blk1 - 1, h, v0, tvw);
     cp_async_commit();
     {
         BwdStaging<KP, TV, TB, bwd_threads(W), UNC> s;
         load(s, tid, 0, 0);
+        scale(s, tid, 0);
         store(s, tid, 0, 0);
     }
     cp_async_wait<0>();
@@ -444,7 +449,10 @@ bwd_kernel(const BwdArgs a) {
             if (lane == 0) mbar_arrive(&staged[it & 1]);
         };
         arrive_staged(0);
-        if (nblk > 1) load(next, ht, 1, 0);
+        if (nblk > 1) {
+            load(next, ht, 1, 0);
+            scale(next, ht, 1);
+        }
 
         // Two rows of dv / db in one store: d_v even (then a tile's rows are too), both buffers aligned for a pair.
         const bool pairs = V % 2 == 0 && ((reinterpret_cast<uintptr_t>(a.dv) | reinterpret_cast<uintptr_t>(a.db)) & (2 * es - 1)) == 0;
@@ -533,6 +541,7 @@ bwd_kernel(const BwdArgs a) {
                     if (lane == 0) mbar_arrive(&empty[b]);
                 }
             }
+            if (it + 2 < nblk) scale(next, ht, it + 2);  // while nothing waits for it
         }
         cp_async_wait<0>();
         if (wait_fail) *fail_flag = wait_fail;

@@ -12,7 +12,7 @@
 //                   Tile shapes are template parameters: every index in the hot loop is a constant.
 //   staging         blocks of 16 tokens: cp.async (16 B) into a raw double buffer one block ahead,
 //                   then one cooperative pass converts to fp32 operands (q*scale, k; v, b as
-//                   duplicated pairs, divided by F) shared by every thread of the CTA.  k*k is formed in
+//                   duplicated pairs, scaled) shared by every thread of the CTA.  k*k is formed in
 //                   registers.  The scalars of 8 blocks are worked out together (fwd_scalars).
 //   reduction       o[v] = sum_k: in-thread over RK, then one transposed butterfly per 4 tokens over
 //                   the KG lanes of the row group.
@@ -34,7 +34,7 @@ constexpr int FWD_AHEAD = 8;
 
 struct FwdSmem {
     int qs, ks, qqs, vs, bs, ys, yvs;           // fp32 operand / result buffers (byte offsets)
-    int fc, zz, inv, fs, blk;                   // scalars of FWD_AHEAD blocks
+    int fc, zz, ws, fs, blk;                    // scalars of FWD_AHEAD blocks
     int raw;                                    // two raw stages follow each other from here
     int rq, rk, rv, rb, raw_stage;              // offsets inside a stage, stage size
     int total;
@@ -55,9 +55,9 @@ __host__ __device__ inline FwdSmem fwd_smem_layout(int KP, int TV, int es, bool 
     s.bs = take(TB * TV * 8);
     s.fc = take(FWD_AHEAD * TB * 16);   // {s, s, c, c}
     s.zz = take(FWD_AHEAD * TB * 8);    // {Z, Z}
-    s.inv = take(FWD_AHEAD * TB * 4);   // 1 / F
+    s.ws = take(FWD_AHEAD * TB * 4);    // w
     s.fs = take(FWD_AHEAD * TB * 4);    // f
-    s.blk = take(FWD_AHEAD * 16);       // F at the block's end, (1 - F) Ip, BlockScale::special
+    s.blk = take(FWD_AHEAD * 8);        // BlockScale::end, special
     s.ys = take(TB * TV * 4);
     s.yvs = unc ? take(TB * TV * 4) : 0;
     s.raw = off;
@@ -146,29 +146,28 @@ __device__ __forceinline__ void fwd_scalars(const FwdSteps<NTHR>& s, unsigned ch
         if (i >= FWD_AHEAD * TB || i >= round_up(nt, 32)) break;
         BlockScale b;
         if (SCALED) {
-            b = block_scale(s.gt[x], i < nt, gh, iph, i & 31);
+            b = block_scale<false>(s.gt[x], i < nt, gh, iph, i & 31);
         } else {
             b.f = b.s = i < nt ? expf(-s.gt[x] * gh) : 1.f;
             b.c = (1.f - b.s) * iph;
-            b.z = 0.f;
-            b.inv = b.end = 1.f;
+            b.z = b.end = 0.f;
+            b.w = 1.f;
             b.special = 0xffffu;
         }
         reinterpret_cast<float4*>(sm + L.fc)[i] = make_float4(b.s, b.s, b.c, b.c);
         reinterpret_cast<float2*>(sm + L.zz)[i] = make_float2(b.z, b.z);
-        reinterpret_cast<float*>(sm + L.inv)[i] = b.inv;
+        reinterpret_cast<float*>(sm + L.ws)[i] = b.w;
         reinterpret_cast<float*>(sm + L.fs)[i] = b.f;
-        if (i % TB == 0)
-            reinterpret_cast<float4*>(sm + L.blk)[i / TB] = make_float4(b.end, (1.f - b.end) * iph, __uint_as_float(b.special), 0.f);
+        if (i % TB == 0) reinterpret_cast<float2*>(sm + L.blk)[i / TB] = make_float2(b.end, __uint_as_float(b.special));
     }
 }
 
-// Convert one block to fp32 operands (v and b as v / F and b / F, with 1 / F of its tokens in `inv`).  ALIGNED: read the raw stage; otherwise read global memory
-// element by element (any K, V, alignment).
+// Convert one block to fp32 operands (v and b times w of block_scale, which is in `ws` for the block's tokens).  ALIGNED: read
+// the raw stage; otherwise read global memory element by element (any K, V, alignment).
 template <int DT, bool ALIGNED, bool UNC>
 __device__ __forceinline__ void fwd_convert(const FwdArgs& a, unsigned char* sm, const unsigned char* stage,
                                             const FwdSmem& L, int KP, int TV, long long tok0, int nt, int h, int v0,
-                                            const float* inv) {
+                                            const float* ws) {
     const palimpsa_problem& p = a.p;
     const int nthr = blockDim.x, tid = threadIdx.x;
     const int K4 = KP / 4, V4 = TV / 4;
@@ -192,7 +191,7 @@ __device__ __forceinline__ void fwd_convert(const FwdArgs& a, unsigned char* sm,
         qs[i] = make_float4(qv.x * sc, qv.y * sc, qv.z * sc, qv.w * sc);
         ks[i] = kv;
         if (UNC) {
-            const float scv = sc * inv[t];
+            const float scv = sc * ws[t];
             qqs[i] = make_float4(scv * qv.x * qv.x, scv * qv.y * qv.y, scv * qv.z * qv.z, scv * qv.w * qv.w);
         }
     }
@@ -211,7 +210,7 @@ __device__ __forceinline__ void fwd_convert(const FwdArgs& a, unsigned char* sm,
                 bv = ld4_guarded<DT>(p.b, row + v0 + c4 * 4, row + p.V);
             }
         }
-        const float m = inv[t];
+        const float m = ws[t];
         st_dup4(vs, i, make_float4(vv.x * m, vv.y * m, vv.z * m, vv.w * m));
         st_dup4(bs, i, make_float4(bv.x * m, bv.y * m, bv.z * m, bv.w * m));
     }
@@ -228,13 +227,15 @@ __host__ __device__ constexpr int fwd_sums(int RK) { return RK >= 12 ? 2 : 1; }
 template <int RK, int KG, int RV, int TV, bool UNC, bool SUM, int G, bool SCALED>
 __device__ __forceinline__ void fwd_group(float2 (&M)[RV][RK / 4][2], float2 (&I)[RV][RK / 4][2], const float4* ks4,
                                           const float4* qs4, const float4* qqs4, const float2* vs2, const float2* bs2,
-                                          const float4* fc, const float2* zz, float* ys, float* yvs, int tg, int kg, int row0, int lane) {
+                                          const float4* fc, const float2* zz, float missing, float* ys, float* yvs, int tg, int kg, int row0,
+                                          int lane) {
     constexpr int KP = RK * KG, J4 = RK / 4, NA = fwd_sums(RK), NRED = G * RV * (UNC ? 2 : 1);
     float red[NRED];
 #pragma unroll
     for (int jt = 0; jt < G; ++jt) {
         const int t = tg + jt;
-        const float4 fcv = SCALED ? fc[t] : make_float4(1.f, 1.f, 0.f, 0.f);
+        float4 fcv = SCALED ? fc[t] : make_float4(1.f, 1.f, 0.f, 0.f);
+        if (SCALED && KP > 16 && t == 0) fcv.z = fcv.w = fcv.x * missing;
         const float2 ff = make_float2(fcv.x, fcv.y), cc = make_float2(fcv.z, fcv.w), z = SUM ? make_float2(0.f, 0.f) : zz[t];
         float2 vr[RV], br[RV], acc[RV][NA], accv[RV][NA];
         if constexpr (RV % 2 == 0) {  // two adjacent duplicated pairs come in as one 16-byte load (row0 and TV are even)
@@ -272,9 +273,14 @@ __device__ __forceinline__ void fwd_group(float2 (&M)[RV][RK / 4][2], float2 (&I
             for (int r = 0; r < RV; ++r) {
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    M[r][j][e] = SCALED ? ffma2(ff, M[r][j][e], fmul2(vr[r], kp[e])) : ffma2(vr[r], kp[e], M[r][j][e]);
                     // summaries: J = f*J + b k^2, no prior term (Ip = 0, so c = 0) and no output
-                    I[r][j][e] = SCALED ? ffma2(ff, I[r][j][e], ffma2(br[r], kkp[e], cc)) : ffma2(br[r], kkp[e], I[r][j][e]);
+                    if (KP == 16) {
+                        M[r][j][e] = ffma2(ff, M[r][j][e], fmul2(vr[r], kp[e]));
+                        I[r][j][e] = ffma2(ff, I[r][j][e], ffma2(br[r], kkp[e], cc));
+                    } else {  // the same result from either copy
+                        M[r][j][e] = ffma2(vr[r], kp[e], SCALED ? fmul2(ff, M[r][j][e]) : M[r][j][e]);
+                        I[r][j][e] = ffma2(br[r], kkp[e], SCALED ? ffma2(ff, I[r][j][e], cc) : I[r][j][e]);
+                    }
                     if (!SUM) {
                         const float2 rr = rcp2(KP == 16 ? I[r][j][e] : fadd2(I[r][j][e], z));
                         acc[r][RK == 16 ? j % NA : e % NA] = ffma2(fmul2(M[r][j][e], rr), qp[e], acc[r][RK == 16 ? j % NA : e % NA]);
@@ -313,7 +319,7 @@ __device__ __forceinline__ void fwd_group(float2 (&M)[RV][RK / 4][2], float2 (&I
 
 // The d_k = 128 tiling (16 state elements per thread, 16 lanes per row) reduces 8 tokens' outputs in one butterfly
 // and is held to 128 registers (4 CTAs of 4 warps per SM): 1.57 -> 1.49 ms on the 170M shape.  The other tilings
-// keep batches of 4 and the compiler's own register count (8 there costs them spills).
+// keep batches of 4 and the compiler's own register count (8 there costs them spills).  (It spilled nothing then, 8 bytes now.)
 template <int RK, int KG, int RV, bool UNC>
 constexpr bool fwd_small_tile = RK * RV <= 16 && KG == 16 && !UNC;
 
@@ -411,6 +417,7 @@ __global__ void __launch_bounds__(32 * W, fwd_small_tile<RK, KG, RV, UNC> ? 4 : 
         cp_async_commit();
     }
 
+    float missing = 0.f;  // from I since the last block: u Ip (block_scale)
     for (int blk = blk0; blk < nblk; ++blk) {
         const int t0 = blk * TB, ahead = (blk - blk0) % FWD_AHEAD;
         if (ahead == 0) {  // the scalars before these have been used: a barrier ago
@@ -419,7 +426,7 @@ __global__ void __launch_bounds__(32 * W, fwd_small_tile<RK, KG, RV, UNC> ? 4 : 
         }
         const float4* fc = reinterpret_cast<const float4*>(sm + L.fc) + ahead * TB;
         const float2* zz = reinterpret_cast<const float2*>(sm + L.zz) + ahead * TB;
-        const float* inv = reinterpret_cast<const float*>(sm + L.inv) + ahead * TB;
+        const float* ws = reinterpret_cast<const float*>(sm + L.ws) + ahead * TB;
         const float* fs = reinterpret_cast<const float*>(sm + L.fs) + ahead * TB;
         const int nt = min(TB, s1 - t0);
         const long long tok0 = (long long)bos + t0;
@@ -437,18 +444,18 @@ __global__ void __launch_bounds__(32 * W, fwd_small_tile<RK, KG, RV, UNC> ? 4 : 
         __syncthreads();
         if (a.aligned) {
             if (p.io_dtype == PALIMPSA_BF16)
-                fwd_convert<PALIMPSA_BF16, true, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, inv);
+                fwd_convert<PALIMPSA_BF16, true, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, ws);
             else if (p.io_dtype == PALIMPSA_F32)
-                fwd_convert<PALIMPSA_F32, true, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, inv);
+                fwd_convert<PALIMPSA_F32, true, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, ws);
             else
-                fwd_convert<PALIMPSA_F16, true, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, inv);
+                fwd_convert<PALIMPSA_F16, true, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, ws);
         } else {
             if (p.io_dtype == PALIMPSA_BF16)
-                fwd_convert<PALIMPSA_BF16, false, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, inv);
+                fwd_convert<PALIMPSA_BF16, false, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, ws);
             else if (p.io_dtype == PALIMPSA_F32)
-                fwd_convert<PALIMPSA_F32, false, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, inv);
+                fwd_convert<PALIMPSA_F32, false, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, ws);
             else
-                fwd_convert<PALIMPSA_F16, false, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, inv);
+                fwd_convert<PALIMPSA_F16, false, UNC>(a, sm, stage, L, KP, TV, tok0, nt, h, v0, ws);
         }
         __syncthreads();
 
@@ -466,38 +473,47 @@ __global__ void __launch_bounds__(32 * W, fwd_small_tile<RK, KG, RV, UNC> ? 4 : 
                         const long long e = (cbase + vrow) * KP + 4 * (j * KG + kg);
                         *reinterpret_cast<float4*>(a.ckpt_M + e) =
                             make_float4(M[r][j][0].x, M[r][j][0].y, M[r][j][1].x, M[r][j][1].y);
-                        *reinterpret_cast<float4*>(a.ckpt_I + e) =
-                            make_float4(I[r][j][0].x, I[r][j][0].y, I[r][j][1].x, I[r][j][1].y);
+                        *reinterpret_cast<float4*>(a.ckpt_I + e) = make_float4(
+                            I[r][j][0].x + missing, I[r][j][0].y + missing, I[r][j][1].x + missing, I[r][j][1].y + missing);
                     }
                 }
             }
         }
 
         // ---- the recurrence: full groups of GF tokens, then the remaining tokens one by one --------
-        const float4 blk_end = reinterpret_cast<const float4*>(sm + L.blk)[ahead];
-        const unsigned special = __float_as_uint(blk_end.z);
+        const float2 blk_end = reinterpret_cast<const float2*>(sm + L.blk)[ahead];
+        const unsigned special = __float_as_uint(blk_end.y);
         int tg = 0;
+        // A window that begins with the group: the state is scaled here, and the group has nothing more to scale.
+        auto edge = [&](int t) __attribute__((always_inline)) {
+            float4 fcv = fc[t];
+            if (t == 0) fcv.z = fcv.w = fcv.x * missing;
+#pragma unroll
+            for (int r = 0; r < RV; ++r)
+#pragma unroll
+                for (int j = 0; j < J4; ++j)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        M[r][j][e] = fmul2(make_float2(fcv.x, fcv.y), M[r][j][e]);
+                        I[r][j][e] = ffma2(make_float2(fcv.x, fcv.y), I[r][j][e], make_float2(fcv.z, fcv.w));
+                    }
+        };
 #define PALIMPSA_GROUP(G)                                                                                                            \
     do {                                                                                                                             \
-        if (KP == 16 || ((special >> tg) & ((1u << G) - 1u)))                                                                        \
-            fwd_group<RK, KG, RV, TV, UNC, SUM, G, true>(M, I, ks4, qs4, qqs4, vs2, bs2, fc, zz, ys, yvs, tg, kg, row0, lane);       \
-        else                                                                                                                         \
-            fwd_group<RK, KG, RV, TV, UNC, SUM, G, false>(M, I, ks4, qs4, qqs4, vs2, bs2, fc, zz, ys, yvs, tg, kg, row0, lane);      \
+        const unsigned bits = (special >> tg) & ((1u << G) - 1u);                                                                    \
+        if (KP == 16 || (bits & ~1u)) {                                                                                              \
+            fwd_group<RK, KG, RV, TV, UNC, SUM, G, true>(M, I, ks4, qs4, qqs4, vs2, bs2, fc, zz, missing, ys, yvs, tg, kg, row0, lane);\
+        } else {                                                                                                                     \
+            if (bits) edge(tg);                                                                                                      \
+            fwd_group<RK, KG, RV, TV, UNC, SUM, G, false>(M, I, ks4, qs4, qqs4, vs2, bs2, fc, zz, missing, ys, yvs, tg, kg, row0, lane);\
+        }                                                                                                                            \
     } while (0)
 #pragma unroll 1
         for (; tg + GF <= nt; tg += GF) PALIMPSA_GROUP(GF);
 #pragma unroll 1
         for (; tg < nt; ++tg) PALIMPSA_GROUP(1);
 #undef PALIMPSA_GROUP
-#pragma unroll
-        for (int r = 0; r < RV; ++r)
-#pragma unroll
-            for (int j = 0; j < J4; ++j)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    M[r][j][e] = fmul2(dup2(blk_end.x), M[r][j][e]);
-                    I[r][j][e] = ffma2(dup2(blk_end.x), I[r][j][e], dup2(blk_end.y));
-                }
+        missing = blk_end.x;
         __syncthreads();
 
         // ---- write the block's outputs -----------------------------------------------------------
@@ -539,7 +555,8 @@ __global__ void __launch_bounds__(32 * W, fwd_small_tile<RK, KG, RV, UNC> ? 4 : 
             for (int j = 0; j < J4; ++j) {
                 const int kc = 4 * (j * KG + kg);
                 if (vrow < V && kc < K) {
-                    const float4 i4 = make_float4(I[r][j][0].x, I[r][j][0].y, I[r][j][1].x, I[r][j][1].y);
+                    const float4 i4 = make_float4(I[r][j][0].x + missing, I[r][j][0].y + missing, I[r][j][1].x + missing,
+                                                  I[r][j][1].y + missing);
                     const float4 mu4 = make_float4(M[r][j][0].x / i4.x, M[r][j][0].y / i4.y, M[r][j][1].x / i4.z,
                                                    M[r][j][1].y / i4.w);
                     const long long e = (st_base + vrow) * K + kc;

@@ -56,7 +56,7 @@ __host__ __device__ inline TallSmem tall_smem_layout(int KP, int TV, int es, boo
     s.vb = take(TB * TV * 16);
     s.fc = take(TB * 16);  // {s, s, c, c}
     s.zz = take(TB * 8);   // {Z, Z}
-    s.blk = take(16);      // F at the block's end, (1 - F) Ip, BlockScale::special
+    s.blk = take(16);      // BlockScale::end, special
     s.op_stage = off;
     off *= 2;
     s.ys = off;
@@ -104,28 +104,28 @@ __device__ __forceinline__ void tall_issue(const FwdArgs& a, int ht, unsigned ch
     }
 }
 
-// One block of fp32 operands (v and b as v / F and b / F: block_scale), by the helper warps.  ALIGNED: from the raw stage;
+// One block of fp32 operands (v and b times w: block_scale), by the helper warps.  ALIGNED: from the raw stage;
 // otherwise element by element from global memory (any K, V, alignment).
 template <int DT, bool ALIGNED, bool UNC, int KP, int TV>
 __device__ __forceinline__ void tall_convert(const FwdArgs& a, int ht, const unsigned char* raw, unsigned char* op,
-                                             const TallSmem& L, long long tok0, int nt, int h, int v0, int tvw, float iph,
-                                             const BlockScale& bs) {
+                                             const TallSmem& L, long long tok0, int nt, int h, int v0, int tvw,
+                                             const BlockScale& bs, int half) {  // half: the block's first lane in bs
     const palimpsa_problem& p = a.p;
     constexpr int K4 = KP / 4, V4 = TV / 4;
     float4* qs = reinterpret_cast<float4*>(op + L.qs);
     float4* ks = reinterpret_cast<float4*>(op + L.ks);
     float4* qqs = reinterpret_cast<float4*>(op + L.qqs);
-    if (ht < TB) {
-        reinterpret_cast<float4*>(op + L.fc)[ht] = make_float4(bs.s, bs.s, bs.c, bs.c);
-        reinterpret_cast<float2*>(op + L.zz)[ht] = make_float2(bs.z, bs.z);
-        if (ht == 0)
-            *reinterpret_cast<float4*>(op + L.blk) = make_float4(bs.end, (1.f - bs.end) * iph, __uint_as_float(bs.special), 0.f);
+    if ((ht ^ half) < TB) {
+        const int t = ht ^ half;
+        reinterpret_cast<float4*>(op + L.fc)[t] = make_float4(bs.s, bs.s, bs.c, bs.c);
+        reinterpret_cast<float2*>(op + L.zz)[t] = make_float2(bs.z, bs.z);
+        if (t == 0) *reinterpret_cast<float2*>(op + L.blk) = make_float2(bs.end, __uint_as_float(bs.special));
     }
     const float sc = p.scale;
 #pragma unroll 2
     for (int i0 = 0; i0 < TB * K4; i0 += FT_HT) {
         const int i = i0 + ht, t = i / K4, c4 = i - t * K4;
-        const float scv = UNC ? sc * __shfl_sync(0xffffffffu, bs.inv, t & 15) : 0.f;
+        const float scv = UNC ? sc * __shfl_sync(0xffffffffu, bs.w, half | (t & 15)) : 0.f;
         if (i >= TB * K4) break;
         float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), kv = qv;
         if (t < nt && c4 * 4 < p.K) {
@@ -146,7 +146,7 @@ __device__ __forceinline__ void tall_convert(const FwdArgs& a, int ht, const uns
 #pragma unroll 2
     for (int i0 = 0; i0 < TB * V4; i0 += FT_HT) {
         const int i = i0 + ht, t = i / V4, r = 4 * (i - t * V4);
-        const float inv = __shfl_sync(0xffffffffu, bs.inv, t & 15);
+        const float wt = __shfl_sync(0xffffffffu, bs.w, half | (t & 15));
         if (i >= TB * V4 || r >= tvw) continue;  // rows past the tile belong to idle warps, or are never written out
         float4 vv = make_float4(0.f, 0.f, 0.f, 0.f), bv = vv;
         if (t < nt) {
@@ -159,8 +159,8 @@ __device__ __forceinline__ void tall_convert(const FwdArgs& a, int ht, const uns
                 bv = ld4_guarded<DT>(p.b, row + r, row + tvw);
             }
         }
-        vv = make_float4(vv.x * inv, vv.y * inv, vv.z * inv, vv.w * inv);
-        bv = make_float4(bv.x * inv, bv.y * inv, bv.z * inv, bv.w * inv);
+        vv = make_float4(vv.x * wt, vv.y * wt, vv.z * wt, vv.w * wt);
+        bv = make_float4(bv.x * wt, bv.y * wt, bv.z * wt, bv.w * wt);
         vb[4 * i] = make_float4(vv.x, vv.x, bv.x, bv.x);
         vb[4 * i + 1] = make_float4(vv.y, vv.y, bv.y, bv.y);
         vb[4 * i + 2] = make_float4(vv.z, vv.z, bv.z, bv.z);
@@ -235,24 +235,30 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
             cp_async_commit();
         };
         auto bar_helpers = [&]() __attribute__((always_inline)) { asm volatile("bar.sync 1, %0;" ::"n"(FT_HT) : "memory"); };
-        float gt = 0.f;  // step size of token lane & 15 of the block that is converted next
+        // Scalars are worked out for two blocks at a time, by every warp for itself: lanes 0 to 15 have the tokens of block it, an even
+        // one, 16 to 31 those of the next.
+        float gt = 0.f;
+        bool live = false;
         auto load_gt = [&](int it) __attribute__((always_inline)) {
-            if (it < nblk && (lane & 15) < tokens(it)) gt = p.gt[(token0(it) + (lane & 15)) * p.H + h];
+            const int b = it + (lane >> 4);
+            live = b < nblk && (lane & 15) < tokens(b);
+            if (live) gt = p.gt[(token0(b) + (lane & 15)) * p.H + h];
         };
         // and that block's scalars: before the wait for the walk, or after it where 16 elements a thread leave no registers to keep
         // them (B=8 T=4096 H=6 d=128: 1.13 after, 1.16 before; B=2 T=3001 H=16 96x192 0.70 after, 0.68 before)
         constexpr bool EARLY = RK * RV < 16;
         BlockScale bs;
         auto scale = [&](int it) __attribute__((always_inline)) {  // while the rows arrive, or the walk goes on
-            bs = block_scale(gt, (lane & 15) < tokens(it), gh, iph, lane);
-            load_gt(it + 1);
+            if (it & 1) return;
+            bs = block_scale<false>(gt, live, gh, iph, lane);
+            load_gt(it + 2);
         };
         auto convert = [&](int it) __attribute__((always_inline)) {
             cp_async_wait<0>();
             bar_helpers();  // every lane's copies have landed
             unsigned char* op = sm + (it & 1) * L.op_stage;
 #define PALIMPSA_CONVERT(DT, AL) \
-    tall_convert<DT, AL, UNC, KP, TV>(a, ht, raw, op, L, token0(it), tokens(it), h, v0, tvw, iph, bs)
+    tall_convert<DT, AL, UNC, KP, TV>(a, ht, raw, op, L, token0(it), tokens(it), h, v0, tvw, bs, 16 * (it & 1))
             if (a.aligned) {
                 if (p.io_dtype == PALIMPSA_BF16) PALIMPSA_CONVERT(PALIMPSA_BF16, true);
                 else if (p.io_dtype == PALIMPSA_F32) PALIMPSA_CONVERT(PALIMPSA_F32, true);
@@ -386,6 +392,7 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
             }
         }
     }
+    float missing = 0.f;  // from I since the last block: u Ip (block_scale)
     for (int it = 0; it < nblk; ++it) {
         if (idle) {
             if (!wait_fail && !mbar_wait_idle(&staged[it & 1], (it >> 1) & 1, POLLS)) wait_fail = 8;
@@ -403,7 +410,10 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
                     for (int j = 0; j < J; ++j) {
                         const long long e = (cbase + row0 + r) * KP + col0 + j * GS;
                         st_cols<CW>(a.ckpt_M + e, M[r][j]);
-                        st_cols<CW>(a.ckpt_I + e, I[r][j]);
+                        float2 i[E];
+#pragma unroll
+                        for (int c = 0; c < E; ++c) i[c] = fadd2(I[r][j][c], dup2(missing));
+                        st_cols<CW>(a.ckpt_I + e, i);
                     }
                 }
             }
@@ -419,15 +429,16 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
         float* yvs = reinterpret_cast<float*>(sm + L.yvs + (it & 1) * L.y_stage);
         if (!wait_fail && !tc::mbar_wait(&staged[it & 1], (it >> 1) & 1, POLLS)) wait_fail = 8;
         const int end = min(TB, s1 - (blk0 + it) * TB);
-        const float4 blk = *reinterpret_cast<const float4*>(op + L.blk);
-        const unsigned special = __float_as_uint(blk.z);
+        const float2 blk = *reinterpret_cast<const float2*>(op + L.blk);
+        const unsigned special = __float_as_uint(blk.y);
         // GF tokens from tg on; `scaled`: some of them scale the state first
         auto group = [&](auto scaled, int tg, auto& red) __attribute__((always_inline)) {
             constexpr bool SCALED = decltype(scaled)::value;
 #pragma unroll
             for (int jt = 0; jt < GF; ++jt) {
                 const int t = tg + jt;
-                const float4 fcv = SCALED ? fc[t] : make_float4(1.f, 1.f, 0.f, 0.f);
+                float4 fcv = SCALED ? fc[t] : make_float4(1.f, 1.f, 0.f, 0.f);
+                if (SCALED && t == 0) fcv.z = fcv.w = fcv.x * missing;
                 const float2 ff = make_float2(fcv.x, fcv.y), cc = make_float2(fcv.z, fcv.w), z = zz[t];
                 float2 vr[RV], br[RV], acc[RV], accv[RV];
 #pragma unroll
@@ -450,8 +461,8 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
                     for (int r = 0; r < RV; ++r) {
 #pragma unroll
                         for (int e = 0; e < E; ++e) {
-                            M[r][j][e] = SCALED ? ffma2(ff, M[r][j][e], fmul2(vr[r], kp[e])) : ffma2(vr[r], kp[e], M[r][j][e]);
-                            I[r][j][e] = SCALED ? ffma2(ff, I[r][j][e], ffma2(br[r], kkp[e], cc)) : ffma2(br[r], kkp[e], I[r][j][e]);
+                            M[r][j][e] = ffma2(vr[r], kp[e], SCALED ? fmul2(ff, M[r][j][e]) : M[r][j][e]);
+                            I[r][j][e] = ffma2(br[r], kkp[e], SCALED ? ffma2(ff, I[r][j][e], cc) : I[r][j][e]);
                             const float2 rr = rcp2(fadd2(I[r][j][e], z));
                             acc[r] = ffma2(fmul2(M[r][j][e], rr), qp[e], acc[r]);
                             if (UNC) accv[r] = ffma2(rr, qqp[e], accv[r]);
@@ -468,8 +479,25 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
 #pragma unroll 1
         for (int tg = 0; tg < end; tg += GF) {
             float red[NRED];
-            if ((special >> tg) & ((1u << GF) - 1u)) group(std::true_type{}, tg, red);
-            else group(std::false_type{}, tg, red);
+            const unsigned bits = (special >> tg) & ((1u << GF) - 1u);
+            if (bits & ~1u) {
+                group(std::true_type{}, tg, red);
+            } else {
+                if (bits) {  // a window begins with the group: the state is scaled here, and the group has nothing more to scale
+                    float4 fcv = fc[tg];
+                    if (tg == 0) fcv.z = fcv.w = fcv.x * missing;
+#pragma unroll
+                    for (int r = 0; r < RV; ++r)
+#pragma unroll
+                        for (int j = 0; j < J; ++j)
+#pragma unroll
+                            for (int e = 0; e < E; ++e) {
+                                M[r][j][e] = fmul2(make_float2(fcv.x, fcv.y), M[r][j][e]);
+                                I[r][j][e] = ffma2(make_float2(fcv.x, fcv.y), I[r][j][e], make_float2(fcv.z, fcv.w));
+                            }
+                }
+                group(std::false_type{}, tg, red);
+            }
             xreduce<NRED, KG>(red, lane);
             const int base = xreduce_index<NRED, KG>(lane), count = xreduce_count<NRED, KG>(lane);
 #pragma unroll
@@ -480,15 +508,7 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
                     (which ? yvs : ys)[(tg + jt) * TV + row0 + r] = red[i];
                 }
         }
-#pragma unroll
-        for (int r = 0; r < RV; ++r)
-#pragma unroll
-            for (int j = 0; j < J; ++j)
-#pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    M[r][j][e] = fmul2(dup2(blk.x), M[r][j][e]);
-                    I[r][j][e] = ffma2(dup2(blk.x), I[r][j][e], dup2(blk.y));
-                }
+        missing = blk.x;
         __syncwarp();
         if (lane == 0) mbar_arrive(&done[it & 1]);
     }
@@ -500,6 +520,8 @@ __global__ void __launch_bounds__(FT_NTHR + FT_HT, 1) fwd_tall_kernel(const FwdA
             for (int j = 0; j < J; ++j) {
                 const int kc = col0 + j * GS;
                 if (row0 + r < tvw && kc < K) {
+#pragma unroll
+                    for (int e = 0; e < E; ++e) I[r][j][e] = fadd2(I[r][j][e], dup2(missing));
                     float2 mu[E];
 #pragma unroll
                     for (int e = 0; e < E; ++e) mu[e] = make_float2(M[r][j][e].x / I[r][j][e].x, M[r][j][e].y / I[r][j][e].y);

@@ -52,3 +52,19 @@ def test_matches_oracle(N, H, T, K, V, dtype, unc, init):
         I0 = 0.5 + torch.rand(N, H, V, K, generator=g)
     got, ref = run_cuda(inp, "chunk", unc=unc, mu0=mu0, I0=I0), run_oracle(inp, unc=unc, mu0=mu0, I0=I0)
     compare(got, ref, tol_for(dtype), names=["o", "final_mu", "final_I", "dq", "dk", "dv", "db", "dgt"], what=f"{N}x{H} {K}x{V}")
+
+
+@pytest.mark.parametrize("N,H,K,V", [(64, 2, 48, 96), (24, 16, 48, 48), (64, 2, 96, 192), (48, 4, 192, 48)])
+@pytest.mark.parametrize("decay", [1.0, 6.0, 40.0])
+def test_nor_the_uncertainty_and_the_states(N, H, K, V, decay):
+    """Also where blocks have several windows, or none: the kernels' groups of tokens differ."""
+    from palimpsa_b200.ops import chunk_palimpsa
+    inp = orc.make_inputs(9, B=N, T=45, H=H, K=K, V=V, dtype=torch.bfloat16)
+    a = [inp[n].to(DEV) for n in ("q", "k", "v", "b", "gt", "g", "Ip")]
+    a[4] = decay * a[4]
+    flat = lambda out: [*out[0], *out[1:]]
+    with torch.no_grad():
+        every = flat(chunk_palimpsa(*a, output_final_state=True, output_uncertainty=True))
+        one = [flat(chunk_palimpsa(*[x[i:i + 1] for x in a[:5]], *a[5:], output_final_state=True, output_uncertainty=True)) for i in range(N)]
+    for x, *parts in zip(every, *one):
+        assert torch.equal(x, torch.cat(parts))
