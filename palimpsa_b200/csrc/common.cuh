@@ -177,11 +177,12 @@ __device__ __forceinline__ ChunkSplit chunk_split(int chunks, int nthr, int tid)
 // 0.45 to 1.0.  With I0 = 0.01, Ip = 1000 and decays near 0.99, 48x48, o was off by 7.5e-5, now by 5e-7.)  What that costs is the
 // helper warps' time between two hand-overs: backward 0.99 -> 1.02 ms at B=8 T=2048 H=16 48x48, whose two helpers have none to
 // spare, 2.16 -> 2.18 at H=6 d=128; the forward, two blocks at a time, 0.57 -> 0.574 (0.595 one at a time).
-// Scales reach 2^-64 (SCALE_LO).  Where the decays are faster, a new window begins in front of a group of 4 tokens, and in a group
-// that is too fast by itself (or has an f above 1) every token is alone: in the backward without any scale (F = 1), its s and c
-// those of the plain recurrence.
+// Scales reach 2^-48 (SCALE_LO): the float range that is left holds states and gradients from 1e-20 to 1e20 in all their bits (at
+// 2^-64 v of 1e20 gave NaN, d_o of 1e-20 lost 10 bits), and g * gt may be 2 a token for a block to be one window.  Where the
+// decays are faster, a new one begins in front of a group of 4 tokens, and in a group that is too fast by itself (or has an f
+// above 1) every token is alone: in the backward without any scale (F = 1), its s and c those of the plain recurrence.
 // ---------------------------------------------------------------------------------------------
-constexpr double SCALE_LO = 0x1p-64;
+constexpr double SCALE_LO = 0x1p-48;
 
 struct BlockScale {
     float f;           // decay of this lane's token (1 past the end)

@@ -112,6 +112,18 @@ def test_slow_decay_towards_a_large_prior(K, V, unc):
     assert max(errs.values()) < 3e-6, errs  # some fifty roundings of 2^-24
 
 
+@pytest.mark.parametrize("K,V", [(48, 40), (128, 24)])
+@pytest.mark.parametrize("vs,dos", [(1e20, 1.0), (1e-20, 1.0), (1.0, 1e20), (1.0, 1e-20)])
+def test_large_and_small_values_keep_their_bits(vs, dos, K, V):
+    """At decays just too slow for a second window, and faster ones: the scales reach 2^48."""
+    inp = orc.make_inputs(13, B=1, T=70, H=3, K=K, V=V)
+    inp["gt"], inp["g"] = torch.ones(1, 70, 3), torch.tensor([2.05, 2.7, 9.0])
+    inp["v"], inp["do"] = vs * inp["v"], dos * inp["do"]
+    got, ref = run_cuda(inp, "chunk"), run_oracle(inp)
+    errs = {n: _norm_err(got[n], ref[n]) for n in ("o", "final_mu", "final_I", "dq", "dk", "dv", "db", "dgt")}
+    assert max(errs.values()) < 2e-6, errs
+
+
 @pytest.mark.parametrize("K,V", [(16, 9), (48, 33), (128, 24)])
 def test_growing_states(K, V):
     """f above 1 (a negative step) now and then: those groups go token by token, the last ones before a sequence's ragged end too."""
