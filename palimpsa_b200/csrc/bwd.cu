@@ -683,7 +683,7 @@ bwd_kernel(const BwdArgs a) {
             const float2* zz2 = reinterpret_cast<const float2*>(op + L.zz2);
             // one forward step of the recurrence on token tl of the staged block: P to s; `scaled`: its s may differ from 1
             auto fstep = [&](auto scaled, const State<RV, NP>& from, State<RV, NP>& s, int tl) __attribute__((always_inline)) {
-                constexpr bool SCALED = decltype(scaled)::value;
+                constexpr bool SCALED = decltype(scaled)::value == 2;
                 const float4 fv = SCALED ? fc2[tl] : make_float4(1.f, 1.f, 0.f, 0.f);
                 const float2 ff = make_float2(fv.x, fv.y), cc = make_float2(fv.z, fv.w);
                 float2 kpv[NP], kk[NP];
@@ -708,13 +708,28 @@ bwd_kernel(const BwdArgs a) {
             // always processed as NG full groups with no per-token conditionals.
             const float2 blk = *reinterpret_cast<const float2*>(op + L.blk);
             const unsigned special = __float_as_uint(blk.y);
+            // Three copies of the walk: over a block of one window; of windows that begin in front of groups, whose scale is applied to
+            // the state that the group finds; of any windows.
+            static_assert(GR == 4, "the groups that block_scale begins windows in front of");
+            auto edge = [&](State<RV, NP>& s, int g) __attribute__((always_inline)) {
+                const float4 fv = fc2[g * GR];
+                const float2 ff = make_float2(fv.x, fv.y), cc = make_float2(fv.z, fv.w);
+#pragma unroll
+                for (int r = 0; r < RV; ++r)
+#pragma unroll
+                    for (int q = 0; q < NP; ++q) {
+                        s.M[r][q] = fmul2(ff, s.M[r][q]);
+                        s.I[r][q] = ffma2(ff, s.I[r][q], cc);
+                    }
+            };
             auto block = [&](auto scaled) __attribute__((always_inline)) {
-                constexpr bool SCALED = decltype(scaled)::value;
+                constexpr bool EDGES = decltype(scaled)::value == 1, SCALED = decltype(scaled)::value == 2;
                 // ---- forward sweep: park the start states of groups 1 .. NG-2, keep the last group's in registers
                 State<RV, NP> P[GR + 1];
                 load_ck(P[0], st);
 #pragma unroll 1
                 for (int g = 0; g < NG - 1; ++g) {
+                    if (EDGES) edge(P[0], g);
 #pragma unroll
                     for (int j = 0; j < GR; ++j) fstep(scaled, P[0], P[0], g * GR + j);
                     if (g < NG - 2) store_slot(P[0], g);
@@ -728,14 +743,15 @@ bwd_kernel(const BwdArgs a) {
                         nGI[r][q] = fmul2(dup2(blk.x), nGI[r][q]);
                     }
 
-                // Per group: the states of its four tokens from P[0] on, then the reverse walk over them.  With SCALED, a token may have
-                // scaled the state it found, by s, and so does the gradient on its way back.
+                // Per group: the states of its four tokens from P[0] on, then the reverse walk over them.  A token that has
+                // scaled the state it found, by s, scales the gradient on its way back.
 #pragma unroll 1
                 for (int gi = NG - 1; gi >= 0; --gi) {
                     if (gi == 0)
                         load_ck(P[0], st);
                     else if (gi < NG - 1)
                         load_slot(P[0], gi - 1);
+                    if (EDGES) edge(P[0], gi);
                     const int b = gi & (KBUF - 1);
                     float red1[NR1], red2[NR2];
 #pragma unroll
@@ -822,6 +838,16 @@ bwd_kernel(const BwdArgs a) {
                         red2[j * 2 + 0] = SCALED ? s * fdf : fdf;
                         red2[j * 2 + 1] = sc_;
                     }
+                    if (EDGES) {
+                        const float2 ff = dup2(fc2[gi * GR].x);
+#pragma unroll
+                        for (int r = 0; r < RV; ++r)
+#pragma unroll
+                            for (int q = 0; q < NP; ++q) {
+                                GM[r][q] = fmul2(ff, GM[r][q]);
+                                nGI[r][q] = fmul2(ff, nGI[r][q]);
+                            }
+                    }
                     if (!CO) {  // a carry-only pass wants nothing but the state gradients
                         // d_v-indexed sums over the KG lanes of a row; per-token scalars over the whole warp
                         xreduce<NR1, KG>(red1, lane);
@@ -847,8 +873,9 @@ bwd_kernel(const BwdArgs a) {
                     }
                 }
             };
-            if (special) block(std::true_type{});
-            else block(std::false_type{});
+            if (special == 0) block(std::integral_constant<int, 0>{});
+            else if ((special & ~0x1111u) == 0) block(std::integral_constant<int, 1>{});
+            else block(std::integral_constant<int, 2>{});
             __syncwarp();
             if (lane == 0) mbar_arrive(&done[st]);
         }
