@@ -15,8 +15,9 @@
 //      all in the scaled form in which neither the state nor its gradient decays from token to token (block_scale in
 //      common.cuh; GM, GI are the gradients of the scaled M and B): the algebra of chunk_palimpsa_bwd_kernel,
 //      chunk_palimpsa_forgetting_scalar.py:343-434, divided by F, with the previous state carried forward instead of rebuilt
-//      by a division, :409-410.  A block in which a token scales the state it finds takes a second copy of the walk, which
-//      also scales the gradients behind that token.
+//      by a division, :409-410.  Blocks in which the state is scaled on the way take other copies of the walk, one for scales in
+//      front of groups, one for scales in front of any token, which also scale the gradients there (B=8 T=2048 H=6 d=128, ms with
+//      one window, windows in front of groups, tokens by themselves: 2.18, 2.40, 2.49; the plain recurrence 2.38).
 // Reductions: over d_k (dv, db) by xor-shuffles inside the lanes of a row; over d_v (dq, dk) first
 // in registers across a thread's rows, then across the CTA's row groups through shared memory, and
 // across the CTAs of different row tiles through fp32 partial buffers in the workspace, which the
@@ -305,7 +306,7 @@ __host__ __device__ constexpr RegSplit bwd_split(int W, int RV, int RK) {
     return W == 8 && RV * RK == 12 ? RegSplit{168, 208, 88} : RegSplit{0, 0, 0};
 }
 
-// CTAs of an SM that the registers have to do for: two of the smallest tilings.  At d_k = 32 that spills 36 bytes: 148 / 296 / 740
+// CTAs of an SM that the registers have to do for: two of the smallest tilings.  At d_k = 32 that spilled 36 bytes (72 now): 148 / 296 / 740
 // CTAs of 32x32, T = 512, take 175 / 268 / 658 us, with one 148 / 289 / 715; with the uncertainty output it would spill 192:
 // 205 / 340 / 831 us against 164 / 320 / 792.
 __host__ __device__ constexpr int bwd_min_ctas(int RK, int KG, int W, bool unc) {
@@ -314,7 +315,8 @@ __host__ __device__ constexpr int bwd_min_ctas(int RK, int KG, int W, bool unc) 
 
 // Tokens of a block that the helper warps carry through registers at a time (BwdStaging): the whole block where they have the
 // registers, since every step costs a helper its address and type branches again (48x48 on 6 warps, B=8 T=4096 H=16: 1.98 ms, half
-// a block at a time 2.05).  With the uncertainty output half a block at a time is the better one: float32, T=2048, 1.18 and 1.12 ms.
+// a block at a time 2.05).  With the uncertainty output smaller steps are (float32, T=2048, 1.18 and 1.12 ms): what 40 registers hold, a
+// whole block on 4 warps of d_k = 48 and 96, half of one on 6 and on 8 of d_k = 256, a quarter on 6 of d_k = 192.
 __host__ __device__ constexpr int bwd_step_tokens(int KP, int TV, int HT, bool unc, RegSplit split) {
     const int room = split.entry > 0 ? split.helper - 54 : unc ? 40 : 72;
     for (int ts = TB; ts > 4; ts /= 2)
@@ -1087,11 +1089,12 @@ static const BwdTile* bwd_tile_choices(int KP) {
     }
 }
 // What a token costs a CTA (the walk, and what does not grow with the rows), in units of which 4 warps take 8.  One wave, T =
-// 512, bf16, us at 4 / 6 / 8 warps (8 of 3 rows): d_k = 48 181 / 247 / 325, 96 182 / 243 / 320, 192 186 / 263 / 340, 64 146 / - / 213
-// (314), 128 149 / - / 224 (266), 32 164 / - / 216, 16 120 / - / 165, 256 - / - / 358.  With the uncertainty output 207 / 276 / 356,
-// 209 / 285 / 356, 212 / 287 / 381, 160 / - / 229 (317), 160 / - / 250 (306), 159 / - / 234, 124 / - / 178, - / - / 359.  The
-// state-gradient pass of exact segments takes 0.45 to 0.55 of that at every height.  (3 rows of d_k = 64 spill 44 bytes: 285 before
-// the scaled form, when the other heights took 151 and 230.  The costs are those of then: the planner's cuts were fitted with them.)
+// 512, bf16, us at 4 / 6 / 8 warps (8 of 3 rows): d_k = 48 190 / 254 / 330, 96 181 / 247 / 328, 192 189 / 263 / 349, 64 146 / - / 216
+// (286), 128 149 / - / 229 (272), 32 170 / - / 220, 16 117 / - / 165, 256 - / - / 374.  With the uncertainty output 204 / 300 / 362,
+// 211 / 273 / 363, 211 / 284 / 388, 161 / - / 233 (322), 167 / - / 249 (302), 163 / - / 244, 129 / - / 187, - / - / 363.  The
+// state-gradient pass of exact segments takes 0.45 to 0.55 of that at every height.  The costs are those before the scaled form
+// (d_k = 64: 151, 230, 285), with which the planner's cuts were fitted; where they are off most, 44 rows of d_k = 64, the choice is even:
+// three waves of 286 at d_v = 128, four of 216 with 32 rows (B=8 T=4096 H=16: 6.75 ms, 6.83 before the scaled form, 7.2 while 44 rows took 314).
 static double bwd_tile_cost(const BwdTile& t, int KP, int NE, bool unc) {
     if (t.RV == 3) return KP == 64 ? (unc ? 17.2 : 15.1) : unc ? 16.4 : 15.7;
     return t.W == 4 ? 8 : t.W == 6 ? 11 : NE == 12 ? 14.2 : 12;

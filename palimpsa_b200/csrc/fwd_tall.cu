@@ -4,9 +4,9 @@
 // itself, between two CTA barriers per 16 tokens.  Here up to 12 compute warps share one tile: a block's operands are
 // converted once per SM, by helper warps, one block ahead of the walk, and the compute warps meet no barrier: they wait for
 // the staged block (an mbarrier), walk its 16 tokens with the state in registers, and hand the reduced outputs back the same
-// way.  What bounds it is the issue rate: a packed FP32 instruction takes two issue cycles (2.05 measured for FMUL2, 2.3 for
-// FFMA2 with a shared operand), so a pair of state elements takes 11 of them per token, its two reciprocals 16 of the MUFU
-// pipe, and the rest of a token (operand loads, the sums over a row's lanes) must stay small against 6 or 8 pairs.
+// way.  The floor is the MUFU pipe: a pair of state elements takes two reciprocals, 16 cycles of it, per token.  What keeps the
+// kernel from that floor is the issue rate: the pair's packed FP32 instructions take 11 issue cycles (2.05 measured for FMUL2, 2.3 for
+// FFMA2 with a shared operand), and the rest of a token (operand loads, the sums over a row's lanes) and the helper warps come on top.
 // Forward with checkpoints, ms, fwd.cu's kernel -> this one with the decay in every step -> in the scaled form (block_scale in
 // common.cuh; 5 packed operations a pair instead of 6) -> with 2 rows of 6 or 8 columns a thread where it had one row of 12 or 16
 // (d_k other than 128: half the operand loads and squares of k per element, for one more value to sum over the lanes): B=8 T=4096
@@ -567,7 +567,8 @@ struct TallPlan {
     double cost;  // per token of the longest-running SM, cycles
 };
 // Tile height: of all counts of tiles the one that costs least, waves of CTAs (one per SM) times what a token costs a CTA.
-// That is 190 cycles and 8.3 per state element on a scheduler's lanes: measured 588 with 12 warps of 16 elements (48 a
+// That is 190 cycles and 8.3 per state element on a scheduler's lanes: measured, with the decay in every step and one row of
+// twice the columns a thread where there are two rows now, 588 with 12 warps of 16 elements (48 a
 // lane and scheduler: 48 rows of d_k = 128), 490 with 12 of 12, 455 with 8 of 16, 411 with 6 of 12.
 template <int RK, int KG, int RV>
 static TallPlan tall_plan(const palimpsa_problem& p, int num_seg) {
